@@ -1,0 +1,197 @@
+// fp64_alu.cuh -- FP64 division, square root and ordering on the integer
+// units, with the results of the IEEE operations bit for bit.
+//
+// GB300 issues one FP64 warp instruction per SM every 16 cycles, in which the
+// four schedulers can issue 64 others; an FP64 division or square root is
+// seven to nine dependent FP64 instructions, an FP64 comparison one.  Here a
+// division is about 55 integer instructions and a square root about 65, so the
+// FP64 pipe is left to the additions and multiplications of the scheme.
+// On a 1.05M-cell mesh, with the FP64 operations left out that these and exact
+// powers of two make unnecessary (spectral_radius, roe_scaled, faces_cell64),
+// pass A went from 1163 to 457 us per launch, pass B from 990 to 615 us, the FP64
+// pipe still 77-81 % busy.
+//
+// Division: the classical digit recurrence in a high radix with quotient
+// digits selected by multiplication with a short reciprocal of the divisor
+// (Ercegovac and Lang, "Digital Arithmetic", 2004, ch. 5; Wong and Flynn, IEEE
+// Trans. Computers 41, 1992): digits of 30, 19 and 4 bits from a 20-bit
+// underestimate of the reciprocal, each followed by the exact remainder in
+// 64-bit integers.  Every digit is an underestimate, so remainders stay
+// non-negative; the last one is corrected by one.  The quotient's 54 leading
+// bits round to nearest by their last bit, since a quotient of two 53-bit
+// numbers is never half way between two others.  The square root is the same
+// recurrence (30, 18 and 5 bits) with an underestimate of 1 / (2 sqrt(x)).
+//
+// Operands or results outside the normal range (zero numerators apart) take
+// the hardware operation.  Compiles for the host too (the seed is then the
+// host's FP32 division), where tests hold it against the host's own IEEE
+// operations.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define E2D_HD __host__ __device__ __forceinline__
+#define E2D_HD_SLOW static __host__ __device__ __noinline__
+#else
+#define E2D_HD inline
+#define E2D_HD_SLOW inline
+#endif
+
+namespace e2d {
+
+E2D_HD uint64_t bits_of(double v) {
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(v);
+#else
+    uint64_t u;
+    memcpy(&u, &v, 8);
+    return u;
+#endif
+}
+
+E2D_HD double double_of(uint64_t u) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double v;
+    memcpy(&v, &u, 8);
+    return v;
+#endif
+}
+
+E2D_HD uint32_t mul_hi(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+
+#ifndef __CUDA_ARCH__
+#ifndef E2D_SEED_ULPS
+#define E2D_SEED_ULPS 0  // host tests: the seed moved by this many units in the last place
+#endif
+E2D_HD float moved_seed(float v) {
+    uint32_t u;
+    memcpy(&u, &v, 4);
+    u += E2D_SEED_ULPS;
+    memcpy(&v, &u, 4);
+    return v;
+}
+#endif
+
+// FP32 seeds, good to one unit in the last place (rcp) and 2^-22 (rsqrt)
+E2D_HD float seed_rcp(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return moved_seed(1.0f / x);
+#endif
+}
+E2D_HD float seed_rsqrt(float x) {
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return moved_seed((float)(1.0 / sqrt((double)x)));
+#endif
+}
+E2D_HD float float_of(uint32_t u) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float v;
+    memcpy(&v, &u, 4);
+    return v;
+#endif
+}
+
+E2D_HD_SLOW double div_ieee(double a, double b) { return a / b; }
+E2D_HD_SLOW double sqrt_ieee(double a) { return sqrt(a); }
+
+// A divisor prepared for div_by: several numerators share the work.
+struct Divisor {
+    double b;
+    uint64_t m;  // significand, bit 52 set
+    uint32_t y;  // 2^32 / (m / 2^52), an underestimate good to 2^-20
+    int e;       // biased exponent; 0 or 2047 (zero, subnormal, infinity, NaN): not prepared
+};
+
+E2D_HD Divisor divisor(double b) {
+    Divisor d;
+    const uint64_t u = bits_of(b);
+    d.b = b;
+    d.e = (int)(u >> 52) & 0x7ff;
+    d.m = (u & 0xFFFFFFFFFFFFFULL) | 0x10000000000000ULL;
+    // top 24 bits as a float f in [1, 2): f <= m < f + 2^-23.  The factor
+    // 1 - 2^-21 covers the seed's unit and makes y an underestimate.
+    const float f = float_of(0x3f800000u | ((uint32_t)(u >> 29) & 0x7fffffu));
+    d.y = (uint32_t)(seed_rcp(f) * 4294965248.0f);
+    return d;
+}
+
+// a / d.b, rounded to nearest even.
+E2D_HD double div_by(double a, const Divisor &d) {
+    const uint64_t ua = bits_of(a);
+    const int ea = (int)(ua >> 52) & 0x7ff;
+    int e = ea - d.e + 1023;
+    const bool zero = (ua << 1) == 0;
+    const bool a_ok = zero || ((unsigned)(ea - 1) < 2046u && (unsigned)(e - 2) < 2043u);
+    if (!a_ok || (unsigned)(d.e - 1) >= 2046u) return div_ieee(a, d.b);
+    uint64_t r = (ua & 0xFFFFFFFFFFFFFULL) | 0x10000000000000ULL;
+    if (r < d.m) {  // quotient of the significands in [1, 2)
+        r <<= 1;
+        e--;
+    }
+    const uint32_t q1 = mul_hi((uint32_t)(r >> 22), d.y);  // 30 bits of fraction
+    r = (r << 30) - (uint64_t)q1 * d.m;                    // < 2^11 m
+    const uint32_t q2 = mul_hi((uint32_t)(r >> 32), d.y) >> 1;  // the next 19
+    r = (r << 19) - (uint64_t)q2 * d.m;                         // < 2^10 m
+    uint32_t q3 = mul_hi((uint32_t)(r >> 32), d.y) >> 16;  // the last 4
+    r = (r << 4) - (uint64_t)q3 * d.m;
+    if (r >= d.m) q3++;
+    const uint64_t q = ((uint64_t)q1 << 23) + ((uint64_t)q2 << 4) + q3;  // 54 bits
+    const uint64_t sign = (ua ^ bits_of(d.b)) & 0x8000000000000000ULL;
+    const uint64_t mag = ((uint64_t)(uint32_t)(e - 1) << 52) + ((q + 1) >> 1);
+    return double_of(sign | (zero ? 0 : mag));
+}
+
+E2D_HD double ddiv(double a, double b) { return div_by(a, divisor(b)); }
+
+// sqrt(x), rounded to nearest even.
+E2D_HD double dsqrt(double x) {
+    const uint64_t u = bits_of(x);
+    if ((uint32_t)(u >> 32) - 0x00100000u >= 0x7ff00000u - 0x00100000u) return sqrt_ieee(x);
+    const int ex = (int)(u >> 52) - 1023;
+    const uint32_t odd = (uint32_t)ex & 1u;
+    const uint64_t m = ((u & 0xFFFFFFFFFFFFFULL) | 0x10000000000000ULL) << odd;  // in [1, 4) 2^52
+    const float f = float_of((0x3f800000u | ((uint32_t)(u >> 29) & 0x7fffffu)) + (odd << 23));
+    const float y = seed_rsqrt(f);
+    const uint32_t z = (uint32_t)(y * 2147481600.0f);        // 2^32 / (2 s), underestimated by 2^-20
+    const uint32_t s1 = (uint32_t)((f * y) * 1073740800.0f);  // s 2^30, underestimated by 2^-20
+    uint64_t r = (m << 8) - (uint64_t)s1 * s1;                // < 2^44
+    const uint32_t s2 = mul_hi((uint32_t)(r >> 12), z);       // the next 18 bits
+    r = (r << 36) - (((uint64_t)s1 * s2) << 19) - (uint64_t)s2 * s2;  // < 2^62
+    const uint64_t sa = ((uint64_t)s1 << 18) + s2;
+    const uint32_t s3 = mul_hi((uint32_t)(r >> 32), z) >> 11;  // the last 5
+    r = (r << 10) - (sa << 6) * s3 - (uint64_t)s3 * s3;
+    uint64_t s = (sa << 5) + s3;
+    if (r > 2 * s) s++;
+    return double_of(((uint64_t)(uint32_t)(((ex - (int)odd) >> 1) + 1022) << 52) + ((s + 1) >> 1));
+}
+
+// Monotonic integer key of a double: keys of numbers order like the numbers
+// (-0 just below +0); the inverse is the same map.
+E2D_HD int64_t order_key(double v) {
+    const int64_t k = (int64_t)bits_of(v);
+    return k ^ (int64_t)((uint64_t)(k >> 63) >> 1);
+}
+E2D_HD double key_value(int64_t k) { return double_of((uint64_t)(k ^ (int64_t)((uint64_t)(k >> 63) >> 1))); }
+
+// |x| < |y| on the bit patterns (finite values order like their magnitudes'
+// bits; a NaN compares above every finite value)
+E2D_HD bool abs_less(double x, double y) {
+    return (bits_of(x) & 0x7FFFFFFFFFFFFFFFULL) < (bits_of(y) & 0x7FFFFFFFFFFFFFFFULL);
+}
+
+}  // namespace e2d

@@ -23,6 +23,7 @@
 #pragma once
 
 #include "dev_types.h"
+#include "fp64_alu.cuh"
 #include "pdl.cuh"
 
 namespace e2d {
@@ -60,8 +61,8 @@ template <typename T> struct BatchMinBlocks {
 
 // Pass B variant.  FP64 evaluates each interior face inside a block's tile of
 // cells once (flux_tile): the FP64 Roe flux is arithmetic bound on this GPU,
-// and evaluating about half as many cut a whole FP64 iteration on a 51.8k-cell
-// mesh from 1.75 to 1.27 ms.  FP32 is bound by memory latency, where the
+// and evaluating about half as many pays for the tile's list (1.75 against 1.27
+// ms for an iteration on a 51.8k-cell mesh when it was introduced).  FP32 is bound by memory latency, where the
 // tile's work list and barriers cost more than they save (0.152 against
 // 0.110 ms per launch on 4.2M cells), so every cell evaluates its own three
 // faces (flux_cell).  Either way both cells of a face use the same flux bits.
@@ -70,6 +71,9 @@ template <typename T> struct FluxTiled { static constexpr bool value = sizeof(T)
 
 template <typename T> __device__ __forceinline__ T tabs(T v) { return fabs(v); }
 template <typename T> __device__ __forceinline__ T tsqrt(T v) { return sqrt(v); }
+template <> __device__ __forceinline__ double tsqrt<double>(double v) { return dsqrt(v); }
+// |x| < |y| (FP64: fp64_alu.cuh)
+__device__ __forceinline__ bool abs_less(float x, float y) { return fabsf(y) > fabsf(x); }
 template <typename T> __device__ __forceinline__ T tmin(T a, T b) { return fmin(a, b); }
 template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return fmax(a, b); }
 
@@ -79,8 +83,8 @@ template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return fmax(
 template <typename T> __device__ __forceinline__ T madd(T a, T b, T c) { return a * b + c; }
 template <> __device__ __forceinline__ float madd<float>(float a, float b, float c) { return fmaf(a, b, c); }
 
-// Divisions and square roots of the stencil's hot paths: IEEE in FP64 (bit
-// parity with the oracle); in FP32 the special-function unit's approximate
+// Divisions and square roots of the stencil's hot paths: in FP64 the IEEE
+// results (bit parity with the oracle) from the integer units, fp64_alu.cuh; in FP32 the special-function unit's approximate
 // reciprocal, reciprocal square root and square root (rcp / rsqrt /
 // sqrt.approx.f32, a few ulp), one instruction each where the IEEE forms take
 // a refinement sequence: the FP32 gather passes are issue bound.
@@ -101,6 +105,22 @@ __device__ __forceinline__ float fsqrt(float x) {
 }
 template <typename T> __device__ __forceinline__ T fdiv(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ float fdiv<float>(float a, float b) { return a * frcp(b); }
+template <> __device__ __forceinline__ double fdiv<double>(double a, double b) { return ddiv(a, b); }
+// The same with several numerators over one divisor.
+template <typename T> struct Over;
+template <> struct Over<float> {
+    float r;
+    __device__ __forceinline__ explicit Over(float b) : r(frcp(b)) {}
+    __device__ __forceinline__ float operator()(float a) const { return a * r; }
+};
+template <> struct Over<double> {
+    Divisor d;
+    __device__ __forceinline__ explicit Over(double b) : d(divisor(b)) {}
+    __device__ __forceinline__ double operator()(double a) const { return div_by(a, d); }
+};
+// Divisions of the boundary ghosts: the compiler's in FP32.
+template <typename T> __device__ __forceinline__ T gdiv(T a, T b) { return a / b; }
+template <> __device__ __forceinline__ double gdiv<double>(double a, double b) { return ddiv(a, b); }
 
 template <typename T> __device__ __forceinline__ T comp(const V4<T> &v, int k) {
     return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
@@ -108,11 +128,11 @@ template <typename T> __device__ __forceinline__ T comp(const V4<T> &v, int k) {
 
 // gpu_solver.cu:49-60 (kernel_CalculationPTA): pressure and sound speed
 template <typename T> __device__ __forceinline__ void pta(const V4<T> &w, T g, T &P, T &A) {
-    T U = w.y / w.x;
-    T V = w.z / w.x;
-    T E = w.w / w.x - T(0.5) * (U * U + V * V);
+    T U = gdiv(w.y, w.x);
+    T V = gdiv(w.z, w.x);
+    T E = gdiv(w.w, w.x) - T(0.5) * (U * U + V * V);
     P = (g - T(1.0)) * w.x * E;
-    A = tsqrt(g * P / w.x);
+    A = tsqrt(gdiv(g * P, w.x));
 }
 
 // gpu_solver.cu:62-135 (kernel_Far_Boundary): far-field ghost state from the
@@ -122,36 +142,36 @@ __device__ __noinline__ V4<T> far_ghost(const V4<T> dw, T P, T A, T vectorx, T v
                                         const Flow<T> f) {
     const T g = f.gamma;
     T nn = tsqrt(vectorx * vectorx + vectory * vectory);
-    T nx = vectory / nn;
-    T ny = vectorx / nn;
-    T UD = dw.y / dw.x;
-    T VD = dw.z / dw.x;
+    T nx = gdiv(vectory, nn);
+    T ny = gdiv(vectorx, nn);
+    T UD = gdiv(dw.y, dw.x);
+    T VD = gdiv(dw.z, dw.x);
     T Un = tabs(f.ui * nx + f.vi * ny);
     T Uncell = UD * nx + VD * ny;
     V4<T> w0 = dw;
-    if (Un / f.ain > T(1.0)) {
+    if (gdiv(Un, f.ain) > T(1.0)) {
         if (!(Uncell > T(0.0))) {
             w0.x = T(1.0);
             w0.y = f.ui;
             w0.z = f.vi;
-            w0.w = f.R * f.tin / (f.vin * f.vin) / (g - T(1.0)) + T(0.50);
+            w0.w = gdiv(gdiv(f.R * f.tin, f.vin * f.vin), g - T(1.0)) + T(0.50);
         }
     } else {
         T PA = f.pis, PD = P, AD = A, ROUD = dw.x, PB, UB, VB;
         if (Uncell > T(0.0)) {
             PB = PA;
-            w0.x = ROUD + (PB - PD) / AD / AD;
-            UB = UD + nx * (PD - PB) / ROUD / AD;
-            VB = VD + ny * (PD - PB) / ROUD / AD;
+            w0.x = ROUD + gdiv(gdiv(PB - PD, AD), AD);
+            UB = UD + gdiv(gdiv(nx * (PD - PB), ROUD), AD);
+            VB = VD + gdiv(gdiv(ny * (PD - PB), ROUD), AD);
         } else {
             PB = T(0.5) * (PA + PD - ROUD * AD * (nx * (f.ui - UD) + ny * (f.vi - VD)));
-            w0.x = T(1.0) + (PB - PA) / AD / AD;
-            UB = f.ui - nx * (PA - PB) / ROUD / AD;
-            VB = f.vi - ny * (PA - PB) / ROUD / AD;
+            w0.x = T(1.0) + gdiv(gdiv(PB - PA, AD), AD);
+            UB = f.ui - gdiv(gdiv(nx * (PA - PB), ROUD), AD);
+            VB = f.vi - gdiv(gdiv(ny * (PA - PB), ROUD), AD);
         }
         w0.y = UB * w0.x;
         w0.z = VB * w0.x;
-        w0.w = PB / (g - T(1.0)) + T(0.5) * (UB * UB + VB * VB) * w0.x;
+        w0.w = gdiv(PB, g - T(1.0)) + T(0.5) * (UB * UB + VB * VB) * w0.x;
     }
     return w0;
 }
@@ -159,10 +179,10 @@ __device__ __noinline__ V4<T> far_ghost(const V4<T> dw, T P, T A, T vectorx, T v
 // gpu_solver.cu:188-221: slip-wall ghost (velocity mirrored in the face)
 template <typename T>
 __device__ __forceinline__ V4<T> wall_ghost(const V4<T> &dw, T vectorx, T vectory, T vectorn) {
-    T nij0 = vectory / vectorn;
-    T nij1 = vectorx / vectorn;
-    T UU = dw.y / dw.x;
-    T VV = dw.z / dw.x;
+    T nij0 = gdiv(vectory, vectorn);
+    T nij1 = gdiv(vectorx, vectorn);
+    T UU = gdiv(dw.y, dw.x);
+    T VV = gdiv(dw.z, dw.x);
     T UV = UU * nij0 + VV * nij1;
     UU = UU - T(2) * UV * nij0;
     VV = VV - T(2) * UV * nij1;
@@ -186,16 +206,23 @@ __device__ __forceinline__ V4<T> ghost(int code, const V4<T> &U, T Sx, T Sy, con
 
 // gpu_solver.cu:385-454 (kernel_deltT): face spectral radius from the mean of
 // the two unreconstructed states.  Symmetric in (a, b) and in the sign of S.
-template <typename T>
-__device__ __forceinline__ T spectral_radius(const V4<T> &a, const V4<T> &b, T vectorx, T vectory,
-                                             T g) {
-    T rou = (a.x + b.x) * T(0.5);
-    T u = (a.y + b.y) / rou * T(0.5);
-    T v = (a.z + b.z) / rou * T(0.5);
-    T EE = (a.w + b.w) * T(0.5) / rou - (u * u + v * v) * T(0.5);
-    T VC = u * vectory + v * vectorx;
-    T p = rou * EE * (g - T(1.0));
-    T CS = tsqrt((g * p / rou) * (vectorx * vectorx + vectory * vectory));
+// The reference halves the sums of the two states (rou = sum / 2, u = sum_u /
+// rou / 2, p = rou EE (g - 1)); here the halves are left out where they cancel
+// exactly (a power of two goes through a rounding unchanged), and a half that
+// is subtracted is a fused multiply-add with an exact product.  19 FP64
+// additions and multiplications where the reference's form issues about 30.
+template <typename T> __device__ T spectral_radius(const V4<T> &a, const V4<T> &b, T vectorx, T vectory, T g);
+template <>
+__device__ __forceinline__ double spectral_radius<double>(const V4<double> &a, const V4<double> &b, double vectorx,
+                                                         double vectory, double g) {
+    const double rou2 = a.x + b.x;  // 2 rou
+    const Divisor d = divisor(rou2);
+    const double u = div_by(a.y + b.y, d);
+    const double v = div_by(a.z + b.z, d);
+    const double EE = fma(-0.5, u * u + v * v, div_by(a.w + b.w, d));
+    const double VC = u * vectory + v * vectorx;
+    const double p2 = rou2 * EE * (g - 1.0);  // 2 p
+    const double CS = dsqrt(div_by(g * p2, d) * (vectorx * vectorx + vectory * vectory));
     return tabs(VC) + CS;
 }
 
@@ -214,69 +241,65 @@ __device__ __forceinline__ float spectral_radius<float>(const V4<float> &a, cons
     return fabsf(VC) + CS;
 }
 
-// gpu_solver.cu:552-566 (kernel_Calc_Function)
-template <typename T>
-__device__ __forceinline__ void calc_function(const V4<T> &w, T g, T &A, T &U, T &V, T &H, T &P) {
-    T temp = T(1.0) / w.x;
-    U = w.y * temp;
-    V = w.z * temp;
-    P = (g - T(1.0)) * w.x * (w.w * temp - T(0.5) * (U * U + V * V));
-    A = tsqrt(g * P * temp);
-    H = w.w * temp + P * temp;
-}
-
 // gpu_solver.cu:569-647 (kernel_ROE_SCHEME): Roe flux with Harten's entropy
 // fix of width eps through the unit normal (nx, ny).
 template <typename T>
-__device__ __forceinline__ V4<T> roe(const V4<T> &LW, const V4<T> &RW, T nx, T ny, T g, T epsilon) {
-    T A0, U0, V0, H0, P0, A1, U1, V1, H1, P1;
-    calc_function(LW, g, A0, U0, V0, H0, P0);
-    calc_function(RW, g, A1, U1, V1, H1, P1);
-    T M0 = (U0 * nx + V0 * ny);
-    T M1 = (U1 * nx + V1 * ny);
-    T DVC = M1 - M0;
-    T lrou = LW.x, rrou = RW.x;
-    T sl = tsqrt(lrou), sr = tsqrt(rrou);
-    T ROUB = sl * sr;
-    T UB = (U0 * sl + U1 * sr) / (sl + sr);
-    T VB = (V0 * sl + V1 * sr) / (sl + sr);
-    T HB = (H0 * sl + H1 * sr) / (sl + sr);
-    T QB = UB * UB + VB * VB;
-    T AB = tsqrt((g - T(1.0)) * (HB - QB / T(2.0)));
-    T VC = UB * nx + VB * ny;
-    T AD0, AD1, AD2;
-    if (tabs(VC - AB) < epsilon) AD0 = ((VC - AB) * (VC - AB) + epsilon * epsilon) / (T(2) * epsilon);
-    else AD0 = tabs(VC - AB);
-    if (tabs(VC) < epsilon) AD1 = (VC * VC + epsilon * epsilon) / (T(2) * epsilon);
-    else AD1 = tabs(VC);
-    if (tabs(VC + AB) < epsilon) AD2 = ((VC + AB) * (VC + AB) + epsilon * epsilon) / (T(2) * epsilon);
-    else AD2 = tabs(VC + AB);
-    T dP = P1 - P0;
-    T F00 = AD0 * (dP - ROUB * AB * DVC) / (T(2.0) * AB * AB);
-    T F01 = F00 * (UB - AB * nx);
-    T F02 = F00 * (VB - AB * ny);
-    T F03 = F00 * (HB - AB * VC);
-    T F10 = AD1 * ((rrou - lrou) - dP / (AB * AB));
-    T F11 = F10 * UB + AD1 * ROUB * (U1 - U0 - DVC * nx);
-    T F12 = F10 * VB + AD1 * ROUB * (V1 - V0 - DVC * ny);
-    T F13 = F10 * QB * T(0.5) + AD1 * ROUB * (UB * (U1 - U0) + VB * (V1 - V0) - DVC * VC);
-    T F20 = AD2 * (dP + ROUB * AB * DVC) / (T(2.0) * AB * AB);
-    T F21 = F20 * (UB + AB * nx);
-    T F22 = F20 * (VB + AB * ny);
-    T F23 = F20 * (HB + AB * VC);
-    T WL0 = lrou * M0;
-    T WL1 = U0 * WL0 + nx * P0;
-    T WL2 = V0 * WL0 + ny * P0;
-    T WL3 = WL0 * H0;
-    T WR0 = rrou * M1;
-    T WR1 = U1 * WR0 + nx * P1;
-    T WR2 = V1 * WR0 + ny * P1;
-    T WR3 = WR0 * H1;
-    V4<T> F;
-    F.x = T(0.5) * ((WL0 + WR0) - (F00 + F10 + F20));
-    F.y = T(0.5) * ((WL1 + WR1) - (F01 + F11 + F21));
-    F.z = T(0.5) * ((WL2 + WR2) - (F02 + F12 + F22));
-    F.w = T(0.5) * ((WL3 + WR3) - (F03 + F13 + F23));
+__device__ V4<T> roe(const V4<T> &LW, const V4<T> &RW, T nx, T ny, T g, T epsilon);
+
+// |v| of the Harten fix (gpu_solver.cu:603-616): (v^2 + eps^2) / (2 eps) below
+// eps.
+__device__ __forceinline__ double harten(const double v, const double epsilon) {
+    if (!abs_less(v, epsilon)) return fabs(v);
+    return ddiv(v * v + epsilon * epsilon, 2.0 * epsilon);
+}
+
+// FP64: the reference's operations in its order (calc_function,
+// gpu_solver.cu:552-566, and the flux), times the face length.  Powers of two
+// move through the roundings: x - 0.5 y is one fused multiply-add (its product
+// is exact), 2 AB AB is twice AB AB and shares its divisor, and the flux's
+// factor 0.5 goes into the face length.
+__device__ __forceinline__ V4<double> roe_scaled(const V4<double> &LW, const V4<double> &RW, const double nx,
+                                                const double ny, const double g, const double epsilon,
+                                                const double vn) {
+    const double gm1 = g - 1.0;
+    const double t0 = ddiv(1.0, LW.x), t1 = ddiv(1.0, RW.x);
+    const double U0 = LW.y * t0, V0 = LW.z * t0, e0 = LW.w * t0;
+    const double U1 = RW.y * t1, V1 = RW.z * t1, e1 = RW.w * t1;
+    const double P0 = gm1 * LW.x * fma(-0.5, U0 * U0 + V0 * V0, e0);
+    const double P1 = gm1 * RW.x * fma(-0.5, U1 * U1 + V1 * V1, e1);
+    const double H0 = e0 + P0 * t0, H1 = e1 + P1 * t1;
+    const double M0 = U0 * nx + V0 * ny, M1 = U1 * nx + V1 * ny;
+    const double DVC = M1 - M0;
+    const double sl = dsqrt(LW.x), sr = dsqrt(RW.x);
+    const double ROUB = sl * sr;
+    const Divisor ds = divisor(sl + sr);
+    const double UB = div_by(U0 * sl + U1 * sr, ds);
+    const double VB = div_by(V0 * sl + V1 * sr, ds);
+    const double HB = div_by(H0 * sl + H1 * sr, ds);
+    const double QB = UB * UB + VB * VB;
+    const double AB = dsqrt(gm1 * fma(-0.5, QB, HB));
+    const double VC = UB * nx + VB * ny;
+    const double AD0 = harten(VC - AB, epsilon), AD1 = harten(VC, epsilon), AD2 = harten(VC + AB, epsilon);
+    const double dP = P1 - P0, RAD = ROUB * AB * DVC;
+    const Divisor da = divisor(AB * AB);
+    Divisor da2 = da;
+    da2.b = 2.0 * da.b;
+    da2.e = da.e ? da.e + 1 : 0;
+    const double F00 = div_by(AD0 * (dP - RAD), da2);
+    const double F20 = div_by(AD2 * (dP + RAD), da2);
+    const double F10 = AD1 * ((RW.x - LW.x) - div_by(dP, da));
+    const double anx = AB * nx, any = AB * ny, avc = AB * VC;
+    const double dU = U1 - U0, dV = V1 - V0, aR = AD1 * ROUB;
+    const double F11 = F10 * UB + aR * (dU - DVC * nx);
+    const double F12 = F10 * VB + aR * (dV - DVC * ny);
+    const double F13 = fma(F10 * QB, 0.5, aR * (UB * dU + VB * dV - DVC * VC));
+    const double WL0 = LW.x * M0, WR0 = RW.x * M1;
+    const double hv = 0.5 * vn;
+    V4<double> F;
+    F.x = ((WL0 + WR0) - (F00 + F10 + F20)) * hv;
+    F.y = (((U0 * WL0 + nx * P0) + (U1 * WR0 + nx * P1)) - (F00 * (UB - anx) + F11 + F20 * (UB + anx))) * hv;
+    F.z = (((V0 * WL0 + ny * P0) + (V1 * WR0 + ny * P1)) - (F00 * (VB - any) + F12 + F20 * (VB + any))) * hv;
+    F.w = ((WL0 * H0 + WR0 * H1) - (F00 * (HB - avc) + F13 + F20 * (HB + avc))) * hv;
     return F;
 }
 
@@ -502,31 +525,13 @@ __device__ __forceinline__ float faces_cell_ref32(const MeshDev<float> &m, const
     return dti;
 }
 
-// |x| < |y| on the bit patterns (finite values order like their magnitudes'
-// bits; a NaN compares above every finite value)
-__device__ __forceinline__ bool abs_less(double x, double y) {
-    return (unsigned long long)(__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) <
-           (unsigned long long)(__double_as_longlong(y) & 0x7FFFFFFFFFFFFFFFLL);
-}
-
-// SRX: the sum of the three face spectral radii comes in as tsum_ext
-// (faces_tile evaluates each interior face's radius once per tile).
-// LDQ (FP64, reference configuration, called by every lane of the warp; live
-// false for padding lanes, which store nothing): the limiter divisions are
-// shared out over the warp.  min(1, (bound - u) / delt2) is 1 exactly when
-// |bound - u| >= |delt2| (the two have the same sign, and a correctly rounded
-// quotient of magnitude >= 1 is >= 1), so only the other slots divide: each
-// lane parks those (numerator, delt2) pairs in its row of qv (12 slots x 2),
-// the warp lists them in qi, every lane divides list entries lane, lane + 32,
-// ..., and reads its quotients back.  Same operands, same IEEE division: the
-// bits do not change; a warp divides about 2-3 times per lane instead of 12.
-template <typename T, bool OPT, bool SRX = false, bool LDQ = false>
+template <typename T, bool OPT>
 __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, const int i,
                                         const V4<T> *__restrict__ W, V4<T> *__restrict__ FS,
                                         T *__restrict__ dt, V4<T> *__restrict__ phi, const int frozen,
-                                        const bool first = false, const T tsum_ext = T(0),
-                                        T *qv_warp = nullptr, unsigned short *qi = nullptr, const bool live = true) {
-    if constexpr (sizeof(T) == 4 && !OPT && !SRX && !LDQ) return faces_cell_ref32(m, f, i, W, FS, dt);
+                                        const bool first = false) {
+    static_assert(sizeof(T) == 4, "FP64 runs faces_tile");
+    if constexpr (!OPT) return faces_cell_ref32(m, f, i, W, FS, dt);
     const int n = m.n;
     const int4 tp = m.topo[i];
     const int code[3] = {tp.x, tp.y, tp.z};
@@ -555,9 +560,8 @@ __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, c
             g0[q] = madd(T(0.5) * (u + c), S[k].x, g0[q]);
             g1[q] = madd(T(0.5) * (u + c), S[k].y, g1[q]);
         }
-        if (!SRX) Tsum += spectral_radius(U, nbv[k], S[k].y, S[k].x, f.gamma);
+        Tsum += spectral_radius(U, nbv[k], S[k].y, S[k].x, f.gamma);
     }
-    if (SRX) Tsum = tsum_ext;
     const T A = cell_area(m, S, i);
     const T rA = fdiv(T(1.0), A);
     T gx[4], gy[4], umax[4], umin[4];
@@ -588,46 +592,6 @@ __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, c
             }
         }
     }
-    unsigned need = 0;
-    T *qv = nullptr;
-    if constexpr (LDQ) {
-        const int lane = threadIdx.x & 31;
-        qv = qv_warp + lane * 24;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (code[k] < 0) continue;
-            const V2<T> r = face_offset(m, S, k, i);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int sl = 4 * k + q;
-                const T delt2 = madd(gx[q], r.x, gy[q] * r.y);
-                const T num = (delt2 > T(0) ? umax[q] : umin[q]) - comp(U, q);
-                if (live && delt2 != T(0) && abs_less(num, delt2)) {
-                    need |= 1u << sl;
-                    qv[2 * sl] = num;
-                    qv[2 * sl + 1] = delt2;
-                }
-            }
-        }
-        const int cnt = __popc(need);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        int off = incl - cnt;
-        for (unsigned mm = need; mm; mm &= mm - 1) qi[off++] = (unsigned short)((lane << 4) | (__ffs(mm) - 1));
-        __syncwarp();
-        for (int j = lane; j < total; j += 32) {
-            const int e = qi[j];
-            T *pv = qv_warp + (e >> 4) * 24 + 2 * (e & 15);
-            pv[0] = pv[0] / pv[1];
-        }
-        __syncwarp();
-        if (!live) return T(0);
-    }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         V4<T> o = U;
@@ -642,7 +606,6 @@ __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, c
                 T u = comp(U, q);
                 if (reuse) fi = comp(pf, q);
                 else if (cellwise) fi = phic[q];
-                else if (LDQ) fi = (need >> (4 * k + q)) & 1 ? tmin(qv[2 * (4 * k + q)], T(1.0)) : T(1.0);
                 else fi = face_limiter(OPT ? f.limiter : 0, f, A, umax[q], umin[q], u, delt2);
                 ph[q] = fi;
                 d[q] = madd(delt2, fi, u);
@@ -651,7 +614,7 @@ __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, c
             if (OPT && f.positivity) {
                 // positivity fallback (option): a face side with a density or
                 // pressure that is not positive takes the cell state
-                const T q = T(0.5) * (d[1] * d[1] + d[2] * d[2]) / d[0];
+                const T q = gdiv(T(0.5) * (d[1] * d[1] + d[2] * d[2]), d[0]);
                 if (!(d[0] > T(0)) || !((f.gamma - T(1.0)) * (d[3] - q) > T(0))) o = U;
             }
             if (OPT && phi && !frozen) {
@@ -667,35 +630,157 @@ __device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, c
     return dti;
 }
 
-// Pass A for one tile of cells [base, base + nvalid) with each interior
-// face's spectral radius evaluated once (the FP64 path, bound by the FP64
-// rate: the radius takes 4 divisions and a square root): the tile lists the
-// radii it must evaluate (boundary faces, faces to cells outside the tile,
-// and inside faces from their left cell only, as flux_tile does for the Roe
-// flux), spreads that list over its threads with the cell states in shared
-// memory, then every cell sums its three radii in face order and runs the
-// rest of faces_cell.  The radius is symmetric in its two states and in the
-// sign of the face vector, and the two cells of a face hold exactly negated
-// face vectors, so each cell gets the bits of its own evaluation.
-// The limiter divisions are shared out over each warp (faces_cell, LDQ).
-// blockDim.x <= kFacesTile.
-constexpr int kFacesTile = 128;
-template <typename T>
-__device__ __forceinline__ void faces_tile(const MeshDev<T> &m, const Flow<T> &f, const int base, const int nvalid,
-                                           const V4<T> *__restrict__ W, V4<T> *__restrict__ FS,
-                                           T *__restrict__ dt) {
+// Bounds of component values over a cell and its neighbours, minus the cell's
+// own value: x = max - u, y = min - u (gpu_solver.cu:330-375), ordered on
+// integer keys.  (A NaN among them makes the gradient, and with it the
+// component's face states, NaN whatever the bounds.)
+__device__ __forceinline__ double2 cell_bounds(const double c0, const double c1, const double c2, const double u) {
+    const int64_t k0 = order_key(c0), k1 = order_key(c1), k2 = order_key(c2), ku = order_key(u);
+    const int64_t a = k0 > k1 ? k0 : k1, b = k2 > ku ? k2 : ku, c = k0 < k1 ? k0 : k1, d = k2 < ku ? k2 : ku;
+    return make_double2(key_value(a > b ? a : b) - u, key_value(c < d ? c : d) - u);
+}
+
+// Limiter value of one component on one face side (face_limiter) in FP64, from
+// the bounds minus the cell value.  Kind 0, min(1, bound / delt2): the bound
+// has delt2's sign, so a correctly rounded quotient of |bound| >= |delt2| is
+// >= 1 and only smaller bounds divide.  Kind 1, the Venkatakrishnan form with
+// its doubled products as exact fused multiply-adds.
+__device__ __forceinline__ double face_limiter64(const int kind, const double e2, const double2 bnd,
+                                                 const double delt2) {
+    const double d1 = (int64_t)bits_of(delt2) > 0 ? bnd.x : bnd.y;
+    if (kind == 1) {
+        if (delt2 == 0.0) return 1.0;
+        const double q = d1 * d1, p = delt2 * d1;
+        return ddiv(fma(2.0, p, q + e2), fma(2.0, delt2 * delt2, q) + p + e2);
+    }
+    return abs_less(d1, delt2) ? ddiv(d1, delt2) : 1.0;
+}
+
+// The FP64 form of faces_cell with the sum of the cell's three spectral radii
+// given (faces_tile).  It issues about 160 FP64 additions and multiplications
+// per cell in the reference configuration: the reference's halves of the
+// neighbour means are taken into the face vectors (exact), the first term of a
+// sum is not added to zero, the bounds are subtracted once per component and
+// divisions, comparisons and selections run on the integer units.
+template <bool OPT>
+__device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
+                                               const V4<double> *__restrict__ W, V4<double> *__restrict__ FS,
+                                               double *__restrict__ dt, V4<double> *__restrict__ phi,
+                                               const int frozen, const bool first, const V4<double> U,
+                                               const int4 tp, const double Tsum) {
+    const int n = m.n;
+    const int code[3] = {tp.x, tp.y, tp.z};
+    V2<double> S[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) S[k] = m.S[k * n + i];
+    V4<double> nbv[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        nbv[k] = code[k] >= 0 ? W[code[k] >> 3] : ghost(code[k], U, S[k].x, S[k].y, f);
+    const double A = m.area[i];
+    const double rA = ddiv(1.0, A);
+    double gx[4], gy[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const double s = comp(U, q) + comp(nbv[k], q);
+            const double px = s * (0.5 * S[k].x), py = s * (0.5 * S[k].y);
+            gx[q] = k == 0 ? px : gx[q] + px;
+            gy[q] = k == 0 ? py : gy[q] + py;
+        }
+        gx[q] *= rA;
+        gy[q] *= rA;
+    }
+    const bool reuse = OPT && phi && frozen;
+    double2 bnd[4];
+    if (!reuse && !(OPT && first)) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            bnd[q] = cell_bounds(comp(nbv[0], q), comp(nbv[1], q), comp(nbv[2], q), comp(U, q));
+    }
+    const int kind = OPT ? f.limiter & 1 : 0;
+    const double e2 = OPT && kind == 1 && !reuse ? f.venk_k3 * A * dsqrt(A) : 0.0;
+    // cell-wise limiter options (2, 3): see faces_cell
+    const bool cellwise = OPT && f.limiter >= 2;
+    double phic[4] = {1.0, 1.0, 1.0, 1.0};
+    if (cellwise && !reuse && !first) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) phic[q] = (double)INFINITY;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (code[k] < 0) continue;
+            const V2<double> r = m.R[k * n + i];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                phic[q] = fmin(phic[q], face_limiter64(kind, e2, bnd[q], gx[q] * r.x + gy[q] * r.y));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        V4<double> o = U;
+        if (code[k] >= 0 && !(OPT && first)) {
+            const V2<double> r = m.R[k * n + i];
+            V4<double> pf;
+            if (reuse) pf = phi[k * n + i];
+            double d[4], ph[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const double delt2 = gx[q] * r.x + gy[q] * r.y;
+                if (reuse) ph[q] = comp(pf, q);
+                else if (cellwise) ph[q] = phic[q];
+                else ph[q] = face_limiter64(kind, e2, bnd[q], delt2);
+                d[q] = delt2 * ph[q] + comp(U, q);
+            }
+            o.x = d[0]; o.y = d[1]; o.z = d[2]; o.w = d[3];
+            if (OPT && f.positivity) {
+                // positivity fallback (option): see faces_cell
+                const double q = ddiv(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
+                if (!(d[0] > 0.0) || !((f.gamma - 1.0) * (d[3] - q) > 0.0)) o = U;
+            }
+            if (OPT && phi && !frozen) {
+                V4<double> pw;
+                pw.x = ph[0]; pw.y = ph[1]; pw.z = ph[2]; pw.w = ph[3];
+                phi[k * n + i] = pw;
+            }
+        }
+        FS[k * n + i] = o;
+    }
+    const double dti = tmin(ddiv(A * f.cfl, Tsum), f.dt_cap);
+    dt[i] = dti;
+    return dti;
+}
+
+// Pass A in FP64 for one tile of cells [base, base + nvalid), each interior
+// face's spectral radius evaluated once: the tile lists the radii it must
+// evaluate (boundary faces, faces to cells outside the tile, and inside faces
+// from their left cell only, as flux_tile does for the Roe flux), spreads that
+// list over its threads with the cell states in shared memory, then every cell
+// sums its three radii in face order and runs faces_cell64.  The radius is
+// symmetric in its two states and in the sign of the face vector, and the two
+// cells of a face hold exactly negated face vectors, so each cell gets the
+// bits of its own evaluation.  Returns the thread's time step (+inf for a
+// padding lane).  blockDim.x <= kFacesTile.
+constexpr int kFacesTile = 256;
+template <bool OPT>
+__device__ __forceinline__ double faces_tile(const MeshDev<double> &m, const Flow<double> &f, const int base,
+                                             const int nvalid, const V4<double> *__restrict__ W,
+                                             V4<double> *__restrict__ FS, double *__restrict__ dt,
+                                             V4<double> *__restrict__ phi, const int frozen, const bool first) {
+    using T = double;
     __shared__ V4<T> Us[kFacesTile];
     __shared__ int4 tps[kFacesTile];
     __shared__ T SRs[kFacesTile * 3];
     __shared__ unsigned short items[kFacesTile * 3];
     __shared__ int wtot[kFacesTile / 32];
-    __shared__ T qv[kFacesTile * 24];
-    __shared__ unsigned short qi[kFacesTile * 12];
     const int n = m.n, t = threadIdx.x, i = base + t;
     const bool live = t < nvalid;
+    __syncthreads();  // the previous tile of this block may still read the shared arrays
     const int4 tp = live ? m.topo[i] : make_int4(-3, -3, -3, 0);
     tps[t] = tp;
-    if (live) Us[t] = W[i];
+    V4<T> U = {};
+    if (live) U = W[i];
+    Us[t] = U;
     const int code[3] = {tp.x, tp.y, tp.z};
     unsigned mask = 0;
 #pragma unroll
@@ -741,34 +826,16 @@ __device__ __forceinline__ void faces_tile(const MeshDev<T> &m, const Flow<T> &f
         SRs[tt * 3 + k] = spectral_radius(Uo, nb, S.y, S.x, f.gamma);
     }
     __syncthreads();
-    T Tsum = T(1);
-    if (live) {
-        Tsum = T(0);
+    if (!live) return (double)INFINITY;
+    T Tsum = T(0);
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int c = code[k];
-            Tsum += (mask & (1u << k)) ? SRs[t * 3 + k] : SRs[((c >> 3) - base) * 3 + (c & 3)];
-        }
+    for (int k = 0; k < 3; k++) {
+        const int c = code[k];
+        const T r = (mask & (1u << k)) ? SRs[t * 3 + k] : SRs[((c >> 3) - base) * 3 + (c & 3)];
+        Tsum = k == 0 ? r : Tsum + r;
     }
-    // every lane of a warp takes part in the shared limiter divisions; a
-    // padding lane computes on the tile's first cell and stores nothing
-    const int w = t >> 5;
-    faces_cell<T, false, true, true>(m, f, live ? i : base, W, FS, dt, nullptr, 0, false, Tsum, qv + w * 32 * 24,
-                                     qi + w * 32 * 12, live);
+    return faces_cell64<OPT>(m, f, i, W, FS, dt, phi, frozen, first, U, tp, Tsum);
 }
-
-// Pass A of the reference configuration in tiles (FP64, see faces_tile).
-template <typename T>
-__global__ void E2D_LB_FACES k_faces_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
-                                          V4<T> *__restrict__ FS, T *__restrict__ dt, Ctl *__restrict__ ctl,
-                                          V4<T> *__restrict__ phi, const int st) {
-    wait_prior_grid();
-    if (ctl->halt) return;
-    const int base = blockIdx.x * blockDim.x;
-    faces_tile(m, f, base, min((int)blockDim.x, m.n - base), W, FS, dt);
-}
-template <typename T> struct FacesTiled { static constexpr bool value = sizeof(T) == 8; };
-template <typename T> inline bool faces_tiled(int block) { return FacesTiled<T>::value && block <= kFacesTile; }
 
 // Global time-step option: the block's smallest step folded into *slot.
 // Every thread of the block must call it (v = +inf for no cell).  A time
@@ -789,8 +856,23 @@ __device__ __forceinline__ void block_min_dt(double v, unsigned long long *slot)
     }
 }
 
-// OPT: the variant with the scheme options (smooth limiter, limiter freezing,
-// global time step); faces_options picks it.
+// FP64: pass A in tiles of blockDim.x cells (faces_tile).
+template <bool OPT>
+__global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<double> f,
+                                                       const V4<double> *__restrict__ W,
+                                                       V4<double> *__restrict__ FS, double *__restrict__ dt,
+                                                       Ctl *__restrict__ ctl, V4<double> *__restrict__ phi,
+                                                       const int st) {
+    wait_prior_grid();
+    if (ctl->halt) return;
+    const int base = blockIdx.x * blockDim.x;
+    const double v = faces_tile<OPT>(m, f, base, min((int)blockDim.x, m.n - base), W, FS, dt, phi,
+                                     OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order);
+    if (OPT && f.global_dt) block_min_dt(v, &ctl->dtmin[st]);
+}
+
+// FP32.  OPT: the variant with the scheme options (smooth limiter, limiter
+// freezing, global time step); faces_options picks it.
 template <typename T, bool OPT>
 __global__ void E2D_LB_FACES k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
                                      V4<T> *__restrict__ FS, T *__restrict__ dt,
@@ -807,6 +889,12 @@ __global__ void E2D_LB_FACES k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__res
     double v = __longlong_as_double((long long)kDtNone);
     if (i < m.n) v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, phi ? ctl->frozen : 0, first);
     block_min_dt(v, &ctl->dtmin[st]);
+}
+
+// The pass-A kernel of a precision.
+template <typename T> auto faces_kernel(bool opt) {
+    if constexpr (sizeof(T) == 8) return opt ? &k_faces_tile<true> : &k_faces_tile<false>;
+    else return opt ? &k_faces<T, true> : &k_faces<T, false>;
 }
 
 // True when a pass-A launch needs the option variant.
@@ -866,8 +954,9 @@ __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f,
 // with S negated, gets the exact negative).
 template <typename T> __device__ __forceinline__ void unit_normal(const V2<T> S, T &nx, T &ny, T &vn) {
     vn = tsqrt(S.y * S.y + S.x * S.x);
-    nx = S.x / vn;
-    ny = S.y / vn;
+    const Over<T> by(vn);
+    nx = by(S.x);
+    ny = by(S.y);
 }
 template <> __device__ __forceinline__ void unit_normal<float>(const V2<float> S, float &nx, float &ny, float &vn) {
     const float q = fmaf(S.y, S.y, S.x * S.x), r = frsqrt(q);
@@ -910,16 +999,16 @@ __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, 
     T nx, ny, vn;
     face_inputs(f, code, S, own, oth, a, b, nx, ny, vn, right);
     // one Roe call site for every face
-    V4<T> F = roe(a, b, nx, ny, f.gamma, f.eps_entropy);
     if constexpr (sizeof(T) == 4) {
+        V4<T> F = roe(a, b, nx, ny, f.gamma, f.eps_entropy);
         // two packed multiplies, the same products
         const float2 xy = __fmul2_rn(make_float2(F.x, F.y), make_float2(vn, vn));
         const float2 zw = __fmul2_rn(make_float2(F.z, F.w), make_float2(vn, vn));
         F.x = xy.x; F.y = xy.y; F.z = zw.x; F.w = zw.y;
+        return F;
     } else {
-        F.x *= vn; F.y *= vn; F.z *= vn; F.w *= vn;
+        return roe_scaled(a, b, nx, ny, f.gamma, f.eps_entropy, vn);
     }
-    return F;
 }
 
 template <typename T>
@@ -1038,6 +1127,7 @@ __device__ __forceinline__ V4<T> nb_sum(const int4 tp, const V4<T> *__restrict__
     for (int k = 0; k < 3; k++)
         if (code[k] >= 0) {
             const V4<T> v = src[code[k] >> 3];
+            if (sizeof(T) == 8 && k == 0) { d = v; continue; }  // no addition to zero
             d.x += v.x; d.y += v.y; d.z += v.z; d.w += v.w;
         }
     return d;
@@ -1053,12 +1143,12 @@ __device__ __forceinline__ void smooth_cell(const MeshDev<T> &m, const T eps, co
     const int4 tp = m.topo[i];
     const V4<T> d = nb_sum(tp, src);
     const V4<T> r0 = res[i];
-    const T den = T(1.0) + (eps) * T(tp.w);
+    const Over<T> den(T(1.0) + (eps) * T(tp.w));
     V4<T> o;
-    o.x = fdiv(madd(d.x, eps, r0.x), den);
-    o.y = fdiv(madd(d.y, eps, r0.y), den);
-    o.z = fdiv(madd(d.z, eps, r0.z), den);
-    o.w = fdiv(madd(d.w, eps, r0.w), den);
+    o.x = den(madd(d.x, eps, r0.x));
+    o.y = den(madd(d.y, eps, r0.y));
+    o.z = den(madd(d.z, eps, r0.z));
+    o.w = den(madd(d.w, eps, r0.w));
     dst[i] = o;
 }
 
@@ -1089,29 +1179,29 @@ __device__ __forceinline__ void update_cell(const MeshDev<T> &m, const Flow<T> &
         if (smooth) {
             const V4<T> d = nb_sum(tp, src);
             const T eps = f.irs_eps;
-            const T den = T(1.0) + (eps) * T(tp.w);
-            T s0 = fdiv(madd(d.x, eps, r.x), den), s1 = fdiv(madd(d.y, eps, r.y), den);
-            T s2 = fdiv(madd(d.z, eps, r.z), den), s3 = fdiv(madd(d.w, eps, r.w), den);
-            if (tabs(r.x) > tabs(s0)) r.x = s0;
-            if (tabs(r.y) > tabs(s1)) r.y = s1;
-            if (tabs(r.z) > tabs(s2)) r.z = s2;
-            if (tabs(r.w) > tabs(s3)) r.w = s3;
+            const Over<T> den(T(1.0) + (eps) * T(tp.w));
+            T s0 = den(madd(d.x, eps, r.x)), s1 = den(madd(d.y, eps, r.y));
+            T s2 = den(madd(d.z, eps, r.z)), s3 = den(madd(d.w, eps, r.w));
+            if (abs_less(s0, r.x)) r.x = s0;
+            if (abs_less(s1, r.y)) r.y = s1;
+            if (abs_less(s2, r.z)) r.z = s2;
+            if (abs_less(s3, r.w)) r.w = s3;
         }
         T RK = rk;
         RK *= dti;
-        const T A = m.area[i];
+        const Over<T> A(m.area[i]);
         const V4<T> w0 = W0[i];
         V4<T> w;
-        w.x = w0.x - fdiv(RK * r.x, A);
-        w.y = w0.y - fdiv(RK * r.y, A);
-        w.z = w0.z - fdiv(RK * r.z, A);
-        w.w = w0.w - fdiv(RK * r.w, A);
+        w.x = w0.x - A(RK * r.x);
+        w.y = w0.y - A(RK * r.y);
+        w.z = w0.z - A(RK * r.z);
+        w.w = w0.w - A(RK * r.w);
         Wout[i] = w;
         if (want) {
             // rho - rho0 in the stencil's precision: exact in FP32 as long as the
             // two densities are within a factor of two (Sterbenz)
             drho = w.x - w0.x;
-            const T q = T(0.5) * (w.y * w.y + w.z * w.z) / w.x;
+            const T q = gdiv(T(0.5) * (w.y * w.y + w.z * w.z), w.x);
             bad = !(w.x > T(0)) || !(w.w - q > T(0));
         }
     }
@@ -1221,9 +1311,13 @@ __global__ void __launch_bounds__(256, BatchMinBlocks<T>::faces) kb_faces(MeshDe
         if (b.ctl[tc].halt) continue;                // uniform over the block
         const Flow<T> f = b.flows[tc];
         double v = __longlong_as_double((long long)kDtNone);
-        if (i < b.case_end[tc])
-            v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, OPT && phi ? b.ctl[tc].frozen : 0,
-                                           OPT && b.ctl[tc].step < f.first_order);
+        const int frozen = OPT && phi ? b.ctl[tc].frozen : 0;
+        const bool first = OPT && b.ctl[tc].step < f.first_order;
+        if constexpr (sizeof(T) == 8)
+            v = faces_tile<OPT>(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, dt, phi,
+                                frozen, first);
+        else if (i < b.case_end[tc])
+            v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, frozen, first);
         if (OPT && f.global_dt) block_min_dt(v, &b.ctl[tc].dtmin[st]);  // uniform over the block
     }
 }
@@ -1355,10 +1449,7 @@ template <typename T> void enqueue_iteration(const Plan<T> &p, cudaStream_t s) {
         const bool last = st == p.stages - 1;
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
-        if (opt) launch_chained(k_faces<T, true>, G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
-        else if (faces_tiled<T>(B))
-            launch_chained(k_faces_tile<T>, G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
-        else launch_chained(k_faces<T, false>, G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
+        launch_chained(faces_kernel<T>(opt), G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
         if (FluxTiled<T>::value) launch_chained(k_flux_tile<T>, G, B, s, p.m, p.f, p.FS, p.res, p.ctl);
         else launch_chained(k_flux<T>, G, B, s, p.m, p.f, p.FS, p.res, p.ctl);
         const V4<T> *src = p.res;
@@ -1392,9 +1483,7 @@ int enqueue_iteration_timed(const Plan<T> &p, cudaStream_t s, cudaEvent_t *ev, i
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
         mark(0);
-        if (opt) k_faces<T, true><<<G, B, 0, s>>>(p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
-        else if (faces_tiled<T>(B)) k_faces_tile<T><<<G, B, 0, s>>>(p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
-        else k_faces<T, false><<<G, B, 0, s>>>(p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
+        faces_kernel<T>(opt)<<<G, B, 0, s>>>(p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
         done();
         mark(1);
         if (FluxTiled<T>::value) k_flux_tile<T><<<G, B, 0, s>>>(p.m, p.f, p.FS, p.res, p.ctl);
