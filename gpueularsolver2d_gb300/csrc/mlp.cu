@@ -18,6 +18,7 @@
 
 #include <cudaTypedefs.h>
 
+#include "fp64_alu.cuh"
 #include "mlp_kernels.cuh"
 #include "mlp_tma.cuh"
 #include "solver_internal.h"
@@ -155,30 +156,105 @@ __global__ void k_to_bf16(int n, const float *__restrict__ a, bf16 *__restrict__
     if (bT) bT[(size_t)(i % cols) * rows + i / cols] = __float2bfloat16_rn(a[i]);
 }
 
-// Minimum distance from each point to a set of segments (wall faces).
-__global__ void __launch_bounds__(256) k_wall_distance(int n, const double *__restrict__ px,
-                                                       const double *__restrict__ py, int nseg,
-                                                       const double4 *__restrict__ seg, double *__restrict__ d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    __shared__ double4 s[256];
+// Rows of NIN FP32 inputs to rows of bf16 with pitch ld; rows from cnt on are
+// zero.  One thread per eight columns.
+__global__ void __launch_bounds__(256) k_pack(int cnt, int rows, const float *__restrict__ x, bf16 *__restrict__ xb,
+                                              int ld) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, r = j / (NIN / 8), c = j % (NIN / 8) * 8;
+    if (r >= rows) return;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (r < cnt) {
+        a = *(const float4 *)(x + (size_t)r * NIN + c);
+        b = *(const float4 *)(x + (size_t)r * NIN + c + 4);
+    }
+    __align__(16) __nv_bfloat162 o[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
+                                         __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
+    *(uint4 *)(xb + (size_t)r * ld + c) = *(const uint4 *)o;
+}
+
+// Wall faces as segments (x0, y0, x1, y1), in boxes of kBox consecutive ones:
+// box = their bounds in FP32.  scale bounds the coordinates' magnitude.
+constexpr int kBox = 16;
+struct Walls {
+    int nseg;
+    const double4 *seg;
+    const float4 *box;
+    float scale;
+};
+
+// Minimum distance from (x, y) to the segments.  A box is passed over when its
+// distance in FP32 is above the best distance so far by more than FP32's
+// rounding of the coordinates (slack); every other segment is evaluated in
+// FP64, its division on the integer units: 14 FP64 operations each, which is
+// what the kernel is bound by (33.6k cells and 251 segments: 0.3 ms before the
+// boxes).
+__device__ __forceinline__ double wall_distance(const Walls &w, const double x, const double y) {
+    const float fx = (float)x, fy = (float)y;
+    const float slack = 2e-6f * (fabsf(fx) + fabsf(fy) + w.scale);
+    const int nbox = (w.nseg + kBox - 1) / kBox;
+    float near = INFINITY;  // an upper bound of the distance
+    for (int k = 0; k < nbox; k++) {
+        const double4 q = w.seg[k * kBox];
+        const float dx = fx - (float)q.x, dy = fy - (float)q.y;
+        near = fminf(near, sqrtf(dx * dx + dy * dy) + slack);
+    }
     double best = 1e300;
-    const double x = i < n ? px[i] : 0.0, y = i < n ? py[i] : 0.0;
-    for (int base = 0; base < nseg; base += 256) {
-        __syncthreads();
-        if (base + (int)threadIdx.x < nseg) s[threadIdx.x] = seg[base + threadIdx.x];
-        __syncthreads();
-        const int cnt = min(256, nseg - base);
-        for (int k = 0; k < cnt; k++) {
-            const double4 q = s[k];
+    for (int k = 0; k < nbox; k++) {
+        const float4 b = w.box[k];
+        const float bx = fmaxf(fmaxf(b.x - fx, fx - b.z), 0.f), by = fmaxf(fmaxf(b.y - fy, fy - b.w), 0.f);
+        if (sqrtf(bx * bx + by * by) - slack > near) continue;
+        const int end = min(w.nseg, (k + 1) * kBox);
+        for (int j = k * kBox; j < end; j++) {
+            const double4 q = w.seg[j];
             const double ex = q.z - q.x, ey = q.w - q.y;
             const double L2 = ex * ex + ey * ey;
-            double t = L2 > 0 ? ((x - q.x) * ex + (y - q.y) * ey) / L2 : 0.0;
+            double t = L2 > 0 ? ddiv((x - q.x) * ex + (y - q.y) * ey, L2) : 0.0;
             t = fmin(1.0, fmax(0.0, t));
             const double dx = x - (q.x + t * ex), dy = y - (q.y + t * ey);
             best = fmin(best, dx * dx + dy * dy);
         }
+        near = fminf(near, (float)sqrt(best) + slack);
     }
-    if (i < n) d[i] = sqrt(best);
+    return sqrt(best);
+}
+
+__global__ void __launch_bounds__(128) k_wall_distance(int n, const double *__restrict__ px,
+                                                       const double *__restrict__ py, Walls w,
+                                                       double *__restrict__ d) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) d[i] = wall_distance(w, px[i], py[i]);
+}
+
+// The features of every cell (e2d_mlp_features), one thread per cell.
+struct FeatureArgs {
+    double f[8][2];
+    float mach, sa, ca;
+};
+__global__ void __launch_bounds__(128) k_features(int n, const double *__restrict__ px, const double *__restrict__ py,
+                                                  Walls w, FeatureArgs a, float4 *__restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = px[i], y = py[i];
+    const double d = w.nseg ? wall_distance(w, x, y) : 1e300;
+    float4 *o = out + (size_t)i * (NIN / 4);
+    float v[E2D_MLP_FEATURES];
+    v[0] = (float)x; v[1] = (float)y; v[2] = (float)log(d + 1e-3);
+    v[3] = a.mach; v[4] = a.sa; v[5] = a.ca;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const double ph = 6.283185307179586 * __dadd_rn(__dmul_rn(a.f[j][0], x), __dmul_rn(a.f[j][1], y));
+        double sn, cs;
+        sincos(ph, &sn, &cs);
+        v[6 + 2 * j] = (float)sn;
+        v[7 + 2 * j] = (float)cs;
+    }
+#pragma unroll
+    for (int j = 0; j < NIN / 4; j++) {
+        float q[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = 4 * j + k < E2D_MLP_FEATURES ? v[4 * j + k] : 0.f;
+        o[j] = make_float4(q[0], q[1], q[2], q[3]);
+    }
 }
 
 struct Tensor {
@@ -199,6 +275,7 @@ struct e2d_mlp {
     // batch buffers
     int B = 0;
     bf16 *xb = nullptr;  // [B][KX], the inputs in the first NIN columns
+    float *xf = nullptr;  // [cfg.batch][NIN], the caller's FP32 rows on their way into xb or X
     float *tb = nullptr, *y = nullptr, *dy = nullptr;
     std::vector<bf16 *> Gd, Hh;  // [nhidden] of [B][H]: gelu'(z) and gelu(z) of each hidden layer
     bf16 *dz[2] = {nullptr, nullptr};  // [B][H]
@@ -412,6 +489,21 @@ int ensure_batch(e2d_mlp *m, int B) {
     return build_ws_maps(m);
 }
 
+// cnt rows of the caller's inputs (at most cfg.batch) to the device and as bf16
+// to dst (row pitch ld), rows cnt .. rows - 1 zero, on the training stream.
+// (A prediction of 33.6k rows takes 0.17 ms, 1.12 ms when the host converted and
+// padded to the full batch of 65536.)
+int stage_rows(e2d_mlp *m, const float *x, int cnt, int rows, bf16 *dst, int ld) {
+    if (!m->xf) {
+        int rc = m->alloc(&m->xf, sizeof(float) * (size_t)m->cfg.batch * NIN);
+        if (rc) return rc;
+    }
+    CK(cudaMemcpyAsync(m->xf, x, sizeof(float) * (size_t)cnt * NIN, cudaMemcpyHostToDevice, m->stream));
+    k_pack<<<(int)(((size_t)rows * (NIN / 8) + 255) / 256), 256, 0, m->stream>>>(cnt, rows, m->xf, dst, ld);
+    CK(cudaGetLastError());
+    return E2D_OK;
+}
+
 AdamSeg adam_seg(const Tensor &t, const float *part, int nparts, size_t pstride, float *grad_out, int pld = 0) {
     AdamSeg g{};
     g.part = part; g.pstride = pstride; g.nparts = nparts; g.count = t.count();
@@ -447,10 +539,9 @@ int check_flag(e2d_mlp *m) {
     return E2D_OK;
 }
 
-// Forward on the batch in xb (rows B) through the hidden layers; without
-// targets (inference) also the output layer into y.
-void forward(e2d_mlp *m, cudaStream_t s, bool with_loss) {
-    const int B = m->B;
+// Forward on the first B rows of xb (a multiple of 128) through the hidden
+// layers; without targets (inference) also the output layer into y.
+void forward(e2d_mlp *m, cudaStream_t s, bool with_loss, int B) {
     for (int l = 0; l < m->nhidden; l++) {
         if (m->use_ws) {
             ws::Args a{};
@@ -570,6 +661,55 @@ void backward(e2d_mlp *m, cudaStream_t s, const float *lr, bool want_grad) {
     claim(1);
 }
 
+// The cell centroids and the wall faces of a mesh on the device, with room for
+// a result: one allocation, freed on every return path.
+struct CellsAndWalls {
+    char *base = nullptr;
+    double *px = nullptr, *py = nullptr;
+    void *out = nullptr;
+    Walls walls{};
+    ~CellsAndWalls() { cudaFree(base); }
+
+    int upload(const e2d_mesh *mesh, size_t out_bytes) {
+        const MeshTopo &t = mesh->topo;
+        const int n = mesh->ncell;
+        std::vector<double4> seg;
+        double scale = 0.0;
+        for (int e = 0; e < t.nedge; e++)
+            if (t.elog[e] == 2) {
+                seg.push_back(make_double4(mesh->x[t.en1[e] - 1], mesh->y[t.en1[e] - 1], mesh->x[t.en2[e] - 1],
+                                           mesh->y[t.en2[e] - 1]));
+                const double4 &q = seg.back();
+                for (double v : {q.x, q.y, q.z, q.w}) scale = std::max(scale, std::fabs(v));
+            }
+        const int nseg = (int)seg.size();
+        std::vector<float4> box((nseg + kBox - 1) / kBox, make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY));
+        for (int k = 0; k < nseg; k++) {
+            float4 &b = box[k / kBox];
+            b.x = std::min({b.x, (float)seg[k].x, (float)seg[k].z});
+            b.y = std::min({b.y, (float)seg[k].y, (float)seg[k].w});
+            b.z = std::max({b.z, (float)seg[k].x, (float)seg[k].z});
+            b.w = std::max({b.w, (float)seg[k].y, (float)seg[k].w});
+        }
+        const size_t cells = Arena::up(sizeof(double) * n), segs = Arena::up(sizeof(double4) * seg.size()),
+                     boxes = Arena::up(sizeof(float4) * box.size());
+        CK(cudaMalloc((void **)&base, 2 * cells + segs + boxes + out_bytes));
+        px = (double *)base;
+        py = (double *)(base + cells);
+        CK(cudaMemcpyAsync(px, t.cx.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(py, t.cy.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+        if (nseg) {
+            CK(cudaMemcpyAsync(base + 2 * cells, seg.data(), sizeof(double4) * nseg, cudaMemcpyHostToDevice));
+            CK(cudaMemcpyAsync(base + 2 * cells + segs, box.data(), sizeof(float4) * box.size(),
+                               cudaMemcpyHostToDevice));
+        }
+        out = base + 2 * cells + segs + boxes;
+        walls = Walls{nseg, (const double4 *)(base + 2 * cells), (const float4 *)(base + 2 * cells + segs),
+                      (float)scale};
+        return E2D_OK;
+    }
+};
+
 int build_train_graph(e2d_mlp *m) {
     if (m->gexec) return E2D_OK;
     cudaGraph_t g = nullptr;
@@ -579,7 +719,7 @@ int build_train_graph(e2d_mlp *m) {
     // the gather reads the step from device memory through its seed argument
     k_gather<<<(m->B + 255) / 256, 256, 0, s>>>(m->B, NIN, KX, NOUT, m->cfg.seed, m->step_dev, m->nsamples, m->X,
                                                   m->T, m->xb, m->tb);
-    forward(m, s, true);
+    forward(m, s, true, m->B);
     backward(m, s, m->lr_dev, false);
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess) { set_error(std::string("graph capture: ") + cudaGetErrorString(e)); return E2D_ERR_CUDA; }
@@ -728,12 +868,15 @@ int e2d_mlp_set_data(e2d_mlp *m, int64_t nsamples, const float *x, const float *
     if (!m || !x || !t || nsamples < 1) { set_error("bad argument"); return E2D_ERR_ARG; }
     if (m->X) { cudaFree(m->X); m->X = nullptr; }
     if (m->T) { cudaFree(m->T); m->T = nullptr; }
-    std::vector<bf16> xb((size_t)nsamples * NIN);
-    for (size_t i = 0; i < xb.size(); i++) xb[i] = __float2bfloat16_rn(x[i]);
-    CK(cudaMalloc((void **)&m->X, sizeof(bf16) * xb.size()));
+    CK(cudaMalloc((void **)&m->X, sizeof(bf16) * (size_t)nsamples * NIN));
     CK(cudaMalloc((void **)&m->T, sizeof(float) * (size_t)nsamples * NOUT));
-    CK(cudaMemcpy(m->X, xb.data(), sizeof(bf16) * xb.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(m->T, t, sizeof(float) * (size_t)nsamples * NOUT, cudaMemcpyHostToDevice));
+    for (int64_t r0 = 0; r0 < nsamples; r0 += m->cfg.batch) {
+        const int cnt = (int)std::min<int64_t>(m->cfg.batch, nsamples - r0);
+        int rc = stage_rows(m, x + (size_t)r0 * NIN, cnt, cnt, m->X + (size_t)r0 * NIN, NIN);
+        if (rc) return rc;
+    }
+    CK(cudaMemcpyAsync(m->T, t, sizeof(float) * (size_t)nsamples * NOUT, cudaMemcpyHostToDevice, m->stream));
+    CK(cudaStreamSynchronize(m->stream));
     m->nsamples = nsamples;
     if (m->gexec) { cudaGraphExecDestroy(m->gexec); m->gexec = nullptr; }
     return E2D_OK;
@@ -764,14 +907,11 @@ int e2d_mlp_forward(e2d_mlp *m, int64_t n, const float *x, float *y) {
     if (!m || !x || !y || n < 1) { set_error("bad argument"); return E2D_ERR_ARG; }
     int rc = ensure_batch(m, m->cfg.batch);
     if (rc) return rc;
-    std::vector<bf16> xb((size_t)m->B * KX, __float2bfloat16_rn(0.f));
     for (int64_t r0 = 0; r0 < n; r0 += m->B) {
         const int64_t cnt = std::min<int64_t>(m->B, n - r0);
-        for (size_t r = 0; r < (size_t)m->B; r++)
-            for (int c = 0; c < NIN; c++)
-                xb[r * KX + c] = __float2bfloat16_rn(r < (size_t)cnt ? x[(size_t)(r0 + r) * NIN + c] : 0.f);
-        CK(cudaMemcpyAsync(m->xb, xb.data(), sizeof(bf16) * xb.size(), cudaMemcpyHostToDevice, m->stream));
-        forward(m, m->stream, false);
+        const int rows = (int)((cnt + 255) / 256 * 256);  // whole tiles; B is a multiple of 2048
+        if ((rc = stage_rows(m, x + (size_t)r0 * NIN, (int)cnt, rows, m->xb, KX))) return rc;
+        forward(m, m->stream, false, rows);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(y + (size_t)r0 * NOUT, m->y, sizeof(float) * cnt * NOUT, cudaMemcpyDeviceToHost, m->stream));
         CK(cudaStreamSynchronize(m->stream));
@@ -783,12 +923,9 @@ int e2d_mlp_gradient(e2d_mlp *m, const float *x, const float *t, double *loss, f
     if (!m || !x || !t || !grad) { set_error("bad argument"); return E2D_ERR_ARG; }
     int rc = ensure_batch(m, m->cfg.batch);
     if (rc) return rc;
-    std::vector<bf16> xb((size_t)m->B * KX, __float2bfloat16_rn(0.f));
-    for (size_t r = 0; r < (size_t)m->B; r++)
-        for (int c = 0; c < NIN; c++) xb[r * KX + c] = __float2bfloat16_rn(x[r * NIN + c]);
-    CK(cudaMemcpy(m->xb, xb.data(), sizeof(bf16) * xb.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(m->tb, t, sizeof(float) * (size_t)m->B * NOUT, cudaMemcpyHostToDevice));
-    forward(m, m->stream, true);
+    if ((rc = stage_rows(m, x, m->B, m->B, m->xb, KX))) return rc;
+    CK(cudaMemcpyAsync(m->tb, t, sizeof(float) * (size_t)m->B * NOUT, cudaMemcpyHostToDevice, m->stream));
+    forward(m, m->stream, true, m->B);
     backward(m, m->stream, nullptr, true);
     CK(cudaGetLastError());
     const int nlp = m->B / 256;
@@ -806,66 +943,47 @@ int e2d_wall_distance(e2d_mesh *mesh, double wall_box, double *d) {
     if (!mesh || !d) { set_error("null argument"); return E2D_ERR_ARG; }
     int rc = build_topology(mesh, wall_box);
     if (rc) return rc;
-    const MeshTopo &t = mesh->topo;
-    std::vector<double4> seg;
-    for (int e = 0; e < t.nedge; e++)
-        if (t.elog[e] == 2)
-            seg.push_back(make_double4(mesh->x[t.en1[e] - 1], mesh->y[t.en1[e] - 1], mesh->x[t.en2[e] - 1],
-                                       mesh->y[t.en2[e] - 1]));
     const int n = mesh->ncell;
-    if (seg.empty()) { for (int i = 0; i < n; i++) d[i] = 1e300; return E2D_OK; }
-    struct Bufs {  // freed on every return path
-        double *px = nullptr, *py = nullptr, *dd = nullptr;
-        double4 *sg = nullptr;
-        ~Bufs() { cudaFree(px); cudaFree(py); cudaFree(dd); cudaFree(sg); }
-    } b;
-    CK(cudaMalloc((void **)&b.px, sizeof(double) * n));
-    CK(cudaMalloc((void **)&b.py, sizeof(double) * n));
-    CK(cudaMalloc((void **)&b.dd, sizeof(double) * n));
-    CK(cudaMalloc((void **)&b.sg, sizeof(double4) * seg.size()));
-    CK(cudaMemcpy(b.px, t.cx.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b.py, t.cy.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(b.sg, seg.data(), sizeof(double4) * seg.size(), cudaMemcpyHostToDevice));
-    k_wall_distance<<<(n + 255) / 256, 256>>>(n, b.px, b.py, (int)seg.size(), b.sg, b.dd);
+    CellsAndWalls c;
+    if ((rc = c.upload(mesh, sizeof(double) * (size_t)n))) return rc;
+    if (!c.walls.nseg) { for (int i = 0; i < n; i++) d[i] = 1e300; return E2D_OK; }
+    k_wall_distance<<<(n + 127) / 128, 128>>>(n, c.px, c.py, c.walls, (double *)c.out);
     CK(cudaGetLastError());
-    CK(cudaMemcpy(d, b.dd, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(d, c.out, sizeof(double) * n, cudaMemcpyDeviceToHost));
     return E2D_OK;
 }
 
 // Features per cell: x, y, log(d_wall + 1e-3), Mach, sin a, cos a, then for
 // j = 0..7: sin(2 pi f_j . (x, y)), cos(2 pi f_j . (x, y)), f_j ~ N(0, sigma^2).
+// Computed on the GPU: the call takes 0.52 ms for 33.6k cells and 251 wall faces,
+// 4.98 ms when the host evaluated the logarithms, sines and cosines.
 int e2d_mlp_features(e2d_mesh *mesh, double wall_box, double mach, double alpha_deg, uint64_t seed, double sigma,
                      float *out) {
     if (!mesh || !out) { set_error("null argument"); return E2D_ERR_ARG; }
-    const int n = mesh->ncell;
-    std::vector<double> d(n);
-    int rc = e2d_wall_distance(mesh, wall_box, d.data());
+    int rc = build_topology(mesh, wall_box);
     if (rc) return rc;
+    const int n = mesh->ncell;
     uint64_t st = seed * 0x9e3779b97f4a7c15ULL + 777;
     auto rnd = [&]() {
         st ^= st >> 12; st ^= st << 25; st ^= st >> 27;
         return ((st * 0x2545F4914F6CDD1DULL) >> 11) * (1.0 / 9007199254740992.0);
     };
-    double f[8][2];
-    for (auto &fj : f)
+    FeatureArgs a;
+    for (auto &fj : a.f)
         for (double &c : fj) {
             double u1 = rnd() + 1e-300, u2 = rnd();
             c = sigma * std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2);
         }
-    const double a = alpha_deg * 3.14159265358979 / 180.0, sa = std::sin(a), ca = std::cos(a);
-    const MeshTopo &t = mesh->topo;
-    for (int i = 0; i < n; i++) {
-        float *o = out + (size_t)i * NIN;
-        const double x = t.cx[i], y = t.cy[i];
-        o[0] = (float)x; o[1] = (float)y; o[2] = (float)std::log(d[i] + 1e-3);
-        o[3] = (float)mach; o[4] = (float)sa; o[5] = (float)ca;
-        for (int j = 0; j < 8; j++) {
-            const double ph = 6.283185307179586 * (f[j][0] * x + f[j][1] * y);
-            o[6 + 2 * j] = (float)std::sin(ph);
-            o[7 + 2 * j] = (float)std::cos(ph);
-        }
-        for (int k = E2D_MLP_FEATURES; k < NIN; k++) o[k] = 0.f;
-    }
+    const double al = alpha_deg * 3.14159265358979 / 180.0;
+    a.mach = (float)mach;
+    a.sa = (float)std::sin(al);
+    a.ca = (float)std::cos(al);
+    CellsAndWalls c;
+    const size_t bytes = sizeof(float) * (size_t)n * NIN;
+    if ((rc = c.upload(mesh, bytes))) return rc;
+    k_features<<<(n + 127) / 128, 128>>>(n, c.px, c.py, c.walls, a, (float4 *)c.out);
+    CK(cudaGetLastError());
+    CK(cudaMemcpy(out, c.out, bytes, cudaMemcpyDeviceToHost));
     return E2D_OK;
 }
 
