@@ -42,6 +42,7 @@ struct BatchBase {
     virtual int launches() const = 0;
     virtual int upload_case(int c, const double *w_file, cudaStream_t s) = 0;
     virtual int download_case(int c, double *w_file, cudaStream_t s) = 0;
+    virtual int download_walls(int c, double *w_wall, cudaStream_t s) = 0;
     virtual int save_state(cudaStream_t s) = 0;
     virtual int restore_state(cudaStream_t s) = 0;
     virtual const void *topo_ptr() const = 0;
@@ -55,6 +56,9 @@ template <typename T> struct BatchT : BatchBase {
     BPlan<T> plan;
     int *perm_dev = nullptr;      // [ntot] internal -> file index within the case
     double *wfile_dev = nullptr;  // [4 * max n_c]
+    int *wall_dev = nullptr;      // [wall faces of all cases] internal cell of each, case by case
+    double *wwall_dev = nullptr;  // [4 * most wall faces of a case]
+    std::vector<size_t> wall_off;  // [ncase] first wall face of each case
     int2 *case_tiles = nullptr;   // [ncase]
     V4<T> *backup = nullptr;      // [ntot] (autotune)
     std::vector<int2> ct_host;
@@ -70,14 +74,23 @@ template <typename T> struct BatchT : BatchBase {
             plan.options = plan.options || p.limiter != 0 || p.global_dt != 0 || p.first_order_iters > 0 ||
                            p.positivity_fix != 0;
         int nmax = 0;
-        for (auto &l : *L) nmax = std::max(nmax, l.n);
+        size_t wmax = 0;
+        std::vector<int> hw;
+        for (size_t c = 0; c < L->size(); c++) {
+            const HostLayout &l = (*L)[c];
+            nmax = std::max(nmax, l.n);
+            wmax = std::max(wmax, l.wall_cell.size());
+            wall_off.push_back(hw.size());
+            for (int i : l.wall_cell) hw.push_back((*off)[c] + i);
+        }
         const int maxtiles = (n + 31) / 32;
         size_t bytes = Arena::up(sizeof(int4) * n) + 2 * Arena::up(sizeof(V2<T>) * 3 * n) +
                        2 * Arena::up(sizeof(T) * n) + 6 * Arena::up(sizeof(V4<T>) * n) +
                        Arena::up(sizeof(V4<T>) * 3 * n) * (freeze ? 2 : 1) + Arena::up(sizeof(double) * maxtiles) +
                        Arena::up(sizeof(int) * n) + Arena::up(sizeof(double) * 4 * nmax) +
                        Arena::up(sizeof(Flow<T>) * ncase) + Arena::up(sizeof(int) * (n / kChunk + 1)) +
-                       2 * Arena::up(sizeof(int2) * ncase);
+                       2 * Arena::up(sizeof(int2) * ncase) + Arena::up(sizeof(int) * hw.size()) +
+                       Arena::up(sizeof(double) * 4 * wmax);
         CK(cudaMalloc((void **)&arena.base, bytes));
         arena.cap = bytes;
         int4 *topo = (int4 *)arena.take(sizeof(int4) * n);
@@ -100,6 +113,9 @@ template <typename T> struct BatchT : BatchBase {
         int *chunk_case = (int *)arena.take(sizeof(int) * (n / kChunk + 1));
         int *case_end = (int *)arena.take(sizeof(int) * ncase);
         case_tiles = (int2 *)arena.take(sizeof(int2) * ncase);
+        wall_dev = (int *)arena.take(sizeof(int) * hw.size());
+        wwall_dev = (double *)arena.take(sizeof(double) * 4 * wmax);
+        if (!hw.empty()) CK(cudaMemcpy(wall_dev, hw.data(), sizeof(int) * hw.size(), cudaMemcpyHostToDevice));
         // concatenated mesh (padding cells stay zero and are never touched)
         std::vector<int32_t> ht(4 * (size_t)n, 0);
         std::vector<T> hS(6 * (size_t)n, T(0)), hR(6 * (size_t)n, T(0)), ha(n, T(1));
@@ -190,6 +206,16 @@ template <typename T> struct BatchT : BatchBase {
         enqueue_export<T>(n, perm_dev + o, plan.W[0] + o, wfile_dev, s);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(w, wfile_dev, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        return E2D_OK;
+    }
+
+    int download_walls(int c, double *w, cudaStream_t s) override {
+        const int cnt = (int)(*L)[c].wall_cell.size();
+        if (!cnt) return E2D_OK;
+        enqueue_export_cells<T>(cnt, wall_dev + wall_off[c], plan.W[0], wwall_dev, s);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(w, wwall_dev, sizeof(double) * 4 * cnt, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         return E2D_OK;
     }
@@ -498,10 +524,10 @@ int e2d_batch_residual_history(e2d_batch *b, int32_t c, double *out, int32_t cap
 
 int e2d_batch_forces(e2d_batch *b, int32_t c, double *cl, double *cd) {
     if (!b || c < 0 || c >= b->ncase) { set_error("bad argument"); return E2D_ERR_ARG; }
-    std::vector<double> w(4 * (size_t)b->L[c].n);
-    int rc = b->impl->download_case(c, w.data(), b->stream);
+    std::vector<double> w(4 * b->L[c].wall_cell.size());
+    int rc = b->impl->download_walls(c, w.data(), b->stream);
     if (rc) return rc;
-    forces_from_state(b->L[c], b->fs[c], b->prm[c].gamma, w.data(), cl, cd);
+    forces_from_walls(b->L[c], b->fs[c], b->prm[c].gamma, w.data(), cl, cd);
     return E2D_OK;
 }
 

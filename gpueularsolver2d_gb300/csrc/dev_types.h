@@ -138,6 +138,10 @@ void enqueue_import(int n, const int *perm, const double *wfile, V4<T> *W, cudaS
 template <typename T>
 void enqueue_export(int n, const int *perm, const V4<T> *W, double *wfile, cudaStream_t s);
 
+// The states of cells[0 .. cnt), FP64.
+template <typename T>
+void enqueue_export_cells(int cnt, const int *cells, const V4<T> *W, double *w, cudaStream_t s);
+
 // Residual kernel launcher (resid.cu).
 void enqueue_resid(double *part, int nparts, Ctl *ctl, double *hist, int hist_cap, bool pairs,
                    cudaStream_t s);

@@ -1,5 +1,5 @@
 // integrals.cu -- FP64 integrals of a conserved state, on the host: lift and
-// drag (forces_from_state), total mass, and the mass fluxes through the
+// drag (forces_from_walls), total mass, and the mass fluxes through the
 // far-field and wall faces.  No reference counterpart.
 //
 // The boundary fluxes are the scheme's own first-order boundary flux, the one
@@ -135,7 +135,10 @@ double roe_mass(const Cons &LW, const Cons &RW, double nx, double ny, double g, 
 
 void integrals_from_state(const HostLayout &L, const FreeStream &fs, const e2d_params &p, const double *w,
                           e2d_integrals *out) {
-    forces_from_state(L, fs, p.gamma, w, &out->cl, &out->cd);
+    std::vector<double> ww(4 * L.wall_cell.size());
+    for (size_t q = 0; q < L.wall_cell.size(); q++)
+        for (int c = 0; c < 4; c++) ww[4 * q + c] = w[4 * (size_t)L.perm[L.wall_cell[q]] + c];
+    forces_from_walls(L, fs, p.gamma, ww.data(), &out->cl, &out->cd);
     const int n = L.n;
     double mass = 0.0, far = 0.0, wall = 0.0;
     for (int i = 0; i < n; i++) {

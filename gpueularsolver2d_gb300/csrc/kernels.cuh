@@ -1426,6 +1426,22 @@ __global__ void k_export(int n, const int *__restrict__ perm, const V4<T> *__res
     d[0] = (double)v.x; d[1] = (double)v.y; d[2] = (double)v.z; d[3] = (double)v.w;
 }
 
+// The states of a list of cells (the wall cells of the forces), FP64.
+template <typename T>
+__global__ void k_export_cells(int cnt, const int *__restrict__ cells, const V4<T> *__restrict__ W,
+                               double *__restrict__ w) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= cnt) return;
+    const V4<T> v = W[cells[j]];
+    double *d = w + 4 * (size_t)j;
+    d[0] = (double)v.x; d[1] = (double)v.y; d[2] = (double)v.z; d[3] = (double)v.w;
+}
+
+template <typename T>
+void enqueue_export_cells(int cnt, const int *cells, const V4<T> *W, double *w, cudaStream_t s) {
+    if (cnt > 0) k_export_cells<T><<<(cnt + 255) / 256, 256, 0, s>>>(cnt, cells, W, w);
+}
+
 template <typename T>
 void enqueue_import(int n, const int *perm, const double *wfile, V4<T> *W, cudaStream_t s) {
     k_import<T><<<(n + 255) / 256, 256, 0, s>>>(n, perm, wfile, W);

@@ -14,4 +14,5 @@ template void enqueue_batch_iteration<float>(const BPlan<float> &p, cudaStream_t
 template int enqueue_iteration_timed<float>(const Plan<float> &p, cudaStream_t s, cudaEvent_t *ev, int *kind);
 template void enqueue_import<float>(int n, const int *perm, const double *wfile, V4<float> *W, cudaStream_t s);
 template void enqueue_export<float>(int n, const int *perm, const V4<float> *W, double *wfile, cudaStream_t s);
+template void enqueue_export_cells<float>(int cnt, const int *cells, const V4<float> *W, double *w, cudaStream_t s);
 }

@@ -9,4 +9,5 @@ template void enqueue_batch_iteration<double>(const BPlan<double> &p, cudaStream
 template int enqueue_iteration_timed<double>(const Plan<double> &p, cudaStream_t s, cudaEvent_t *ev, int *kind);
 template void enqueue_import<double>(int n, const int *perm, const double *wfile, V4<double> *W, cudaStream_t s);
 template void enqueue_export<double>(int n, const int *perm, const V4<double> *W, double *wfile, cudaStream_t s);
+template void enqueue_export_cells<double>(int cnt, const int *cells, const V4<double> *W, double *w, cudaStream_t s);
 }

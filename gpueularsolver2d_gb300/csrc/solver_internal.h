@@ -32,8 +32,9 @@ struct HostLayout {
 
 int build_layout(e2d_mesh *m, const e2d_params &p, HostLayout &L);
 
-// CL, CD from a file-order state (see e2d_forces).
-void forces_from_state(const HostLayout &L, const FreeStream &fs, double gamma, const double *w_file,
+// CL, CD from the states of the wall faces' cells, in the order of L.wall_cell
+// (see e2d_forces).
+void forces_from_walls(const HostLayout &L, const FreeStream &fs, double gamma, const double *w_wall,
                        double *cl, double *cd);
 
 // CL, CD, total mass and boundary mass fluxes of a file-order state (see
