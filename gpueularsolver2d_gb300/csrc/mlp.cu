@@ -20,7 +20,7 @@
 
 #include "fp64_alu.cuh"
 #include "mlp_kernels.cuh"
-#include "mlp_tma.cuh"
+#include "mlp_chain.cuh"
 #include "solver_internal.h"
 
 using namespace e2d;
@@ -44,10 +44,18 @@ constexpr int NIN = E2D_MLP_INPUTS;  // padded input width
 constexpr int KX = 64;
 constexpr int NOUT = 4;
 constexpr int H = 256;
-constexpr int kSplits = 64;          // split-K over the batch for weight gradients
+constexpr int kSplits = 64;          // split-K over the batch for weight gradients (per-tile kernels)
+constexpr int kLossSlots = 1024;     // training steps whose losses stay on the device before they are read
+// Below this many bytes of weight-gradient partials (all hidden layers, half of
+// L2) every layer keeps its own, and a step runs one weight-gradient launch and
+// one Adam launch; above it, layer by layer with two alternating sets, so that
+// Adam still finds its partials in L2.
+constexpr size_t kMergeBytes = (size_t)64 << 20;
 
+// step[0]: Adam steps done; step[1]: loss slot of the current step.
 __global__ void k_step_update(int *step, float beta1, float beta2, float *bc) {
     const int s = ++*step;
+    step[1]++;
     bc[0] = 1.f - powf(beta1, (float)s);
     bc[1] = 1.f - powf(beta2, (float)s);
 }
@@ -55,35 +63,42 @@ __global__ void k_step_update(int *step, float beta1, float beta2, float *bc) {
 // One parameter tensor's Adam step: the gradient of element i = (r, c) is the
 // sum of nparts partials part[p * pstride + r * pld + c]; wbf (may be null,
 // row pitch wld) is the bf16 copy used by
-// the GEMMs, wbfT (may be null) its transpose ([cols][rows], the data-gradient
-// GEMM's K-major operand); grad_out (may be null) receives the gradient.
+// the GEMMs; grad_out (may be null) receives the gradient.
 struct AdamSeg {
     const float *part;
     size_t pstride;
     int nparts, count, rows, cols;
     int pld, wld;  // row pitch of a partial and of wbf (elements; cols unless padded)
     float *w32, *m, *v;
-    bf16 *wbf, *wbfT;
+    bf16 *wbf;
     float *grad_out;
 };
 
-// Adam on two tensors (a layer's weights and bias) in one launch: blocks
-// [0, nb0) take seg0, the rest seg1, 128 parameters per 256-thread block
-// (every count, stride and partial offset a multiple of 4).  Lane l of warp j
-// sums parameters 4l .. 4l + 3 of the block over partials j, j + 8, ...
-// (16-byte loads, sixteen in flight: one round for up to 128 partials; the
-// partials are still in L2, so the kernel is bound by the latency of its
-// rounds), the eight warp sums are added in a fixed tree (deterministic), and
-// warp 0 applies the step with its moments and weights requested up front.  lr (device, read at run
-// time so that the host can schedule it) null: gradient only.
-__global__ void __launch_bounds__(256) k_adam_seg(AdamSeg seg0, AdamSeg seg1, int nb0,
+// Adam on a list of tensors (a layer's weights and bias, or every tensor of the
+// network) in one launch: tensor k takes blocks [first[k], first[k + 1]), 128
+// parameters per 256-thread block (every count, stride and partial offset a
+// multiple of 4).  Lane l of warp j sums parameters 4l .. 4l + 3 of the block over
+// partials j, j + 8, ... (16-byte loads, sixteen in flight: one round for up to
+// 128 partials; the partials are still in L2, so the kernel is bound by the
+// latency of its rounds), the eight warp sums are added in a fixed tree
+// (deterministic), and warp 0 applies the step with its moments and weights
+// requested up front.  lr (device, read at run time so that the host can
+// schedule it) null: gradient only.
+constexpr int kMaxSegs = 2 * (ws::MAXL + 1);
+struct AdamList {
+    AdamSeg seg[kMaxSegs];
+    int first[kMaxSegs + 1];
+    int n = 0;
+};
+__global__ void __launch_bounds__(256) k_adam_seg(const __grid_constant__ AdamList list,
                                                   const float *__restrict__ lr_dev, float beta1, float beta2,
                                                   float eps, const float *__restrict__ bc) {
     __shared__ float4 red[8][32];
-    const bool first = (int)blockIdx.x < nb0;
-    const AdamSeg &S = first ? seg0 : seg1;
+    int k = 0;
+    while ((int)blockIdx.x >= list.first[k + 1]) k++;
+    const AdamSeg &S = list.seg[k];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int i = (((int)blockIdx.x - (first ? 0 : nb0)) * 32 + lane) * 4;
+    const int i = (((int)blockIdx.x - list.first[k]) * 32 + lane) * 4;
     const int ri = i / S.cols, ci = i % S.cols;  // cols is 1 or a multiple of 4
     const bool live = i < S.count;
     // the step's other operands are requested first: they do not depend on the sum
@@ -122,7 +137,7 @@ __global__ void __launch_bounds__(256) k_adam_seg(AdamSeg seg0, AdamSeg seg1, in
     for (int q = 0; q < 4; q++) {
         float r[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++) r[k] = ((const float *)&red[k][lane])[q];
+        for (int w = 0; w < 8; w++) r[w] = ((const float *)&red[w][lane])[q];
         g[q] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
     }
     if (S.grad_out) *(float4 *)(S.grad_out + i) = make_float4(g[0], g[1], g[2], g[3]);
@@ -141,19 +156,12 @@ __global__ void __launch_bounds__(256) k_adam_seg(AdamSeg seg0, AdamSeg seg1, in
         __align__(8) __nv_bfloat162 h2[2] = {__floats2bfloat162_rn(wo[0], wo[1]), __floats2bfloat162_rn(wo[2], wo[3])};
         *(uint2 *)(S.wbf + (size_t)ri * S.wld + ci) = *(const uint2 *)h2;
     }
-    if (S.wbfT)
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            S.wbfT[(size_t)((i + q) % S.cols) * S.rows + (i + q) / S.cols] = __float2bfloat16_rn(wo[q]);
 }
 
-// bf16 copy (row pitch ld) of a [rows][cols] matrix, and (bT non-null) of its transpose
-__global__ void k_to_bf16(int n, const float *__restrict__ a, bf16 *__restrict__ b, bf16 *__restrict__ bT, int rows,
-                          int cols, int ld) {
+// bf16 copy (row pitch ld) of a matrix of n elements in rows of cols
+__global__ void k_to_bf16(int n, const float *__restrict__ a, bf16 *__restrict__ b, int cols, int ld) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    b[(size_t)(i / cols) * ld + i % cols] = __float2bfloat16_rn(a[i]);
-    if (bT) bT[(size_t)(i % cols) * rows + i / cols] = __float2bfloat16_rn(a[i]);
+    if (i < n) b[(size_t)(i / cols) * ld + i % cols] = __float2bfloat16_rn(a[i]);
 }
 
 // Rows of NIN FP32 inputs to rows of bf16 with pitch ld; rows from cnt on are
@@ -261,7 +269,6 @@ struct Tensor {
     int rows, cols;
     float *w32 = nullptr, *m = nullptr, *v = nullptr;
     bf16 *wbf = nullptr;   // hidden layers: [rows][wld()] (the first layer padded to KX columns)
-    bf16 *wbfT = nullptr;  // hidden layers after the first: [cols][rows]
     int count() const { return rows * cols; }
     int wld() const { return cols == NIN ? KX : cols; }
 };
@@ -278,13 +285,16 @@ struct e2d_mlp {
     float *xf = nullptr;  // [cfg.batch][NIN], the caller's FP32 rows on their way into xb or X
     float *tb = nullptr, *y = nullptr, *dy = nullptr;
     std::vector<bf16 *> Gd, Hh;  // [nhidden] of [B][H]: gelu'(z) and gelu(z) of each hidden layer
-    bf16 *dz[2] = {nullptr, nullptr};  // [B][H]
-    // weight- and bias-gradient partials, two sets: a layer's Adam step reads
-    // one on the side stream while the next layer's gradient fills the other
-    float *part[2] = {nullptr, nullptr};
-    float *bpart[2] = {nullptr, nullptr};
-    double *loss_part = nullptr;
-    int *step_dev = nullptr;
+    std::vector<bf16 *> dz;  // [nhidden] of [B][H]: gradient at each hidden layer's pre-activation
+    // weight- and bias-gradient partials of each hidden layer (merged: its own;
+    // otherwise one of two sets in turn, a layer's Adam step reading one on
+    // the side stream while the next layer's gradient fills the other), and
+    // of the output layer
+    bool merged = false;
+    std::vector<float *> part, bpart;
+    float *opart = nullptr;
+    double *loss_part = nullptr;  // [kLossSlots][B / 256]
+    int *step_dev = nullptr;      // k_step_update
     int *flag_dev = nullptr;    // set by a tensor-core GEMM whose wait timed out
     float *bc_dev = nullptr;
     float *lr_dev = nullptr;    // Adam step size, read by every step
@@ -298,16 +308,13 @@ struct e2d_mlp {
     cudaStream_t side = nullptr;  // Adam steps, overlapping the next layer's gradient
     cudaEvent_t ev_fork = nullptr, ev_done[2] = {nullptr, nullptr};
     cudaGraphExec_t gexec = nullptr;
-    // TMA tensor maps of the 256 x 256 GEMMs (ws::k_gemm_ws), per hidden layer
-    // l >= 1: forward A = Hh[l-1], W_l; data gradient A = dz[0] / dz[1], W_l^T
+    // the TMA / tcgen05 kernels: tensor maps of the forward chain (step l is
+    // layer l), of the data-gradient chain (step k is layer L - 1 - k, whose
+    // output is the gradient of the layer before) and of the weight gradients
     bool use_ws = false;
     int nsm = 0;
-    std::vector<CUtensorMap> mapHf, mapW, mapWT, mapHw;
-    std::vector<CUtensorMap> mapHo, mapGo;  // Hh[l], Gd[l] in 32 x 32 epilogue slabs
-    // dz[0] / dz[1] with 128-row boxes (data gradient), 64-row boxes (weights), 32 x 32 slabs
-    CUtensorMap mapDz[2], mapDzw[2], mapDzo[2];
-    CUtensorMap mapPart[2], mapPart0[2];  // weight-gradient partials: 256 x 256 layers, the first layer (256 x KX)
-    CUtensorMap mapX, mapXw, mapW0;   // the first layer's inputs (128- and 64-row boxes) and BF16 weights
+    ws::ChainMaps fwd, bwd;
+    ws::WgradMaps wgrad;
     int wrows = ws::WROWS;  // batch rows per weight-gradient split
     std::vector<double> loss_host;
 
@@ -347,11 +354,9 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// 2D map of a row-major [rows][cols] bf16 matrix, box 64 columns x box_rows,
-// 128-byte swizzle (the layout the ws kernel's descriptors describe)
 // Row-major [rows][cols] bf16 tensor, boxes of box_rows x 64 columns with the
-// 128-byte swizzle (MMA operands) or, slab = true, 32 x 32 with the 64-byte
-// swizzle (the epilogue slabs of ws::k_gemm_ws).
+// 128-byte swizzle (MMA operands, and the 32-row parts of them that an epilogue
+// stores) or, slab = true, 32 x 32 with the 64-byte swizzle (gelu'(z)).
 bool map_2d(CUtensorMap *map, const bf16 *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, bool slab = false) {
     auto enc = tensor_map_encoder();
     if (!enc) return false;
@@ -378,7 +383,7 @@ bool map_part(CUtensorMap *map, const float *ptr, uint64_t rows, uint64_t cols) 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of the warp-specialised GEMMs once the batch buffers exist;
+// Tensor maps of the TMA / tcgen05 kernels once the batch buffers exist;
 // use_ws stays false (the per-tile kernel runs every layer) when the driver
 // entry point, a map or the shared-memory size is not available, or
 // E2D_MLP_WS=0.  With E2D_MLP_WS=1 that is an error instead.
@@ -394,57 +399,36 @@ int build_ws_maps(e2d_mlp *m) {
         if (required) { set_error("E2D_MLP_WS=1: no device attributes"); return E2D_ERR_CUDA; }
         return E2D_OK;
     }
-    m->mapHf.assign(m->nhidden, CUtensorMap{});
-    m->mapW.assign(m->nhidden, CUtensorMap{});
-    m->mapWT.assign(m->nhidden, CUtensorMap{});
-    m->mapHw.assign(m->nhidden, CUtensorMap{});
-    m->mapHo.assign(m->nhidden, CUtensorMap{});
-    m->mapGo.assign(m->nhidden, CUtensorMap{});
     bool ok = m->wrows >= ws::WCH && m->wrows % ws::WCH == 0 && m->B % m->wrows == 0;
-    for (int l = 0; l < m->nhidden && ok; l++) {
-        ok = ok && map_2d(&m->mapHo[l], m->Hh[l], m->B, H, 32, true);
-        ok = ok && map_2d(&m->mapGo[l], m->Gd[l], m->B, H, 32, true);
+    const int L = m->nhidden;
+    const uint64_t B = m->B, prows = (uint64_t)(m->B / m->wrows) * H;
+    ok = ok && map_2d(&m->fwd.in, m->xb, B, KX, ws::BM) && map_2d(&m->bwd.in, m->dz[L - 1], B, H, ws::BM);
+    for (int l = 0; l < L && ok; l++) {
+        ok = ok && map_2d(&m->fwd.w[l], m->W[l].wbf, H, l ? H : KX, ws::ND);
+        ok = ok && map_2d(&m->fwd.out[l], m->Hh[l], B, H, 32) && map_2d(&m->fwd.aux[l], m->Gd[l], B, H, 32, true);
+        ok = ok && map_2d(&m->wgrad.dz[l], m->dz[l], B, H, ws::WCH);
+        ok = ok && (l ? map_2d(&m->wgrad.h[l], m->Hh[l - 1], B, H, ws::WCH)
+                      : map_2d(&m->wgrad.h[l], m->xb, B, KX, ws::WCH));
+        ok = ok && map_part(&m->wgrad.part[l], m->part[l], prows, l ? H : KX);
+        m->wgrad.bpart[l] = m->bpart[l];
+        if (l == 0) continue;
+        const int k = L - 1 - l;
+        ok = ok && map_2d(&m->bwd.w[k], m->W[l].wbf, H, H, ws::KC);
+        ok = ok && map_2d(&m->bwd.out[k], m->dz[l - 1], B, H, 32) && map_2d(&m->bwd.aux[k], m->Gd[l - 1], B, H, 32, true);
     }
-    for (int l = 1; l < m->nhidden && ok; l++) {
-        ok = ok && map_2d(&m->mapHf[l], m->Hh[l - 1], m->B, H, ws::BM);
-        ok = ok && map_2d(&m->mapW[l], m->W[l].wbf, H, H, ws::ND);
-        ok = ok && map_2d(&m->mapWT[l], m->W[l].wbfT, H, H, ws::ND);
-        ok = ok && map_2d(&m->mapHw[l], m->Hh[l - 1], m->B, H, ws::WCH);
-    }
-    for (int k = 0; k < 2 && ok; k++) {
-        ok = ok && map_2d(&m->mapDz[k], m->dz[k], m->B, H, ws::BM);
-        ok = ok && map_2d(&m->mapDzw[k], m->dz[k], m->B, H, ws::WCH);
-        ok = ok && map_2d(&m->mapDzo[k], m->dz[k], m->B, H, 32, true);
-    }
-    for (int k = 0; k < 2 && ok; k++) {
-        ok = ok && map_part(&m->mapPart[k], m->part[k], (uint64_t)(m->B / m->wrows) * H, H);
-        ok = ok && map_part(&m->mapPart0[k], m->part[k], (uint64_t)(m->B / m->wrows) * H, KX);
-    }
-    ok = ok && map_2d(&m->mapX, m->xb, m->B, KX, ws::BM);
-    ok = ok && map_2d(&m->mapXw, m->xb, m->B, KX, ws::WCH);
-    ok = ok && map_2d(&m->mapW0, m->W[0].wbf, H, KX, ws::ND);
     const auto smem_ok = [](const void *f, int bytes) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    if (ok && smem_ok((const void *)ws::k_gemm_ws<EPI_BIAS_GELU, 4>, ws::Gemm<4>::SMEM) &&
-        smem_ok((const void *)ws::k_gemm_ws<EPI_BIAS_GELU, 1>, ws::Gemm<1>::SMEM) &&
-        smem_ok((const void *)ws::k_gemm_ws<EPI_GELU_BWD, 4>, ws::Gemm<4>::SMEM) &&
+    if (ok && smem_ok((const void *)ws::k_chain<EPI_BIAS_GELU>, ws::CHAIN_SMEM) &&
+        smem_ok((const void *)ws::k_chain<EPI_GELU_BWD>, ws::CHAIN_SMEM) &&
         smem_ok((const void *)ws::k_wgrad_ws<4>, ws::WSMEM) && smem_ok((const void *)ws::k_wgrad_ws<1>, ws::WSMEM))
         m->use_ws = true;
     cudaGetLastError();
     if (required && !m->use_ws) {
-        set_error("E2D_MLP_WS=1: the warp-specialised GEMMs cannot run here (tensor maps or shared memory)");
+        set_error("E2D_MLP_WS=1: the TMA / tcgen05 kernels cannot run here (tensor maps or shared memory)");
         return E2D_ERR_CUDA;
     }
     return E2D_OK;
-}
-
-template <int EPI, int NK>
-void gemm_ws(e2d_mlp *m, const CUtensorMap &a, const CUtensorMap &w, const CUtensorMap &out, const CUtensorMap &aux,
-             ws::Args g, cudaStream_t s) {
-    g.flag = m->flag_dev;
-    const int ntiles = g.M / ws::BM, grid = ntiles < m->nsm ? ntiles : m->nsm;
-    ws::k_gemm_ws<EPI, NK><<<grid, ws::THREADS, ws::Gemm<NK>::SMEM, s>>>(a, w, out, aux, g);
 }
 
 size_t param_count(const e2d_mlp *m) {
@@ -472,20 +456,29 @@ int ensure_batch(e2d_mlp *m, int B) {
         if ((rc = m->alloc(&m->Gd[l], sizeof(bf16) * (size_t)B * H))) return rc;
         if ((rc = m->alloc(&m->Hh[l], sizeof(bf16) * (size_t)B * H))) return rc;
     }
-    for (int k = 0; k < 2; k++)
-        if ((rc = m->alloc(&m->dz[k], sizeof(bf16) * (size_t)B * H))) return rc;
+    m->dz.resize(m->nhidden);
+    for (int l = 0; l < m->nhidden; l++)
+        if ((rc = m->alloc(&m->dz[l], sizeof(bf16) * (size_t)B * H))) return rc;
     // weight-gradient partials: kSplits of the per-tile kernel, or one per
-    // wrows rows of the batch for the warp-specialised one (512 rows: 128
-    // CTAs at batch 65536, 20.7 us per layer against 26.9 us for 1024 rows,
-    // with Adam summing twice the partials)
+    // wrows rows of the batch for the TMA one (512 rows: 128 CTAs at batch
+    // 65536, 20.7 us per layer against 26.9 us for 1024 rows, with Adam
+    // summing twice the partials)
     const int nparts = std::max(kSplits, B / m->wrows);
-    for (int k = 0; k < 2; k++)
-        if ((rc = m->alloc(&m->part[k], sizeof(float) * (size_t)nparts * H * H))) return rc;
-    // bias / output-layer partials: the same, or one per 256 rows for the output layer
-    for (int k = 0; k < 2; k++)
-        if ((rc = m->alloc(&m->bpart[k], sizeof(float) * (size_t)std::max(nparts, B / 256) * (NOUT * H + NOUT + H))))
-            return rc;
-    if ((rc = m->alloc(&m->loss_part, sizeof(double) * (B / 256)))) return rc;
+    m->merged = (size_t)m->nhidden * (B / m->wrows) * H * H * sizeof(float) <= kMergeBytes;
+    m->part.resize(m->nhidden);
+    m->bpart.resize(m->nhidden);
+    for (int l = m->nhidden - 1; l >= 0; l--) {
+        const int share = l + 2;  // the set of the layer two up, unless merged
+        if (!m->merged && share < m->nhidden) {
+            m->part[l] = m->part[share];
+            m->bpart[l] = m->bpart[share];
+            continue;
+        }
+        if ((rc = m->alloc(&m->part[l], sizeof(float) * (size_t)nparts * H * H))) return rc;
+        if ((rc = m->alloc(&m->bpart[l], sizeof(float) * (size_t)nparts * H))) return rc;
+    }
+    if ((rc = m->alloc(&m->opart, sizeof(float) * (size_t)(B / 256) * (NOUT * H + NOUT)))) return rc;
+    if ((rc = m->alloc(&m->loss_part, sizeof(double) * kLossSlots * (B / 256)))) return rc;
     return build_ws_maps(m);
 }
 
@@ -509,16 +502,22 @@ AdamSeg adam_seg(const Tensor &t, const float *part, int nparts, size_t pstride,
     g.part = part; g.pstride = pstride; g.nparts = nparts; g.count = t.count();
     g.rows = t.rows; g.cols = t.cols;
     g.pld = pld ? pld : t.cols; g.wld = t.wld();
-    g.w32 = t.w32; g.m = t.m; g.v = t.v; g.wbf = t.wbf; g.wbfT = t.wbfT;
+    g.w32 = t.w32; g.m = t.m; g.v = t.v; g.wbf = t.wbf;
     g.grad_out = grad_out;
     return g;
 }
 
-// Adam on a weight tensor and its bias in one launch.
-void adam2(e2d_mlp *m, cudaStream_t s, const AdamSeg &w, const AdamSeg &b, const float *lr) {
+void adam_add(AdamList &list, const AdamSeg &g) {
+    if (list.n == 0) list.first[0] = 0;
+    list.seg[list.n] = g;
+    list.first[list.n + 1] = list.first[list.n] + (g.count + 127) / 128;
+    list.n++;
+}
+
+// Adam on the listed tensors in one launch.
+void adam(e2d_mlp *m, cudaStream_t s, const AdamList &list, const float *lr) {
     const auto &c = m->cfg;
-    const int nb0 = (w.count + 127) / 128, nb1 = (b.count + 127) / 128;
-    k_adam_seg<<<nb0 + nb1, 256, 0, s>>>(w, b, nb0, lr, (float)c.beta1, (float)c.beta2, (float)c.eps, m->bc_dev);
+    k_adam_seg<<<list.first[list.n], 256, 0, s>>>(list, lr, (float)c.beta1, (float)c.beta2, (float)c.eps, m->bc_dev);
 }
 
 template <bool TA, bool TB, int EPI> void gemm(e2d_mlp *m, GemmArgs g, dim3 grid, cudaStream_t s) {
@@ -542,14 +541,18 @@ int check_flag(e2d_mlp *m) {
 // Forward on the first B rows of xb (a multiple of 128) through the hidden
 // layers; without targets (inference) also the output layer into y.
 void forward(e2d_mlp *m, cudaStream_t s, bool with_loss, int B) {
-    for (int l = 0; l < m->nhidden; l++) {
-        if (m->use_ws) {
-            ws::Args a{};
-            a.M = B; a.bias = m->b[l].w32;
-            if (l == 0) gemm_ws<EPI_BIAS_GELU, 1>(m, m->mapX, m->mapW0, m->mapHo[0], m->mapGo[0], a, s);
-            else gemm_ws<EPI_BIAS_GELU, 4>(m, m->mapHf[l], m->mapW[l], m->mapHo[l], m->mapGo[l], a, s);
-            continue;
-        }
+    if (m->use_ws) {
+        ws::ChainArgs a{};
+        a.M = B;
+        a.steps = m->nhidden;
+        a.first = KX / ws::KC;
+        a.keep = with_loss ? 0 : m->nhidden - 1;
+        a.aux = with_loss;
+        for (int l = 0; l < m->nhidden; l++) a.bias[l] = m->b[l].w32;
+        a.flag = m->flag_dev;
+        ws::k_chain<EPI_BIAS_GELU><<<std::min(B / ws::BM, m->nsm), ws::THREADS, ws::CHAIN_SMEM, s>>>(m->fwd, a);
+    }
+    for (int l = 0; l < m->nhidden && !m->use_ws; l++) {
         GemmArgs g{};
         g.M = B; g.N = H; g.K = l == 0 ? NIN : H;
         g.A = l == 0 ? m->xb : m->Hh[l - 1];
@@ -577,88 +580,102 @@ void backward(e2d_mlp *m, cudaStream_t s, const float *lr, bool want_grad) {
         goff -= t.count();
         return m->grad + goff;
     };
-    // Each layer's Adam step runs on the side stream, forked after the
-    // layer's weight gradient, while the main stream goes on with the next
-    // layer (which needs neither the updated weights nor these partials);
-    // the partial sets alternate, and a set is only refilled after the Adam
-    // step that read it.  Both streams join at the end.
-    bool used[2] = {false, false};
-    auto claim = [&](int k) {
-        if (used[k]) cudaStreamWaitEvent(s, m->ev_done[k], 0);
-    };
-    auto fork_adam = [&](int k, const AdamSeg &w, const AdamSeg &bias) {
-        cudaEventRecord(m->ev_fork, s);
-        cudaStreamWaitEvent(m->side, m->ev_fork, 0);
-        adam2(m, m->side, w, bias, lr);
-        cudaEventRecord(m->ev_done[k], m->side);
-        used[k] = true;
-    };
     // output layer, forward and backward in one pass (loss, its weight / bias
     // partials, and the gradient at the last pre-activation: the output
     // layer's data gradient times the stored gelu'(z))
     Tensor &Wo = m->W[L], &bo = m->b[L];
     const int oparts = B / 256;
     k_out_train<H, NOUT><<<oparts, 256, 0, s>>>(B, m->Hh[L - 1], Wo.w32, bo.w32, m->tb, m->Gd[L - 1], m->y, m->dy,
-                                                m->dz[0], m->bpart[0], m->loss_part);
+                                                m->dz[L - 1], m->opart, m->loss_part, m->step_dev + 1);
     const size_t ostride = NOUT * H + NOUT;
     float *gbo = gslot(bo);
     float *gWo = gslot(Wo);
-    fork_adam(0, adam_seg(Wo, m->bpart[0], oparts, ostride, gWo),
-              adam_seg(bo, m->bpart[0] + NOUT * H, oparts, ostride, gbo));
-    int cur = 0;
-    for (int l = L - 1; l >= 0; l--) {
-        const int kin = l == 0 ? NIN : H, pk = (L - l) & 1;  // partial set of this layer
-        // gradient at the previous pre-activation, first (it reads W_l before
-        // this layer's Adam step changes it): dz W_l, W_l read MN-major
-        // ([out][in] = [K][N]); then the weight gradient, whose partials the
-        // Adam step reads straight after, while they are still in L2
-        if (l > 0 && m->use_ws) {
-            ws::Args a{};
-            a.M = B;
-            gemm_ws<EPI_GELU_BWD, 4>(m, m->mapDz[cur], m->mapWT[l], m->mapDzo[cur ^ 1], m->mapGo[l - 1], a, s);
-        } else if (l > 0) {
-            GemmArgs gd{};
-            gd.M = B; gd.N = H; gd.K = H;
-            gd.A = m->dz[cur]; gd.lda = H;
-            gd.B = m->W[l].wbf; gd.ldb = H;
-            gd.zin = m->Gd[l - 1]; gd.out = m->dz[cur ^ 1]; gd.ldc = H;
-            gemm<false, true, EPI_GELU_BWD>(m, gd, dim3(H / BN, (B + BM - 1) / BM, 1), s);
+    // Adam steps: all in one list (merged), or each on the side stream, forked
+    // after the gradient it reads, while the main stream goes on with the
+    // next layer; a partial set is only refilled after the Adam step that
+    // read it, and both streams join at the end.
+    AdamList all;
+    bool used[2] = {false, false};
+    auto claim = [&](int k) {
+        if (used[k]) cudaStreamWaitEvent(s, m->ev_done[k], 0);
+    };
+    auto step = [&](int k, const AdamSeg &w, const AdamSeg &bias) {
+        if (m->merged) {
+            adam_add(all, w);
+            adam_add(all, bias);
+            return;
         }
-        claim(pk);
-        // dW_l = dz^T hin (split over the batch; both operands are read
-        // MN-major, the batch index being their slow one), db_l = column sums
-        // of dz
-        int wparts = kSplits, pld = kin;
+        AdamList one;
+        adam_add(one, w);
+        adam_add(one, bias);
+        cudaEventRecord(m->ev_fork, s);
+        cudaStreamWaitEvent(m->side, m->ev_fork, 0);
+        adam(m, m->side, one, lr);
+        cudaEventRecord(m->ev_done[k], m->side);
+        used[k] = true;
+    };
+    step(0, adam_seg(Wo, m->opart, oparts, ostride, gWo), adam_seg(bo, m->opart + NOUT * H, oparts, ostride, gbo));
+    // the data gradients of every layer first: they read the weights that the
+    // Adam steps change
+    if (m->use_ws && L > 1) {
+        ws::ChainArgs a{};
+        a.M = B;
+        a.steps = L - 1;
+        a.first = 4;
+        a.flag = m->flag_dev;
+        ws::k_chain<EPI_GELU_BWD><<<std::min(B / ws::BM, m->nsm), ws::THREADS, ws::CHAIN_SMEM, s>>>(m->bwd, a);
+    }
+    for (int l = L - 1; l > 0 && !m->use_ws; l--) {
+        // dz W_l, W_l read MN-major ([out][in] = [K][N])
+        GemmArgs gd{};
+        gd.M = B; gd.N = H; gd.K = H;
+        gd.A = m->dz[l]; gd.lda = H;
+        gd.B = m->W[l].wbf; gd.ldb = H;
+        gd.zin = m->Gd[l - 1]; gd.out = m->dz[l - 1]; gd.ldc = H;
+        gemm<false, true, EPI_GELU_BWD>(m, gd, dim3(H / BN, (B + BM - 1) / BM, 1), s);
+    }
+    // weight gradients dW_l = dz^T hin (split over the batch; both operands are
+    // read MN-major, the batch index being their slow one), db_l = column sums
+    // of dz
+    const int wparts = m->use_ws ? B / m->wrows : kSplits;
+    if (m->use_ws && m->merged && L > 1) {
+        // the first layer's beside the others'
+        cudaEventRecord(m->ev_fork, s);
+        cudaStreamWaitEvent(m->side, m->ev_fork, 0);
+        ws::k_wgrad_ws<1><<<wparts, ws::WTHREADS, ws::WSMEM, m->side>>>(m->wgrad, 0, B, m->wrows, m->flag_dev);
+        cudaEventRecord(m->ev_done[0], m->side);
+        ws::k_wgrad_ws<4><<<dim3(wparts, L - 1), ws::WTHREADS, ws::WSMEM, s>>>(m->wgrad, 1, B, m->wrows, m->flag_dev);
+        used[0] = true;
+    }
+    for (int l = L - 1; l >= 0; l--) {
+        const int kin = l == 0 ? NIN : H, pk = l & 1;  // partial set of this layer
+        // the first layer's TMA partials are 256 x KX (its padding columns get zero)
+        const int pld = m->use_ws && l == 0 ? KX : kin;
+        if (!m->merged) claim(pk);
         if (m->use_ws) {
-            // the first layer's partials are 256 x KX (its padding columns get zero)
-            wparts = B / m->wrows;
-            if (l == 0) {
-                pld = KX;
-                ws::k_wgrad_ws<1><<<wparts, ws::WTHREADS, ws::WSMEM, s>>>(m->mapDzw[cur], m->mapXw, m->mapPart0[pk],
-                                                                          B, m->wrows, m->bpart[pk], m->flag_dev);
-            } else {
-                ws::k_wgrad_ws<4><<<wparts, ws::WTHREADS, ws::WSMEM, s>>>(m->mapDzw[cur], m->mapHw[l], m->mapPart[pk],
-                                                                          B, m->wrows, m->bpart[pk], m->flag_dev);
-            }
+            if (l == 0 && (!m->merged || L == 1))
+                ws::k_wgrad_ws<1><<<wparts, ws::WTHREADS, ws::WSMEM, s>>>(m->wgrad, l, B, m->wrows, m->flag_dev);
+            else if (l > 0 && !m->merged)
+                ws::k_wgrad_ws<4><<<wparts, ws::WTHREADS, ws::WSMEM, s>>>(m->wgrad, l, B, m->wrows, m->flag_dev);
         } else {
             GemmArgs gw{};
             gw.M = H; gw.N = kin; gw.K = B;
-            gw.A = m->dz[cur]; gw.lda = H;
+            gw.A = m->dz[l]; gw.lda = H;
             gw.B = l == 0 ? m->xb : m->Hh[l - 1]; gw.ldb = l == 0 ? KX : H;
-            gw.part = m->part[pk];
+            gw.part = m->part[l];
             gemm<true, true, EPI_PARTIAL>(m, gw, dim3((kin + BN - 1) / BN, H / BM, kSplits), s);
-            // (the warp-specialised weight-gradient kernel also writes the
-            // bias gradient's partials, one per split)
-            k_colsum<<<dim3(H / 32, kSplits), 256, 0, s>>>(B, H, rows, m->dz[cur], m->bpart[pk]);
+            // (the TMA weight-gradient kernel also writes the bias gradient's
+            // partials, one per split)
+            k_colsum<<<dim3(H / 32, kSplits), 256, 0, s>>>(B, H, rows, m->dz[l], m->bpart[l]);
         }
         float *gb = gslot(m->b[l]);
         float *gW = gslot(m->W[l]);
-        fork_adam(pk, adam_seg(m->W[l], m->part[pk], wparts, (size_t)H * pld, gW, pld),
-                  adam_seg(m->b[l], m->bpart[pk], wparts, H, gb));
-        cur ^= 1;
+        step(pk, adam_seg(m->W[l], m->part[l], wparts, (size_t)H * pld, gW, pld),
+             adam_seg(m->b[l], m->bpart[l], wparts, H, gb));
     }
     claim(0);
     claim(1);
+    if (m->merged) adam(m, s, all, lr);
 }
 
 // The cell centroids and the wall faces of a mesh on the device, with room for
@@ -717,7 +734,7 @@ int build_train_graph(e2d_mlp *m) {
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     k_step_update<<<1, 1, 0, s>>>(m->step_dev, (float)m->cfg.beta1, (float)m->cfg.beta2, m->bc_dev);
     // the gather reads the step from device memory through its seed argument
-    k_gather<<<(m->B + 255) / 256, 256, 0, s>>>(m->B, NIN, KX, NOUT, m->cfg.seed, m->step_dev, m->nsamples, m->X,
+    k_gather<NIN, NOUT><<<m->B * (NIN / 8) / 256, 256, 0, s>>>(m->B, KX, m->cfg.seed, m->step_dev, m->nsamples, m->X,
                                                   m->T, m->xb, m->tb);
     forward(m, s, true, m->B);
     backward(m, s, m->lr_dev, false);
@@ -790,18 +807,16 @@ int e2d_mlp_create(const e2d_mlp_config *cfg, e2d_mlp **out) {
             if ((rc = m->alloc(&t->m, sizeof(float) * n))) return rc;
             if ((rc = m->alloc(&t->v, sizeof(float) * n))) return rc;
             if (!last && t == &W && (rc = m->alloc(&t->wbf, sizeof(bf16) * (size_t)t->rows * t->wld()))) return rc;
-            if (!last && l > 0 && t == &W && (rc = m->alloc(&t->wbfT, sizeof(bf16) * n))) return rc;
         }
         CK(cudaMemcpy(W.w32, hw.data(), sizeof(float) * hw.size(), cudaMemcpyHostToDevice));
         CK(cudaMemcpy(b.w32, hb.data(), sizeof(float) * hb.size(), cudaMemcpyHostToDevice));
         if (W.wbf)
-            k_to_bf16<<<(W.count() + 255) / 256, 256, 0, m->stream>>>(W.count(), W.w32, W.wbf, W.wbfT, W.rows,
-                                                                       W.cols, W.wld());
+            k_to_bf16<<<(W.count() + 255) / 256, 256, 0, m->stream>>>(W.count(), W.w32, W.wbf, W.cols, W.wld());
         m->W.push_back(W);
         m->b.push_back(b);
     }
     int rc;
-    if ((rc = m->alloc(&m->step_dev, sizeof(int)))) return rc;
+    if ((rc = m->alloc(&m->step_dev, 2 * sizeof(int)))) return rc;
     if ((rc = m->alloc(&m->flag_dev, sizeof(int)))) return rc;
     CK(cudaFuncSetAttribute(k_gemm_tc<false, false, EPI_BIAS_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             tc::SMEM));
@@ -845,8 +860,7 @@ int e2d_mlp_set_params(e2d_mlp *m, const float *in) {
         for (Tensor *t : {&m->W[l], &m->b[l]}) {
             CK(cudaMemcpy(t->w32, in + off, sizeof(float) * t->count(), cudaMemcpyHostToDevice));
             if (t->wbf)
-                k_to_bf16<<<(t->count() + 255) / 256, 256, 0, m->stream>>>(t->count(), t->w32, t->wbf, t->wbfT,
-                                                                            t->rows, t->cols, t->wld());
+                k_to_bf16<<<(t->count() + 255) / 256, 256, 0, m->stream>>>(t->count(), t->w32, t->wbf, t->cols, t->wld());
             off += t->count();
         }
     CK(cudaStreamSynchronize(m->stream));
@@ -887,19 +901,23 @@ int e2d_mlp_train(e2d_mlp *m, int32_t steps, double *loss) {
     int rc = ensure_batch(m, m->cfg.batch);
     if (rc) return rc;
     if ((rc = build_train_graph(m))) return rc;
+    // the steps run back to back; their loss partials stay on the device until
+    // kLossSlots steps are done
     const int nlp = m->B / 256;
-    std::vector<double> lp(nlp);
-    for (int k = 0; k < steps; k++) {
-        CK(cudaGraphLaunch(m->gexec, m->stream));
-        if (loss) {
-            CK(cudaMemcpyAsync(lp.data(), m->loss_part, sizeof(double) * nlp, cudaMemcpyDeviceToHost, m->stream));
-            CK(cudaStreamSynchronize(m->stream));
+    std::vector<double> lp(loss ? (size_t)std::min(steps, kLossSlots) * nlp : 0);
+    for (int k0 = 0; k0 < steps; k0 += kLossSlots) {
+        const int cnt = std::min(steps - k0, kLossSlots);
+        CK(cudaMemsetAsync(m->step_dev + 1, 0xff, sizeof(int), m->stream));  // -1: the first step takes slot 0
+        for (int k = 0; k < cnt; k++) CK(cudaGraphLaunch(m->gexec, m->stream));
+        if (loss)
+            CK(cudaMemcpyAsync(lp.data(), m->loss_part, sizeof(double) * cnt * nlp, cudaMemcpyDeviceToHost, m->stream));
+        CK(cudaStreamSynchronize(m->stream));
+        for (int k = 0; loss && k < cnt; k++) {
             double s = 0.0;
-            for (double v : lp) s += v;
-            loss[k] = s / ((double)m->B * NOUT);
+            for (int j = 0; j < nlp; j++) s += lp[(size_t)k * nlp + j];
+            loss[k0 + k] = s / ((double)m->B * NOUT);
         }
     }
-    CK(cudaStreamSynchronize(m->stream));
     return check_flag(m);
 }
 
@@ -925,6 +943,7 @@ int e2d_mlp_gradient(e2d_mlp *m, const float *x, const float *t, double *loss, f
     if (rc) return rc;
     if ((rc = stage_rows(m, x, m->B, m->B, m->xb, KX))) return rc;
     CK(cudaMemcpyAsync(m->tb, t, sizeof(float) * (size_t)m->B * NOUT, cudaMemcpyHostToDevice, m->stream));
+    CK(cudaMemsetAsync(m->step_dev + 1, 0, sizeof(int), m->stream));  // loss slot 0
     forward(m, m->stream, true, m->B);
     backward(m, m->stream, nullptr, true);
     CK(cudaGetLastError());

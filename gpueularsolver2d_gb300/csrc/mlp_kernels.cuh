@@ -367,113 +367,127 @@ __global__ void __launch_bounds__(256) k_out_bwd_data(int B, const float *__rest
 }
 
 // Output layer of a training step, forward and backward in one pass over the
-// last hidden layer (256 -> NOUT on the CUDA cores), one warp per row: lane l
-// holds h[b][8l .. 8l + 7] (one 16-byte load), the NOUT dot products are
-// butterfly-reduced over the warp, then y, the squared-error loss, dY = 2 (y - t)
-// / (B NOUT), the gradient dz[b][k] = (sum_o dY[b][o] W[o][k]) gd[b][k] (bf16,
-// gd = gelu'(z) stored by the forward epilogue) and the lane's share of
-// dW = dY^T h, db = sum dY.  Block c (256 rows, 8 warps of 32 rows) writes
-// part[c][o * H + k] and part[c][NOUT * H + o] (its warps added in a fixed
-// order) and loss_part[c]: deterministic.
+// last hidden layer (256 -> NOUT = 4 on the CUDA cores), one warp per row: lane
+// l holds h[b][8l .. 8l + 7] (one 16-byte load); the four dot products are
+// reduced over the warp together (each exchange also halves the number of
+// outputs a lane carries, until lanes 8 o .. 8 o + 7 hold output o), then y, the
+// error e = y - t, dY = 2 e / (B NOUT), the gradient dz[b][k] = (sum_o dY[b][o]
+// W[o][k]) gd[b][k] (bf16, gd = gelu'(z) stored by the forward epilogue) and the
+// lane's share of dW = dY^T h, db = sum dY.  Block c (256 rows, 8 warps of 32
+// rows) writes part[c][o * H + k] and part[c][NOUT * H + o] (its warps added in a
+// fixed order) and loss_part[*slot][c], the sum of e^2 in FP64: deterministic.
+// The errors wait in shared memory and eight lanes of one warp add them at the
+// end, each its warp's 128 in order: added row by row, the FP64 pipe (one warp
+// instruction per SM in 16 cycles, whatever its active lanes) was 69 % busy and
+// bound the kernel (46 us at batch 65536).
 template <int H, int NOUT>
 __global__ void __launch_bounds__(256, 2) k_out_train(int B, const bf16 *__restrict__ h, const float *__restrict__ W,
                                                    const float *__restrict__ bias, const float *__restrict__ t,
                                                    const bf16 *__restrict__ gd, float *__restrict__ y,
                                                    float *__restrict__ dy, bf16 *__restrict__ dz,
-                                                   float *__restrict__ part, double *__restrict__ loss_part) {
+                                                   float *__restrict__ part, double *__restrict__ loss_part,
+                                                   const int *__restrict__ slot) {
     static_assert(H == 256, "one 16-byte load per lane covers a row");
+    static_assert(NOUT == 4, "the reduction splits four outputs over the warp");
     __shared__ float red[8][NOUT * H + NOUT];
     __shared__ __align__(16) float Ws[NOUT * H];
-    __shared__ double lred[8];
+    __shared__ float errs[8][32 * NOUT + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k0 = lane * 8;
     for (int e = threadIdx.x; e < NOUT * H; e += blockDim.x) Ws[e] = W[e];
     __syncthreads();
-    float acc[NOUT][8], dacc[NOUT];
+    float acc[NOUT][8], dacc = 0.f;
 #pragma unroll
-    for (int o = 0; o < NOUT; o++) {
-        dacc[o] = 0.f;
+    for (int o = 0; o < NOUT; o++)
 #pragma unroll
         for (int q = 0; q < 8; q++) acc[o][q] = 0.f;
-    }
-    double l = 0.0;
+    const bool hi = lane & 16, mid = lane & 8;
+    const int mine = lane >> 3;  // this lane's output after the reduction
+    const float bo = bias[mine];
     const int r0 = blockIdx.x * 256 + warp * 32;  // B is a multiple of 256
     constexpr int RB = 2;                          // rows whose loads are in flight together
     for (int rb = 0; rb < 32; rb += RB) {
         uint4 hvs[RB], gvs[RB];
+        float tv[RB];
 #pragma unroll
         for (int j = 0; j < RB; j++) {
             hvs[j] = *(const uint4 *)(h + (size_t)(r0 + rb + j) * H + k0);
             gvs[j] = *(const uint4 *)(gd + (size_t)(r0 + rb + j) * H + k0);
+            tv[j] = t[(size_t)(r0 + rb + j) * NOUT + mine];
         }
 #pragma unroll
-    for (int j = 0; j < RB; j++) {
-        const int b = r0 + rb + j;
-        const uint4 hv = hvs[j], gv = gvs[j];
-        const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&hv;
-        float x[8];
+        for (int j = 0; j < RB; j++) {
+            const int b = r0 + rb + j;
+            const uint4 hv = hvs[j], gv = gvs[j];
+            const __nv_bfloat162 *h2 = (const __nv_bfloat162 *)&hv;
+            float x[8];
 #pragma unroll
-        for (int q = 0; q < 4; q++) { x[2 * q] = __low2float(h2[q]); x[2 * q + 1] = __high2float(h2[q]); }
-        float p[NOUT];
-#pragma unroll
-        for (int o = 0; o < NOUT; o++) {
-            const float4 wa = *(const float4 *)&Ws[o * H + k0], wb = *(const float4 *)&Ws[o * H + k0 + 4];
-            p[o] = fmaf(x[0], wa.x, fmaf(x[1], wa.y, fmaf(x[2], wa.z, fmaf(x[3], wa.w,
-                   fmaf(x[4], wb.x, fmaf(x[5], wb.y, fmaf(x[6], wb.z, x[7] * wb.w)))))));
-        }
-#pragma unroll
-        for (int o = 0; o < NOUT; o++)
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) p[o] += __shfl_xor_sync(0xffffffffu, p[o], sh);
-        float d[NOUT];
-#pragma unroll
-        for (int o = 0; o < NOUT; o++) {
-            const float yo = p[o] + bias[o];
-            const float e = yo - t[(size_t)b * NOUT + o];
-            if (lane == 0) {
-                y[(size_t)b * NOUT + o] = yo;
-                l += (double)e * e;
-            }
-            d[o] = 2.0f * e / (float)(B * NOUT);
-            if (lane == o) dy[(size_t)b * NOUT + o] = d[o];
-            dacc[o] += d[o];
-#pragma unroll
-            for (int q = 0; q < 8; q++) acc[o][q] = fmaf(d[o], x[q], acc[o][q]);
-        }
-        const __nv_bfloat162 *g2 = (const __nv_bfloat162 *)&gv;
-        __align__(16) __nv_bfloat162 o2[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            float s0 = 0.f, s1 = 0.f;
+            for (int q = 0; q < 4; q++) { x[2 * q] = __low2float(h2[q]); x[2 * q + 1] = __high2float(h2[q]); }
+            float p[NOUT];
 #pragma unroll
             for (int o = 0; o < NOUT; o++) {
-                const float2 wo = *(const float2 *)&Ws[o * H + k0 + 2 * q];
-                s0 = fmaf(d[o], wo.x, s0);
-                s1 = fmaf(d[o], wo.y, s1);
+                const float4 wa = *(const float4 *)&Ws[o * H + k0], wb = *(const float4 *)&Ws[o * H + k0 + 4];
+                p[o] = fmaf(x[0], wa.x, fmaf(x[1], wa.y, fmaf(x[2], wa.z, fmaf(x[3], wa.w,
+                       fmaf(x[4], wb.x, fmaf(x[5], wb.y, fmaf(x[6], wb.z, x[7] * wb.w)))))));
             }
-            o2[q] = __floats2bfloat162_rn(s0 * __low2float(g2[q]), s1 * __high2float(g2[q]));
+            float v0 = hi ? p[2] : p[0], v1 = hi ? p[3] : p[1];
+            v0 += __shfl_xor_sync(0xffffffffu, hi ? p[0] : p[2], 16);
+            v1 += __shfl_xor_sync(0xffffffffu, hi ? p[1] : p[3], 16);
+            float s = mid ? v1 : v0;
+            s += __shfl_xor_sync(0xffffffffu, mid ? v0 : v1, 8);
+#pragma unroll
+            for (int sh = 4; sh > 0; sh >>= 1) s += __shfl_xor_sync(0xffffffffu, s, sh);
+            const float yo = s + bo, e = yo - tv[j], de = 2.0f * e / (float)(B * NOUT);
+            dacc += de;
+            if ((lane & 7) == 0) {
+                y[(size_t)b * NOUT + mine] = yo;
+                dy[(size_t)b * NOUT + mine] = de;
+                errs[warp][(rb + j) * NOUT + mine] = e;
+            }
+            float d[NOUT];
+#pragma unroll
+            for (int o = 0; o < NOUT; o++) {
+                d[o] = __shfl_sync(0xffffffffu, de, 8 * o);
+#pragma unroll
+                for (int q = 0; q < 8; q++) acc[o][q] = fmaf(d[o], x[q], acc[o][q]);
+            }
+            const __nv_bfloat162 *g2 = (const __nv_bfloat162 *)&gv;
+            __align__(16) __nv_bfloat162 o2[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+                for (int o = 0; o < NOUT; o++) {
+                    const float2 wo = *(const float2 *)&Ws[o * H + k0 + 2 * q];
+                    s0 = fmaf(d[o], wo.x, s0);
+                    s1 = fmaf(d[o], wo.y, s1);
+                }
+                o2[q] = __floats2bfloat162_rn(s0 * __low2float(g2[q]), s1 * __high2float(g2[q]));
+            }
+            *(uint4 *)(dz + (size_t)b * H + k0) = *(const uint4 *)o2;
         }
-        *(uint4 *)(dz + (size_t)b * H + k0) = *(const uint4 *)o2;
-    }
     }
 #pragma unroll
-    for (int o = 0; o < NOUT; o++) {
+    for (int o = 0; o < NOUT; o++)
 #pragma unroll
         for (int q = 0; q < 8; q++) red[warp][o * H + k0 + q] = acc[o][q];
-        if (lane == 0) red[warp][NOUT * H + o] = dacc[o];
-    }
-    if (lane == 0) lred[warp] = l;
+    if ((lane & 7) == 0) red[warp][NOUT * H + mine] = dacc;
     __syncthreads();
+    if (warp == 7) {  // the other warps go on with the partials below
+        double l = 0.0;
+        if (lane < 8)
+            for (int k = 0; k < 32 * NOUT; k++) l = fma((double)errs[lane][k], (double)errs[lane][k], l);
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) s += __shfl_sync(0xffffffffu, l, k);
+        if (lane == 0) loss_part[(size_t)*slot * gridDim.x + blockIdx.x] = s;
+        return;
+    }
     float *pc = part + (size_t)blockIdx.x * (NOUT * H + NOUT);
-    for (int e = threadIdx.x; e < NOUT * H + NOUT; e += blockDim.x) {
+    for (int e = threadIdx.x; e < NOUT * H + NOUT; e += 224) {
         float s = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; k++) s += red[k][e];
         pc[e] = s;
-    }
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < 8; k++) s += lred[k];
-        loss_part[blockIdx.x] = s;
     }
 }
 
@@ -539,14 +553,16 @@ __global__ void __launch_bounds__(256) k_colsum(int B, int N, int rows_per_split
     }
 }
 
-// Random mini-batch gather: rows idx(step, j) of the training set (nin
-// columns) into row j of xb (row pitch ldx), with the step counter read from
-// device memory (the training step is a static graph).
-__global__ void __launch_bounds__(256) k_gather(int B, int nin, int ldx, int nout, unsigned long long seed,
-                                                const int *__restrict__ stepp, long long nsamples,
-                                                const bf16 *__restrict__ X, const float *__restrict__ T,
-                                                bf16 *__restrict__ xb, float *__restrict__ tb) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// Random mini-batch gather: rows idx(step, j) of the training set into row j of
+// xb (row pitch ldx) and tb, with the step counter read from device memory (the
+// training step is a static graph).  One thread per eight columns.
+template <int NIN, int NOUT>
+__global__ void __launch_bounds__(256) k_gather(int B, int ldx, unsigned long long seed, const int *__restrict__ stepp,
+                                                long long nsamples, const bf16 *__restrict__ X,
+                                                const float *__restrict__ T, bf16 *__restrict__ xb,
+                                                float *__restrict__ tb) {
+    static_assert(NOUT == 4, "one 16-byte target per row");
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = i / (NIN / 8), c = i % (NIN / 8);
     if (j >= B) return;
     const int step = *stepp;
     unsigned long long z = seed + 0x9e3779b97f4a7c15ULL * ((unsigned long long)step * 1315423911ULL + j + 1);
@@ -554,9 +570,8 @@ __global__ void __launch_bounds__(256) k_gather(int B, int nin, int ldx, int nou
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
     z ^= z >> 31;
     const long long r = (long long)(z % (unsigned long long)nsamples);
-    for (int k = 0; k < nin; k += 8)
-        *(uint4 *)(xb + (size_t)j * ldx + k) = *(const uint4 *)(X + (size_t)r * nin + k);
-    for (int o = 0; o < nout; o++) tb[(size_t)j * nout + o] = T[(size_t)r * nout + o];
+    *(uint4 *)(xb + (size_t)j * ldx + 8 * c) = *(const uint4 *)(X + (size_t)r * NIN + 8 * c);
+    if (c == 0) *(float4 *)(tb + (size_t)j * NOUT) = *(const float4 *)(T + (size_t)r * NOUT);
 }
 
 }  // namespace mlp
