@@ -74,22 +74,52 @@ struct AdamSeg {
     float *grad_out;
 };
 
+// The Adam step of parameters i .. i + 3 with gradient g (lr null: the gradient
+// is written only); m4, v4, w4: their moments and weights.
+struct AdamCoef {
+    float lr, bc0, bc1, beta1, beta2, eps;
+};
+__device__ __forceinline__ void adam_apply(const AdamSeg &S, const int i, const int ri, const int ci, const float *g,
+                                           const float4 m4, const float4 v4, const float4 w4, const bool step,
+                                           const AdamCoef c) {
+    if (S.grad_out) *(float4 *)(S.grad_out + i) = make_float4(g[0], g[1], g[2], g[3]);
+    if (!step) return;
+    float mo[4], vo[4], wo[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        mo[q] = c.beta1 * ((const float *)&m4)[q] + (1.f - c.beta1) * g[q];
+        vo[q] = c.beta2 * ((const float *)&v4)[q] + (1.f - c.beta2) * g[q] * g[q];
+        wo[q] = ((const float *)&w4)[q] - c.lr * (mo[q] / c.bc0) / (sqrtf(vo[q] / c.bc1) + c.eps);
+    }
+    *(float4 *)(S.m + i) = make_float4(mo[0], mo[1], mo[2], mo[3]);
+    *(float4 *)(S.v + i) = make_float4(vo[0], vo[1], vo[2], vo[3]);
+    *(float4 *)(S.w32 + i) = make_float4(wo[0], wo[1], wo[2], wo[3]);
+    if (S.wbf) {
+        __align__(8) __nv_bfloat162 h2[2] = {__floats2bfloat162_rn(wo[0], wo[1]), __floats2bfloat162_rn(wo[2], wo[3])};
+        *(uint2 *)(S.wbf + (size_t)ri * S.wld + ci) = *(const uint2 *)h2;
+    }
+}
+
 // Adam on a list of tensors (a layer's weights and bias, or every tensor of the
-// network) in one launch: tensor k takes blocks [first[k], first[k + 1]), 128
-// parameters per 256-thread block (every count, stride and partial offset a
-// multiple of 4).  Lane l of warp j sums parameters 4l .. 4l + 3 of the block over
-// partials j, j + 8, ... (16-byte loads, sixteen in flight: one round for up to
-// 128 partials; the partials are still in L2, so the kernel is bound by the
-// latency of its rounds), the eight warp sums are added in a fixed tree
-// (deterministic), and warp 0 applies the step with its moments and weights
-// requested up front.  lr (device, read at run time so that the host can
-// schedule it) null: gradient only.
+// network) in one launch: tensor k takes blocks [first[k], first[k + 1]) of 256
+// threads (every count, stride and partial offset a multiple of 4), four
+// parameters to a lane.  The gradient is the sum of the partials in a fixed
+// order: eight sums over partials j, j + 8, ... (even and odd terms apart), added
+// in a tree.  lr (device, read at run time so that the host can schedule it)
+// null: gradient only.
+// ALONE (every tensor has at most kWarpParts partials): a lane adds all eight sums itself, 1024 parameters
+// to a block; otherwise the block's eight warps take one sum each of the same 128
+// parameters (sixteen 16-byte loads in flight, one round for up to 128
+// partials, which are still in L2) and warp 0 applies the step.  With 8 partials
+// (batch 4096, 8 layers) the second form took 21 us, most of its warps idle.
 constexpr int kMaxSegs = 2 * (ws::MAXL + 1);
+constexpr int kWarpParts = 32;
 struct AdamList {
     AdamSeg seg[kMaxSegs];
     int first[kMaxSegs + 1];
     int n = 0;
 };
+template <bool ALONE>  // every tensor of the list has at most kWarpParts partials
 __global__ void __launch_bounds__(256) k_adam_seg(const __grid_constant__ AdamList list,
                                                   const float *__restrict__ lr_dev, float beta1, float beta2,
                                                   float eps, const float *__restrict__ bc) {
@@ -97,31 +127,60 @@ __global__ void __launch_bounds__(256) k_adam_seg(const __grid_constant__ AdamLi
     int k = 0;
     while ((int)blockIdx.x >= list.first[k + 1]) k++;
     const AdamSeg &S = list.seg[k];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int i = (((int)blockIdx.x - list.first[k]) * 32 + lane) * 4;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, block = (int)blockIdx.x - list.first[k];
+    const int i = (ALONE ? block * 256 + (int)threadIdx.x : block * 32 + lane) * 4;
     const int ri = i / S.cols, ci = i % S.cols;  // cols is 1 or a multiple of 4
     const bool live = i < S.count;
     // the step's other operands are requested first: they do not depend on the sum
     float4 m4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = m4, w4 = m4;
-    float lr = 0.f, bc0 = 1.f, bc1 = 1.f;
-    if (wp == 0 && live && lr_dev) {
+    AdamCoef c{0.f, 1.f, 1.f, beta1, beta2, eps};
+    if ((ALONE || wp == 0) && live && lr_dev) {
         m4 = *(const float4 *)(S.m + i);
         v4 = *(const float4 *)(S.v + i);
         w4 = *(const float4 *)(S.w32 + i);
-        lr = *lr_dev;
-        bc0 = bc[0];
-        bc1 = bc[1];
+        c.lr = *lr_dev;
+        c.bc0 = bc[0];
+        c.bc1 = bc[1];
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float *pp = S.part + (size_t)ri * S.pld + ci;
+    float g[4];
+    if constexpr (ALONE) {
+        if (!live) return;
+        float4 a[8][2];
+#pragma unroll
+        for (int w = 0; w < 8; w++) a[w][0] = a[w][1] = zero;
+#pragma unroll
+        for (int j = 0; j < kWarpParts / 8; j++) {
+            if (8 * j >= S.nparts) break;
+            float4 v[8];
+#pragma unroll
+            for (int w = 0; w < 8; w++)
+                v[w] = 8 * j + w < S.nparts ? *(const float4 *)(pp + (size_t)(8 * j + w) * S.pstride) : zero;
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                float4 &t = a[w][j & 1];
+                t.x += v[w].x; t.y += v[w].y; t.z += v[w].z; t.w += v[w].w;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            float r[8];
+#pragma unroll
+            for (int w = 0; w < 8; w++) r[w] = ((const float *)&a[w][0])[q] + ((const float *)&a[w][1])[q];
+            g[q] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
+        }
+        adam_apply(S, i, ri, ci, g, m4, v4, w4, lr_dev != nullptr, c);
+        return;
     }
     // partials wp, wp + 8, ..., sixteen 16-byte loads in flight per round
-    float4 a[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    float4 a[2] = {zero, zero};
     if (live) {
-        const float *pp = S.part + (size_t)ri * S.pld + ci;
         for (int p0 = wp; p0 < S.nparts; p0 += 128) {
             float4 v[16];
 #pragma unroll
             for (int j = 0; j < 16; j++)
-                v[j] = p0 + 8 * j < S.nparts ? *(const float4 *)(pp + (size_t)(p0 + 8 * j) * S.pstride)
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[j] = p0 + 8 * j < S.nparts ? *(const float4 *)(pp + (size_t)(p0 + 8 * j) * S.pstride) : zero;
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 float4 &t = a[j & 1];
@@ -132,7 +191,6 @@ __global__ void __launch_bounds__(256) k_adam_seg(const __grid_constant__ AdamLi
     red[wp][lane] = make_float4(a[0].x + a[1].x, a[0].y + a[1].y, a[0].z + a[1].z, a[0].w + a[1].w);
     __syncthreads();
     if (wp != 0 || !live) return;
-    float g[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         float r[8];
@@ -140,22 +198,7 @@ __global__ void __launch_bounds__(256) k_adam_seg(const __grid_constant__ AdamLi
         for (int w = 0; w < 8; w++) r[w] = ((const float *)&red[w][lane])[q];
         g[q] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
     }
-    if (S.grad_out) *(float4 *)(S.grad_out + i) = make_float4(g[0], g[1], g[2], g[3]);
-    if (!lr_dev) return;
-    float mo[4], vo[4], wo[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        mo[q] = beta1 * ((const float *)&m4)[q] + (1.f - beta1) * g[q];
-        vo[q] = beta2 * ((const float *)&v4)[q] + (1.f - beta2) * g[q] * g[q];
-        wo[q] = ((const float *)&w4)[q] - lr * (mo[q] / bc0) / (sqrtf(vo[q] / bc1) + eps);
-    }
-    *(float4 *)(S.m + i) = make_float4(mo[0], mo[1], mo[2], mo[3]);
-    *(float4 *)(S.v + i) = make_float4(vo[0], vo[1], vo[2], vo[3]);
-    *(float4 *)(S.w32 + i) = make_float4(wo[0], wo[1], wo[2], wo[3]);
-    if (S.wbf) {
-        __align__(8) __nv_bfloat162 h2[2] = {__floats2bfloat162_rn(wo[0], wo[1]), __floats2bfloat162_rn(wo[2], wo[3])};
-        *(uint2 *)(S.wbf + (size_t)ri * S.wld + ci) = *(const uint2 *)h2;
-    }
+    adam_apply(S, i, ri, ci, g, m4, v4, w4, lr_dev != nullptr, c);
 }
 
 // bf16 copy (row pitch ld) of a matrix of n elements in rows of cols
@@ -356,16 +399,16 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // Row-major [rows][cols] bf16 tensor, boxes of box_rows x 64 columns with the
 // 128-byte swizzle (MMA operands, and the 32-row parts of them that an epilogue
-// stores) or, slab = true, 32 x 32 with the 64-byte swizzle (gelu'(z)).
-bool map_2d(CUtensorMap *map, const bf16 *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, bool slab = false) {
+// stores).
+bool map_2d(CUtensorMap *map, const bf16 *ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
     auto enc = tensor_map_encoder();
     if (!enc) return false;
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {cols * sizeof(bf16)};
-    const cuuint32_t box[2] = {slab ? 32u : (cuuint32_t)ws::KC, slab ? 32u : box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)ws::KC, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)ptr, dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, slab ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -405,7 +448,7 @@ int build_ws_maps(e2d_mlp *m) {
     ok = ok && map_2d(&m->fwd.in, m->xb, B, KX, ws::BM) && map_2d(&m->bwd.in, m->dz[L - 1], B, H, ws::BM);
     for (int l = 0; l < L && ok; l++) {
         ok = ok && map_2d(&m->fwd.w[l], m->W[l].wbf, H, l ? H : KX, ws::ND);
-        ok = ok && map_2d(&m->fwd.out[l], m->Hh[l], B, H, 32) && map_2d(&m->fwd.aux[l], m->Gd[l], B, H, 32, true);
+        ok = ok && map_2d(&m->fwd.out[l], m->Hh[l], B, H, 32);
         ok = ok && map_2d(&m->wgrad.dz[l], m->dz[l], B, H, ws::WCH);
         ok = ok && (l ? map_2d(&m->wgrad.h[l], m->Hh[l - 1], B, H, ws::WCH)
                       : map_2d(&m->wgrad.h[l], m->xb, B, KX, ws::WCH));
@@ -414,13 +457,15 @@ int build_ws_maps(e2d_mlp *m) {
         if (l == 0) continue;
         const int k = L - 1 - l;
         ok = ok && map_2d(&m->bwd.w[k], m->W[l].wbf, H, H, ws::KC);
-        ok = ok && map_2d(&m->bwd.out[k], m->dz[l - 1], B, H, 32) && map_2d(&m->bwd.aux[k], m->Gd[l - 1], B, H, 32, true);
+        ok = ok && map_2d(&m->bwd.out[k], m->dz[l - 1], B, H, 32);
     }
     const auto smem_ok = [](const void *f, int bytes) {
         return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    if (ok && smem_ok((const void *)ws::k_chain<EPI_BIAS_GELU>, ws::CHAIN_SMEM) &&
-        smem_ok((const void *)ws::k_chain<EPI_GELU_BWD>, ws::CHAIN_SMEM) &&
+    if (ok && smem_ok((const void *)ws::k_chain<EPI_BIAS_GELU, 1>, ws::Chain<1>::SMEM) &&
+        smem_ok((const void *)ws::k_chain<EPI_BIAS_GELU, 2>, ws::Chain<2>::SMEM) &&
+        smem_ok((const void *)ws::k_chain<EPI_GELU_BWD, 1>, ws::Chain<1>::SMEM) &&
+        smem_ok((const void *)ws::k_chain<EPI_GELU_BWD, 2>, ws::Chain<2>::SMEM) &&
         smem_ok((const void *)ws::k_wgrad_ws<4>, ws::WSMEM) && smem_ok((const void *)ws::k_wgrad_ws<1>, ws::WSMEM))
         m->use_ws = true;
     cudaGetLastError();
@@ -507,17 +552,18 @@ AdamSeg adam_seg(const Tensor &t, const float *part, int nparts, size_t pstride,
     return g;
 }
 
-void adam_add(AdamList &list, const AdamSeg &g) {
-    if (list.n == 0) list.first[0] = 0;
-    list.seg[list.n] = g;
-    list.first[list.n + 1] = list.first[list.n] + (g.count + 127) / 128;
-    list.n++;
-}
+void adam_add(AdamList &list, const AdamSeg &g) { list.seg[list.n++] = g; }
 
 // Adam on the listed tensors in one launch.
-void adam(e2d_mlp *m, cudaStream_t s, const AdamList &list, const float *lr) {
+void adam(e2d_mlp *m, cudaStream_t s, AdamList &list, const float *lr) {
     const auto &c = m->cfg;
-    k_adam_seg<<<list.first[list.n], 256, 0, s>>>(list, lr, (float)c.beta1, (float)c.beta2, (float)c.eps, m->bc_dev);
+    bool alone = true;
+    for (int k = 0; k < list.n; k++) alone = alone && list.seg[k].nparts <= kWarpParts;
+    const int per = alone ? 1024 : 128;  // parameters of a block
+    list.first[0] = 0;
+    for (int k = 0; k < list.n; k++) list.first[k + 1] = list.first[k] + (list.seg[k].count + per - 1) / per;
+    const auto kernel = alone ? k_adam_seg<true> : k_adam_seg<false>;
+    kernel<<<list.first[list.n], 256, 0, s>>>(list, lr, (float)c.beta1, (float)c.beta2, (float)c.eps, m->bc_dev);
 }
 
 template <bool TA, bool TB, int EPI> void gemm(e2d_mlp *m, GemmArgs g, dim3 grid, cudaStream_t s) {
@@ -538,6 +584,16 @@ int check_flag(e2d_mlp *m) {
     return E2D_OK;
 }
 
+// One direction's chain: two tiles to a CTA once there are more tiles than SMs
+// (batch 65536, 5 layers: forward 111 -> 77 us, data gradient 91 -> 67 us; with one
+// tile per SM the larger ring is the better use of shared memory).
+template <int EPI> void chain(e2d_mlp *m, const ws::ChainMaps &maps, ws::ChainArgs &a, cudaStream_t s) {
+    a.flag = m->flag_dev;
+    const int ntiles = a.M / ws::BM, grid = std::min(ntiles, m->nsm);
+    if (ntiles > m->nsm) ws::k_chain<EPI, 2><<<grid, ws::THREADS, ws::Chain<2>::SMEM, s>>>(maps, a);
+    else ws::k_chain<EPI, 1><<<grid, ws::THREADS, ws::Chain<1>::SMEM, s>>>(maps, a);
+}
+
 // Forward on the first B rows of xb (a multiple of 128) through the hidden
 // layers; without targets (inference) also the output layer into y.
 void forward(e2d_mlp *m, cudaStream_t s, bool with_loss, int B) {
@@ -547,10 +603,12 @@ void forward(e2d_mlp *m, cudaStream_t s, bool with_loss, int B) {
         a.steps = m->nhidden;
         a.first = KX / ws::KC;
         a.keep = with_loss ? 0 : m->nhidden - 1;
-        a.aux = with_loss;
-        for (int l = 0; l < m->nhidden; l++) a.bias[l] = m->b[l].w32;
-        a.flag = m->flag_dev;
-        ws::k_chain<EPI_BIAS_GELU><<<std::min(B / ws::BM, m->nsm), ws::THREADS, ws::CHAIN_SMEM, s>>>(m->fwd, a);
+        a.store_aux = with_loss;
+        for (int l = 0; l < m->nhidden; l++) {
+            a.bias[l] = m->b[l].w32;
+            a.aux[l] = m->Gd[l];
+        }
+        chain<EPI_BIAS_GELU>(m, m->fwd, a, s);
     }
     for (int l = 0; l < m->nhidden && !m->use_ws; l++) {
         GemmArgs g{};
@@ -585,8 +643,9 @@ void backward(e2d_mlp *m, cudaStream_t s, const float *lr, bool want_grad) {
     // layer's data gradient times the stored gelu'(z))
     Tensor &Wo = m->W[L], &bo = m->b[L];
     const int oparts = B / 256;
-    k_out_train<H, NOUT><<<oparts, 256, 0, s>>>(B, m->Hh[L - 1], Wo.w32, bo.w32, m->tb, m->Gd[L - 1], m->y, m->dy,
-                                                m->dz[L - 1], m->opart, m->loss_part, m->step_dev + 1);
+    const auto out_train = oparts > m->nsm ? k_out_train<H, NOUT, 2, 2> : k_out_train<H, NOUT, 8, 1>;
+    out_train<<<oparts, 256, 0, s>>>(B, m->Hh[L - 1], Wo.w32, bo.w32, m->tb, m->Gd[L - 1], m->y, m->dy, m->dz[L - 1],
+                                     m->opart, m->loss_part, m->step_dev + 1);
     const size_t ostride = NOUT * H + NOUT;
     float *gbo = gslot(bo);
     float *gWo = gslot(Wo);
@@ -622,8 +681,8 @@ void backward(e2d_mlp *m, cudaStream_t s, const float *lr, bool want_grad) {
         a.M = B;
         a.steps = L - 1;
         a.first = 4;
-        a.flag = m->flag_dev;
-        ws::k_chain<EPI_GELU_BWD><<<std::min(B / ws::BM, m->nsm), ws::THREADS, ws::CHAIN_SMEM, s>>>(m->bwd, a);
+        for (int l = L - 1; l > 0; l--) a.aux[L - 1 - l] = m->Gd[l - 1];
+        chain<EPI_GELU_BWD>(m, m->bwd, a, s);
     }
     for (int l = L - 1; l > 0 && !m->use_ws; l--) {
         // dz W_l, W_l read MN-major ([out][in] = [K][N])

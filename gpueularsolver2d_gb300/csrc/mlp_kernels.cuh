@@ -379,9 +379,12 @@ __global__ void __launch_bounds__(256) k_out_bwd_data(int B, const float *__rest
 // The errors wait in shared memory and eight lanes of one warp add them at the
 // end, each its warp's 128 in order: added row by row, the FP64 pipe (one warp
 // instruction per SM in 16 cycles, whatever its active lanes) was 69 % busy and
-// bound the kernel (46 us at batch 65536).
-template <int H, int NOUT>
-__global__ void __launch_bounds__(256, 2) k_out_train(int B, const bf16 *__restrict__ h, const float *__restrict__ W,
+// bound the kernel (46 us at batch 65536, now 36).  RB rows' loads are in flight
+// together, MINB blocks share an SM: 2 and 2 for large batches, 8 and 1 when there
+// is at most one block per SM and the latency of the rows is all there is
+// (batch 4096: 26 -> 22 us).
+template <int H, int NOUT, int RB, int MINB>
+__global__ void __launch_bounds__(256, MINB) k_out_train(int B, const bf16 *__restrict__ h, const float *__restrict__ W,
                                                    const float *__restrict__ bias, const float *__restrict__ t,
                                                    const bf16 *__restrict__ gd, float *__restrict__ y,
                                                    float *__restrict__ dy, bf16 *__restrict__ dz,
@@ -404,7 +407,6 @@ __global__ void __launch_bounds__(256, 2) k_out_train(int B, const bf16 *__restr
     const int mine = lane >> 3;  // this lane's output after the reduction
     const float bo = bias[mine];
     const int r0 = blockIdx.x * 256 + warp * 32;  // B is a multiple of 256
-    constexpr int RB = 2;                          // rows whose loads are in flight together
     for (int rb = 0; rb < 32; rb += RB) {
         uint4 hvs[RB], gvs[RB];
         float tv[RB];

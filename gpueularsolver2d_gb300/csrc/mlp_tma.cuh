@@ -17,8 +17,6 @@ constexpr int KC = 64;                       // K columns per A slice: one 128-b
 constexpr int SLICE_BYTES = BM * KC * 2;     // 16 KB
 constexpr int WSLICE_BYTES = ND * KC * 2;    // 32 KB
 constexpr int NEPI = 16;                     // epilogue warps: 4 per 32-lane quarter of tensor memory
-constexpr int SLAB = 32 * 32 * 2;            // one epilogue slab: 32 rows x 32 columns of bf16
-constexpr int SLABS_BYTES = NEPI * 2 * SLAB; // two slabs per epilogue warp
 constexpr int THREADS = 32 * (2 + NEPI);
 constexpr uint32_t TMEM_COLS = 512;          // two 256-column FP32 accumulators
 constexpr int WAIT_LIMIT = 1 << 22;          // try_wait calls before giving up
@@ -71,12 +69,6 @@ __device__ __forceinline__ void tma_store(const CUtensorMap *map, uint32_t src, 
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n"
                  :: "l"((uint64_t)map), "r"(x), "r"(y), "r"(src) : "memory");
 }
-
-// Byte offset of 16-byte unit u (0..3) of row r in a slab of 64-byte rows
-// with the 64-byte swizzle (unit index XOR bits 1-2 of the row), the layout
-// of a TMA box of 32 bf16 columns under CU_TENSOR_MAP_SWIZZLE_64B.  A
-// quarter-warp (8 consecutive rows, same u) covers all 32 banks.
-__device__ __forceinline__ uint32_t slab_off(int r, int u) { return (uint32_t)(r * 64 + ((u ^ ((r >> 1) & 3)) << 4)); }
 
 __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" :: "r"(bar)
