@@ -121,6 +121,12 @@ template <> struct Over<double> {
 // Divisions of the boundary ghosts: the compiler's in FP32.
 template <typename T> __device__ __forceinline__ T gdiv(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ double gdiv<double>(double a, double b) { return ddiv(a, b); }
+template <typename T> struct GOver {
+    T b;
+    __device__ __forceinline__ explicit GOver(T v) : b(v) {}
+    __device__ __forceinline__ T operator()(T a) const { return a / b; }
+};
+template <> struct GOver<double> : Over<double> { using Over<double>::Over; };
 
 template <typename T> __device__ __forceinline__ T comp(const V4<T> &v, int k) {
     return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
@@ -128,11 +134,12 @@ template <typename T> __device__ __forceinline__ T comp(const V4<T> &v, int k) {
 
 // gpu_solver.cu:49-60 (kernel_CalculationPTA): pressure and sound speed
 template <typename T> __device__ __forceinline__ void pta(const V4<T> &w, T g, T &P, T &A) {
-    T U = gdiv(w.y, w.x);
-    T V = gdiv(w.z, w.x);
-    T E = gdiv(w.w, w.x) - T(0.5) * (U * U + V * V);
+    const GOver<T> by(w.x);
+    T U = by(w.y);
+    T V = by(w.z);
+    T E = by(w.w) - T(0.5) * (U * U + V * V);
     P = (g - T(1.0)) * w.x * E;
-    A = tsqrt(gdiv(g * P, w.x));
+    A = tsqrt(by(g * P));
 }
 
 // gpu_solver.cu:62-135 (kernel_Far_Boundary): far-field ghost state from the
@@ -176,13 +183,52 @@ __device__ __noinline__ V4<T> far_ghost(const V4<T> dw, T P, T A, T vectorx, T v
     return w0;
 }
 
+// FP64: the same operations; divisions by one divisor share its preparation,
+// and the supersonic test's quotient exceeds 1 only where Un > AIN.
+template <>
+inline __device__ __noinline__ V4<double> far_ghost<double>(const V4<double> dw, double P, double A, double vectorx,
+                                                     double vectory, const Flow<double> f) {
+    const double g = f.gamma;
+    const Divisor dn = divisor(tsqrt(vectorx * vectorx + vectory * vectory)), dr = divisor(dw.x);
+    const double nx = div_by(vectory, dn), ny = div_by(vectorx, dn);
+    const double UD = div_by(dw.y, dr), VD = div_by(dw.z, dr);
+    const double Un = fabs(f.ui * nx + f.vi * ny);
+    const double Uncell = UD * nx + VD * ny;
+    V4<double> w0 = dw;
+    if (Un > f.ain && ddiv(Un, f.ain) > 1.0) {
+        if (!(Uncell > 0.0)) {
+            w0.x = 1.0;
+            w0.y = f.ui;
+            w0.z = f.vi;
+            w0.w = ddiv(ddiv(f.R * f.tin, f.vin * f.vin), g - 1.0) + 0.50;
+        }
+    } else {
+        const Divisor da = divisor(A);
+        const bool out = Uncell > 0.0;
+        // outflow: the ghost's pressure is the free stream's, its state follows
+        // from the cell's; inflow: from the free stream's (gpu_solver.cu:98-130)
+        const double PA = f.pis;
+        double PB = PA;
+        if (!out) PB = 0.5 * (PA + P - dw.x * A * (nx * (f.ui - UD) + ny * (f.vi - VD)));
+        const double dp = out ? PB - P : PB - PA, pd = out ? P - PB : PA - PB;
+        w0.x = (out ? dw.x : 1.0) + div_by(div_by(dp, da), da);
+        const double du = div_by(div_by(nx * pd, dr), da), dv = div_by(div_by(ny * pd, dr), da);
+        const double UB = out ? UD + du : f.ui - du, VB = out ? VD + dv : f.vi - dv;
+        w0.y = UB * w0.x;
+        w0.z = VB * w0.x;
+        w0.w = ddiv(PB, g - 1.0) + 0.5 * (UB * UB + VB * VB) * w0.x;
+    }
+    return w0;
+}
+
 // gpu_solver.cu:188-221: slip-wall ghost (velocity mirrored in the face)
 template <typename T>
 __device__ __forceinline__ V4<T> wall_ghost(const V4<T> &dw, T vectorx, T vectory, T vectorn) {
-    T nij0 = gdiv(vectory, vectorn);
-    T nij1 = gdiv(vectorx, vectorn);
-    T UU = gdiv(dw.y, dw.x);
-    T VV = gdiv(dw.z, dw.x);
+    const GOver<T> n(vectorn), r(dw.x);
+    T nij0 = n(vectory);
+    T nij1 = n(vectorx);
+    T UU = r(dw.y);
+    T VV = r(dw.z);
     T UV = UU * nij0 + VV * nij1;
     UU = UU - T(2) * UV * nij0;
     VV = VV - T(2) * UV * nij1;
@@ -657,34 +703,49 @@ __device__ __forceinline__ double face_limiter64(const int kind, const double e2
 }
 
 // The FP64 form of faces_cell with the sum of the cell's three spectral radii
-// given (faces_tile).  It issues about 160 FP64 additions and multiplications
-// per cell in the reference configuration: the reference's halves of the
-// neighbour means are taken into the face vectors (exact), the first term of a
-// sum is not added to zero, the bounds are subtracted once per component and
-// divisions, comparisons and selections run on the integer units.
-template <bool OPT>
+// given (faces_tile), by LPC lanes per cell: lane part takes the NQ = 4 / LPC
+// components from part NQ on.  It issues about 160 FP64 additions and
+// multiplications per cell in the reference configuration: the reference's
+// halves of the neighbour means are taken into the face vectors (exact), the
+// first term of a sum is not added to zero, the bounds are subtracted once per
+// component and divisions, comparisons and selections run on the integer units.
+// gs: the ghost states of the cell's boundary faces.
+template <bool OPT, int LPC>
 __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
-                                               const V4<double> *__restrict__ W, V4<double> *__restrict__ FS,
-                                               double *__restrict__ dt, V4<double> *__restrict__ phi,
-                                               const int frozen, const bool first, const V4<double> U,
-                                               const int4 tp, const double Tsum) {
-    const int n = m.n;
+                                               const int part, const V4<double> *__restrict__ W,
+                                               V4<double> *__restrict__ FS, double *__restrict__ dt,
+                                               V4<double> *__restrict__ phi, const int frozen, const bool first,
+                                               const V4<double> *__restrict__ Uc, const int4 tp,
+                                               const V4<double> *gs, const double Tsum) {
+    constexpr int NQ = 4 / LPC;
+    const int n = m.n, q0 = part * NQ;
     const int code[3] = {tp.x, tp.y, tp.z};
+    auto values = [&](const V4<double> *p, double *v) {
+        const double *d = reinterpret_cast<const double *>(p) + q0;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) v[q] = d[q];
+    };
+    auto store = [&](V4<double> *p, const double *v) {
+        double *d = reinterpret_cast<double *>(p) + q0;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) d[q] = v[q];
+    };
     V2<double> S[3];
+    double u[NQ], nb[3][NQ];
 #pragma unroll
-    for (int k = 0; k < 3; k++) S[k] = m.S[k * n + i];
-    V4<double> nbv[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-        nbv[k] = code[k] >= 0 ? W[code[k] >> 3] : ghost(code[k], U, S[k].x, S[k].y, f);
+    for (int k = 0; k < 3; k++) {
+        S[k] = m.S[k * n + i];
+        values(code[k] >= 0 ? W + (code[k] >> 3) : gs + k, nb[k]);
+    }
+    values(Uc, u);
     const double A = m.area[i];
     const double rA = ddiv(1.0, A);
-    double gx[4], gy[4];
+    double gx[NQ], gy[NQ];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < NQ; q++) {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const double s = comp(U, q) + comp(nbv[k], q);
+            const double s = u[q] + nb[k][q];
             const double px = s * (0.5 * S[k].x), py = s * (0.5 * S[k].y);
             gx[q] = k == 0 ? px : gx[q] + px;
             gy[q] = k == 0 ? py : gy[q] + py;
@@ -693,103 +754,112 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
         gy[q] *= rA;
     }
     const bool reuse = OPT && phi && frozen;
-    double2 bnd[4];
+    double2 bnd[NQ];
     if (!reuse && !(OPT && first)) {
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-            bnd[q] = cell_bounds(comp(nbv[0], q), comp(nbv[1], q), comp(nbv[2], q), comp(U, q));
+        for (int q = 0; q < NQ; q++) bnd[q] = cell_bounds(nb[0][q], nb[1][q], nb[2][q], u[q]);
     }
     const int kind = OPT ? f.limiter & 1 : 0;
     const double e2 = OPT && kind == 1 && !reuse ? f.venk_k3 * A * dsqrt(A) : 0.0;
     // cell-wise limiter options (2, 3): see faces_cell
     const bool cellwise = OPT && f.limiter >= 2;
-    double phic[4] = {1.0, 1.0, 1.0, 1.0};
+    double phic[NQ];
     if (cellwise && !reuse && !first) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) phic[q] = (double)INFINITY;
+        for (int q = 0; q < NQ; q++) phic[q] = (double)INFINITY;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             if (code[k] < 0) continue;
             const V2<double> r = m.R[k * n + i];
 #pragma unroll
-            for (int q = 0; q < 4; q++)
+            for (int q = 0; q < NQ; q++)
                 phic[q] = fmin(phic[q], face_limiter64(kind, e2, bnd[q], gx[q] * r.x + gy[q] * r.y));
         }
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        V4<double> o = U;
+        double d[NQ];
         if (code[k] >= 0 && !(OPT && first)) {
             const V2<double> r = m.R[k * n + i];
-            V4<double> pf;
-            if (reuse) pf = phi[k * n + i];
-            double d[4], ph[4];
+            double ph[NQ];
+            if (reuse) values(phi + k * n + i, ph);
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
+            for (int q = 0; q < NQ; q++) {
                 const double delt2 = gx[q] * r.x + gy[q] * r.y;
-                if (reuse) ph[q] = comp(pf, q);
-                else if (cellwise) ph[q] = phic[q];
-                else ph[q] = face_limiter64(kind, e2, bnd[q], delt2);
-                d[q] = delt2 * ph[q] + comp(U, q);
+                if (cellwise && !reuse) ph[q] = phic[q];
+                else if (!reuse) ph[q] = face_limiter64(kind, e2, bnd[q], delt2);
+                d[q] = delt2 * ph[q] + u[q];
             }
-            o.x = d[0]; o.y = d[1]; o.z = d[2]; o.w = d[3];
-            if (OPT && f.positivity) {
-                // positivity fallback (option): see faces_cell
-                const double q = ddiv(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
-                if (!(d[0] > 0.0) || !((f.gamma - 1.0) * (d[3] - q) > 0.0)) o = U;
-            }
-            if (OPT && phi && !frozen) {
-                V4<double> pw;
-                pw.x = ph[0]; pw.y = ph[1]; pw.z = ph[2]; pw.w = ph[3];
-                phi[k * n + i] = pw;
-            }
+            if constexpr (OPT && LPC == 1)
+                if (f.positivity) {
+                    // positivity fallback (option): see faces_cell
+                    const double q = ddiv(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
+                    if (!(d[0] > 0.0) || !((f.gamma - 1.0) * (d[3] - q) > 0.0))
+                        for (int c = 0; c < 4; c++) d[c] = u[c];
+                }
+            if (OPT && phi && !frozen) store(phi + k * n + i, ph);
+        } else {
+#pragma unroll
+            for (int q = 0; q < NQ; q++) d[q] = u[q];
         }
-        FS[k * n + i] = o;
+        store(FS + k * n + i, d);
     }
+    if (part != 0) return (double)INFINITY;
     const double dti = tmin(ddiv(A * f.cfl, Tsum), f.dt_cap);
     dt[i] = dti;
     return dti;
 }
 
-// Pass A in FP64 for one tile of cells [base, base + nvalid), each interior
-// face's spectral radius evaluated once: the tile lists the radii it must
-// evaluate (boundary faces, faces to cells outside the tile, and inside faces
-// from their left cell only, as flux_tile does for the Roe flux), spreads that
-// list over its threads with the cell states in shared memory, then every cell
-// sums its three radii in face order and runs faces_cell64.  The radius is
+// Pass A in FP64 for one tile of cells [base, base + nvalid), nvalid <=
+// blockDim.x / LPC, each interior face's spectral radius evaluated once: the tile
+// lists the radii it must evaluate (boundary faces, faces to cells outside the
+// tile, and inside faces from their left cell only, as flux_tile does for the
+// Roe flux), spreads that list over its threads with the cell states in shared
+// memory (boundary faces leave their ghost states there), then every cell sums
+// its three radii in face order and LPC lanes run faces_cell64.  The radius is
 // symmetric in its two states and in the sign of the face vector, and the two
-// cells of a face hold exactly negated face vectors, so each cell gets the
-// bits of its own evaluation.  Returns the thread's time step (+inf for a
-// padding lane).  blockDim.x <= kFacesTile.
-constexpr int kFacesTile = 256;
-template <bool OPT>
+// cells of a face hold exactly negated face vectors, so each cell gets the bits
+// of its own evaluation.  Returns the cell's time step (+inf for other lanes).
+// LPC 2 and 4 shorten the chain of a thread where a mesh leaves the GPU's
+// schedulers with few warps (gather_shape).
+struct FacesSmem {
+    V4<double> *Us, *Gs;    // [cells] states, [3 cells] ghost states
+    double *SRs;            // [3 cells] spectral radii
+    int4 *tps;              // [cells] face codes
+    unsigned short *items;  // [3 cells] radii to evaluate
+    static constexpr size_t per_cell = 4 * sizeof(V4<double>) + 3 * sizeof(double) + sizeof(int4) + 3 * sizeof(unsigned short);
+    __device__ __forceinline__ FacesSmem(unsigned char *p, int cells)
+        : Us(reinterpret_cast<V4<double> *>(p)), Gs(Us + cells), SRs(reinterpret_cast<double *>(Gs + 3 * cells)),
+          tps(reinterpret_cast<int4 *>(SRs + 3 * cells)), items(reinterpret_cast<unsigned short *>(tps + cells)) {}
+};
+template <bool OPT, int LPC>
 __device__ __forceinline__ double faces_tile(const MeshDev<double> &m, const Flow<double> &f, const int base,
                                              const int nvalid, const V4<double> *__restrict__ W,
                                              V4<double> *__restrict__ FS, double *__restrict__ dt,
-                                             V4<double> *__restrict__ phi, const int frozen, const bool first) {
+                                             V4<double> *__restrict__ phi, const int frozen, const bool first,
+                                             unsigned char *smem) {
     using T = double;
-    __shared__ V4<T> Us[kFacesTile];
-    __shared__ int4 tps[kFacesTile];
-    __shared__ T SRs[kFacesTile * 3];
-    __shared__ unsigned short items[kFacesTile * 3];
-    __shared__ int wtot[kFacesTile / 32];
-    const int n = m.n, t = threadIdx.x, i = base + t;
-    const bool live = t < nvalid;
+    __shared__ int wtot[8];
+    const FacesSmem sm(smem, blockDim.x / LPC);
+    V4<T> *Us = sm.Us, *Gs = sm.Gs;
+    T *SRs = sm.SRs;
+    int4 *tps = sm.tps;
+    unsigned short *items = sm.items;
+    const int n = m.n, t = threadIdx.x;
+    const bool owner = t < nvalid;
     __syncthreads();  // the previous tile of this block may still read the shared arrays
-    const int4 tp = live ? m.topo[i] : make_int4(-3, -3, -3, 0);
-    tps[t] = tp;
-    V4<T> U = {};
-    if (live) U = W[i];
-    Us[t] = U;
-    const int code[3] = {tp.x, tp.y, tp.z};
     unsigned mask = 0;
+    if (owner) {
+        const int4 tp = m.topo[base + t];
+        tps[t] = tp;
+        Us[t] = W[base + t];
+        const int code[3] = {tp.x, tp.y, tp.z};
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        if (!live) continue;
-        const int c = code[k];
-        if (c < 0) { mask |= 1u << k; continue; }
-        const bool inside = (unsigned)((c >> 3) - base) < (unsigned)nvalid;
-        if (!inside || !((c >> 2) & 1)) mask |= 1u << k;
+        for (int k = 0; k < 3; k++) {
+            const int c = code[k];
+            const bool inside = c >= 0 && (unsigned)((c >> 3) - base) < (unsigned)nvalid;
+            if (!inside || !((c >> 2) & 1)) mask |= 1u << k;
+        }
     }
     // exclusive prefix sum of the per-cell counts over the block
     const int cnt = __popc(mask), lane = t & 31, wid = t >> 5;
@@ -822,19 +892,28 @@ __device__ __forceinline__ double faces_tile(const MeshDev<double> &m, const Flo
             nb = (unsigned)(nj - base) < (unsigned)nvalid ? Us[nj - base] : W[nj];
         } else {
             nb = ghost(c, Uo, S.x, S.y, f);
+            Gs[tt * 3 + k] = nb;
         }
         SRs[tt * 3 + k] = spectral_radius(Uo, nb, S.y, S.x, f.gamma);
     }
     __syncthreads();
-    if (!live) return (double)INFINITY;
+    const int tt = t / LPC;
+    if (tt >= nvalid) return (double)INFINITY;
+    const int4 tp = tps[tt];
+    const int code[3] = {tp.x, tp.y, tp.z};
     T Tsum = T(0);
+    if (t % LPC == 0) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int c = code[k];
-        const T r = (mask & (1u << k)) ? SRs[t * 3 + k] : SRs[((c >> 3) - base) * 3 + (c & 3)];
-        Tsum = k == 0 ? r : Tsum + r;
+        for (int k = 0; k < 3; k++) {
+            // an inside face of which the cell is the right one: its left cell has it
+            const int c = code[k], q = (c >> 3) - base;
+            const bool other = c >= 0 && (unsigned)q < (unsigned)nvalid && ((c >> 2) & 1);
+            const T r = other ? SRs[q * 3 + (c & 3)] : SRs[tt * 3 + k];
+            Tsum = k == 0 ? r : Tsum + r;
+        }
     }
-    return faces_cell64<OPT>(m, f, i, W, FS, dt, phi, frozen, first, U, tp, Tsum);
+    return faces_cell64<OPT, LPC>(m, f, base + tt, t % LPC, W, FS, dt, phi, frozen, first, Us + tt, tp, Gs + tt * 3,
+                                  Tsum);
 }
 
 // Global time-step option: the block's smallest step folded into *slot.
@@ -856,18 +935,19 @@ __device__ __forceinline__ void block_min_dt(double v, unsigned long long *slot)
     }
 }
 
-// FP64: pass A in tiles of blockDim.x cells (faces_tile).
-template <bool OPT>
+// FP64: pass A in tiles of blockDim.x / LPC cells (faces_tile).
+template <bool OPT, int LPC>
 __global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<double> f,
                                                        const V4<double> *__restrict__ W,
                                                        V4<double> *__restrict__ FS, double *__restrict__ dt,
                                                        Ctl *__restrict__ ctl, V4<double> *__restrict__ phi,
                                                        const int st) {
+    extern __shared__ __align__(32) unsigned char smem[];
     wait_prior_grid();
     if (ctl->halt) return;
-    const int base = blockIdx.x * blockDim.x;
-    const double v = faces_tile<OPT>(m, f, base, min((int)blockDim.x, m.n - base), W, FS, dt, phi,
-                                     OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order);
+    const int tile = blockDim.x / LPC, base = blockIdx.x * tile;
+    const double v = faces_tile<OPT, LPC>(m, f, base, min(tile, m.n - base), W, FS, dt, phi,
+                                          OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order, smem);
     if (OPT && f.global_dt) block_min_dt(v, &ctl->dtmin[st]);
 }
 
@@ -892,9 +972,14 @@ __global__ void E2D_LB_FACES k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__res
 }
 
 // The pass-A kernel of a precision.
-template <typename T> auto faces_kernel(bool opt) {
-    if constexpr (sizeof(T) == 8) return opt ? &k_faces_tile<true> : &k_faces_tile<false>;
-    else return opt ? &k_faces<T, true> : &k_faces<T, false>;
+template <typename T> auto faces_kernel(bool opt, int lanes) {
+    if constexpr (sizeof(T) == 8) {
+        if (lanes == 4) return opt ? &k_faces_tile<true, 4> : &k_faces_tile<false, 4>;
+        if (lanes == 2) return opt ? &k_faces_tile<true, 2> : &k_faces_tile<false, 2>;
+        return opt ? &k_faces_tile<true, 1> : &k_faces_tile<false, 1>;
+    } else {
+        return opt ? &k_faces<T, true> : &k_faces<T, false>;
+    }
 }
 
 // True when a pass-A launch needs the option variant.
@@ -1028,18 +1113,21 @@ __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f
 // their left cell only), spreads that list over its threads, keeps the
 // fluxes in shared memory, and then every cell sums its three faces in face
 // order with the reference's signs.  The fluxes are the same bits as in
-// flux_cell and are summed in the same order.  blockDim.x <= 256.
-template <typename T>
+// flux_cell and are summed in the same order.  nvalid <= blockDim.x / R,
+// blockDim.x <= 256: with R = 2 the list (about 1.7 faces per cell) takes the
+// threads once instead of twice.
+template <typename T, int R = 1>
 __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f, const int base, const int nvalid,
                                           const V4<T> *__restrict__ FS, V4<T> *__restrict__ res) {
-    __shared__ V4<T> Fs[256 * 3];
-    __shared__ int4 tps[256];
-    __shared__ unsigned short items[256 * 3];
+    constexpr int CELLS = 256 / R;
+    __shared__ V4<T> Fs[CELLS * 3];
+    __shared__ int4 tps[CELLS];
+    __shared__ unsigned short items[CELLS * 3];
     __shared__ int wtot[8];
     const int t = threadIdx.x, i = base + t;
     const bool live = t < nvalid;
     const int4 tp = live ? m.topo[i] : make_int4(-3, -3, -3, 0);
-    tps[t] = tp;
+    if (live) tps[t] = tp;
     const int code[3] = {tp.x, tp.y, tp.z};
     unsigned mask = 0;
 #pragma unroll
@@ -1098,13 +1186,13 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
     res[i] = r;
 }
 
-template <typename T>
+template <typename T, int R>
 __global__ void E2D_LB_FLUX k_flux_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ FS,
                                         V4<T> *__restrict__ res, const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
-    const int base = blockIdx.x * blockDim.x;
-    flux_tile(m, f, base, min((int)blockDim.x, m.n - base), FS, res);
+    const int tile = blockDim.x / R, base = blockIdx.x * tile;
+    flux_tile<T, R>(m, f, base, min(tile, m.n - base), FS, res);
 }
 
 template <typename T>
@@ -1115,6 +1203,31 @@ __global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restr
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
     flux_cell(m, f, i, FS, res);
+}
+
+// The pass-B kernel of a precision.
+template <typename T> auto flux_kernel(int lanes) {
+    if constexpr (FluxTiled<T>::value) return lanes == 2 ? &k_flux_tile<T, 2> : &k_flux_tile<T, 1>;
+    else return &k_flux<T>;
+}
+
+// Threads per cell of passes A and B.  FP32: one.  FP64: a mesh of up to some
+// 40k cells has one or two warps for each of the GPU's 608 schedulers, and a
+// launch takes as long as one thread's chain of some 2500 instructions, so the
+// cell's work is spread over more threads; on large meshes that only repeats
+// loads and the work per cell, and smaller tiles evaluate more faces twice.
+// us per launch with 1 / 2 / 4 threads in pass A and 1 / 2 in pass B: 2k cells 27 /
+// 20 / 17 and 30 / 21; 8k 31 / 21 / 18 and 33 / 22; 34k (limiter option) 29 / 25 /
+// 29 and 40 / 37; 80k 61 / 54 / 54 and 77 / 79; 131k 72 / 70 / 79 and 100 / 106;
+// 1.05M 436 / 461 / 554 and 615 / 691.  (The positivity option compares a cell's
+// components: one thread.)
+struct Gather {
+    int faces, flux;
+};
+template <typename T> Gather gather_shape(const Plan<T> &p) {
+    if (sizeof(T) == 4) return {1, 1};
+    const int n = p.m.n;
+    return {p.f.positivity || n > 200000 ? 1 : n > 12000 ? 2 : 4, n > 40000 ? 1 : 2};
 }
 
 // Sum of the interior neighbours' values in face order (gpu_solver.cu:1658-1666)
@@ -1304,6 +1417,7 @@ template <typename T, bool OPT>
 __global__ void __launch_bounds__(256, BatchMinBlocks<T>::faces) kb_faces(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W,
                                       V4<T> *__restrict__ FS, T *__restrict__ dt, V4<T> *__restrict__ phi,
                                       const int st) {
+    extern __shared__ __align__(32) unsigned char smem[];
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int base = t * blockDim.x, i = base + threadIdx.x;
@@ -1314,8 +1428,8 @@ __global__ void __launch_bounds__(256, BatchMinBlocks<T>::faces) kb_faces(MeshDe
         const int frozen = OPT && phi ? b.ctl[tc].frozen : 0;
         const bool first = OPT && b.ctl[tc].step < f.first_order;
         if constexpr (sizeof(T) == 8)
-            v = faces_tile<OPT>(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, dt, phi,
-                                frozen, first);
+            v = faces_tile<OPT, 1>(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, dt, phi,
+                                frozen, first, smem);
         else if (i < b.case_end[tc])
             v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, frozen, first);
         if (OPT && f.global_dt) block_min_dt(v, &b.ctl[tc].dtmin[st]);  // uniform over the block
@@ -1384,8 +1498,8 @@ template <typename T> void enqueue_batch_iteration(const BPlan<T> &p, cudaStream
         const bool last = st == p.stages - 1;
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
-        if (p.options) launch_chained(kb_faces<T, true>, G, B, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi, st);
-        else launch_chained(kb_faces<T, false>, G, B, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi, st);
+        launch_chained_smem(p.options ? kb_faces<T, true> : kb_faces<T, false>, G, B,
+                            sizeof(T) == 8 ? B * FacesSmem::per_cell : 0, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi, st);
         launch_chained(kb_flux<T>, G, B, s, p.m, p.b, NT, p.FS, p.res);
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {
@@ -1458,69 +1572,57 @@ void enqueue_export(int n, const int *perm, const V4<T> *W, double *wfile, cudaS
 // update W[1] in place, and the last stage writes the result back into W[0]
 // (each cell reads its own W0 before overwriting it), so W[0] is also the
 // next iteration's W0.
-template <typename T> void enqueue_iteration(const Plan<T> &p, cudaStream_t s) {
+// mark(kind) and done() bracket each launch (kind: 0 faces, 1 flux, 2 smooth,
+// 3 update, 4 resid).
+template <typename T, typename Mark, typename Done>
+void enqueue_passes(const Plan<T> &p, cudaStream_t s, Mark mark, Done done) {
     const int n = p.m.n, B = p.block, G = (n + B - 1) / B;
     const bool opt = faces_options(p.f, p.phi);
-    for (int st = 0; st < p.stages; st++) {
-        const bool last = st == p.stages - 1;
-        V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
-        V4<T> *Wout = last ? p.W[0] : p.W[1];
-        launch_chained(faces_kernel<T>(opt), G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
-        if (FluxTiled<T>::value) launch_chained(k_flux_tile<T>, G, B, s, p.m, p.f, p.FS, p.res, p.ctl);
-        else launch_chained(k_flux<T>, G, B, s, p.m, p.f, p.FS, p.res, p.ctl);
-        const V4<T> *src = p.res;
-        for (int sw = 0; sw + 1 < p.sweeps; sw++) {
-            V4<T> *dst = p.sm[sw & 1];
-            launch_chained(k_smooth<T>, G, B, s, p.m, p.f.irs_eps, src, p.res, dst, p.ctl);
-            src = dst;
-        }
-        if (p.f.global_dt)
-            launch_chained(k_update<T, true>, G, B, s, p.m, p.f, p.rk[st], p.sweeps > 0 ? 1 : 0, src, p.res, p.dt,
-                           p.W[0], Wout, last ? p.part : nullptr, p.ctl, st);
-        else
-            launch_chained(k_update<T, false>, G, B, s, p.m, p.f, p.rk[st], p.sweeps > 0 ? 1 : 0, src, p.res, p.dt,
-                           p.W[0], Wout, last ? p.part : nullptr, p.ctl, st);
-    }
-    enqueue_resid(p.part, G, p.ctl, p.hist, p.hist_cap, sizeof(T) == 4, s);
-}
-
-// Same launches as enqueue_iteration, with events recorded around each one.
-// ev[2*j], ev[2*j+1] bracket launch j; kind[j] is 0 faces, 1 flux, 2 smooth,
-// 3 update, 4 resid.  Returns the number of launches.
-template <typename T>
-int enqueue_iteration_timed(const Plan<T> &p, cudaStream_t s, cudaEvent_t *ev, int *kind) {
-    const int n = p.m.n, B = p.block, G = (n + B - 1) / B;
-    const bool opt = faces_options(p.f, p.phi);
-    int j = 0;
-    auto mark = [&](int k) { kind[j] = k; cudaEventRecord(ev[2 * j], s); };
-    auto done = [&]() { cudaEventRecord(ev[2 * j + 1], s); j++; };
+    const Gather ga = gather_shape(p);
+    const auto grid = [&](int lanes) { return (n + B / lanes - 1) / (B / lanes); };
     for (int st = 0; st < p.stages; st++) {
         const bool last = st == p.stages - 1;
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
         mark(0);
-        faces_kernel<T>(opt)<<<G, B, 0, s>>>(p.m, p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
+        launch_chained_smem(faces_kernel<T>(opt, ga.faces), grid(ga.faces), B,
+                            sizeof(T) == 8 ? B / ga.faces * FacesSmem::per_cell : 0, s, p.m, p.f, Wcur, p.FS, p.dt,
+                            p.ctl, p.phi, st);
         done();
         mark(1);
-        if (FluxTiled<T>::value) k_flux_tile<T><<<G, B, 0, s>>>(p.m, p.f, p.FS, p.res, p.ctl);
-        else k_flux<T><<<G, B, 0, s>>>(p.m, p.f, p.FS, p.res, p.ctl);
+        launch_chained(flux_kernel<T>(ga.flux), grid(ga.flux), B, s, p.m, p.f, p.FS, p.res, p.ctl);
         done();
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {
             V4<T> *dst = p.sm[sw & 1];
-            mark(2); k_smooth<T><<<G, B, 0, s>>>(p.m, p.f.irs_eps, src, p.res, dst, p.ctl); done();
+            mark(2);
+            launch_chained(k_smooth<T>, G, B, s, p.m, p.f.irs_eps, src, p.res, dst, p.ctl);
+            done();
             src = dst;
         }
         mark(3);
-        if (p.f.global_dt)
-            k_update<T, true><<<G, B, 0, s>>>(p.m, p.f, p.rk[st], p.sweeps > 0 ? 1 : 0, src, p.res, p.dt,
-                                              p.W[0], Wout, last ? p.part : nullptr, p.ctl, st);
-        else
-            k_update<T, false><<<G, B, 0, s>>>(p.m, p.f, p.rk[st], p.sweeps > 0 ? 1 : 0, src, p.res, p.dt,
-                                               p.W[0], Wout, last ? p.part : nullptr, p.ctl, st);
+        launch_chained(p.f.global_dt ? k_update<T, true> : k_update<T, false>, G, B, s, p.m, p.f, p.rk[st],
+                       p.sweeps > 0 ? 1 : 0, src, p.res, p.dt, p.W[0], Wout, last ? p.part : nullptr, p.ctl, st);
         done();
     }
-    mark(4); enqueue_resid(p.part, G, p.ctl, p.hist, p.hist_cap, sizeof(T) == 4, s); done();
+    mark(4);
+    enqueue_resid(p.part, G, p.ctl, p.hist, p.hist_cap, sizeof(T) == 4, s);
+    done();
+}
+
+template <typename T> void enqueue_iteration(const Plan<T> &p, cudaStream_t s) {
+    enqueue_passes(p, s, [](int) {}, [] {});
+}
+
+// Same launches as enqueue_iteration, with events recorded around each one.
+// ev[2*j], ev[2*j+1] bracket launch j; kind[j] is its kind.  Returns the
+// number of launches.
+template <typename T>
+int enqueue_iteration_timed(const Plan<T> &p, cudaStream_t s, cudaEvent_t *ev, int *kind) {
+    int j = 0;
+    enqueue_passes(
+        p, s, [&](int k) { kind[j] = k; cudaEventRecord(ev[2 * j], s); },
+        [&] { cudaEventRecord(ev[2 * j + 1], s); j++; });
     return j;
 }
 
