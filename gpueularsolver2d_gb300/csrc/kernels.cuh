@@ -50,7 +50,11 @@ template <> struct MinBlocks<float> {
     static constexpr int faces = E2D_MINB_FACES > 0 ? E2D_MINB_FACES : 1;
     static constexpr int flux = E2D_MINB_FLUX > 0 ? E2D_MINB_FLUX : 1;
 };
-#define E2D_LB_FACES __launch_bounds__(256, MinBlocks<T>::faces)
+// FP32 pass A with the scheme options needs 64 registers not to spill (at 40 it
+// spilled 148 / 416 bytes per thread): an iteration of 131k cells with the
+// cell-wise limiter 63.2 -> 60.5 us, of 24 batched cases of 33k cells with the
+// smooth limiter (48 registers before) 295 -> 281 us.
+constexpr int kOptBlocks = 4;
 // The batched (persistent, tile-walking) FP32 kernels hold a few more live
 // values across their tile loop: one block fewer per SM, so that they do not
 // spill (at the single-case targets ptxas spilled 144 / 60 bytes per thread).
@@ -435,21 +439,9 @@ __device__ __forceinline__ V4<float> roe<float>(const V4<float> &LW, const V4<fl
 // Face midpoint minus cell centroid of face k.  FP64 reads the value the host
 // computed with the reference's formulas (midpoint and centroid averages,
 // gpu_init.cu:100-228), which keeps the FP64 parity bit for bit.  FP32
-// derives it from the face vectors already in registers instead of reading 24
-// bytes per cell: with e_j = (-S_j.y, S_j.x) the edge opposite node j,
-// mid_k - centroid = (e_{k+2} - e_{k+1}) / 6 exactly.
-template <typename T>
-__device__ __forceinline__ V2<T> face_offset(const MeshDev<T> &m, const V2<T> *S, int k, int i) {
-    return m.R[k * m.n + i];
-}
-template <>
-__device__ __forceinline__ V2<float> face_offset<float>(const MeshDev<float> &m, const V2<float> *S, int k, int i) {
-    const V2<float> a = S[(k + 1) % 3], b = S[(k + 2) % 3];
-    V2<float> r;
-    r.x = (a.y - b.y) * (1.0f / 6.0f);
-    r.y = (b.x - a.x) * (1.0f / 6.0f);
-    return r;
-}
+// (offset32) derives it from the face vectors already in registers instead of
+// reading 24 bytes per cell: with e_j = (-S_j.y, S_j.x) the edge opposite node
+// j, mid_k - centroid = (e_{k+2} - e_{k+1}) / 6 exactly.
 
 // Cell area: FP64 reads the host value (Calc_area, gpu_init.cu:95-98); FP32
 // takes half the cross product of two edge vectors, (S_1.x S_2.y - S_1.y S_2.x) / 2
@@ -483,19 +475,194 @@ __device__ __forceinline__ T face_limiter(const int kind, const Flow<T> &f, cons
     return delt2 == T(0) ? T(1.0) : tmin(fdiv(bound - u, delt2), T(1.0));
 }
 
-// Returns the cell's local time step (also stored in dt[i]).  OPT compiles in
-// the scheme options (smooth limiter, frozen limiter values, first-order
-// faces, positivity fallback); without them the reference configuration runs
-// in fewer registers (no spills at the FP32 occupancy target) with the same
-// arithmetic.  first: this iteration uses first-order faces (option).
-// FP32, reference configuration: the arithmetic of faces_cell with the
-// component pairs (rho, rho u) and (rho v, rho E) on the packed FP32 units
-// (two lanes per instruction, each with the scalar operation order, so the
-// bits are those of the scalar form): the gradient sums, the gradients, the
-// reconstruction differences, the limiter quotients and the face states.
-__device__ __forceinline__ float faces_cell_ref32(const MeshDev<float> &m, const Flow<float> &f, const int i,
-                                                  const V4<float> *__restrict__ W, V4<float> *__restrict__ FS,
-                                                  float *__restrict__ dt) {
+// FP32 pass A.  The component pairs (rho, rho u) and (rho v, rho E) run on the
+// packed FP32 units (two lanes per instruction, each with the scalar operation
+// order): the gradient sums, the gradients, the reconstruction differences,
+// the limiter quotients and the face states.
+
+// Gradient and bounds of one cell: what its face states are reconstructed from.
+struct Recon32 {
+    float2 U01, U23, gxa, gxb, gya, gyb;
+    float umax[4], umin[4];
+};
+
+// From the cell's state U, its face vectors S and its neighbours' (or ghost)
+// states nbv; SR: also the sum of the three face spectral radii.
+template <bool SR>
+__device__ __forceinline__ Recon32 reconstruct32(const Flow<float> &f, const V4<float> &U, const V2<float> *S,
+                                                 const V4<float> *nbv, const float A, float &Tsum) {
+    Recon32 c;
+    c.U01 = make_float2(U.x, U.y);
+    c.U23 = make_float2(U.z, U.w);
+    const float2 half = make_float2(0.5f, 0.5f);
+    float2 g0a = make_float2(0.f, 0.f), g0b = g0a, g1a = g0a, g1b = g0a;
+    float jmax[4], jmin[4];
+    Tsum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float v = comp(nbv[k], q);
+            if (k == 0) { jmax[q] = v; jmin[q] = v; }
+            else {
+                if (v < jmin[q]) jmin[q] = v;
+                if (v > jmax[q]) jmax[q] = v;
+            }
+        }
+        const float2 ha = __fmul2_rn(half, __fadd2_rn(c.U01, make_float2(nbv[k].x, nbv[k].y)));
+        const float2 hb = __fmul2_rn(half, __fadd2_rn(c.U23, make_float2(nbv[k].z, nbv[k].w)));
+        const float2 sx = make_float2(S[k].x, S[k].x), sy = make_float2(S[k].y, S[k].y);
+        g0a = __ffma2_rn(ha, sx, g0a);
+        g0b = __ffma2_rn(hb, sx, g0b);
+        g1a = __ffma2_rn(ha, sy, g1a);
+        g1b = __ffma2_rn(hb, sy, g1b);
+        if (SR) Tsum += spectral_radius(U, nbv[k], S[k].y, S[k].x, f.gamma);
+    }
+    const float rA = fdiv(1.0f, A);
+    const float2 rA2 = make_float2(rA, rA);
+    c.gxa = __fmul2_rn(g0a, rA2);
+    c.gxb = __fmul2_rn(g0b, rA2);
+    c.gya = __fmul2_rn(g1a, rA2);
+    c.gyb = __fmul2_rn(g1b, rA2);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        c.umax[q] = tmax(comp(U, q), jmax[q]);
+        c.umin[q] = tmin(comp(U, q), jmin[q]);
+    }
+    return c;
+}
+
+// How a cell limits its face states under the scheme options.
+struct Limit32 {
+    bool reuse;     // frozen values from phi
+    bool cellwise;  // one value per cell and component (options 2, 3)
+    float A;
+    float phic[4];
+};
+
+// State on the cell's side of the face with midpoint offset r: the limited
+// reconstruction.  ph: the limiter values (in: the frozen ones when reused).
+template <bool OPT>
+__device__ __forceinline__ V4<float> face_state32(const Recon32 &c, const Flow<float> &f, const Limit32 &lim,
+                                                  const V2<float> r, V4<float> &ph) {
+    const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y);
+    const float2 da = __ffma2_rn(c.gxa, rx, __fmul2_rn(c.gya, ry));  // delt2 of components 0, 1
+    const float2 db = __ffma2_rn(c.gxb, rx, __fmul2_rn(c.gyb, ry));  // and 2, 3
+    float2 fa, fb;
+    if (OPT && lim.reuse) {
+        fa = make_float2(ph.x, ph.y);
+        fb = make_float2(ph.z, ph.w);
+    } else if (OPT && lim.cellwise) {
+        fa = make_float2(lim.phic[0], lim.phic[1]);
+        fb = make_float2(lim.phic[2], lim.phic[3]);
+    } else if (OPT && f.limiter == 1) {
+        fa = make_float2(face_limiter(1, f, lim.A, c.umax[0], c.umin[0], c.U01.x, da.x),
+                         face_limiter(1, f, lim.A, c.umax[1], c.umin[1], c.U01.y, da.y));
+        fb = make_float2(face_limiter(1, f, lim.A, c.umax[2], c.umin[2], c.U23.x, db.x),
+                         face_limiter(1, f, lim.A, c.umax[3], c.umin[3], c.U23.y, db.y));
+    } else {
+        // limiter (kind 0): min(1, (bound - u) / delt2), bound - u as
+        // u * (-1) + bound (one rounding, the same bits)
+        const float2 mone = make_float2(-1.0f, -1.0f);
+        const float2 na = __ffma2_rn(c.U01, mone, make_float2(da.x > 0.f ? c.umax[0] : c.umin[0],
+                                                              da.y > 0.f ? c.umax[1] : c.umin[1]));
+        const float2 nb = __ffma2_rn(c.U23, mone, make_float2(db.x > 0.f ? c.umax[2] : c.umin[2],
+                                                              db.y > 0.f ? c.umax[3] : c.umin[3]));
+        const float2 qa = __fmul2_rn(na, make_float2(frcp(da.x), frcp(da.y)));
+        const float2 qb = __fmul2_rn(nb, make_float2(frcp(db.x), frcp(db.y)));
+        fa = make_float2(da.x == 0.f ? 1.0f : tmin(qa.x, 1.0f), da.y == 0.f ? 1.0f : tmin(qa.y, 1.0f));
+        fb = make_float2(db.x == 0.f ? 1.0f : tmin(qb.x, 1.0f), db.y == 0.f ? 1.0f : tmin(qb.y, 1.0f));
+    }
+    const float2 wa = __ffma2_rn(da, fa, c.U01), wb = __ffma2_rn(db, fb, c.U23);
+    V4<float> o;
+    o.x = wa.x; o.y = wa.y; o.z = wb.x; o.w = wb.y;
+    ph.x = fa.x; ph.y = fa.y; ph.z = fb.x; ph.w = fb.y;
+    if (OPT && f.positivity) {
+        // positivity fallback (option): a face side with a density or
+        // pressure that is not positive takes the cell state
+        const float q = 0.5f * (o.y * o.y + o.z * o.z) / o.x;
+        if (!(o.x > 0.f) || !((f.gamma - 1.0f) * (o.w - q) > 0.f)) {
+            o.x = c.U01.x; o.y = c.U01.y; o.z = c.U23.x; o.w = c.U23.y;
+        }
+    }
+    return o;
+}
+
+// Face offsets of a cell from its face vectors (face_offset, FP32).
+__device__ __forceinline__ V2<float> offset32(const V2<float> a, const V2<float> b) {
+    V2<float> r;
+    r.x = (a.y - b.y) * (1.0f / 6.0f);
+    r.y = (b.x - a.x) * (1.0f / 6.0f);
+    return r;
+}
+
+// The limiter settings of a cell; the cell-wise options (2, 3) take the
+// smallest of the per-face values (reference form, Venkatakrishnan form) of
+// the cell's interior faces.
+template <bool OPT>
+__device__ __forceinline__ Limit32 limits32(const Recon32 &c, const Flow<float> &f, const int *code,
+                                            const V2<float> *S, const float A, const bool reuse, const bool first) {
+    Limit32 lim;
+    lim.reuse = reuse;
+    lim.cellwise = OPT && f.limiter >= 2;
+    lim.A = A;
+    if (lim.cellwise && !reuse && !first) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) lim.phic[q] = INFINITY;
+        const float2 u[2] = {c.U01, c.U23};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (code[k] < 0) continue;
+            const V2<float> r = offset32(S[(k + 1) % 3], S[(k + 2) % 3]);
+            const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y);
+            const float2 d[2] = {__ffma2_rn(c.gxa, rx, __fmul2_rn(c.gya, ry)),
+                                 __ffma2_rn(c.gxb, rx, __fmul2_rn(c.gyb, ry))};
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                lim.phic[q] = tmin(lim.phic[q],
+                                   face_limiter(f.limiter - 2, f, A, c.umax[q], c.umin[q],
+                                                q & 1 ? u[q >> 1].y : u[q >> 1].x, q & 1 ? d[q >> 1].y : d[q >> 1].x));
+        }
+    }
+    return lim;
+}
+
+// Pass A of one cell from its neighbours' (or ghost) states: its three face
+// states go to out(k, state), its local time step is returned.  OPT compiles in
+// the scheme options (smooth limiter, frozen limiter values, first-order faces,
+// positivity fallback); without them the reference configuration runs in fewer
+// registers.  first: this iteration uses first-order faces.
+template <bool OPT, typename Out>
+__device__ __forceinline__ float faces_cell32(const MeshDev<float> &m, const Flow<float> &f, const int i,
+                                              const int *code, const V2<float> *S, const V4<float> &U,
+                                              const V4<float> *nbv, V4<float> *__restrict__ phi, const int frozen,
+                                              const bool first, Out out) {
+    const int n = m.n;
+    const float A = cell_area(m, S, i);
+    float Tsum;
+    const Recon32 c = reconstruct32<true>(f, U, S, nbv, A, Tsum);
+    const bool reuse = OPT && phi && frozen;
+    const Limit32 lim = limits32<OPT>(c, f, code, S, A, reuse, first);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        V4<float> o = U;
+        if (code[k] >= 0 && !(OPT && first)) {
+            V4<float> ph;
+            if (reuse) ph = phi[k * n + i];
+            o = face_state32<OPT>(c, f, lim, offset32(S[(k + 1) % 3], S[(k + 2) % 3]), ph);
+            if (OPT && phi && !frozen) phi[k * n + i] = ph;
+        }
+        out(k, o);
+    }
+    return tmin(fdiv(A * f.cfl, Tsum), f.dt_cap);
+}
+
+// The same from global memory; the face states go to FS, the step to dt[i].
+template <bool OPT>
+__device__ __forceinline__ float faces_cell(const MeshDev<float> &m, const Flow<float> &f, const int i,
+                                            const V4<float> *__restrict__ W, V4<float> *__restrict__ FS,
+                                            float *__restrict__ dt, V4<float> *__restrict__ phi, const int frozen,
+                                            const bool first) {
     const int n = m.n;
     const int4 tp = m.topo[i];
     const int code[3] = {tp.x, tp.y, tp.z};
@@ -507,171 +674,8 @@ __device__ __forceinline__ float faces_cell_ref32(const MeshDev<float> &m, const
 #pragma unroll
     for (int k = 0; k < 3; k++)
         nbv[k] = code[k] >= 0 ? W[code[k] >> 3] : ghost(code[k], U, S[k].x, S[k].y, f);
-    const float2 U01 = make_float2(U.x, U.y), U23 = make_float2(U.z, U.w), half = make_float2(0.5f, 0.5f);
-    float2 g0a = make_float2(0.f, 0.f), g0b = g0a, g1a = g0a, g1b = g0a;
-    float jmax[4], jmin[4];
-    float Tsum = 0.f;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float c = comp(nbv[k], q);
-            if (k == 0) { jmax[q] = c; jmin[q] = c; }
-            else {
-                if (c < jmin[q]) jmin[q] = c;
-                if (c > jmax[q]) jmax[q] = c;
-            }
-        }
-        const float2 ha = __fmul2_rn(half, __fadd2_rn(U01, make_float2(nbv[k].x, nbv[k].y)));
-        const float2 hb = __fmul2_rn(half, __fadd2_rn(U23, make_float2(nbv[k].z, nbv[k].w)));
-        const float2 sx = make_float2(S[k].x, S[k].x), sy = make_float2(S[k].y, S[k].y);
-        g0a = __ffma2_rn(ha, sx, g0a);
-        g0b = __ffma2_rn(hb, sx, g0b);
-        g1a = __ffma2_rn(ha, sy, g1a);
-        g1b = __ffma2_rn(hb, sy, g1b);
-        Tsum += spectral_radius(U, nbv[k], S[k].y, S[k].x, f.gamma);
-    }
-    const float A = cell_area(m, S, i);
-    const float rA = fdiv(1.0f, A);
-    const float2 rA2 = make_float2(rA, rA);
-    const float2 gxa = __fmul2_rn(g0a, rA2), gxb = __fmul2_rn(g0b, rA2);
-    const float2 gya = __fmul2_rn(g1a, rA2), gyb = __fmul2_rn(g1b, rA2);
-    float umax[4], umin[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        umax[q] = tmax(comp(U, q), jmax[q]);
-        umin[q] = tmin(comp(U, q), jmin[q]);
-    }
-    const float2 mone = make_float2(-1.0f, -1.0f);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        V4<float> o = U;
-        if (code[k] >= 0) {
-            const V2<float> r = face_offset(m, S, k, i);
-            const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y);
-            const float2 da = __ffma2_rn(gxa, rx, __fmul2_rn(gya, ry));  // delt2 of components 0, 1
-            const float2 db = __ffma2_rn(gxb, rx, __fmul2_rn(gyb, ry));  // and 2, 3
-            // limiter (kind 0): min(1, (bound - u) / delt2), bound - u as
-            // u * (-1) + bound (one rounding, the same bits)
-            const float2 na = __ffma2_rn(U01, mone, make_float2(da.x > 0.f ? umax[0] : umin[0],
-                                                                  da.y > 0.f ? umax[1] : umin[1]));
-            const float2 nb = __ffma2_rn(U23, mone, make_float2(db.x > 0.f ? umax[2] : umin[2],
-                                                                  db.y > 0.f ? umax[3] : umin[3]));
-            const float2 qa = __fmul2_rn(na, make_float2(frcp(da.x), frcp(da.y)));
-            const float2 qb = __fmul2_rn(nb, make_float2(frcp(db.x), frcp(db.y)));
-            const float2 fa = make_float2(da.x == 0.f ? 1.0f : tmin(qa.x, 1.0f), da.y == 0.f ? 1.0f : tmin(qa.y, 1.0f));
-            const float2 fb = make_float2(db.x == 0.f ? 1.0f : tmin(qb.x, 1.0f), db.y == 0.f ? 1.0f : tmin(qb.y, 1.0f));
-            const float2 wa = __ffma2_rn(da, fa, U01), wb = __ffma2_rn(db, fb, U23);
-            o.x = wa.x; o.y = wa.y; o.z = wb.x; o.w = wb.y;
-        }
-        FS[k * n + i] = o;
-    }
-    const float dti = tmin(fdiv(A * f.cfl, Tsum), f.dt_cap);
-    dt[i] = dti;
-    return dti;
-}
-
-template <typename T, bool OPT>
-__device__ __forceinline__ T faces_cell(const MeshDev<T> &m, const Flow<T> &f, const int i,
-                                        const V4<T> *__restrict__ W, V4<T> *__restrict__ FS,
-                                        T *__restrict__ dt, V4<T> *__restrict__ phi, const int frozen,
-                                        const bool first = false) {
-    static_assert(sizeof(T) == 4, "FP64 runs faces_tile");
-    if constexpr (!OPT) return faces_cell_ref32(m, f, i, W, FS, dt);
-    const int n = m.n;
-    const int4 tp = m.topo[i];
-    const int code[3] = {tp.x, tp.y, tp.z};
-    const V4<T> U = W[i];
-    V2<T> S[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) S[k] = m.S[k * n + i];
-    V4<T> nbv[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-        nbv[k] = code[k] >= 0 ? W[code[k] >> 3] : ghost(code[k], U, S[k].x, S[k].y, f);
-    T g0[4] = {T(0.0), T(0.0), T(0.0), T(0.0)}, g1[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
-    T jmax[4], jmin[4];
-    T Tsum = T(0);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            T c = comp(nbv[k], q);
-            if (k == 0) { jmax[q] = c; jmin[q] = c; }
-            else {
-                if (c < jmin[q]) jmin[q] = c;
-                if (c > jmax[q]) jmax[q] = c;
-            }
-            T u = comp(U, q);
-            g0[q] = madd(T(0.5) * (u + c), S[k].x, g0[q]);
-            g1[q] = madd(T(0.5) * (u + c), S[k].y, g1[q]);
-        }
-        Tsum += spectral_radius(U, nbv[k], S[k].y, S[k].x, f.gamma);
-    }
-    const T A = cell_area(m, S, i);
-    const T rA = fdiv(T(1.0), A);
-    T gx[4], gy[4], umax[4], umin[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        gx[q] = g0[q] * rA;
-        gy[q] = g1[q] * rA;
-        umax[q] = tmax(comp(U, q), jmax[q]);
-        umin[q] = tmin(comp(U, q), jmin[q]);
-    }
-    const bool reuse = OPT && phi && frozen;
-    // cell-wise limiter options (2, 3): the smallest of the per-face values of
-    // the cell's interior faces (reference form, Venkatakrishnan form), the
-    // same value on every face of the cell
-    const bool cellwise = OPT && f.limiter >= 2;
-    T phic[4] = {T(1.0), T(1.0), T(1.0), T(1.0)};
-    if (cellwise && !reuse && !first) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) phic[q] = T(INFINITY);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (code[k] < 0) continue;
-            const V2<T> r = face_offset(m, S, k, i);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const T delt2 = madd(gx[q], r.x, gy[q] * r.y);
-                phic[q] = tmin(phic[q], face_limiter(f.limiter - 2, f, A, umax[q], umin[q], comp(U, q), delt2));
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        V4<T> o = U;
-        if (code[k] >= 0 && !(OPT && first)) {
-            const V2<T> r = face_offset(m, S, k, i);
-            V4<T> pf;
-            if (reuse) pf = phi[k * n + i];
-            T fi = T(1.0), d[4], ph[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                T delt2 = madd(gx[q], r.x, gy[q] * r.y);
-                T u = comp(U, q);
-                if (reuse) fi = comp(pf, q);
-                else if (cellwise) fi = phic[q];
-                else fi = face_limiter(OPT ? f.limiter : 0, f, A, umax[q], umin[q], u, delt2);
-                ph[q] = fi;
-                d[q] = madd(delt2, fi, u);
-            }
-            o.x = d[0]; o.y = d[1]; o.z = d[2]; o.w = d[3];
-            if (OPT && f.positivity) {
-                // positivity fallback (option): a face side with a density or
-                // pressure that is not positive takes the cell state
-                const T q = gdiv(T(0.5) * (d[1] * d[1] + d[2] * d[2]), d[0]);
-                if (!(d[0] > T(0)) || !((f.gamma - T(1.0)) * (d[3] - q) > T(0))) o = U;
-            }
-            if (OPT && phi && !frozen) {
-                V4<T> pw;
-                pw.x = ph[0]; pw.y = ph[1]; pw.z = ph[2]; pw.w = ph[3];
-                phi[k * n + i] = pw;
-            }
-        }
-        FS[k * n + i] = o;
-    }
-    const T dti = tmin(fdiv(A * f.cfl, Tsum), f.dt_cap);
+    const float dti = faces_cell32<OPT>(m, f, i, code, S, U, nbv, phi, frozen, first,
+                                        [&](int k, const V4<float> &o) { FS[k * n + i] = o; });
     dt[i] = dti;
     return dti;
 }
@@ -761,7 +765,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
     }
     const int kind = OPT ? f.limiter & 1 : 0;
     const double e2 = OPT && kind == 1 && !reuse ? f.venk_k3 * A * dsqrt(A) : 0.0;
-    // cell-wise limiter options (2, 3): see faces_cell
+    // cell-wise limiter options (2, 3): see limits32
     const bool cellwise = OPT && f.limiter >= 2;
     double phic[NQ];
     if (cellwise && !reuse && !first) {
@@ -792,7 +796,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
             }
             if constexpr (OPT && LPC == 1)
                 if (f.positivity) {
-                    // positivity fallback (option): see faces_cell
+                    // positivity fallback (option): see face_state32
                     const double q = ddiv(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
                     if (!(d[0] > 0.0) || !((f.gamma - 1.0) * (d[3] - q) > 0.0))
                         for (int c = 0; c < 4; c++) d[c] = u[c];
@@ -954,7 +958,7 @@ __global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<d
 // FP32.  OPT: the variant with the scheme options (smooth limiter, limiter
 // freezing, global time step); faces_options picks it.
 template <typename T, bool OPT>
-__global__ void E2D_LB_FACES k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
+__global__ void __launch_bounds__(256, OPT ? kOptBlocks : MinBlocks<T>::faces) k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
                                      V4<T> *__restrict__ FS, T *__restrict__ dt,
                                      Ctl *__restrict__ ctl, V4<T> *__restrict__ phi, const int st) {
     wait_prior_grid();
@@ -963,11 +967,11 @@ __global__ void E2D_LB_FACES k_faces(MeshDev<T> m, Flow<T> f, const V4<T> *__res
     const bool first = OPT && ctl->step < f.first_order;
     if (!OPT || !f.global_dt) {
         if (i >= m.n) return;
-        faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, OPT && phi ? ctl->frozen : 0, first);
+        faces_cell<OPT>(m, f, i, W, FS, dt, phi, OPT && phi ? ctl->frozen : 0, first);
         return;
     }
     double v = __longlong_as_double((long long)kDtNone);
-    if (i < m.n) v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, phi ? ctl->frozen : 0, first);
+    if (i < m.n) v = (double)faces_cell<OPT>(m, f, i, W, FS, dt, phi, phi ? ctl->frozen : 0, first);
     block_min_dt(v, &ctl->dtmin[st]);
 }
 
@@ -999,6 +1003,21 @@ __device__ __forceinline__ T stage_dt(const Flow<T> &f, const Ctl *ctl, const in
 // three faces, summed as gpu_solver.cu:798-825 (+F where the cell is the
 // edge's left cell, -F where it is the right cell, in face order).
 template <typename T>
+__device__ __forceinline__ void add_flux(V4<T> &r, const V4<T> &F, const bool right) {
+    if constexpr (sizeof(T) == 4) {
+        // r +- F as r + (+-1) F: the product is exact, one rounding, the
+        // same bits as the add or subtract; two packed instructions
+        const float sg = right ? -1.0f : 1.0f;
+        const float2 xy = __ffma2_rn(make_float2(F.x, F.y), make_float2(sg, sg), make_float2(r.x, r.y));
+        const float2 zw = __ffma2_rn(make_float2(F.z, F.w), make_float2(sg, sg), make_float2(r.z, r.w));
+        r.x = xy.x; r.y = xy.y; r.z = zw.x; r.w = zw.y;
+    } else {
+        if (right) { r.x -= F.x; r.y -= F.y; r.z -= F.z; r.w -= F.w; }
+        else { r.x += F.x; r.y += F.y; r.z += F.z; r.w += F.w; }
+    }
+}
+
+template <typename T>
 __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f, const int i,
                                           const V4<T> *__restrict__ FS, V4<T> *__restrict__ res) {
     const int n = m.n;
@@ -1019,17 +1038,7 @@ __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f,
     for (int k = 0; k < 3; k++) {
         bool right;
         const V4<T> F = face_flux_of(f, code[k], S[k], own[k], oth[k], right);
-        if constexpr (sizeof(T) == 4) {
-            // r +- F as r + (+-1) F: the product is exact, one rounding, the
-            // same bits as the add or subtract; two packed instructions
-            const float sg = right ? -1.0f : 1.0f;
-            const float2 xy = __ffma2_rn(make_float2(F.x, F.y), make_float2(sg, sg), make_float2(r.x, r.y));
-            const float2 zw = __ffma2_rn(make_float2(F.z, F.w), make_float2(sg, sg), make_float2(r.z, r.w));
-            r.x = xy.x; r.y = xy.y; r.z = zw.x; r.w = zw.y;
-        } else {
-            if (right) { r.x -= F.x; r.y -= F.y; r.z -= F.z; r.w -= F.w; }
-            else { r.x += F.x; r.y += F.y; r.z += F.z; r.w += F.w; }
-        }
+        add_flux(r, F, right);
     }
     res[i] = r;
 }
@@ -1250,19 +1259,22 @@ __device__ __forceinline__ V4<T> nb_sum(const int4 tp, const V4<T> *__restrict__
 // Pass C: gpu_solver.cu:1635-1673 (kernel_Smooth1): one Jacobi-type sweep
 // dst = (eps * sum_interior src + res) / (1 + eps * CLog).
 template <typename T>
-__device__ __forceinline__ void smooth_cell(const MeshDev<T> &m, const T eps, const int i,
-                                            const V4<T> *__restrict__ src, const V4<T> *__restrict__ res,
-                                            V4<T> *__restrict__ dst) {
-    const int4 tp = m.topo[i];
-    const V4<T> d = nb_sum(tp, src);
-    const V4<T> r0 = res[i];
-    const Over<T> den(T(1.0) + (eps) * T(tp.w));
+__device__ __forceinline__ V4<T> smooth_value(const T eps, const int clog, const V4<T> &d, const V4<T> &r0) {
+    const Over<T> den(T(1.0) + (eps) * T(clog));
     V4<T> o;
     o.x = den(madd(d.x, eps, r0.x));
     o.y = den(madd(d.y, eps, r0.y));
     o.z = den(madd(d.z, eps, r0.z));
     o.w = den(madd(d.w, eps, r0.w));
-    dst[i] = o;
+    return o;
+}
+
+template <typename T>
+__device__ __forceinline__ void smooth_cell(const MeshDev<T> &m, const T eps, const int i,
+                                            const V4<T> *__restrict__ src, const V4<T> *__restrict__ res,
+                                            V4<T> *__restrict__ dst) {
+    const int4 tp = m.topo[i];
+    dst[i] = smooth_value(eps, tp.w, nb_sum(tp, src), res[i]);
 }
 
 template <typename T>
@@ -1280,44 +1292,51 @@ __global__ void __launch_bounds__(256) k_smooth(MeshDev<T> m, T eps, const V4<T>
 // Pass D: gpu_solver.cu:1675-1720 (kernel_Smooth2, last sweep + clamp) fused
 // with 938-966 (kernel_RKStep); on the last stage also 968-1020 (kernel_drou)
 // as FP64 block partials and a count of unphysical cells.
+// The new state from the start state w0, the residual r and (smooth) the sum d of
+// the neighbours' smoothed residuals; want: also rho - rho0 and whether the state
+// is unphysical.
+template <typename T>
+__device__ __forceinline__ V4<T> update_value(const Flow<T> &f, const T rk, const int smooth, const int clog, V4<T> r,
+                                              const V4<T> &d, const T dti, const T area, const V4<T> &w0,
+                                              const bool want, T &drho, int &bad) {
+    if (smooth) {
+        const T eps = f.irs_eps;
+        const Over<T> den(T(1.0) + (eps) * T(clog));
+        T s0 = den(madd(d.x, eps, r.x)), s1 = den(madd(d.y, eps, r.y));
+        T s2 = den(madd(d.z, eps, r.z)), s3 = den(madd(d.w, eps, r.w));
+        if (abs_less(s0, r.x)) r.x = s0;
+        if (abs_less(s1, r.y)) r.y = s1;
+        if (abs_less(s2, r.z)) r.z = s2;
+        if (abs_less(s3, r.w)) r.w = s3;
+    }
+    T RK = rk;
+    RK *= dti;
+    const Over<T> A(area);
+    V4<T> w;
+    w.x = w0.x - A(RK * r.x);
+    w.y = w0.y - A(RK * r.y);
+    w.z = w0.z - A(RK * r.z);
+    w.w = w0.w - A(RK * r.w);
+    if (want) {
+        // rho - rho0 in the stencil's precision: exact in FP32 as long as the
+        // two densities are within a factor of two (Sterbenz)
+        drho = w.x - w0.x;
+        const T q = gdiv(T(0.5) * (w.y * w.y + w.z * w.z), w.x);
+        bad = !(w.x > T(0)) || !(w.w - q > T(0));
+    }
+    return w;
+}
+
 template <typename T>
 __device__ __forceinline__ void update_cell(const MeshDev<T> &m, const Flow<T> &f, const T rk,
                                             const int smooth, const int i, const V4<T> *__restrict__ src,
                                             const V4<T> *__restrict__ res, const T dti,
                                             const V4<T> *W0, V4<T> *Wout, const bool want, T &drho,
                                             int &bad) {
-    {
-        const int4 tp = m.topo[i];
-        V4<T> r = res[i];
-        if (smooth) {
-            const V4<T> d = nb_sum(tp, src);
-            const T eps = f.irs_eps;
-            const Over<T> den(T(1.0) + (eps) * T(tp.w));
-            T s0 = den(madd(d.x, eps, r.x)), s1 = den(madd(d.y, eps, r.y));
-            T s2 = den(madd(d.z, eps, r.z)), s3 = den(madd(d.w, eps, r.w));
-            if (abs_less(s0, r.x)) r.x = s0;
-            if (abs_less(s1, r.y)) r.y = s1;
-            if (abs_less(s2, r.z)) r.z = s2;
-            if (abs_less(s3, r.w)) r.w = s3;
-        }
-        T RK = rk;
-        RK *= dti;
-        const Over<T> A(m.area[i]);
-        const V4<T> w0 = W0[i];
-        V4<T> w;
-        w.x = w0.x - A(RK * r.x);
-        w.y = w0.y - A(RK * r.y);
-        w.z = w0.z - A(RK * r.z);
-        w.w = w0.w - A(RK * r.w);
-        Wout[i] = w;
-        if (want) {
-            // rho - rho0 in the stencil's precision: exact in FP32 as long as the
-            // two densities are within a factor of two (Sterbenz)
-            drho = w.x - w0.x;
-            const T q = gdiv(T(0.5) * (w.y * w.y + w.z * w.z), w.x);
-            bad = !(w.x > T(0)) || !(w.w - q > T(0));
-        }
-    }
+    const int4 tp = m.topo[i];
+    V4<T> d = {};
+    if (smooth) d = nb_sum(tp, src);
+    Wout[i] = update_value(f, rk, smooth, tp.w, res[i], d, dti, m.area[i], W0[i], want, drho, bad);
 }
 
 // Deterministic block sum of (rho - rho0)^2 (fixed shuffle tree, then the
@@ -1361,7 +1380,8 @@ __device__ __forceinline__ void pair_add(float &ah, float &al, const float bh, c
     al = t - (ah - s);
 }
 
-__device__ __forceinline__ void block_partial(float drho, int bad, double *slot, int *nbad) {
+// The warp's sum of drho^2 as a pair, in lane 0.
+__device__ __forceinline__ float2 warp_squares(const float drho) {
     float hi = drho * drho;
     float lo = fmaf(drho, drho, -hi);
 #pragma unroll
@@ -1369,12 +1389,17 @@ __device__ __forceinline__ void block_partial(float drho, int bad, double *slot,
         const float bh = __shfl_down_sync(0xffffffffu, hi, o), bl = __shfl_down_sync(0xffffffffu, lo, o);
         pair_add(hi, lo, bh, bl);
     }
+    return make_float2(hi, lo);
+}
+
+__device__ __forceinline__ void block_partial(float drho, int bad, double *slot, int *nbad) {
+    const float2 sq = warp_squares(drho);
     unsigned badmask = __ballot_sync(0xffffffffu, bad);
     __shared__ float2 wsf[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __syncthreads();  // wsf may still be read by the previous use in this block
     if (lane == 0) {
-        wsf[wid] = make_float2(hi, lo);
+        wsf[wid] = sq;
         if (badmask) atomicAdd(nbad, __popc(badmask));
     }
     __syncthreads();
@@ -1414,7 +1439,7 @@ __global__ void __launch_bounds__(256) k_update(MeshDev<T> m, Flow<T> f, T rk, i
 // (converged) cases and padding cells are skipped.
 
 template <typename T, bool OPT>
-__global__ void __launch_bounds__(256, BatchMinBlocks<T>::faces) kb_faces(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W,
+__global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : BatchMinBlocks<T>::faces) kb_faces(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W,
                                       V4<T> *__restrict__ FS, T *__restrict__ dt, V4<T> *__restrict__ phi,
                                       const int st) {
     extern __shared__ __align__(32) unsigned char smem[];
@@ -1431,7 +1456,7 @@ __global__ void __launch_bounds__(256, BatchMinBlocks<T>::faces) kb_faces(MeshDe
             v = faces_tile<OPT, 1>(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, dt, phi,
                                 frozen, first, smem);
         else if (i < b.case_end[tc])
-            v = (double)faces_cell<T, OPT>(m, f, i, W, FS, dt, phi, frozen, first);
+            v = (double)faces_cell<OPT>(m, f, i, W, FS, dt, phi, frozen, first);
         if (OPT && f.global_dt) block_min_dt(v, &b.ctl[tc].dtmin[st]);  // uniform over the block
     }
 }
