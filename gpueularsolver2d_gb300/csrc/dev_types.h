@@ -129,6 +129,11 @@ void enqueue_batch_resid(double *part, const int2 *case_tiles, int ncase, Ctl *c
 // Instantiated for double in kernels_f64.cu and for float in kernels_f32.cu.
 template <typename T> void enqueue_iteration(const Plan<T> &p, cudaStream_t s);
 
+// Up to `iters` iterations of a small FP32 mesh in one launch (small32.cuh); it
+// stops by itself like the passes do.  False when it does not apply to the plan
+// (probe: asked once, nothing is launched) or the launch failed.
+bool small_iterations(const Plan<float> &p, int iters, cudaStream_t s, bool probe);
+
 // Same, with an event pair around every launch (per-pass timing).
 template <typename T> int enqueue_iteration_timed(const Plan<T> &p, cudaStream_t s, cudaEvent_t *ev, int *kind);
 

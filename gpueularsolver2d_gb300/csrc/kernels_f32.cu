@@ -7,6 +7,7 @@
 // explicitly with fmaf.  Division and square root are the fast (non-IEEE)
 // forms, denormals flush to zero.
 #include "kernels.cuh"
+#include "small32.cuh"
 
 namespace e2d {
 template void enqueue_iteration<float>(const Plan<float> &p, cudaStream_t s);

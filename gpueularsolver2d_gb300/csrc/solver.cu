@@ -218,6 +218,8 @@ struct SolverBase {
     virtual int download_walls(double *w_wall) = 0;
     virtual int enqueue(cudaStream_t s) = 0;
     virtual int launches() const = 0;
+    virtual bool small() const = 0;  // iterations run in one launch (small32.cuh)
+    virtual int run_small(cudaStream_t s, int iters) = 0;
     virtual int nblocks() const = 0;
     virtual int enqueue_timed(cudaStream_t s, cudaEvent_t *ev, int *kind) = 0;
     virtual const void *topo_ptr() const = 0;
@@ -232,6 +234,7 @@ template <typename T> struct SolverT : SolverBase {
     int *wall_dev = nullptr;       // [wall faces] internal cell of each
     double *wwall_dev = nullptr;   // [4 wall faces] their states
     cudaStream_t *stream = nullptr;
+    bool small_ = false;
 
     explicit SolverT(HostLayout *l) : L(l) {}
 
@@ -290,6 +293,7 @@ template <typename T> struct SolverT : SolverBase {
         for (int k = 0; k < 8; k++) plan.rk[k] = (T)p.rk_coef[k];
         plan.sweeps = p.irs_sweeps;
         plan.block = block;
+        if constexpr (sizeof(T) == 4) small_ = small_iterations(plan, 0, nullptr, true);
         return E2D_OK;
     }
 
@@ -335,7 +339,16 @@ template <typename T> struct SolverT : SolverBase {
         return E2D_OK;
     }
 
-    int launches() const override { return launches_per_iteration(plan); }
+    bool small() const override { return small_; }
+    int run_small(cudaStream_t s, int iters) override {
+        if constexpr (sizeof(T) == 4)
+            if (small_iterations(plan, iters, s, false)) return E2D_OK;
+        CK(cudaGetLastError());
+        set_error("the small-mesh kernel could not be launched");
+        return E2D_ERR_CUDA;
+    }
+
+    int launches() const override { return small_ ? 1 : launches_per_iteration(plan); }
     const void *topo_ptr() const override { return plan.m.topo; }
     int nblocks() const override { return (L->n + plan.block - 1) / plan.block; }
 };
@@ -434,10 +447,14 @@ int capture(e2d_solver *s, int iters, cudaGraphExec_t *out) {
     return E2D_OK;
 }
 
-int build_graph(e2d_solver *s) {
-    if (s->gexec && s->gexec1) return E2D_OK;
+void bind_hist(e2d_solver *s) {
     if (s->prm.precision == E2D_FP64) set_hist<double>(s->impl.get(), s->hist_dev, s->hist_cap);
     else set_hist<float>(s->impl.get(), s->hist_dev, s->hist_cap);
+}
+
+int build_graph(e2d_solver *s) {
+    if (s->gexec && s->gexec1) return E2D_OK;
+    bind_hist(s);
     drop_graphs(s);
     int rc = capture(s, s->graph_iters, &s->gexec);
     if (rc == E2D_OK) rc = capture(s, 1, &s->gexec1);
@@ -476,12 +493,17 @@ int sync_hist(e2d_solver *s) {
     return E2D_OK;
 }
 
+// Iterations of one small-mesh launch (a few milliseconds at most).
+constexpr int kSmallIters = 256;
+
 // Runs up to n iterations (fewer if the residual test stops the loop).
 int run(e2d_solver *s, int n, bool check, double epsl, int poll_every) {
     if (n <= 0) return E2D_OK;
     int rc = ensure_hist(s, s->ctl_host->step + n);
     if (rc) return rc;
-    if ((rc = build_graph(s))) return rc;
+    const bool small = s->impl->small();
+    if (small) bind_hist(s);
+    else if ((rc = build_graph(s))) return rc;
     Ctl &c = *s->ctl_host;
     c.halt = 0;
     c.nbad = 0;
@@ -489,10 +511,18 @@ int run(e2d_solver *s, int n, bool check, double epsl, int poll_every) {
     c.check_epsl = check ? 1 : 0;
     c.epsl = epsl;
     if ((rc = push_ctl(s))) return rc;
-    // whole graphs of graph_iters iterations, then single-iteration graphs for
-    // the remainder (no launches of iterations that would only find the halt flag)
-    const int full = n / s->graph_iters, rem = n % s->graph_iters;
+    // small meshes: launches of up to kSmallIters iterations.  Otherwise whole
+    // graphs of graph_iters iterations, then single-iteration graphs for the
+    // remainder (no launches of iterations that would only find the halt flag)
+    const int full = small ? 0 : n / s->graph_iters, rem = small ? 0 : n % s->graph_iters;
     CK(cudaEventRecord(s->ev0, s->stream));
+    for (int k = 0; small && k < n && !c.halt; k += kSmallIters) {
+        if ((rc = s->impl->run_small(s->stream, std::min(kSmallIters, n - k)))) return rc;
+        if (check && k + kSmallIters < n) {
+            if ((rc = pull_ctl(s))) return rc;
+            if ((rc = sync_hist(s))) return rc;
+        }
+    }
     for (int k = 0; k < full; k++) {
         CK(cudaGraphLaunch(s->gexec, s->stream));
         if (check && poll_every > 0 && (k + 1) % poll_every == 0 && (k + 1 < full || rem)) {
