@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kSmallThreads + 32, 1) k_small32(const __grid_
                 if (live[j]) {
                     V4<float> d = {};
                     if (g.sweeps > 0) d = nb_values(j, src);
-                    const V4<float> w = update_value(g.f, g.rk[st], g.sweeps > 0 ? 1 : 0, clog[j], r[j], d, dt[j],
+                    const V4<float> w = update_value(g.f.irs_eps, g.rk[st], g.sweeps > 0 ? 1 : 0, clog[j], r[j], d, dt[j],
                                                      area[j], w0[j], last, drho, bad);
                     Ws[at[j]] = w;
                     if (last) w0[j] = w;
