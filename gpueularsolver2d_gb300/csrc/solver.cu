@@ -218,6 +218,7 @@ struct SolverBase {
     virtual int download_walls(double *w_wall) = 0;
     virtual int enqueue(cudaStream_t s) = 0;
     virtual int launches() const = 0;
+    virtual int passes() const = 0;  // launches of enqueue and enqueue_timed
     virtual bool small() const = 0;  // iterations run in one launch (small32.cuh)
     virtual int run_small(cudaStream_t s, int iters) = 0;
     virtual int nblocks() const = 0;
@@ -348,7 +349,8 @@ template <typename T> struct SolverT : SolverBase {
         return E2D_ERR_CUDA;
     }
 
-    int launches() const override { return small_ ? 1 : launches_per_iteration(plan); }
+    int passes() const override { return launches_per_iteration(plan); }
+    int launches() const override { return small_ ? 1 : passes(); }
     const void *topo_ptr() const override { return plan.m.topo; }
     int nblocks() const override { return (L->n + plan.block - 1) / plan.block; }
 };
@@ -656,7 +658,7 @@ int e2d_profile_passes(e2d_solver *s, int32_t iters, double *ms, int32_t *launch
     Ctl &c = *s->ctl_host;
     c.halt = 0; c.nbad = 0; c.target = c.step + iters; c.check_epsl = 0;
     if ((rc = push_ctl(s))) return rc;
-    const int per = s->impl->launches();
+    const int per = s->impl->passes();
     std::vector<cudaEvent_t> ev(2 * (size_t)per * iters);
     std::vector<int> kind((size_t)per * iters);
     for (auto &e : ev) CK(cudaEventCreate(&e));

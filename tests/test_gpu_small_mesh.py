@@ -53,3 +53,14 @@ def test_stops_at_the_residual(lib):
     a.step(300)
     b.step(300)
     assert np.array_equal(a.state(), b.state())
+
+
+def test_profiled_passes_advance_like_steps(lib):
+    """e2d_profile_passes launches the passes one by one whatever the mesh."""
+    mesh = e2d.Mesh.ogrid(64, 16, seed=2)
+    a = e2d.Solver(mesh, e2d.default_params(**KW))
+    b = e2d.Solver(mesh, e2d.default_params(**KW))
+    ms, launches = a.profile_passes(5)
+    b.step(5)
+    assert launches.tolist() == [20, 20, 20, 20, 5] and np.all(ms > 0)
+    assert np.array_equal(a.state(), b.state()) and np.array_equal(a.history(), b.history())
