@@ -427,9 +427,13 @@ __device__ __forceinline__ V4<float> roe<float>(const V4<float> &LW, const V4<fl
 // Pass A: gpu_solver.cu:137-223 (kernel_Boundary), 225-383 (kernel_Gradient),
 // 385-454 (kernel_deltT), 456-549 (kernel_Limiter / kernel_LBJinterpolate),
 // and the dt part of 768-878 (kernel_Flux_e2c).
-// FS[k*n+i] receives the state on the cell's own side of face k: the limited
-// reconstruction for an interior face, the cell state itself for a boundary
-// face (the reference's boundary faces are first order).
+// FS[k*n+i] receives the state on the cell's own side of face k, the limited
+// reconstruction, for an interior face, and the ghost state for a boundary face
+// (the reference's boundary faces are first order: the cell's own side is the
+// cell state, and pass B would evaluate the ghost again from it: on small
+// O-grids most warps hold a boundary cell.  us per iteration without and with
+// this: FP32 4.2M cells 940 and 925, 60 batched cases 508 and 500, 2k cells in one
+// launch 18.4 and 14.7; FP64 33.6k cells 252 and 243).
 //
 // Limiter freezing (an option with no reference counterpart, off when phi is
 // null): while not frozen the limiter values of every face are recorded in
@@ -627,8 +631,10 @@ __device__ __forceinline__ Limit32 limits32(const Recon32 &c, const Flow<float> 
     return lim;
 }
 
-// Pass A of one cell from its neighbours' (or ghost) states: its three face
-// states go to out(k, state), its local time step is returned.  OPT compiles in
+// Pass A of one cell from its neighbours' (or ghost) states: the states of its
+// interior faces go to out(k, state), its local time step is returned.  (On a
+// boundary face the cell's side is the cell state itself; what pass B needs
+// there is the ghost, which the caller leaves in the face's place.)  OPT compiles in
 // the scheme options (smooth limiter, frozen limiter values, first-order faces,
 // positivity fallback); without them the reference configuration runs in fewer
 // registers.  first: this iteration uses first-order faces.
@@ -645,8 +651,9 @@ __device__ __forceinline__ float faces_cell32(const MeshDev<float> &m, const Flo
     const Limit32 lim = limits32<OPT>(c, f, code, S, A, reuse, first);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
+        if (code[k] < 0) continue;
         V4<float> o = U;
-        if (code[k] >= 0 && !(OPT && first)) {
+        if (!(OPT && first)) {
             V4<float> ph;
             if (reuse) ph = phi[k * n + i];
             o = face_state32<OPT>(c, f, lim, offset32(S[(k + 1) % 3], S[(k + 2) % 3]), ph);
@@ -671,8 +678,10 @@ __device__ __forceinline__ float faces_cell(const MeshDev<float> &m, const Flow<
     for (int k = 0; k < 3; k++) S[k] = m.S[k * n + i];
     V4<float> nbv[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++)
-        nbv[k] = code[k] >= 0 ? W[code[k] >> 3] : ghost(code[k], U, S[k].x, S[k].y, f);
+    for (int k = 0; k < 3; k++) {
+        if (code[k] >= 0) nbv[k] = W[code[k] >> 3];
+        else FS[k * n + i] = nbv[k] = ghost(code[k], U, S[k].x, S[k].y, f);
+    }
     const float dti = faces_cell32<OPT>(m, f, i, code, S, U, nbv, phi, frozen, first,
                                         [&](int k, const V4<float> &o) { FS[k * n + i] = o; });
     dt[i] = dti;
@@ -801,9 +810,9 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
                         for (int c = 0; c < 4; c++) d[c] = u[c];
                 }
             if (OPT && phi && !frozen) store(phi + k * n + i, ph);
-        } else {
+        } else {  // a boundary face's place takes the ghost (for pass B)
 #pragma unroll
-            for (int q = 0; q < NQ; q++) d[q] = u[q];
+            for (int q = 0; q < NQ; q++) d[q] = code[k] < 0 ? nb[k][q] : u[q];
         }
         store(FS + k * n + i, d);
     }
@@ -1018,7 +1027,8 @@ __device__ __forceinline__ void add_flux(V4<T> &r, const V4<T> &F, const bool ri
 
 template <typename T>
 __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f, const int i,
-                                          const V4<T> *__restrict__ FS, V4<T> *__restrict__ res, const int4 tp) {
+                                          const V4<T> *__restrict__ W, const V4<T> *__restrict__ FS,
+                                          V4<T> *__restrict__ res, const int4 tp) {
     const int n = m.n;
     const int code[3] = {tp.x, tp.y, tp.z};
     V4<T> r;
@@ -1029,8 +1039,8 @@ __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f,
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         S[k] = m.S[k * n + i];
-        own[k] = FS[k * n + i];
-        if (code[k] >= 0) oth[k] = FS[(code[k] & 3) * n + (code[k] >> 3)];
+        own[k] = code[k] >= 0 ? FS[k * n + i] : W[i];
+        oth[k] = FS[code[k] >= 0 ? (code[k] & 3) * n + (code[k] >> 3) : k * n + i];
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -1059,26 +1069,20 @@ template <> __device__ __forceinline__ void unit_normal<float>(const V2<float> S
 }
 
 // Inputs of the Roe flux of one face in the edge's orientation: left state a,
-// right state b (the ghost across a boundary face), unit normal (nx, ny) of
+// right state b (oth: the neighbour's side, the ghost of a boundary face), unit normal (nx, ny) of
 // the edge and the face length vn; *right tells whether the cell is the
 // edge's right cell.
 template <typename T>
-__device__ __forceinline__ void face_inputs(const Flow<T> &f, const int code, const V2<T> S, const V4<T> own,
-                                            const V4<T> oth, V4<T> &a, V4<T> &b, T &nx, T &ny, T &vn,
-                                            bool &right) {
+__device__ __forceinline__ void face_inputs(const int code, const V2<T> S, const V4<T> own, const V4<T> oth, V4<T> &a,
+                                            V4<T> &b, T &nx, T &ny, T &vn, bool &right) {
     unit_normal(S, nx, ny, vn);
     // the left state first: both cells of a face run the same instructions on
     // the same inputs (their normals are exact negatives), so they get the
     // same bits
     a = own;
-    right = false;
-    if (code >= 0) {
-        right = (code >> 2) & 1;
-        if (right) { a = oth; b = own; nx = -nx; ny = -ny; }
-        else b = oth;
-    } else {
-        b = ghost(code, own, S.x, S.y, f);
-    }
+    b = oth;
+    right = code >= 0 && ((code >> 2) & 1);
+    if (right) { a = oth; b = own; nx = -nx; ny = -ny; }
 }
 
 // Flux of face k of cell i, times |S|, in the edge's orientation (the
@@ -1089,7 +1093,7 @@ __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, 
                                               const V4<T> oth, bool &right) {
     V4<T> a, b;
     T nx, ny, vn;
-    face_inputs(f, code, S, own, oth, a, b, nx, ny, vn, right);
+    face_inputs(code, S, own, oth, a, b, nx, ny, vn, right);
     // one Roe call site for every face
     if constexpr (sizeof(T) == 4) {
         V4<T> F = roe(a, b, nx, ny, f.gamma, f.eps_entropy);
@@ -1105,12 +1109,12 @@ __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, 
 
 template <typename T>
 __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f, const int i, const int k,
-                                           const int code, const V4<T> *__restrict__ FS, bool &right) {
+                                           const int code, const V4<T> *__restrict__ W,
+                                           const V4<T> *__restrict__ FS, bool &right) {
     const int n = m.n;
     const V2<T> S = m.S[k * n + i];
-    const V4<T> own = FS[k * n + i];
-    V4<T> oth = own;
-    if (code >= 0) oth = FS[(code & 3) * n + (code >> 3)];
+    const V4<T> own = code >= 0 ? FS[k * n + i] : W[i];
+    const V4<T> oth = code >= 0 ? FS[(code & 3) * n + (code >> 3)] : FS[k * n + i];
     return face_flux_of(f, code, S, own, oth, right);
 }
 
@@ -1125,7 +1129,8 @@ __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f
 // threads once instead of twice.
 template <typename T, int R = 1>
 __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f, const int base, const int nvalid,
-                                          const V4<T> *__restrict__ FS, V4<T> *__restrict__ res) {
+                                          const V4<T> *__restrict__ W, const V4<T> *__restrict__ FS,
+                                          V4<T> *__restrict__ res) {
     constexpr int CELLS = 256 / R;
     __shared__ V4<T> Fs[CELLS * 3];
     __shared__ int4 tps[CELLS];
@@ -1169,7 +1174,7 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
         const int4 q = tps[tt];
         const int c = k == 0 ? q.x : k == 1 ? q.y : q.z;
         bool right;
-        Fs[tt * 3 + k] = face_flux(m, f, base + tt, k, c, FS, right);
+        Fs[tt * 3 + k] = face_flux(m, f, base + tt, k, c, W, FS, right);
     }
     __syncthreads();
     if (!live) return;
@@ -1194,22 +1199,24 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
 }
 
 template <typename T, int R>
-__global__ void E2D_LB_FLUX k_flux_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ FS,
+__global__ void E2D_LB_FLUX k_flux_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
+                                        const V4<T> *__restrict__ FS,
                                         V4<T> *__restrict__ res, const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
     const int tile = blockDim.x / R, base = blockIdx.x * tile;
-    flux_tile<T, R>(m, f, base, min(tile, m.n - base), FS, res);
+    flux_tile<T, R>(m, f, base, min(tile, m.n - base), W, FS, res);
 }
 
 template <typename T>
-__global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ FS,
+__global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
+                                   const V4<T> *__restrict__ FS,
                                    V4<T> *__restrict__ res, const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
-    flux_cell(m, f, i, FS, res, m.topo[i]);
+    flux_cell(m, f, i, W, FS, res, m.topo[i]);
 }
 
 // The pass-B kernel of a precision.
@@ -1466,7 +1473,7 @@ __global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : Batc
 }
 
 template <typename T, bool LOOP>
-__global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlocks<T>::flux) kb_flux(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ FS,
+__global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlocks<T>::flux) kb_flux(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W, const V4<T> *__restrict__ FS,
                                     V4<T> *__restrict__ res) {
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += LOOP ? gridDim.x : ntiles) {
@@ -1477,9 +1484,9 @@ __global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlock
         if (b.ctl[tc].halt) continue;                // uniform over the block
         const Flow<T> &f = b.flows[tc];
         if constexpr (FluxTiled<T>::value) {
-            flux_tile(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), FS, res);
+            flux_tile(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, res);
         } else {
-            if (i < b.case_end[tc]) flux_cell(m, f, i, FS, res, tp);
+            if (i < b.case_end[tc]) flux_cell(m, f, i, W, FS, res, tp);
         }
     }
 }
@@ -1537,7 +1544,7 @@ template <typename T, bool LOOP> void enqueue_batch_passes(const BPlan<T> &p, cu
         V4<T> *Wout = last ? p.W[0] : p.W[1];
         launch_chained_smem(p.options ? kb_faces<T, true, LOOP> : kb_faces<T, false, LOOP>, G, B,
                             sizeof(T) == 8 ? B * FacesSmem::per_cell : 0, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi, st);
-        launch_chained(kb_flux<T, LOOP>, G, B, s, p.m, p.b, NT, p.FS, p.res);
+        launch_chained(kb_flux<T, LOOP>, G, B, s, p.m, p.b, NT, Wcur, p.FS, p.res);
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {
             V4<T> *dst = p.sm[sw & 1];
@@ -1628,7 +1635,7 @@ void enqueue_passes(const Plan<T> &p, cudaStream_t s, Mark mark, Done done) {
                             p.ctl, p.phi, st);
         done();
         mark(1);
-        launch_chained(flux_kernel<T>(ga.flux), grid(ga.flux), B, s, p.m, p.f, p.FS, p.res, p.ctl);
+        launch_chained(flux_kernel<T>(ga.flux), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
         done();
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {

@@ -155,9 +155,10 @@ __global__ void __launch_bounds__(kSmallThreads + 32, 1) k_small32(const __grid_
                 const V4<float> U = Ws[at[j]];
                 V4<float> nbv[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++)
-                    nbv[k] = code[j][k] >= 0 ? load_cluster(nb[j][k])
-                                             : ghost(code[j][k], U, S[j][k].x, S[j][k].y, g.f);
+                for (int k = 0; k < 3; k++) {
+                    if (code[j][k] >= 0) nbv[k] = load_cluster(nb[j][k]);
+                    else FSs[k * C + at[j]] = nbv[k] = ghost(code[j][k], U, S[j][k].x, S[j][k].y, g.f);
+                }
                 dt[j] = faces_cell32<OPT>(g.m, g.f, id[j], code[j], S[j], U, nbv, g.phi, frozen, first,
                                           [&](int k, const V4<float> &o) { FSs[k * C + at[j]] = o; });
             }
@@ -175,8 +176,9 @@ __global__ void __launch_bounds__(kSmallThreads + 32, 1) k_small32(const __grid_
                 V4<float> own[3], oth[3];
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
-                    own[k] = FSs[k * C + at[j]];
+                    own[k] = code[j][k] >= 0 ? FSs[k * C + at[j]] : Ws[at[j]];
                     if (code[j][k] >= 0) oth[k] = load_cluster(nb[j][k] + (1 + (code[j][k] & 3)) * row);
+                    else oth[k] = FSs[k * C + at[j]];
                 }
                 V4<float> s = {};
 #pragma unroll
@@ -294,9 +296,9 @@ template <bool OPT, int CPT> bool small_launch(const SmallArgs &a, cudaStream_t 
     return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess;
 }
 
-// us per iteration of 4 stages, this against one launch per pass: 2k cells 18.4 and
-// 37.8; 8k 23.7 and 38.7, with the cell-wise limiter 29.5 and 41.7; 12k 32.2 and 39.5;
-// 16k 36.4 and 41.0, with the smooth limiter 47.5 and 41.8 (two cells to a thread
+// us per iteration of 4 stages, this against one launch per pass: 2k cells 14.7 and
+// 35.6; 8k 21.2 and 36.4, with the cell-wise limiter 27.5 and 38.9; 12k 29.1 and 36.3;
+// 16k 33.6 and 37.8 (two cells to a thread
 // spill with the options: they stop at one).
 bool small_iterations(const Plan<float> &p, int iters, cudaStream_t s, bool probe) {
     const bool opt = faces_options(p.f, p.phi);
