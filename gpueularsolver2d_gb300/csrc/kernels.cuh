@@ -303,53 +303,65 @@ __device__ __forceinline__ double harten(const double v, const double epsilon) {
     return ddiv(v * v + epsilon * epsilon, 2.0 * epsilon);
 }
 
+// A product on the FP64 pipe or (INT) the integer units, the same bits.  On
+// meshes that fill the GPU the FP64 pipe is the bound and the integer units have
+// most of their issue slots left: 48 of pass B's 78 products and half of pass A's
+// run there (1.05M cells: pass B 608 -> 525 us, with two thirds of the rest too 557; pass A 435 -> 402,
+// with a third more 425).  On small meshes a launch is as long as one thread's
+// chain, which forty instructions for one only lengthen (2k cells: pass B 22 -> 27).
+template <bool INT> __device__ __forceinline__ double mul(double a, double b) {
+    if constexpr (INT) return imul(a, b);
+    else return a * b;
+}
+
 // FP64: the reference's operations in its order (calc_function,
 // gpu_solver.cu:552-566, and the flux), times the face length.  Powers of two
 // move through the roundings: x - 0.5 y is one fused multiply-add (its product
 // is exact), 2 AB AB is twice AB AB and shares its divisor, and the flux's
 // factor 0.5 goes into the face length.
+template <bool IM>
 __device__ __forceinline__ V4<double> roe_scaled(const V4<double> &LW, const V4<double> &RW, const double nx,
                                                 const double ny, const double g, const double epsilon,
                                                 const double vn) {
     const double gm1 = g - 1.0;
     const double t0 = ddiv(1.0, LW.x), t1 = ddiv(1.0, RW.x);
-    const double U0 = LW.y * t0, V0 = LW.z * t0, e0 = LW.w * t0;
-    const double U1 = RW.y * t1, V1 = RW.z * t1, e1 = RW.w * t1;
-    const double P0 = gm1 * LW.x * fma(-0.5, U0 * U0 + V0 * V0, e0);
-    const double P1 = gm1 * RW.x * fma(-0.5, U1 * U1 + V1 * V1, e1);
-    const double H0 = e0 + P0 * t0, H1 = e1 + P1 * t1;
-    const double M0 = U0 * nx + V0 * ny, M1 = U1 * nx + V1 * ny;
+    const double U0 = mul<IM>(LW.y, t0), V0 = mul<IM>(LW.z, t0), e0 = mul<IM>(LW.w, t0);
+    const double U1 = mul<IM>(RW.y, t1), V1 = mul<IM>(RW.z, t1), e1 = mul<IM>(RW.w, t1);
+    const double P0 = mul<IM>(gm1, LW.x) * fma(-0.5, mul<IM>(U0, U0) + V0 * V0, e0);
+    const double P1 = mul<IM>(gm1, RW.x) * fma(-0.5, mul<IM>(U1, U1) + V1 * V1, e1);
+    const double H0 = e0 + mul<IM>(P0, t0), H1 = e1 + mul<IM>(P1, t1);
+    const double M0 = mul<IM>(U0, nx) + V0 * ny, M1 = mul<IM>(U1, nx) + V1 * ny;
     const double DVC = M1 - M0;
     const double sl = dsqrt(LW.x), sr = dsqrt(RW.x);
-    const double ROUB = sl * sr;
+    const double ROUB = mul<IM>(sl, sr);
     const Divisor ds = divisor(sl + sr);
-    const double UB = div_by(U0 * sl + U1 * sr, ds);
-    const double VB = div_by(V0 * sl + V1 * sr, ds);
-    const double HB = div_by(H0 * sl + H1 * sr, ds);
-    const double QB = UB * UB + VB * VB;
+    const double UB = div_by(mul<IM>(U0, sl) + U1 * sr, ds);
+    const double VB = div_by(mul<IM>(V0, sl) + V1 * sr, ds);
+    const double HB = div_by(mul<IM>(H0, sl) + H1 * sr, ds);
+    const double QB = mul<IM>(UB, UB) + VB * VB;
     const double AB = dsqrt(gm1 * fma(-0.5, QB, HB));
-    const double VC = UB * nx + VB * ny;
+    const double VC = mul<IM>(UB, nx) + VB * ny;
     const double AD0 = harten(VC - AB, epsilon), AD1 = harten(VC, epsilon), AD2 = harten(VC + AB, epsilon);
-    const double dP = P1 - P0, RAD = ROUB * AB * DVC;
-    const Divisor da = divisor(AB * AB);
+    const double dP = P1 - P0, RAD = mul<IM>(ROUB, AB) * DVC;
+    const Divisor da = divisor(mul<IM>(AB, AB));
     Divisor da2 = da;
     da2.b = 2.0 * da.b;
     da2.e = da.e ? da.e + 1 : 0;
-    const double F00 = div_by(AD0 * (dP - RAD), da2);
-    const double F20 = div_by(AD2 * (dP + RAD), da2);
+    const double F00 = div_by(mul<IM>(AD0, dP - RAD), da2);
+    const double F20 = div_by(mul<IM>(AD2, dP + RAD), da2);
     const double F10 = AD1 * ((RW.x - LW.x) - div_by(dP, da));
-    const double anx = AB * nx, any = AB * ny, avc = AB * VC;
-    const double dU = U1 - U0, dV = V1 - V0, aR = AD1 * ROUB;
-    const double F11 = F10 * UB + aR * (dU - DVC * nx);
-    const double F12 = F10 * VB + aR * (dV - DVC * ny);
-    const double F13 = fma(F10 * QB, 0.5, aR * (UB * dU + VB * dV - DVC * VC));
-    const double WL0 = LW.x * M0, WR0 = RW.x * M1;
+    const double anx = mul<IM>(AB, nx), any = mul<IM>(AB, ny), avc = mul<IM>(AB, VC);
+    const double dU = U1 - U0, dV = V1 - V0, aR = mul<IM>(AD1, ROUB);
+    const double F11 = mul<IM>(F10, UB) + aR * (dU - mul<IM>(DVC, nx));
+    const double F12 = mul<IM>(F10, VB) + aR * (dV - mul<IM>(DVC, ny));
+    const double F13 = fma(mul<IM>(F10, QB), 0.5, aR * (mul<IM>(UB, dU) + VB * dV - mul<IM>(DVC, VC)));
+    const double WL0 = mul<IM>(LW.x, M0), WR0 = mul<IM>(RW.x, M1);
     const double hv = 0.5 * vn;
     V4<double> F;
     F.x = ((WL0 + WR0) - (F00 + F10 + F20)) * hv;
-    F.y = (((U0 * WL0 + nx * P0) + (U1 * WR0 + nx * P1)) - (F00 * (UB - anx) + F11 + F20 * (UB + anx))) * hv;
-    F.z = (((V0 * WL0 + ny * P0) + (V1 * WR0 + ny * P1)) - (F00 * (VB - any) + F12 + F20 * (VB + any))) * hv;
-    F.w = ((WL0 * H0 + WR0 * H1) - (F00 * (HB - avc) + F13 + F20 * (HB + avc))) * hv;
+    F.y = ((mul<IM>(U0, WL0) + mul<IM>(nx, P0)) + (mul<IM>(U1, WR0) + nx * P1) - (mul<IM>(F00, UB - anx) + F11 + F20 * (UB + anx))) * hv;
+    F.z = ((mul<IM>(V0, WL0) + mul<IM>(ny, P0)) + (mul<IM>(V1, WR0) + ny * P1) - (mul<IM>(F00, VB - any) + F12 + F20 * (VB + any))) * hv;
+    F.w = ((mul<IM>(WL0, H0) + mul<IM>(WR0, H1)) - (mul<IM>(F00, HB - avc) + F13 + F20 * (HB + avc))) * hv;
     return F;
 }
 
@@ -722,7 +734,8 @@ __device__ __forceinline__ double face_limiter64(const int kind, const double e2
 // first term of a sum is not added to zero, the bounds are subtracted once per
 // component and divisions, comparisons and selections run on the integer units.
 // gs: the ghost states of the cell's boundary faces.
-template <bool OPT, int LPC>
+// IM: half of the products on the integer units (mul).
+template <bool OPT, int LPC, bool IM = (LPC < 4)>
 __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
                                                const int part, const V4<double> *__restrict__ W,
                                                V4<double> *__restrict__ FS, double *__restrict__ dt,
@@ -758,7 +771,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const double s = u[q] + nb[k][q];
-            const double px = s * (0.5 * S[k].x), py = s * (0.5 * S[k].y);
+            const double px = mul<IM>(s, 0.5 * S[k].x), py = s * (0.5 * S[k].y);
             gx[q] = k == 0 ? px : gx[q] + px;
             gy[q] = k == 0 ? py : gy[q] + py;
         }
@@ -785,7 +798,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
             const V2<double> r = m.R[k * n + i];
 #pragma unroll
             for (int q = 0; q < NQ; q++)
-                phic[q] = fmin(phic[q], face_limiter64(kind, e2, bnd[q], gx[q] * r.x + gy[q] * r.y));
+                phic[q] = fmin(phic[q], face_limiter64(kind, e2, bnd[q], mul<IM>(gx[q], r.x) + gy[q] * r.y));
         }
     }
 #pragma unroll
@@ -797,7 +810,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
             if (reuse) values(phi + k * n + i, ph);
 #pragma unroll
             for (int q = 0; q < NQ; q++) {
-                const double delt2 = gx[q] * r.x + gy[q] * r.y;
+                const double delt2 = mul<IM>(gx[q], r.x) + gy[q] * r.y;
                 if (cellwise && !reuse) ph[q] = phic[q];
                 else if (!reuse) ph[q] = face_limiter64(kind, e2, bnd[q], delt2);
                 d[q] = delt2 * ph[q] + u[q];
@@ -1088,7 +1101,7 @@ __device__ __forceinline__ void face_inputs(const int code, const V2<T> S, const
 // Flux of face k of cell i, times |S|, in the edge's orientation (the
 // reference's Res_e.left of gpu_solver.cu:738-745); *right tells whether cell
 // i is the edge's right cell.
-template <typename T>
+template <typename T, bool IM = false>
 __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, const V2<T> S, const V4<T> own,
                                               const V4<T> oth, bool &right) {
     V4<T> a, b;
@@ -1103,11 +1116,11 @@ __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, 
         F.x = xy.x; F.y = xy.y; F.z = zw.x; F.w = zw.y;
         return F;
     } else {
-        return roe_scaled(a, b, nx, ny, f.gamma, f.eps_entropy, vn);
+        return roe_scaled<IM>(a, b, nx, ny, f.gamma, f.eps_entropy, vn);
     }
 }
 
-template <typename T>
+template <typename T, bool IM>
 __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f, const int i, const int k,
                                            const int code, const V4<T> *__restrict__ W,
                                            const V4<T> *__restrict__ FS, bool &right) {
@@ -1115,7 +1128,7 @@ __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f
     const V2<T> S = m.S[k * n + i];
     const V4<T> own = code >= 0 ? FS[k * n + i] : W[i];
     const V4<T> oth = code >= 0 ? FS[(code & 3) * n + (code >> 3)] : FS[k * n + i];
-    return face_flux_of(f, code, S, own, oth, right);
+    return face_flux_of<T, IM>(f, code, S, own, oth, right);
 }
 
 // Pass B for one tile of cells [base, base + nvalid) with each interior face
@@ -1127,7 +1140,7 @@ __device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f
 // flux_cell and are summed in the same order.  nvalid <= blockDim.x / R,
 // blockDim.x <= 256: with R = 2 the list (about 1.7 faces per cell) takes the
 // threads once instead of twice.
-template <typename T, int R = 1>
+template <typename T, int R = 1, bool IM = true>
 __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f, const int base, const int nvalid,
                                           const V4<T> *__restrict__ W, const V4<T> *__restrict__ FS,
                                           V4<T> *__restrict__ res) {
@@ -1174,7 +1187,7 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
         const int4 q = tps[tt];
         const int c = k == 0 ? q.x : k == 1 ? q.y : q.z;
         bool right;
-        Fs[tt * 3 + k] = face_flux(m, f, base + tt, k, c, W, FS, right);
+        Fs[tt * 3 + k] = face_flux<T, IM>(m, f, base + tt, k, c, W, FS, right);
     }
     __syncthreads();
     if (!live) return;
@@ -1198,14 +1211,14 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
     res[i] = r;
 }
 
-template <typename T, int R>
+template <typename T, int R, bool IM>
 __global__ void E2D_LB_FLUX k_flux_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
                                         const V4<T> *__restrict__ FS,
                                         V4<T> *__restrict__ res, const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
     const int tile = blockDim.x / R, base = blockIdx.x * tile;
-    flux_tile<T, R>(m, f, base, min(tile, m.n - base), W, FS, res);
+    flux_tile<T, R, IM>(m, f, base, min(tile, m.n - base), W, FS, res);
 }
 
 template <typename T>
@@ -1220,9 +1233,13 @@ __global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restr
 }
 
 // The pass-B kernel of a precision.
-template <typename T> auto flux_kernel(int lanes) {
-    if constexpr (FluxTiled<T>::value) return lanes == 2 ? &k_flux_tile<T, 2> : &k_flux_tile<T, 1>;
-    else return &k_flux<T>;
+template <typename T> auto flux_kernel(int lanes, bool im) {
+    if constexpr (FluxTiled<T>::value) {
+        if (lanes == 1) return &k_flux_tile<T, 1, true>;
+        return im ? &k_flux_tile<T, 2, true> : &k_flux_tile<T, 2, false>;
+    } else {
+        return &k_flux<T>;
+    }
 }
 
 // Threads per cell of passes A and B.  FP32: one.  FP64: a mesh of up to some
@@ -1230,7 +1247,8 @@ template <typename T> auto flux_kernel(int lanes) {
 // launch takes as long as one thread's chain of some 2500 instructions, so the
 // cell's work is spread over more threads; on large meshes that only repeats
 // loads and the work per cell, and smaller tiles evaluate more faces twice.
-// us per launch with 1 / 2 / 4 threads in pass A and 1 / 2 in pass B: 2k cells 27 /
+// us per launch with 1 / 2 / 4 threads in pass A and 1 / 2 in pass B (all products on
+// the FP64 pipe; from 12k cells on some leave it, see mul): 2k cells 27 /
 // 20 / 17 and 30 / 21; 8k 31 / 21 / 18 and 33 / 22; 34k (limiter option) 29 / 25 /
 // 29 and 40 / 37; 80k 61 / 54 / 54 and 77 / 79; 131k 72 / 70 / 79 and 100 / 106;
 // 1.05M 436 / 461 / 554 and 615 / 691.  (The positivity option compares a cell's
@@ -1635,7 +1653,7 @@ void enqueue_passes(const Plan<T> &p, cudaStream_t s, Mark mark, Done done) {
                             p.ctl, p.phi, st);
         done();
         mark(1);
-        launch_chained(flux_kernel<T>(ga.flux), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
+        launch_chained(flux_kernel<T>(ga.flux, ga.faces < 4), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
         done();
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {

@@ -42,6 +42,9 @@ int main(int argc, char **argv) {
         if (!same(e2d::dsqrt(a), std::sqrt(a))) {
             if (bad++ < 5) printf("sqrt %a: %a, not %a\n", a, e2d::dsqrt(a), std::sqrt(a));
         }
+        if (!same(e2d::imul(a, b), a * b)) {
+            if (bad++ < 5) printf("mul %a %a: %a, not %a\n", a, b, e2d::imul(a, b), a * b);
+        }
         const bool lt = e2d::order_key(a) < e2d::order_key(b);
         if (a == a && b == b && a != b && lt != (a < b)) bad++;
         if (!same(e2d::key_value(e2d::order_key(a)), a)) bad++;
@@ -59,6 +62,10 @@ int main(int argc, char **argv) {
         check(std::fabs(b), a);
         check(a * b, b);  // quotients close to representable numbers
         check(a * a, a);
+        // products half way between two numbers, and next to it
+        const uint64_t odd = (rnd() & 0x3ffffff) | 1, big = (1ULL << 52) | (rnd() & 0xFFFFFFFFFFFFFULL);
+        check((double)(odd | 0x4000000), (double)(rnd() & 0x7ffffff));
+        check((double)big, (double)(odd & 7));
     }
     printf("%ld\n", bad);
     return bad != 0;
