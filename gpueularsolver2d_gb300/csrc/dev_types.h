@@ -56,6 +56,23 @@ template <typename T> struct MeshDev {
     const T *__restrict__ area;
 };
 
+// Every face once (FP64 on large meshes), in the order of the left cells:
+// at[j] = {entry k * n + i of the left (or boundary) cell i, the right cell's entry
+// or -1 on a boundary face, i, the right cell}; geo: unit normal, half the length,
+// face vector and its square, [6][count]; radius: [3n] a face's spectral radius at
+// its left cell's entry.
+struct FaceList {
+    const int4 *at;
+    double *geo, *radius;
+    int count;  // 0: passes A and B work in tiles of cells
+};
+
+// Cells from which a single FP64 mesh takes a face list.  Below, a launch is as
+// long as one thread's chain and several threads per cell shorten it (gather_shape).
+// us per iteration in tiles and with the list: 8k cells 164 and 201, 20k 210 and
+// 217, 34k 249 and 237, 131k 640 and 566, 1.05M 4291 and 3680.
+constexpr int face_list_cells = 24000;
+
 // Everything one iteration needs.
 template <typename T> struct Plan {
     MeshDev<T> m;
@@ -74,10 +91,11 @@ template <typename T> struct Plan {
     T rk[8];
     int sweeps;
     int block;
+    FaceList faces;
 };
 
 template <typename T> int launches_per_iteration(const Plan<T> &p) {
-    return p.stages * (3 + (p.sweeps > 1 ? p.sweeps - 1 : 0)) + 1;
+    return p.stages * (3 + (p.faces.count ? 1 : 0) + (p.sweeps > 1 ? p.sweeps - 1 : 0)) + 1;
 }
 
 // Batched cases: the cells of all cases in one array, case c in
@@ -146,6 +164,9 @@ void enqueue_export(int n, const int *perm, const V4<T> *W, double *wfile, cudaS
 // The states of cells[0 .. cnt), FP64.
 template <typename T>
 void enqueue_export_cells(int cnt, const int *cells, const V4<T> *W, double *w, cudaStream_t s);
+
+// Geometry of a face list from the mesh's face vectors.
+void enqueue_face_geometry(const MeshDev<double> &m, const FaceList &l, cudaStream_t s);
 
 // Residual kernel launcher (resid.cu).
 void enqueue_resid(double *part, int nparts, Ctl *ctl, double *hist, int hist_cap, bool pairs,

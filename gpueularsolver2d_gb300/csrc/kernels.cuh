@@ -16,7 +16,9 @@
 // Every cell gathers its own faces, so nothing is accumulated with atomics
 // and the result does not depend on scheduling.  An interior face inside one
 // block's tile of cells is evaluated once; a face between two tiles is
-// evaluated by both cells from identical inputs, so both see the same value.  The arithmetic of each quantity follows the reference kernel
+// evaluated by both cells from identical inputs, so both see the same value.
+// (Large FP64 meshes evaluate every face once from a list and split pass B in
+// two: k_face_flux, k_face_sum.)  The arithmetic of each quantity follows the reference kernel
 // it replaces operation by operation (cited per function); compiled without
 // FMA contraction, the FP64 instantiation reproduces the CPU oracle bit for
 // bit.
@@ -262,9 +264,9 @@ __device__ __forceinline__ V4<T> ghost(int code, const V4<T> &U, T Sx, T Sy, con
 // is subtracted is a fused multiply-add with an exact product.  19 FP64
 // additions and multiplications where the reference's form issues about 30.
 template <typename T> __device__ T spectral_radius(const V4<T> &a, const V4<T> &b, T vectorx, T vectory, T g);
-template <>
-__device__ __forceinline__ double spectral_radius<double>(const V4<double> &a, const V4<double> &b, double vectorx,
-                                                         double vectory, double g) {
+// FP64, with the face vector's square q given.
+__device__ __forceinline__ double spectral_radius64(const V4<double> &a, const V4<double> &b, double vectorx,
+                                                    double vectory, double q, double g) {
     const double rou2 = a.x + b.x;  // 2 rou
     const Divisor d = divisor(rou2);
     const double u = div_by(a.y + b.y, d);
@@ -272,8 +274,13 @@ __device__ __forceinline__ double spectral_radius<double>(const V4<double> &a, c
     const double EE = fma(-0.5, u * u + v * v, div_by(a.w + b.w, d));
     const double VC = u * vectory + v * vectorx;
     const double p2 = rou2 * EE * (g - 1.0);  // 2 p
-    const double CS = dsqrt(div_by(g * p2, d) * (vectorx * vectorx + vectory * vectory));
+    const double CS = dsqrt(div_by(g * p2, d) * q);
     return tabs(VC) + CS;
+}
+template <>
+__device__ __forceinline__ double spectral_radius<double>(const V4<double> &a, const V4<double> &b, double vectorx,
+                                                         double vectory, double g) {
+    return spectral_radius64(a, b, vectorx, vectory, vectorx * vectorx + vectory * vectory, g);
 }
 
 // FP32: the same quantity with one reciprocal and fused multiply-adds.
@@ -315,14 +322,14 @@ template <bool INT> __device__ __forceinline__ double mul(double a, double b) {
 }
 
 // FP64: the reference's operations in its order (calc_function,
-// gpu_solver.cu:552-566, and the flux), times the face length.  Powers of two
+// gpu_solver.cu:552-566, and the flux), times the face length 2 hv.  Powers of two
 // move through the roundings: x - 0.5 y is one fused multiply-add (its product
 // is exact), 2 AB AB is twice AB AB and shares its divisor, and the flux's
 // factor 0.5 goes into the face length.
 template <bool IM>
 __device__ __forceinline__ V4<double> roe_scaled(const V4<double> &LW, const V4<double> &RW, const double nx,
                                                 const double ny, const double g, const double epsilon,
-                                                const double vn) {
+                                                const double hv) {
     const double gm1 = g - 1.0;
     const double t0 = ddiv(1.0, LW.x), t1 = ddiv(1.0, RW.x);
     const double U0 = mul<IM>(LW.y, t0), V0 = mul<IM>(LW.z, t0), e0 = mul<IM>(LW.w, t0);
@@ -356,7 +363,6 @@ __device__ __forceinline__ V4<double> roe_scaled(const V4<double> &LW, const V4<
     const double F12 = mul<IM>(F10, VB) + aR * (dV - mul<IM>(DVC, ny));
     const double F13 = fma(mul<IM>(F10, QB), 0.5, aR * (mul<IM>(UB, dU) + VB * dV - mul<IM>(DVC, VC)));
     const double WL0 = mul<IM>(LW.x, M0), WR0 = mul<IM>(RW.x, M1);
-    const double hv = 0.5 * vn;
     V4<double> F;
     F.x = ((WL0 + WR0) - (F00 + F10 + F20)) * hv;
     F.y = ((mul<IM>(U0, WL0) + mul<IM>(nx, P0)) + (mul<IM>(U1, WR0) + nx * P1) - (mul<IM>(F00, UB - anx) + F11 + F20 * (UB + anx))) * hv;
@@ -726,22 +732,20 @@ __device__ __forceinline__ double face_limiter64(const int kind, const double e2
     return abs_less(d1, delt2) ? ddiv(d1, delt2) : 1.0;
 }
 
-// The FP64 form of faces_cell with the sum of the cell's three spectral radii
-// given (faces_tile), by LPC lanes per cell: lane part takes the NQ = 4 / LPC
-// components from part NQ on.  It issues about 160 FP64 additions and
+// The face states of the FP64 form of faces_cell, by LPC lanes per cell: lane part
+// takes the NQ = 4 / LPC components from part NQ on.  It issues about 160 FP64 additions and
 // multiplications per cell in the reference configuration: the reference's
 // halves of the neighbour means are taken into the face vectors (exact), the
 // first term of a sum is not added to zero, the bounds are subtracted once per
 // component and divisions, comparisons and selections run on the integer units.
-// gs: the ghost states of the cell's boundary faces.
+// gs: the ghost states of the cell's boundary faces, gstep apart.
 // IM: half of the products on the integer units (mul).
 template <bool OPT, int LPC, bool IM = (LPC < 4)>
-__device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
+__device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
                                                const int part, const V4<double> *__restrict__ W,
-                                               V4<double> *__restrict__ FS, double *__restrict__ dt,
-                                               V4<double> *__restrict__ phi, const int frozen, const bool first,
-                                               const V4<double> *__restrict__ Uc, const int4 tp,
-                                               const V4<double> *gs, const double Tsum) {
+                                               V4<double> *FS, V4<double> *__restrict__ phi, const int frozen,
+                                               const bool first, const V4<double> *__restrict__ Uc, const int4 tp,
+                                               const V4<double> *gs, const int gstep) {
     constexpr int NQ = 4 / LPC;
     const int n = m.n, q0 = part * NQ;
     const int code[3] = {tp.x, tp.y, tp.z};
@@ -760,7 +764,7 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         S[k] = m.S[k * n + i];
-        values(code[k] >= 0 ? W + (code[k] >> 3) : gs + k, nb[k]);
+        values(code[k] >= 0 ? W + (code[k] >> 3) : gs + k * gstep, nb[k]);
     }
     values(Uc, u);
     const double A = m.area[i];
@@ -829,10 +833,12 @@ __device__ __forceinline__ double faces_cell64(const MeshDev<double> &m, const F
         }
         store(FS + k * n + i, d);
     }
-    if (part != 0) return (double)INFINITY;
-    const double dti = tmin(ddiv(A * f.cfl, Tsum), f.dt_cap);
-    dt[i] = dti;
-    return dti;
+}
+
+// Local time step of a cell from the sum of its faces' spectral radii.
+__device__ __forceinline__ double local_dt(const MeshDev<double> &m, const Flow<double> &f, const int i,
+                                           const double Tsum) {
+    return tmin(ddiv(m.area[i] * f.cfl, Tsum), f.dt_cap);
 }
 
 // Pass A in FP64 for one tile of cells [base, base + nvalid), nvalid <=
@@ -937,8 +943,9 @@ __device__ __forceinline__ double faces_tile(const MeshDev<double> &m, const Flo
             Tsum = k == 0 ? r : Tsum + r;
         }
     }
-    return faces_cell64<OPT, LPC>(m, f, base + tt, t % LPC, W, FS, dt, phi, frozen, first, Us + tt, tp, Gs + tt * 3,
-                                  Tsum);
+    faces_cell64<OPT, LPC>(m, f, base + tt, t % LPC, W, FS, phi, frozen, first, Us + tt, tp, Gs + tt * 3, 1);
+    if (t % LPC != 0) return (double)INFINITY;
+    return dt[base + tt] = local_dt(m, f, base + tt, Tsum);
 }
 
 // Global time-step option: the block's smallest step folded into *slot.
@@ -974,6 +981,29 @@ __global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<d
     const double v = faces_tile<OPT, LPC>(m, f, base, min(tile, m.n - base), W, FS, dt, phi,
                                           OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order, smem);
     if (OPT && f.global_dt) block_min_dt(v, &ctl->dtmin[st]);
+}
+
+// FP64 with a face list: the face states only, one cell per thread without tiles;
+// the radii are taken with the fluxes (k_face_flux) and the steps with their sums.
+template <bool OPT>
+__global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<double> f,
+                                                        const V4<double> *__restrict__ W, V4<double> *FS,
+                                                        const Ctl *__restrict__ ctl, V4<double> *__restrict__ phi) {
+    wait_prior_grid();
+    if (ctl->halt) return;
+    const int n = m.n, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int4 tp = m.topo[i];
+    if ((tp.x | tp.y | tp.z) < 0) {
+#pragma unroll 1
+        for (int k = 0; k < 3; k++) {
+            const int c = k == 0 ? tp.x : k == 1 ? tp.y : tp.z;
+            const V2<double> S = m.S[k * n + i];
+            if (c < 0) FS[k * n + i] = ghost(c, W[i], S.x, S.y, f);
+        }
+    }
+    faces_cell64<OPT, 1>(m, f, i, 0, W, FS, phi, OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order,
+                         W + i, tp, FS + i, n);
 }
 
 // FP32.  OPT: the variant with the scheme options (smooth limiter, limiter
@@ -1116,7 +1146,7 @@ __device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, 
         F.x = xy.x; F.y = xy.y; F.z = zw.x; F.w = zw.y;
         return F;
     } else {
-        return roe_scaled<IM>(a, b, nx, ny, f.gamma, f.eps_entropy, vn);
+        return roe_scaled<IM>(a, b, nx, ny, f.gamma, f.eps_entropy, 0.5 * vn);
     }
 }
 
@@ -1232,34 +1262,93 @@ __global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restr
     flux_cell(m, f, i, W, FS, res, m.topo[i]);
 }
 
+// Pass B in FP64 with a face list, in two launches.  First every face once, one
+// thread each: its spectral radius, and its flux, which takes the place of the
+// left cell's side in FS (a face's two sides are read by its thread alone).  Then
+// every cell sums its three in face order with the reference's signs.  Same bits as
+// flux_tile and faces_tile, whose tiles of 128 cells evaluate 1.75 rounds of
+// faces per warp of cells (faces between tiles twice, the last round partly filled)
+// and wait for their slowest warp; this is 1.5, without barriers, and the
+// normals are the list's.  1.05M cells: pass A 401 -> 301 us, pass B 527 -> 480.
+template <typename T> __global__ void __launch_bounds__(256) k_face_geometry(const V2<T> *__restrict__ S, FaceList l) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= l.count) return;
+    const V2<T> v = S[l.at[j].x];
+    T nx, ny, vn;
+    unit_normal(v, nx, ny, vn);
+    const T g[6] = {nx, ny, 0.5 * vn, v.x, v.y, v.y * v.y + v.x * v.x};
+    for (int k = 0; k < 6; k++) l.geo[(size_t)k * l.count + j] = g[k];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2) k_face_flux(FaceList l, Flow<T> f, const V4<T> *__restrict__ W,
+                                                      V4<T> *FS, const Ctl *__restrict__ ctl) {
+    wait_prior_grid();
+    if (ctl->halt) return;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= l.count) return;
+    const int4 at = l.at[j];
+    const double *g = l.geo + j;
+    const size_t nf = l.count;
+    const bool inner = at.y >= 0;
+    const V4<T> Wa = W[at.z], b = FS[inner ? at.y : at.x], a = inner ? FS[at.x] : Wa;
+    l.radius[at.x] = spectral_radius64(Wa, inner ? W[at.w] : b, g[4 * nf], g[3 * nf], g[5 * nf], f.gamma);
+    FS[at.x] = roe_scaled<true>(a, b, g[0], g[nf], f.gamma, f.eps_entropy, g[2 * nf]);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_face_sum(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ F,
+                                                  const T *__restrict__ radius, V4<T> *__restrict__ res,
+                                                  T *__restrict__ dt, Ctl *ctl, const int st) {
+    wait_prior_grid();
+    if (ctl->halt) return;
+    const int n = m.n, i = blockIdx.x * blockDim.x + threadIdx.x;
+    T dti = T(INFINITY);
+    if (i < n) {
+        const int4 tp = m.topo[i];
+        const int code[3] = {tp.x, tp.y, tp.z};
+        V4<T> v[3], r = {};
+        T q[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const int c = code[k], j = c >= 0 && ((c >> 2) & 1) ? (c & 3) * n + (c >> 3) : k * n + i;
+            v[k] = F[j];
+            q[k] = radius[j];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) add_flux(r, v[k], code[k] >= 0 && ((code[k] >> 2) & 1));
+        res[i] = r;
+        dt[i] = dti = local_dt(m, f, i, q[0] + q[1] + q[2]);
+    }
+    if (f.global_dt) block_min_dt(dti, &ctl->dtmin[st]);
+}
+
 // The pass-B kernel of a precision.
-template <typename T> auto flux_kernel(int lanes, bool im) {
+template <typename T> auto flux_kernel(bool im) {
     if constexpr (FluxTiled<T>::value) {
-        if (lanes == 1) return &k_flux_tile<T, 1, true>;
         return im ? &k_flux_tile<T, 2, true> : &k_flux_tile<T, 2, false>;
     } else {
         return &k_flux<T>;
     }
 }
 
-// Threads per cell of passes A and B.  FP32: one.  FP64: a mesh of up to some
-// 40k cells has one or two warps for each of the GPU's 608 schedulers, and a
+// Threads per cell of passes A and B in tiles.  FP32: one.  FP64: a mesh of up to
+// some 40k cells has one or two warps for each of the GPU's 608 schedulers, and a
 // launch takes as long as one thread's chain of some 2500 instructions, so the
 // cell's work is spread over more threads; on large meshes that only repeats
 // loads and the work per cell, and smaller tiles evaluate more faces twice.
 // us per launch with 1 / 2 / 4 threads in pass A and 1 / 2 in pass B (all products on
 // the FP64 pipe; from 12k cells on some leave it, see mul): 2k cells 27 /
 // 20 / 17 and 30 / 21; 8k 31 / 21 / 18 and 33 / 22; 34k (limiter option) 29 / 25 /
-// 29 and 40 / 37; 80k 61 / 54 / 54 and 77 / 79; 131k 72 / 70 / 79 and 100 / 106;
-// 1.05M 436 / 461 / 554 and 615 / 691.  (The positivity option compares a cell's
-// components: one thread.)
+// 29 and 40 / 37; 80k 61 / 54 / 54 and 77 / 79; 131k 72 / 70 / 79 and 100 / 106.
+// Larger meshes take a face list (face_list_cells).  (The positivity option
+// compares a cell's components: one thread.)
 struct Gather {
     int faces, flux;
 };
 template <typename T> Gather gather_shape(const Plan<T> &p) {
     if (sizeof(T) == 4) return {1, 1};
-    const int n = p.m.n;
-    return {p.f.positivity || n > 200000 ? 1 : n > 12000 ? 2 : 4, n > 40000 ? 1 : 2};
+    return {p.f.positivity ? 1 : p.m.n > 12000 ? 2 : 4, 2};
 }
 
 // Sum of the interior neighbours' values in face order (gpu_solver.cu:1658-1666)
@@ -1648,12 +1737,27 @@ void enqueue_passes(const Plan<T> &p, cudaStream_t s, Mark mark, Done done) {
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
         mark(0);
-        launch_chained_smem(faces_kernel<T>(opt, ga.faces), grid(ga.faces), B,
-                            sizeof(T) == 8 ? B / ga.faces * FacesSmem::per_cell : 0, s, p.m, p.f, Wcur, p.FS, p.dt,
-                            p.ctl, p.phi, st);
-        done();
-        mark(1);
-        launch_chained(flux_kernel<T>(ga.flux, ga.faces < 4), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
+        if (p.faces.count) {
+            if constexpr (sizeof(T) == 8) {
+                const int GF = (p.faces.count + B - 1) / B;
+                launch_chained(opt ? k_faces_cells<true> : k_faces_cells<false>, G, B, s, p.m, p.f, Wcur, p.FS, p.ctl,
+                               p.phi);
+                done();
+                mark(1);
+                launch_chained(k_face_flux<T>, GF, B, s, p.faces, p.f, Wcur, p.FS, p.ctl);
+                done();
+                mark(1);
+                launch_chained(k_face_sum<T>, G, B, s, p.m, p.f, p.FS, p.faces.radius, p.res, p.dt, p.ctl, st);
+            }
+        } else {
+            launch_chained_smem(faces_kernel<T>(opt, ga.faces), grid(ga.faces), B,
+                                sizeof(T) == 8 ? B / ga.faces * FacesSmem::per_cell : 0, s, p.m, p.f, Wcur, p.FS, p.dt,
+                                p.ctl, p.phi, st);
+            done();
+            mark(1);
+            launch_chained(flux_kernel<T>(ga.faces < 4), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res,
+                           p.ctl);
+        }
         done();
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {

@@ -10,4 +10,8 @@ template int enqueue_iteration_timed<double>(const Plan<double> &p, cudaStream_t
 template void enqueue_import<double>(int n, const int *perm, const double *wfile, V4<double> *W, cudaStream_t s);
 template void enqueue_export<double>(int n, const int *perm, const V4<double> *W, double *wfile, cudaStream_t s);
 template void enqueue_export_cells<double>(int cnt, const int *cells, const V4<double> *W, double *w, cudaStream_t s);
+
+void enqueue_face_geometry(const MeshDev<double> &m, const FaceList &l, cudaStream_t s) {
+    k_face_geometry<<<(l.count + 255) / 256, 256, 0, s>>>(m.S, l);
+}
 }

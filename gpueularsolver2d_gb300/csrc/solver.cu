@@ -248,6 +248,10 @@ template <typename T> struct SolverT : SolverBase {
                        Arena::up(sizeof(V4<T>) * 3 * n) * (freezes(p) ? 2 : 1) +
                        Arena::up(sizeof(double) * G) +
                        Arena::up(sizeof(int) * n) + Arena::up(sizeof(double) * 4 * n);
+        std::vector<int4> faces;
+        if (sizeof(T) == 8 && n > face_list_cells) faces = face_list();
+        bytes += Arena::up(sizeof(int4) * faces.size()) + Arena::up(sizeof(double) * 6 * faces.size()) +
+                 Arena::up(faces.empty() ? 0 : sizeof(double) * 3 * n);
         CK(cudaMalloc((void **)&arena.base, bytes));
         arena.cap = bytes;
         int4 *topo = (int4 *)arena.take(sizeof(int4) * n);
@@ -280,6 +284,19 @@ template <typename T> struct SolverT : SolverBase {
         CK(cudaMemset(plan.W[1], 0, sizeof(V4<T>) * n));
         CK(cudaMemset(plan.part, 0, sizeof(double) * G));
         plan.m = MeshDev<T>{n, topo, S, R, area};
+        plan.faces = FaceList{};
+        if constexpr (sizeof(T) == 8) {
+            if (!faces.empty()) {
+                const int count = (int)faces.size();
+                int4 *at = (int4 *)arena.take(sizeof(int4) * count);
+                double *geo = (double *)arena.take(sizeof(double) * 6 * count);
+                plan.faces = FaceList{at, geo, (double *)arena.take(sizeof(double) * 3 * n), count};
+                CK(cudaMemcpy(at, faces.data(), sizeof(int4) * count, cudaMemcpyHostToDevice));
+                enqueue_face_geometry(plan.m, plan.faces, nullptr);
+                CK(cudaGetLastError());
+                CK(cudaDeviceSynchronize());
+            }
+        }
         Flow<T> &f = plan.f;
         f.gamma = (T)p.gamma; f.ui = (T)fs.ui; f.vi = (T)fs.vi; f.ain = (T)fs.ain_test; f.tin = (T)p.tin;
         f.vin = (T)fs.vin; f.R = (T)kR; f.pis = (T)fs.pis; f.cfl = (T)p.cfl; f.dt_cap = (T)p.dt_cap;
@@ -296,6 +313,20 @@ template <typename T> struct SolverT : SolverBase {
         plan.block = block;
         if constexpr (sizeof(T) == 4) small_ = small_iterations(plan, 0, nullptr, true);
         return E2D_OK;
+    }
+
+    // Every face once, at its left cell (see FaceList).
+    std::vector<int4> face_list() const {
+        const int n = L->n;
+        std::vector<int4> v;
+        v.reserve(3 * (size_t)n / 2 + 1024);
+        for (int i = 0; i < n; i++)
+            for (int k = 0; k < 3; k++) {
+                const int c = L->topo[4 * (size_t)i + k];
+                if (c < 0) v.push_back(make_int4(k * n + i, -1, i, i));
+                else if (!((c >> 2) & 1)) v.push_back(make_int4(k * n + i, (c & 3) * n + (c >> 3), i, c >> 3));
+            }
+        return v;
     }
 
     // Caller's FP64 file-order buffer -> device (one copy; from pinned memory
