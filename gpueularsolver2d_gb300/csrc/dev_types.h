@@ -67,11 +67,11 @@ struct FaceList {
     int count;  // 0: passes A and B work in tiles of cells
 };
 
-// Cells from which a single FP64 mesh takes a face list.  Below, a launch is as
-// long as one thread's chain and several threads per cell shorten it (gather_shape).
-// us per iteration in tiles and with the list: 8k cells 164 and 201, 20k 210 and
-// 217, 34k 249 and 237, 131k 640 and 566, 1.05M 4291 and 3680.
-constexpr int face_list_cells = 24000;
+// Cells above which a single FP64 mesh takes a face list.  Below, a launch is as
+// long as one thread's chain, and the list's extra launch costs more than it saves.
+// us per iteration in tiles and with the list: 8k cells 141 and 152, 12.8k 158 and
+// 152, 20k 186 and 185, 34k 220 and 207, 80k 436 and 353, 252k 1059 and 907.
+constexpr int face_list_cells = 12000;
 
 // Everything one iteration needs.
 template <typename T> struct Plan {

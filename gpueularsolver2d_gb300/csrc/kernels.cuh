@@ -112,18 +112,15 @@ __device__ __forceinline__ float fsqrt(float x) {
 template <typename T> __device__ __forceinline__ T fdiv(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ float fdiv<float>(float a, float b) { return a * frcp(b); }
 template <> __device__ __forceinline__ double fdiv<double>(double a, double b) { return ddiv(a, b); }
-// The same with several numerators over one divisor.
-template <typename T> struct Over;
-template <> struct Over<float> {
-    float r;
-    __device__ __forceinline__ explicit Over(float b) : r(frcp(b)) {}
-    __device__ __forceinline__ float operator()(float a) const { return a * r; }
+// The same with several numerators over one divisor.  FP64: FastOps, whose user
+// does its formula again with IeeeOps where an operand was out of range.
+struct Ops32 {
+    __device__ __forceinline__ float over(float b) { return frcp(b); }
+    __device__ __forceinline__ float by(float a, float r) { return a * r; }
 };
-template <> struct Over<double> {
-    Divisor d;
-    __device__ __forceinline__ explicit Over(double b) : d(divisor(b)) {}
-    __device__ __forceinline__ double operator()(double a) const { return div_by(a, d); }
-};
+template <typename T> struct OpsFor { typedef Ops32 type; };
+template <> struct OpsFor<double> { typedef FastOps type; };
+template <typename T> using OpsOf = typename OpsFor<T>::type;
 // Divisions of the boundary ghosts: the compiler's in FP32.
 template <typename T> __device__ __forceinline__ T gdiv(T a, T b) { return a / b; }
 template <> __device__ __forceinline__ double gdiv<double>(double a, double b) { return ddiv(a, b); }
@@ -132,7 +129,11 @@ template <typename T> struct GOver {
     __device__ __forceinline__ explicit GOver(T v) : b(v) {}
     __device__ __forceinline__ T operator()(T a) const { return a / b; }
 };
-template <> struct GOver<double> : Over<double> { using Over<double>::Over; };
+template <> struct GOver<double> {
+    Divisor d;
+    __device__ __forceinline__ explicit GOver(double v) : d(divisor(v)) {}
+    __device__ __forceinline__ double operator()(double a) const { return div_by(a, d); }
+};
 
 template <typename T> __device__ __forceinline__ T comp(const V4<T> &v, int k) {
     return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
@@ -265,22 +266,31 @@ __device__ __forceinline__ V4<T> ghost(int code, const V4<T> &U, T Sx, T Sy, con
 // additions and multiplications where the reference's form issues about 30.
 template <typename T> __device__ T spectral_radius(const V4<T> &a, const V4<T> &b, T vectorx, T vectory, T g);
 // FP64, with the face vector's square q given.
-__device__ __forceinline__ double spectral_radius64(const V4<double> &a, const V4<double> &b, double vectorx,
+template <class O>
+__device__ __forceinline__ double spectral_radius64(O &o, const V4<double> &a, const V4<double> &b, double vectorx,
                                                     double vectory, double q, double g) {
     const double rou2 = a.x + b.x;  // 2 rou
-    const Divisor d = divisor(rou2);
-    const double u = div_by(a.y + b.y, d);
-    const double v = div_by(a.z + b.z, d);
-    const double EE = fma(-0.5, u * u + v * v, div_by(a.w + b.w, d));
+    const auto d = o.over(rou2);
+    const double u = o.by(a.y + b.y, d);
+    const double v = o.by(a.z + b.z, d);
+    const double EE = fma(-0.5, u * u + v * v, o.by(a.w + b.w, d));
     const double VC = u * vectory + v * vectorx;
     const double p2 = rou2 * EE * (g - 1.0);  // 2 p
-    const double CS = dsqrt(div_by(g * p2, d) * q);
+    const double CS = o.sqrt(o.by(g * p2, d) * q);
     return tabs(VC) + CS;
+}
+static __device__ __noinline__ double spectral_radius_ieee(const V4<double> a, const V4<double> b, double vectorx,
+                                                           double vectory, double q, double g) {
+    IeeeOps o;
+    return spectral_radius64(o, a, b, vectorx, vectory, q, g);
 }
 template <>
 __device__ __forceinline__ double spectral_radius<double>(const V4<double> &a, const V4<double> &b, double vectorx,
                                                          double vectory, double g) {
-    return spectral_radius64(a, b, vectorx, vectory, vectorx * vectorx + vectory * vectory, g);
+    FastOps o;
+    const double q = vectorx * vectorx + vectory * vectory;
+    const double r = spectral_radius64(o, a, b, vectorx, vectory, q, g);
+    return o.bad ? spectral_radius_ieee(a, b, vectorx, vectory, q, g) : r;
 }
 
 // FP32: the same quantity with one reciprocal and fused multiply-adds.
@@ -305,69 +315,71 @@ __device__ V4<T> roe(const V4<T> &LW, const V4<T> &RW, T nx, T ny, T g, T epsilo
 
 // |v| of the Harten fix (gpu_solver.cu:603-616): (v^2 + eps^2) / (2 eps) below
 // eps.
-__device__ __forceinline__ double harten(const double v, const double epsilon) {
+template <class O> __device__ __forceinline__ double harten(O &o, const double v, const double epsilon) {
     if (!abs_less(v, epsilon)) return fabs(v);
-    return ddiv(v * v + epsilon * epsilon, 2.0 * epsilon);
+    return o.div(v * v + epsilon * epsilon, 2.0 * epsilon);
 }
 
-// A product on the FP64 pipe or (INT) the integer units, the same bits.  On
-// meshes that fill the GPU the FP64 pipe is the bound and the integer units have
-// most of their issue slots left: 48 of pass B's 78 products and half of pass A's
-// run there (1.05M cells: pass B 608 -> 525 us, with two thirds of the rest too 557; pass A 435 -> 402,
-// with a third more 425).  On small meshes a launch is as long as one thread's
-// chain, which forty instructions for one only lengthen (2k cells: pass B 22 -> 27).
-template <bool INT> __device__ __forceinline__ double mul(double a, double b) {
-    if constexpr (INT) return imul(a, b);
-    else return a * b;
+__device__ __forceinline__ double twice(double b) { return 2.0 * b; }
+__device__ __forceinline__ Divisor twice(Divisor d) {  // (exponent 2046 becomes one that is not prepared)
+    d.b = 2.0 * d.b;
+    d.e = d.e ? d.e + 1 : 0;
+    return d;
 }
 
+// Which products go to the integer units (IM, o.mul): on meshes that fill the GPU
+// the FP64 pipe is the bound (81 % busy is the most seen) and the integer units
+// have most of their issue slots left.  us per launch at 1.05M cells: pass A with
+// none / 12 / 24 / 36 of its 68 there 281 / 261 / 256 / 261, the flux and the radii
+// with 42 / 48 / 52 of the flux's 78: 406 / 413 / 419, pass C with none / 1 / 2 of 4:
+// 45 / 43 / 41.  On small meshes a launch is as long as one thread's chain, which
+// forty instructions for one only lengthen (8k cells: pass B 19 -> 24).
 // FP64: the reference's operations in its order (calc_function,
 // gpu_solver.cu:552-566, and the flux), times the face length 2 hv.  Powers of two
 // move through the roundings: x - 0.5 y is one fused multiply-add (its product
 // is exact), 2 AB AB is twice AB AB and shares its divisor, and the flux's
 // factor 0.5 goes into the face length.
-template <bool IM>
-__device__ __forceinline__ V4<double> roe_scaled(const V4<double> &LW, const V4<double> &RW, const double nx,
+// IM: some of the products (o.mul) on the integer units.
+template <bool IM, class O>
+__device__ __forceinline__ V4<double> roe_scaled(O &o, const V4<double> &LW, const V4<double> &RW, const double nx,
                                                 const double ny, const double g, const double epsilon,
                                                 const double hv) {
     const double gm1 = g - 1.0;
-    const double t0 = ddiv(1.0, LW.x), t1 = ddiv(1.0, RW.x);
-    const double U0 = mul<IM>(LW.y, t0), V0 = mul<IM>(LW.z, t0), e0 = mul<IM>(LW.w, t0);
-    const double U1 = mul<IM>(RW.y, t1), V1 = mul<IM>(RW.z, t1), e1 = mul<IM>(RW.w, t1);
-    const double P0 = mul<IM>(gm1, LW.x) * fma(-0.5, mul<IM>(U0, U0) + V0 * V0, e0);
-    const double P1 = mul<IM>(gm1, RW.x) * fma(-0.5, mul<IM>(U1, U1) + V1 * V1, e1);
-    const double H0 = e0 + mul<IM>(P0, t0), H1 = e1 + mul<IM>(P1, t1);
-    const double M0 = mul<IM>(U0, nx) + V0 * ny, M1 = mul<IM>(U1, nx) + V1 * ny;
+    const double t0 = o.div(1.0, LW.x), t1 = o.div(1.0, RW.x);
+    const double U0 = o.template mul<IM>(LW.y, t0), V0 = o.template mul<IM>(LW.z, t0), e0 = o.template mul<IM>(LW.w, t0);
+    const double U1 = o.template mul<IM>(RW.y, t1), V1 = o.template mul<IM>(RW.z, t1), e1 = o.template mul<IM>(RW.w, t1);
+    const double P0 = o.template mul<IM>(gm1, LW.x) * fma(-0.5, o.template mul<IM>(U0, U0) + V0 * V0, e0);
+    const double P1 = o.template mul<IM>(gm1, RW.x) * fma(-0.5, o.template mul<IM>(U1, U1) + V1 * V1, e1);
+    const double H0 = e0 + o.template mul<IM>(P0, t0), H1 = e1 + o.template mul<IM>(P1, t1);
+    const double M0 = o.template mul<IM>(U0, nx) + V0 * ny, M1 = o.template mul<IM>(U1, nx) + V1 * ny;
     const double DVC = M1 - M0;
-    const double sl = dsqrt(LW.x), sr = dsqrt(RW.x);
-    const double ROUB = mul<IM>(sl, sr);
-    const Divisor ds = divisor(sl + sr);
-    const double UB = div_by(mul<IM>(U0, sl) + U1 * sr, ds);
-    const double VB = div_by(mul<IM>(V0, sl) + V1 * sr, ds);
-    const double HB = div_by(mul<IM>(H0, sl) + H1 * sr, ds);
-    const double QB = mul<IM>(UB, UB) + VB * VB;
-    const double AB = dsqrt(gm1 * fma(-0.5, QB, HB));
-    const double VC = mul<IM>(UB, nx) + VB * ny;
-    const double AD0 = harten(VC - AB, epsilon), AD1 = harten(VC, epsilon), AD2 = harten(VC + AB, epsilon);
-    const double dP = P1 - P0, RAD = mul<IM>(ROUB, AB) * DVC;
-    const Divisor da = divisor(mul<IM>(AB, AB));
-    Divisor da2 = da;
-    da2.b = 2.0 * da.b;
-    da2.e = da.e ? da.e + 1 : 0;
-    const double F00 = div_by(mul<IM>(AD0, dP - RAD), da2);
-    const double F20 = div_by(mul<IM>(AD2, dP + RAD), da2);
-    const double F10 = AD1 * ((RW.x - LW.x) - div_by(dP, da));
-    const double anx = mul<IM>(AB, nx), any = mul<IM>(AB, ny), avc = mul<IM>(AB, VC);
-    const double dU = U1 - U0, dV = V1 - V0, aR = mul<IM>(AD1, ROUB);
-    const double F11 = mul<IM>(F10, UB) + aR * (dU - mul<IM>(DVC, nx));
-    const double F12 = mul<IM>(F10, VB) + aR * (dV - mul<IM>(DVC, ny));
-    const double F13 = fma(mul<IM>(F10, QB), 0.5, aR * (mul<IM>(UB, dU) + VB * dV - mul<IM>(DVC, VC)));
-    const double WL0 = mul<IM>(LW.x, M0), WR0 = mul<IM>(RW.x, M1);
+    const double sl = o.sqrt(LW.x), sr = o.sqrt(RW.x);
+    const double ROUB = o.template mul<IM>(sl, sr);
+    const auto ds = o.over(sl + sr);
+    const double UB = o.by(U0 * sl + U1 * sr, ds);
+    const double VB = o.by(V0 * sl + V1 * sr, ds);
+    const double HB = o.by(H0 * sl + H1 * sr, ds);
+    const double QB = o.template mul<IM>(UB, UB) + VB * VB;
+    const double AB = o.sqrt(gm1 * fma(-0.5, QB, HB));
+    const double VC = o.template mul<IM>(UB, nx) + VB * ny;
+    const double AD0 = harten(o, VC - AB, epsilon), AD1 = harten(o, VC, epsilon), AD2 = harten(o, VC + AB, epsilon);
+    const double dP = P1 - P0, RAD = o.template mul<IM>(ROUB, AB) * DVC;
+    const double a2 = o.template mul<IM>(AB, AB);
+    const auto da = o.over(a2), da2 = twice(da);
+    const double F00 = o.by(o.template mul<IM>(AD0, dP - RAD), da2);
+    const double F20 = o.by(o.template mul<IM>(AD2, dP + RAD), da2);
+    const double F10 = AD1 * ((RW.x - LW.x) - o.by(dP, da));
+    const double anx = o.template mul<IM>(AB, nx), any = o.template mul<IM>(AB, ny), avc = o.template mul<IM>(AB, VC);
+    const double dU = U1 - U0, dV = V1 - V0, aR = o.template mul<IM>(AD1, ROUB);
+    const double F11 = o.template mul<IM>(F10, UB) + aR * (dU - o.template mul<IM>(DVC, nx));
+    const double F12 = o.template mul<IM>(F10, VB) + aR * (dV - o.template mul<IM>(DVC, ny));
+    const double F13 = fma(o.template mul<IM>(F10, QB), 0.5, aR * (o.template mul<IM>(UB, dU) + VB * dV - o.template mul<IM>(DVC, VC)));
+    const double WL0 = o.template mul<IM>(LW.x, M0), WR0 = o.template mul<IM>(RW.x, M1);
     V4<double> F;
     F.x = ((WL0 + WR0) - (F00 + F10 + F20)) * hv;
-    F.y = ((mul<IM>(U0, WL0) + mul<IM>(nx, P0)) + (mul<IM>(U1, WR0) + nx * P1) - (mul<IM>(F00, UB - anx) + F11 + F20 * (UB + anx))) * hv;
-    F.z = ((mul<IM>(V0, WL0) + mul<IM>(ny, P0)) + (mul<IM>(V1, WR0) + ny * P1) - (mul<IM>(F00, VB - any) + F12 + F20 * (VB + any))) * hv;
-    F.w = ((mul<IM>(WL0, H0) + mul<IM>(WR0, H1)) - (mul<IM>(F00, HB - avc) + F13 + F20 * (HB + avc))) * hv;
+    F.y = ((o.template mul<IM>(U0, WL0) + o.template mul<IM>(nx, P0)) + (o.template mul<IM>(U1, WR0) + nx * P1) - (F00 * (UB - anx) + F11 + F20 * (UB + anx))) * hv;
+    F.z = ((o.template mul<IM>(V0, WL0) + o.template mul<IM>(ny, P0)) + (o.template mul<IM>(V1, WR0) + ny * P1) - (F00 * (VB - any) + F12 + F20 * (VB + any))) * hv;
+    F.w = ((o.template mul<IM>(WL0, H0) + o.template mul<IM>(WR0, H1)) - (F00 * (HB - avc) + F13 + F20 * (HB + avc))) * hv;
     return F;
 }
 
@@ -721,15 +733,18 @@ __device__ __forceinline__ double2 cell_bounds(const double c0, const double c1,
 // has delt2's sign, so a correctly rounded quotient of |bound| >= |delt2| is
 // >= 1 and only smaller bounds divide.  Kind 1, the Venkatakrishnan form with
 // its doubled products as exact fused multiply-adds.
-__device__ __forceinline__ double face_limiter64(const int kind, const double e2, const double2 bnd,
+template <class O>
+__device__ __forceinline__ double face_limiter64(O &o, const int kind, const double e2, const double2 bnd,
                                                  const double delt2) {
     const double d1 = (int64_t)bits_of(delt2) > 0 ? bnd.x : bnd.y;
     if (kind == 1) {
         if (delt2 == 0.0) return 1.0;
         const double q = d1 * d1, p = delt2 * d1;
-        return ddiv(fma(2.0, p, q + e2), fma(2.0, delt2 * delt2, q) + p + e2);
+        return o.div(fma(2.0, p, q + e2), fma(2.0, delt2 * delt2, q) + p + e2);
     }
-    return abs_less(d1, delt2) ? ddiv(d1, delt2) : 1.0;
+    const bool need = abs_less(d1, delt2);  // else a quotient of at least 1 (or of 0 by 0)
+    const double q = o.div(d1, need ? delt2 : 1.0);
+    return need ? q : 1.0;
 }
 
 // The face states of the FP64 form of faces_cell, by LPC lanes per cell: lane part
@@ -739,9 +754,9 @@ __device__ __forceinline__ double face_limiter64(const int kind, const double e2
 // first term of a sum is not added to zero, the bounds are subtracted once per
 // component and divisions, comparisons and selections run on the integer units.
 // gs: the ghost states of the cell's boundary faces, gstep apart.
-// IM: half of the products on the integer units (mul).
-template <bool OPT, int LPC, bool IM = (LPC < 4)>
-__device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
+// IM: 24 of the 68 products on the integer units (see roe_scaled).
+template <bool OPT, int LPC, bool IM, class O>
+__device__ __forceinline__ void faces_cell64(O &o, const MeshDev<double> &m, const Flow<double> &f, const int i,
                                                const int part, const V4<double> *__restrict__ W,
                                                V4<double> *FS, V4<double> *__restrict__ phi, const int frozen,
                                                const bool first, const V4<double> *__restrict__ Uc, const int4 tp,
@@ -759,23 +774,25 @@ __device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flo
 #pragma unroll
         for (int q = 0; q < NQ; q++) d[q] = v[q];
     };
-    V2<double> S[3];
+    V2<double> h[3];  // halves of the face vectors
     double u[NQ], nb[3][NQ];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        S[k] = m.S[k * n + i];
+        const V2<double> S = m.S[k * n + i];
+        h[k].x = o.half(S.x);
+        h[k].y = o.half(S.y);
         values(code[k] >= 0 ? W + (code[k] >> 3) : gs + k * gstep, nb[k]);
     }
     values(Uc, u);
     const double A = m.area[i];
-    const double rA = ddiv(1.0, A);
+    const double rA = o.div(1.0, A);
     double gx[NQ], gy[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const double s = u[q] + nb[k][q];
-            const double px = mul<IM>(s, 0.5 * S[k].x), py = s * (0.5 * S[k].y);
+            const double px = o.template mul<IM>(s, h[k].x), py = s * h[k].y;
             gx[q] = k == 0 ? px : gx[q] + px;
             gy[q] = k == 0 ? py : gy[q] + py;
         }
@@ -789,7 +806,7 @@ __device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flo
         for (int q = 0; q < NQ; q++) bnd[q] = cell_bounds(nb[0][q], nb[1][q], nb[2][q], u[q]);
     }
     const int kind = OPT ? f.limiter & 1 : 0;
-    const double e2 = OPT && kind == 1 && !reuse ? f.venk_k3 * A * dsqrt(A) : 0.0;
+    const double e2 = OPT && kind == 1 && !reuse ? f.venk_k3 * A * o.sqrt(A) : 0.0;
     // cell-wise limiter options (2, 3): see limits32
     const bool cellwise = OPT && f.limiter >= 2;
     double phic[NQ];
@@ -802,37 +819,60 @@ __device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flo
             const V2<double> r = m.R[k * n + i];
 #pragma unroll
             for (int q = 0; q < NQ; q++)
-                phic[q] = fmin(phic[q], face_limiter64(kind, e2, bnd[q], mul<IM>(gx[q], r.x) + gy[q] * r.y));
+                phic[q] = fmin(phic[q], face_limiter64(o, kind, e2, bnd[q], o.template mul<IM>(gx[q], r.x) + gy[q] * r.y));
         }
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         double d[NQ];
-        if (code[k] >= 0 && !(OPT && first)) {
+        if (!(OPT && first)) {
             const V2<double> r = m.R[k * n + i];
             double ph[NQ];
             if (reuse) values(phi + k * n + i, ph);
 #pragma unroll
             for (int q = 0; q < NQ; q++) {
-                const double delt2 = mul<IM>(gx[q], r.x) + gy[q] * r.y;
+                const double delt2 = o.template mul<IM>(gx[q], r.x) + gy[q] * r.y;
                 if (cellwise && !reuse) ph[q] = phic[q];
-                else if (!reuse) ph[q] = face_limiter64(kind, e2, bnd[q], delt2);
+                else if (!reuse) ph[q] = face_limiter64(o, kind, e2, bnd[q], delt2);
                 d[q] = delt2 * ph[q] + u[q];
             }
             if constexpr (OPT && LPC == 1)
                 if (f.positivity) {
                     // positivity fallback (option): see face_state32
-                    const double q = ddiv(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
+                    const double q = o.div(0.5 * (d[1] * d[1] + d[2] * d[2]), d[0]);
                     if (!(d[0] > 0.0) || !((f.gamma - 1.0) * (d[3] - q) > 0.0))
                         for (int c = 0; c < 4; c++) d[c] = u[c];
                 }
-            if (OPT && phi && !frozen) store(phi + k * n + i, ph);
-        } else {  // a boundary face's place takes the ghost (for pass B)
+            if (OPT && phi && !frozen && code[k] >= 0) store(phi + k * n + i, ph);
+        } else {
 #pragma unroll
-            for (int q = 0; q < NQ; q++) d[q] = code[k] < 0 ? nb[k][q] : u[q];
+            for (int q = 0; q < NQ; q++) d[q] = u[q];
         }
+        // a boundary face's place takes the ghost (for pass B)
+#pragma unroll
+        for (int q = 0; q < NQ; q++) d[q] = code[k] < 0 ? nb[k][q] : d[q];
         store(FS + k * n + i, d);
     }
+}
+
+template <bool OPT, int LPC>
+static __device__ __noinline__ void faces_cell64_ieee(const MeshDev<double> m, const Flow<double> f, const int i,
+                                                      const int part, const V4<double> *W, V4<double> *FS,
+                                                      V4<double> *phi, const int frozen, const bool first,
+                                                      const V4<double> *Uc, const int4 tp, const V4<double> *gs,
+                                                      const int gstep) {
+    IeeeOps o;
+    faces_cell64<OPT, LPC, false>(o, m, f, i, part, W, FS, phi, frozen, first, Uc, tp, gs, gstep);
+}
+template <bool OPT, int LPC, bool IM = (LPC < 4)>
+__device__ __forceinline__ void faces_cell64(const MeshDev<double> &m, const Flow<double> &f, const int i,
+                                             const int part, const V4<double> *__restrict__ W, V4<double> *FS,
+                                             V4<double> *__restrict__ phi, const int frozen, const bool first,
+                                             const V4<double> *__restrict__ Uc, const int4 tp, const V4<double> *gs,
+                                             const int gstep) {
+    FastOps o;
+    faces_cell64<OPT, LPC, IM>(o, m, f, i, part, W, FS, phi, frozen, first, Uc, tp, gs, gstep);
+    if (o.bad) faces_cell64_ieee<OPT, LPC>(m, f, i, part, W, FS, phi, frozen, first, Uc, tp, gs, gstep);
 }
 
 // Local time step of a cell from the sum of its faces' spectral radii.
@@ -852,7 +892,7 @@ __device__ __forceinline__ double local_dt(const MeshDev<double> &m, const Flow<
 // cells of a face hold exactly negated face vectors, so each cell gets the bits
 // of its own evaluation.  Returns the cell's time step (+inf for other lanes).
 // LPC 2 and 4 shorten the chain of a thread where a mesh leaves the GPU's
-// schedulers with few warps (gather_shape).
+// schedulers with few warps (faces_lanes).
 struct FacesSmem {
     V4<double> *Us, *Gs;    // [cells] states, [3 cells] ghost states
     double *SRs;            // [3 cells] spectral radii
@@ -983,18 +1023,17 @@ __global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<d
     if (OPT && f.global_dt) block_min_dt(v, &ctl->dtmin[st]);
 }
 
-// FP64 with a face list: the face states only, one cell per thread without tiles;
+// FP64 with a face list: the face states only, LPC threads per cell without tiles;
 // the radii are taken with the fluxes (k_face_flux) and the steps with their sums.
-template <bool OPT>
+template <bool OPT, int LPC>
 __global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<double> f,
                                                         const V4<double> *__restrict__ W, V4<double> *FS,
                                                         const Ctl *__restrict__ ctl, V4<double> *__restrict__ phi) {
     wait_prior_grid();
     if (ctl->halt) return;
-    const int n = m.n, i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int4 tp = m.topo[i];
-    if ((tp.x | tp.y | tp.z) < 0) {
+    const int n = m.n, t = blockIdx.x * blockDim.x + threadIdx.x, i = t / LPC, part = t % LPC;
+    const int4 tp = i < n ? m.topo[i] : make_int4(0, 0, 0, 0);
+    if ((tp.x | tp.y | tp.z) < 0 && part == 0) {
 #pragma unroll 1
         for (int k = 0; k < 3; k++) {
             const int c = k == 0 ? tp.x : k == 1 ? tp.y : tp.z;
@@ -1002,8 +1041,10 @@ __global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<
             if (c < 0) FS[k * n + i] = ghost(c, W[i], S.x, S.y, f);
         }
     }
-    faces_cell64<OPT, 1>(m, f, i, 0, W, FS, phi, OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order,
-                         W + i, tp, FS + i, n);
+    if (LPC > 1) __syncwarp();  // the cell's other threads read the ghosts
+    if (i >= n) return;
+    faces_cell64<OPT, LPC>(m, f, i, part, W, FS, phi, OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order,
+                           W + i, tp, FS + i, n);
 }
 
 // FP32.  OPT: the variant with the scheme options (smooth limiter, limiter
@@ -1026,15 +1067,16 @@ __global__ void __launch_bounds__(256, OPT ? kOptBlocks : MinBlocks<T>::faces) k
     block_min_dt(v, &ctl->dtmin[st]);
 }
 
-// The pass-A kernel of a precision.
-template <typename T> auto faces_kernel(bool opt, int lanes) {
-    if constexpr (sizeof(T) == 8) {
-        if (lanes == 4) return opt ? &k_faces_tile<true, 4> : &k_faces_tile<false, 4>;
-        if (lanes == 2) return opt ? &k_faces_tile<true, 2> : &k_faces_tile<false, 2>;
-        return opt ? &k_faces_tile<true, 1> : &k_faces_tile<false, 1>;
-    } else {
-        return opt ? &k_faces<T, true> : &k_faces<T, false>;
-    }
+// The FP64 pass-A kernel, in tiles and with a face list.
+inline auto faces_tile_kernel(bool opt, int lanes) {
+    if (lanes == 4) return opt ? &k_faces_tile<true, 4> : &k_faces_tile<false, 4>;
+    if (lanes == 2) return opt ? &k_faces_tile<true, 2> : &k_faces_tile<false, 2>;
+    return opt ? &k_faces_tile<true, 1> : &k_faces_tile<false, 1>;
+}
+inline auto faces_cells_kernel(bool opt, int lanes) {
+    if (lanes == 4) return opt ? &k_faces_cells<true, 4> : &k_faces_cells<false, 4>;
+    if (lanes == 2) return opt ? &k_faces_cells<true, 2> : &k_faces_cells<false, 2>;
+    return opt ? &k_faces_cells<true, 1> : &k_faces_cells<false, 1>;
 }
 
 // True when a pass-A launch needs the option variant.
@@ -1097,13 +1139,14 @@ __device__ __forceinline__ void flux_cell(const MeshDev<T> &m, const Flow<T> &f,
 // Length vn of the face vector S and the unit normal S / vn: IEEE in FP64; in
 // FP32 from one reciprocal square root of |S|^2 (the other cell of the face,
 // with S negated, gets the exact negative).
-template <typename T> __device__ __forceinline__ void unit_normal(const V2<T> S, T &nx, T &ny, T &vn) {
-    vn = tsqrt(S.y * S.y + S.x * S.x);
-    const Over<T> by(vn);
-    nx = by(S.x);
-    ny = by(S.y);
+template <class O>
+__device__ __forceinline__ void unit_normal(O &o, const V2<double> S, double &nx, double &ny, double &vn) {
+    vn = o.sqrt(S.y * S.y + S.x * S.x);
+    const auto by = o.over(vn);
+    nx = o.by(S.x, by);
+    ny = o.by(S.y, by);
 }
-template <> __device__ __forceinline__ void unit_normal<float>(const V2<float> S, float &nx, float &ny, float &vn) {
+__device__ __forceinline__ void unit_normal(Ops32 &, const V2<float> S, float &nx, float &ny, float &vn) {
     const float q = fmaf(S.y, S.y, S.x * S.x), r = frsqrt(q);
     vn = q * r;
     const float2 nn = __fmul2_rn(make_float2(S.x, S.y), make_float2(r, r));
@@ -1115,10 +1158,10 @@ template <> __device__ __forceinline__ void unit_normal<float>(const V2<float> S
 // right state b (oth: the neighbour's side, the ghost of a boundary face), unit normal (nx, ny) of
 // the edge and the face length vn; *right tells whether the cell is the
 // edge's right cell.
-template <typename T>
-__device__ __forceinline__ void face_inputs(const int code, const V2<T> S, const V4<T> own, const V4<T> oth, V4<T> &a,
+template <typename T, class O>
+__device__ __forceinline__ void face_inputs(O &o, const int code, const V2<T> S, const V4<T> own, const V4<T> oth, V4<T> &a,
                                             V4<T> &b, T &nx, T &ny, T &vn, bool &right) {
-    unit_normal(S, nx, ny, vn);
+    unit_normal(o, S, nx, ny, vn);
     // the left state first: both cells of a face run the same instructions on
     // the same inputs (their normals are exact negatives), so they get the
     // same bits
@@ -1131,34 +1174,40 @@ __device__ __forceinline__ void face_inputs(const int code, const V2<T> S, const
 // Flux of face k of cell i, times |S|, in the edge's orientation (the
 // reference's Res_e.left of gpu_solver.cu:738-745); *right tells whether cell
 // i is the edge's right cell.
-template <typename T, bool IM = false>
-__device__ __forceinline__ V4<T> face_flux_of(const Flow<T> &f, const int code, const V2<T> S, const V4<T> own,
-                                              const V4<T> oth, bool &right) {
-    V4<T> a, b;
-    T nx, ny, vn;
-    face_inputs(code, S, own, oth, a, b, nx, ny, vn, right);
-    // one Roe call site for every face
-    if constexpr (sizeof(T) == 4) {
-        V4<T> F = roe(a, b, nx, ny, f.gamma, f.eps_entropy);
-        // two packed multiplies, the same products
-        const float2 xy = __fmul2_rn(make_float2(F.x, F.y), make_float2(vn, vn));
-        const float2 zw = __fmul2_rn(make_float2(F.z, F.w), make_float2(vn, vn));
-        F.x = xy.x; F.y = xy.y; F.z = zw.x; F.w = zw.y;
-        return F;
-    } else {
-        return roe_scaled<IM>(a, b, nx, ny, f.gamma, f.eps_entropy, 0.5 * vn);
-    }
+__device__ __forceinline__ V4<float> face_flux_of(const Flow<float> &f, const int code, const V2<float> S,
+                                                  const V4<float> own, const V4<float> oth, bool &right) {
+    Ops32 o;
+    V4<float> a, b;
+    float nx, ny, vn;
+    face_inputs(o, code, S, own, oth, a, b, nx, ny, vn, right);
+    V4<float> F = roe(a, b, nx, ny, f.gamma, f.eps_entropy);
+    // two packed multiplies, the same products
+    const float2 xy = __fmul2_rn(make_float2(F.x, F.y), make_float2(vn, vn));
+    const float2 zw = __fmul2_rn(make_float2(F.z, F.w), make_float2(vn, vn));
+    F.x = xy.x; F.y = xy.y; F.z = zw.x; F.w = zw.y;
+    return F;
 }
 
-template <typename T, bool IM>
-__device__ __forceinline__ V4<T> face_flux(const MeshDev<T> &m, const Flow<T> &f, const int i, const int k,
-                                           const int code, const V4<T> *__restrict__ W,
-                                           const V4<T> *__restrict__ FS, bool &right) {
+// The same in FP64, from global memory.
+template <bool IM, class O>
+__device__ __forceinline__ V4<double> face_flux64(O &o, const MeshDev<double> &m, const Flow<double> &f, const int i,
+                                                  const int k, const int code, const V4<double> *W,
+                                                  const V4<double> *FS) {
     const int n = m.n;
-    const V2<T> S = m.S[k * n + i];
-    const V4<T> own = code >= 0 ? FS[k * n + i] : W[i];
-    const V4<T> oth = code >= 0 ? FS[(code & 3) * n + (code >> 3)] : FS[k * n + i];
-    return face_flux_of<T, IM>(f, code, S, own, oth, right);
+    const V2<double> S = m.S[k * n + i];
+    const V4<double> own = code >= 0 ? FS[k * n + i] : W[i];
+    const V4<double> oth = code >= 0 ? FS[(code & 3) * n + (code >> 3)] : FS[k * n + i];
+    V4<double> a, b;
+    double nx, ny, vn;
+    bool right;
+    face_inputs(o, code, S, own, oth, a, b, nx, ny, vn, right);
+    return roe_scaled<IM>(o, a, b, nx, ny, f.gamma, f.eps_entropy, 0.5 * vn);
+}
+static __device__ __noinline__ V4<double> face_flux_ieee(const MeshDev<double> m, const Flow<double> f, const int i,
+                                                         const int k, const int code, const V4<double> *W,
+                                                         const V4<double> *FS) {
+    IeeeOps o;
+    return face_flux64<false>(o, m, f, i, k, code, W, FS);
 }
 
 // Pass B for one tile of cells [base, base + nvalid) with each interior face
@@ -1216,8 +1265,10 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
         const int it = items[j], tt = it >> 2, k = it & 3;
         const int4 q = tps[tt];
         const int c = k == 0 ? q.x : k == 1 ? q.y : q.z;
-        bool right;
-        Fs[tt * 3 + k] = face_flux<T, IM>(m, f, base + tt, k, c, W, FS, right);
+        FastOps o;
+        V4<T> F = face_flux64<IM>(o, m, f, base + tt, k, c, W, FS);
+        if (o.bad) F = face_flux_ieee(m, f, base + tt, k, c, W, FS);
+        Fs[tt * 3 + k] = F;
     }
     __syncthreads();
     if (!live) return;
@@ -1241,14 +1292,14 @@ __device__ __forceinline__ void flux_tile(const MeshDev<T> &m, const Flow<T> &f,
     res[i] = r;
 }
 
-template <typename T, int R, bool IM>
+template <typename T>
 __global__ void E2D_LB_FLUX k_flux_tile(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ W,
                                         const V4<T> *__restrict__ FS,
                                         V4<T> *__restrict__ res, const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
-    const int tile = blockDim.x / R, base = blockIdx.x * tile;
-    flux_tile<T, R, IM>(m, f, base, min(tile, m.n - base), W, FS, res);
+    const int tile = blockDim.x / 2, base = blockIdx.x * tile;
+    flux_tile<T, 2, false>(m, f, base, min(tile, m.n - base), W, FS, res);
 }
 
 template <typename T>
@@ -1269,31 +1320,53 @@ __global__ void E2D_LB_FLUX k_flux(MeshDev<T> m, Flow<T> f, const V4<T> *__restr
 // flux_tile and faces_tile, whose tiles of 128 cells evaluate 1.75 rounds of
 // faces per warp of cells (faces between tiles twice, the last round partly filled)
 // and wait for their slowest warp; this is 1.5, without barriers, and the
-// normals are the list's.  1.05M cells: pass A 401 -> 301 us, pass B 527 -> 480.
+// normals are the list's.  1.05M cells, when it was introduced: pass A 401 ->
+// 301 us, pass B 527 -> 480.
 template <typename T> __global__ void __launch_bounds__(256) k_face_geometry(const V2<T> *__restrict__ S, FaceList l) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= l.count) return;
     const V2<T> v = S[l.at[j].x];
     T nx, ny, vn;
-    unit_normal(v, nx, ny, vn);
+    IeeeOps o;
+    unit_normal(o, v, nx, ny, vn);
     const T g[6] = {nx, ny, 0.5 * vn, v.x, v.y, v.y * v.y + v.x * v.x};
     for (int k = 0; k < 6; k++) l.geo[(size_t)k * l.count + j] = g[k];
 }
 
+template <bool IM, class O>
+__device__ __forceinline__ V4<double> listed_face(O &o, const FaceList &l, const Flow<double> &f, const int j,
+                                                  const int4 at, const V4<double> *W, const V4<double> *FS,
+                                                  double &radius) {
+    const double *g = l.geo + j;
+    const size_t nf = l.count;
+    const bool inner = at.y >= 0;
+    const V4<double> Wa = W[at.z], b = FS[inner ? at.y : at.x], a = inner ? FS[at.x] : Wa;
+    radius = spectral_radius64(o, Wa, inner ? W[at.w] : b, g[4 * nf], g[3 * nf], g[5 * nf], f.gamma);
+    return roe_scaled<IM>(o, a, b, g[0], g[nf], f.gamma, f.eps_entropy, g[2 * nf]);
+}
+static __device__ __noinline__ V4<double> listed_face_ieee(const FaceList l, const Flow<double> f, const int j,
+                                                           const V4<double> *W, const V4<double> *FS) {
+    IeeeOps o;
+    double r;
+    const int4 at = l.at[j];
+    const V4<double> F = listed_face<false>(o, l, f, j, at, W, FS, r);
+    l.radius[at.x] = r;
+    return F;
+}
 template <typename T>
-__global__ void __launch_bounds__(256, 2) k_face_flux(FaceList l, Flow<T> f, const V4<T> *__restrict__ W,
-                                                      V4<T> *FS, const Ctl *__restrict__ ctl) {
+__global__ void __launch_bounds__(256, 2) k_face_flux(FaceList l, Flow<T> f, const V4<T> *__restrict__ W, V4<T> *FS,
+                                                      const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= l.count) return;
     const int4 at = l.at[j];
-    const double *g = l.geo + j;
-    const size_t nf = l.count;
-    const bool inner = at.y >= 0;
-    const V4<T> Wa = W[at.z], b = FS[inner ? at.y : at.x], a = inner ? FS[at.x] : Wa;
-    l.radius[at.x] = spectral_radius64(Wa, inner ? W[at.w] : b, g[4 * nf], g[3 * nf], g[5 * nf], f.gamma);
-    FS[at.x] = roe_scaled<true>(a, b, g[0], g[nf], f.gamma, f.eps_entropy, g[2 * nf]);
+    FastOps o;
+    T r;
+    V4<T> F = listed_face<true>(o, l, f, j, at, W, FS, r);
+    l.radius[at.x] = r;
+    if (o.bad) F = listed_face_ieee(l, f, j, W, FS);
+    FS[at.x] = F;
 }
 
 template <typename T>
@@ -1323,32 +1396,21 @@ __global__ void __launch_bounds__(256) k_face_sum(MeshDev<T> m, Flow<T> f, const
     if (f.global_dt) block_min_dt(dti, &ctl->dtmin[st]);
 }
 
-// The pass-B kernel of a precision.
-template <typename T> auto flux_kernel(bool im) {
-    if constexpr (FluxTiled<T>::value) {
-        return im ? &k_flux_tile<T, 2, true> : &k_flux_tile<T, 2, false>;
-    } else {
-        return &k_flux<T>;
-    }
-}
-
-// Threads per cell of passes A and B in tiles.  FP32: one.  FP64: a mesh of up to
-// some 40k cells has one or two warps for each of the GPU's 608 schedulers, and a
-// launch takes as long as one thread's chain of some 2500 instructions, so the
-// cell's work is spread over more threads; on large meshes that only repeats
-// loads and the work per cell, and smaller tiles evaluate more faces twice.
-// us per launch with 1 / 2 / 4 threads in pass A and 1 / 2 in pass B (all products on
-// the FP64 pipe; from 12k cells on some leave it, see mul): 2k cells 27 /
-// 20 / 17 and 30 / 21; 8k 31 / 21 / 18 and 33 / 22; 34k (limiter option) 29 / 25 /
-// 29 and 40 / 37; 80k 61 / 54 / 54 and 77 / 79; 131k 72 / 70 / 79 and 100 / 106.
-// Larger meshes take a face list (face_list_cells).  (The positivity option
-// compares a cell's components: one thread.)
-struct Gather {
-    int faces, flux;
-};
-template <typename T> Gather gather_shape(const Plan<T> &p) {
-    if (sizeof(T) == 4) return {1, 1};
-    return {p.f.positivity ? 1 : p.m.n > 12000 ? 2 : 4, 2};
+// Threads per cell of pass A.  FP32: one.  FP64: a mesh of up to some 100k cells
+// has one to five warps for each of the GPU's 608 schedulers, and a launch takes as
+// long as one thread's chain of some 2500 instructions, so the cell's components
+// are spread over more threads; on large meshes that only repeats loads and the
+// work per cell.  us per iteration with 1 / 2 / 4 and a face list: 12.8k cells 177 /
+// 162 / 152, 34k 221 / 207 / 214, 80k 376 / 353 / 362, 131k 497 / 493 / 512 (with the
+// cell-wise limiter 633 / 658 / 668), 252k 908 / 907 / 938.  In tiles (at most
+// 12k cells, and the allocation-free iteration's 33k) four, then two; pass B's
+// tiles are half a block, one thread per listed face (8k: 22 us a launch, 33 with
+// tiles of a block).  (The positivity option compares a cell's components: one.)
+template <typename T> int faces_lanes(const Plan<T> &p) {
+    const int n = p.m.n;
+    if (sizeof(T) == 4 || p.f.positivity) return 1;
+    if (p.faces.count) return n > 100000 ? 1 : n > 16000 ? 2 : 4;
+    return n > 12000 ? 2 : 4;
 }
 
 // Sum of the interior neighbours' values in face order (gpu_solver.cu:1658-1666)
@@ -1370,15 +1432,33 @@ __device__ __forceinline__ V4<T> nb_sum(const int4 tp, const V4<T> *__restrict__
 // ---------------------------------------------------------------------------
 // Pass C: gpu_solver.cu:1635-1673 (kernel_Smooth1): one Jacobi-type sweep
 // dst = (eps * sum_interior src + res) / (1 + eps * CLog).
+template <typename T, class O>
+__device__ __forceinline__ V4<T> smooth_with(O &q, const T eps, const int clog, const V4<T> &d, const V4<T> &r0) {
+    const auto den = q.over(T(1.0) + (eps) * T(clog));
+    V4<T> o;
+    if constexpr (sizeof(T) == 8) {  // two products on each kind of unit (1.05M cells: 45 -> 41 us, pass D 70 -> 67)
+        o.x = q.by(q.template mul<true>(d.x, eps) + r0.x, den);
+        o.y = q.by(q.template mul<true>(d.y, eps) + r0.y, den);
+    } else {
+        o.x = q.by(madd(d.x, eps, r0.x), den);
+        o.y = q.by(madd(d.y, eps, r0.y), den);
+    }
+    o.z = q.by(madd(d.z, eps, r0.z), den);
+    o.w = q.by(madd(d.w, eps, r0.w), den);
+    return o;
+}
+static __device__ __noinline__ V4<double> smooth_ieee(const double eps, const int clog, const V4<double> d,
+                                                      const V4<double> r0) {
+    IeeeOps o;
+    return smooth_with(o, eps, clog, d, r0);
+}
 template <typename T>
 __device__ __forceinline__ V4<T> smooth_value(const T eps, const int clog, const V4<T> &d, const V4<T> &r0) {
-    const Over<T> den(T(1.0) + (eps) * T(clog));
-    V4<T> o;
-    o.x = den(madd(d.x, eps, r0.x));
-    o.y = den(madd(d.y, eps, r0.y));
-    o.z = den(madd(d.z, eps, r0.z));
-    o.w = den(madd(d.w, eps, r0.w));
-    return o;
+    OpsOf<T> o;
+    V4<T> v = smooth_with(o, eps, clog, d, r0);
+    if constexpr (sizeof(T) == 8)
+        if (o.bad) v = smooth_ieee(eps, clog, d, r0);
+    return v;
 }
 
 template <typename T>
@@ -1407,27 +1487,40 @@ __global__ void __launch_bounds__(256) k_smooth(MeshDev<T> m, T eps, const V4<T>
 // The new state from the start state w0, the residual r and (smooth) the sum d of
 // the neighbours' smoothed residuals; want: also rho - rho0 and whether the state
 // is unphysical.
-template <typename T>
-__device__ __forceinline__ V4<T> update_value(const T eps, const T rk, const int smooth, const int clog, V4<T> r,
-                                              const V4<T> &d, const T dti, const T area, const V4<T> &w0,
-                                              const bool want, T &drho, int &bad) {
+template <typename T, class O>
+__device__ __forceinline__ V4<T> update_with(O &o, const T eps, const T rk, const int smooth, const int clog, V4<T> r,
+                                             const V4<T> &d, const T dti, const T area, const V4<T> &w0) {
     if (smooth) {
-        const Over<T> den(T(1.0) + (eps) * T(clog));
-        T s0 = den(madd(d.x, eps, r.x)), s1 = den(madd(d.y, eps, r.y));
-        T s2 = den(madd(d.z, eps, r.z)), s3 = den(madd(d.w, eps, r.w));
-        if (abs_less(s0, r.x)) r.x = s0;
-        if (abs_less(s1, r.y)) r.y = s1;
-        if (abs_less(s2, r.z)) r.z = s2;
-        if (abs_less(s3, r.w)) r.w = s3;
+        const V4<T> s = smooth_with(o, eps, clog, d, r);
+        if (abs_less(s.x, r.x)) r.x = s.x;
+        if (abs_less(s.y, r.y)) r.y = s.y;
+        if (abs_less(s.z, r.z)) r.z = s.z;
+        if (abs_less(s.w, r.w)) r.w = s.w;
     }
     T RK = rk;
     RK *= dti;
-    const Over<T> A(area);
+    const auto A = o.over(area);
     V4<T> w;
-    w.x = w0.x - A(RK * r.x);
-    w.y = w0.y - A(RK * r.y);
-    w.z = w0.z - A(RK * r.z);
-    w.w = w0.w - A(RK * r.w);
+    w.x = w0.x - o.by(RK * r.x, A);
+    w.y = w0.y - o.by(RK * r.y, A);
+    w.z = w0.z - o.by(RK * r.z, A);
+    w.w = w0.w - o.by(RK * r.w, A);
+    return w;
+}
+static __device__ __noinline__ V4<double> update_ieee(const double eps, const double rk, const int smooth,
+                                                      const int clog, const V4<double> r, const V4<double> d,
+                                                      const double dti, const double area, const V4<double> w0) {
+    IeeeOps o;
+    return update_with(o, eps, rk, smooth, clog, r, d, dti, area, w0);
+}
+template <typename T>
+__device__ __forceinline__ V4<T> update_value(const T eps, const T rk, const int smooth, const int clog, const V4<T> &r,
+                                              const V4<T> &d, const T dti, const T area, const V4<T> &w0,
+                                              const bool want, T &drho, int &bad) {
+    OpsOf<T> o;
+    V4<T> w = update_with(o, eps, rk, smooth, clog, r, d, dti, area, w0);
+    if constexpr (sizeof(T) == 8)
+        if (o.bad) w = update_ieee(eps, rk, smooth, clog, r, d, dti, area, w0);
     if (want) {
         // rho - rho0 in the stencil's precision: exact in FP32 as long as the
         // two densities are within a factor of two (Sterbenz)
@@ -1730,33 +1823,33 @@ template <typename T, typename Mark, typename Done>
 void enqueue_passes(const Plan<T> &p, cudaStream_t s, Mark mark, Done done) {
     const int n = p.m.n, B = p.block, G = (n + B - 1) / B;
     const bool opt = faces_options(p.f, p.phi);
-    const Gather ga = gather_shape(p);
-    const auto grid = [&](int lanes) { return (n + B / lanes - 1) / (B / lanes); };
+    const int lanes = faces_lanes(p);
+    const auto grid = [&](int per_cell) { return (n + B / per_cell - 1) / (B / per_cell); };
     for (int st = 0; st < p.stages; st++) {
         const bool last = st == p.stages - 1;
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
         mark(0);
-        if (p.faces.count) {
-            if constexpr (sizeof(T) == 8) {
-                const int GF = (p.faces.count + B - 1) / B;
-                launch_chained(opt ? k_faces_cells<true> : k_faces_cells<false>, G, B, s, p.m, p.f, Wcur, p.FS, p.ctl,
-                               p.phi);
-                done();
-                mark(1);
-                launch_chained(k_face_flux<T>, GF, B, s, p.faces, p.f, Wcur, p.FS, p.ctl);
-                done();
-                mark(1);
-                launch_chained(k_face_sum<T>, G, B, s, p.m, p.f, p.FS, p.faces.radius, p.res, p.dt, p.ctl, st);
-            }
-        } else {
-            launch_chained_smem(faces_kernel<T>(opt, ga.faces), grid(ga.faces), B,
-                                sizeof(T) == 8 ? B / ga.faces * FacesSmem::per_cell : 0, s, p.m, p.f, Wcur, p.FS, p.dt,
-                                p.ctl, p.phi, st);
+        if constexpr (sizeof(T) == 4) {
+            launch_chained(opt ? k_faces<T, true> : k_faces<T, false>, G, B, s, p.m, p.f, Wcur, p.FS, p.dt, p.ctl,
+                           p.phi, st);
             done();
             mark(1);
-            launch_chained(flux_kernel<T>(ga.faces < 4), grid(ga.flux), B, s, p.m, p.f, Wcur, p.FS, p.res,
-                           p.ctl);
+            launch_chained(k_flux<T>, G, B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
+        } else if (p.faces.count) {
+            launch_chained(faces_cells_kernel(opt, lanes), grid(lanes), B, s, p.m, p.f, Wcur, p.FS, p.ctl, p.phi);
+            done();
+            mark(1);
+            launch_chained(k_face_flux<T>, (p.faces.count + B - 1) / B, B, s, p.faces, p.f, Wcur, p.FS, p.ctl);
+            done();
+            mark(1);
+            launch_chained(k_face_sum<T>, G, B, s, p.m, p.f, p.FS, p.faces.radius, p.res, p.dt, p.ctl, st);
+        } else {
+            launch_chained_smem(faces_tile_kernel(opt, lanes), grid(lanes), B, B / lanes * FacesSmem::per_cell, s, p.m,
+                                p.f, Wcur, p.FS, p.dt, p.ctl, p.phi, st);
+            done();
+            mark(1);
+            launch_chained(k_flux_tile<T>, grid(2), B, s, p.m, p.f, Wcur, p.FS, p.res, p.ctl);
         }
         done();
         const V4<T> *src = p.res;

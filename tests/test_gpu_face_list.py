@@ -1,6 +1,7 @@
-"""FP64 meshes above 24000 cells, whose passes A and B work from a list of the
-faces, against the CPU oracle, bit for bit: both sides of the line, block sizes
-from the smallest to the largest, and the options."""
+"""FP64 meshes above 12000 cells, whose passes A and B work from a list of the
+faces, against the CPU oracle, bit for bit: both sides of the line and
+of the changes of threads per cell, block sizes from the smallest to the largest,
+and the options."""
 import numpy as np
 import pytest
 
@@ -21,13 +22,14 @@ def run(oracle, ni, nj, iters, **kw):
     return s
 
 
-@pytest.mark.parametrize("ni,nj,launches", [(120, 100, 17), (157, 77, 21)])
+@pytest.mark.parametrize("ni,nj,launches", [(100, 60, 17), (101, 60, 21), (157, 77, 21), (251, 200, 21)])
 def test_line(lib, oracle, ni, nj, launches):
     assert run(oracle, ni, nj, 3).launches_per_iteration() == launches
 
 
+@pytest.mark.parametrize("ni", [101, 157])
 @pytest.mark.parametrize("kw", [dict(block_size=32), dict(block_size=256), dict(limiter=1), dict(limiter=2),
                                 dict(limiter=3, limiter_freeze=2), dict(positivity_fix=1), dict(global_dt=1),
                                 dict(first_order_iters=2)])
-def test_options(lib, oracle, kw):
-    run(oracle, 157, 77, 4, **kw)
+def test_options(lib, oracle, kw, ni):
+    run(oracle, ni, 77, 4, **kw)
