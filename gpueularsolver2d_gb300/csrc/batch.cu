@@ -46,6 +46,7 @@ struct BatchBase {
     virtual int save_state(cudaStream_t s) = 0;
     virtual int restore_state(cudaStream_t s) = 0;
     virtual const void *topo_ptr() const = 0;
+    virtual void mark_live(cudaStream_t s) = 0;
 };
 
 template <typename T> struct BatchT : BatchBase {
@@ -88,7 +89,7 @@ template <typename T> struct BatchT : BatchBase {
                        2 * Arena::up(sizeof(T) * n) + 6 * Arena::up(sizeof(V4<T>) * n) +
                        Arena::up(sizeof(V4<T>) * 3 * n) * (freeze ? 2 : 1) + Arena::up(sizeof(double) * maxtiles) +
                        Arena::up(sizeof(int) * n) + Arena::up(sizeof(double) * 4 * nmax) +
-                       Arena::up(sizeof(Flow<T>) * ncase) + Arena::up(sizeof(int) * (n / kChunk + 1)) +
+                       Arena::up(sizeof(Flow<T>) * ncase) + 2 * Arena::up(sizeof(int) * (n / kChunk + 1)) +
                        2 * Arena::up(sizeof(int2) * ncase) + Arena::up(sizeof(int) * hw.size()) +
                        Arena::up(sizeof(double) * 4 * wmax);
         CK(cudaMalloc((void **)&arena.base, bytes));
@@ -111,13 +112,15 @@ template <typename T> struct BatchT : BatchBase {
         wfile_dev = (double *)arena.take(sizeof(double) * 4 * nmax);
         Flow<T> *flows = (Flow<T> *)arena.take(sizeof(Flow<T>) * ncase);
         int *chunk_case = (int *)arena.take(sizeof(int) * (n / kChunk + 1));
+        int *live = (int *)arena.take(sizeof(int) * (n / kChunk + 1));
         int *case_end = (int *)arena.take(sizeof(int) * ncase);
         case_tiles = (int2 *)arena.take(sizeof(int2) * ncase);
         wall_dev = (int *)arena.take(sizeof(int) * hw.size());
         wwall_dev = (double *)arena.take(sizeof(double) * 4 * wmax);
         if (!hw.empty()) CK(cudaMemcpy(wall_dev, hw.data(), sizeof(int) * hw.size(), cudaMemcpyHostToDevice));
-        // concatenated mesh (padding cells stay zero and are never touched)
+        // concatenated mesh (padding cells stay zero, -1 in topo's last place, and are never touched)
         std::vector<int32_t> ht(4 * (size_t)n, 0);
+        for (size_t k = 3; k < ht.size(); k += 4) ht[k] = -1;
         std::vector<T> hS(6 * (size_t)n, T(0)), hR(6 * (size_t)n, T(0)), ha(n, T(1));
         std::vector<int> hp(n, 0), hcc(n / kChunk + 1, 0), hce(ncase);
         std::vector<Flow<T>> hf(ncase);
@@ -161,7 +164,7 @@ template <typename T> struct BatchT : BatchBase {
         CK(cudaMemset(plan.W[1], 0, sizeof(V4<T>) * n));
         plan.m = MeshDev<T>{n, topo, S, R, area};
         plan.f = hf[0];
-        plan.b = BatchDev<T>{flows, chunk_case, case_end, ctl};
+        plan.b = BatchDev<T>{flows, chunk_case, live, case_end, ctl};
         plan.ncase = ncase;
         plan.case_tiles = case_tiles;
         plan.hist = hist;
@@ -191,6 +194,9 @@ template <typename T> struct BatchT : BatchBase {
 
     int launches() const override { return launches_per_iteration(plan); }
     const void *topo_ptr() const override { return plan.m.topo; }
+    void mark_live(cudaStream_t s) override {
+        enqueue_batch_live(plan.b.chunk_case, plan.b.live, ntot / kChunk, plan.b.ctl, s);
+    }
 
     int upload_case(int c, const double *w, cudaStream_t s) override {
         const int n = (*L)[c].n, o = (*off)[c];
@@ -303,6 +309,14 @@ int pull_all(e2d_batch *b) {
     return E2D_OK;
 }
 
+// The cases' control blocks to the device, and the chunks' live table after them.
+int push_all(e2d_batch *b) {
+    CK(cudaMemcpyAsync(b->ctl_dev, b->ctl_host, sizeof(Ctl) * b->ncase, cudaMemcpyHostToDevice, b->stream));
+    b->impl->mark_live(b->stream);
+    CK(cudaGetLastError());
+    return E2D_OK;
+}
+
 int sync_hist_all(e2d_batch *b) {
     for (int c = 0; c < b->ncase; c++) {
         const int step = b->ctl_host[c].step, have = (int)b->hist[c].size();
@@ -328,23 +342,22 @@ int run_batch(e2d_batch *b, int n, bool check, double epsl) {
         C.check_epsl = check ? 1 : 0;
         C.epsl = epsl;
     }
-    CK(cudaMemcpyAsync(b->ctl_dev, b->ctl_host, sizeof(Ctl) * b->ncase, cudaMemcpyHostToDevice, b->stream));
+    int rc = push_all(b);
+    if (rc) return rc;
     const int launches = (n + b->graph_iters - 1) / b->graph_iters;
     const int poll = check ? std::max(1, 64 / b->graph_iters) : 0;
     CK(cudaEventRecord(b->ev0, b->stream));
     for (int k = 0; k < launches; k++) {
         CK(cudaGraphLaunch(b->gexec, b->stream));
         if (poll && (k + 1) % poll == 0 && k + 1 < launches) {
-            int rc = pull_all(b);
-            if (rc) return rc;
+            if ((rc = pull_all(b))) return rc;
             bool all = true;
             for (int c = 0; c < b->ncase && all; c++) all = b->ctl_host[c].halt != 0;
             if (all) break;
         }
     }
     CK(cudaEventRecord(b->ev1, b->stream));
-    int rc = pull_all(b);
-    if (rc) return rc;
+    if ((rc = pull_all(b))) return rc;
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
     b->last_ms = ms;
@@ -645,7 +658,7 @@ int e2d_batch_autotune(e2d_batch *b, const char *cache_path, int32_t iters, int3
                 b->ctl_host[c].check_epsl = 0;
                 b->ctl_host[c].target = 1 << 30;
             }
-            CK(cudaMemcpy(b->ctl_dev, b->ctl_host, sizeof(Ctl) * b->ncase, cudaMemcpyHostToDevice));
+            if ((rc = push_all(b))) return rc;
             CK(cudaGraphLaunch(b->gexec, b->stream));
             const int launches = std::max(1, iters / b->graph_iters);
             CK(cudaEventRecord(b->ev0, b->stream));

@@ -106,6 +106,7 @@ constexpr int kChunk = 256;
 template <typename T> struct BatchDev {
     const Flow<T> *flows;    // [ncase]
     const int *chunk_case;   // [n / kChunk] case of each chunk
+    int *live;               // [n / kChunk] the same, or -1 while the case is halted
     const int *case_end;     // [ncase] one past the last real cell
     Ctl *ctl;                // [ncase]
 };
@@ -141,7 +142,10 @@ template <typename T> void enqueue_batch_iteration(const BPlan<T> &p, cudaStream
 
 // pairs: the partials are float2 pairs (FP32 stencil) rather than doubles.
 void enqueue_batch_resid(double *part, const int2 *case_tiles, int ncase, Ctl *ctl, double *hist,
-                         int hist_cap, bool pairs, cudaStream_t s);
+                         int hist_cap, bool pairs, int *live, int block, cudaStream_t s);
+// The chunks' live table from the cases' halt flags; before the first iteration
+// after the host has set them.
+void enqueue_batch_live(const int *chunk_case, int *live, int nchunk, const Ctl *ctl, cudaStream_t s);
 
 // Enqueue one iteration (all RK stages + the residual) on a stream.
 // Instantiated for double in kernels_f64.cu and for float in kernels_f32.cu.

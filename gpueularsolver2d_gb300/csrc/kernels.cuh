@@ -1638,14 +1638,14 @@ __global__ void __launch_bounds__(256) k_update(MeshDev<T> m, Flow<T> f, T rk, i
 // Batched cases: the same per-cell work as the kernels above, by persistent
 // CTAs that walk the tiles of all cases (tile = blockDim.x consecutive cells,
 // all of one case: cases are padded to kChunk cells and a block has at most
-// kChunk threads).  The tile's case, its halt flag and its flow constants are
-// looked up once per tile (uniform over the block); tiles of halted
-// (converged) cases and padding cells are skipped.  The lookups are a chain of
-// loads, so the cell's face codes are requested beside them.  With a CTA for
-// every tile (LOOP false, the default launch shape) there is no loop to keep
-// values for and pass B has its single-case registers.  60 cases, 1.85M cells: pass A
-// 39.1 -> 38.9 us, B 56.8 -> 49.7, smoothing 21.9 -> 19.5, an iteration 540 -> 508 us;
-// 24 cases of 33k cells with the smooth limiter 281 -> 260 us.
+// kChunk threads).  The tile's case, or that it is halted (converged), is one load
+// beside the cell's face codes, so the cell's gathers wait for no more than in a
+// single case; its flow constants are read beside them, and padding cells have a
+// mark in their face codes.  (With the case, then its halt flag and last cell, read
+// before the gathers an iteration of 60 cases, 1.85M cells, took 507 us; so 453;
+// 24 cases of 33k cells with the smooth limiter 255 -> 241 us.)  With a CTA for every
+// tile (LOOP false, the default launch shape) there is no loop to keep values for
+// and pass B has its single-case registers (540 -> 508 us).
 
 template <typename T, bool OPT, bool LOOP>
 __global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : BatchMinBlocks<T>::faces) kb_faces(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W,
@@ -1655,10 +1655,10 @@ __global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : Batc
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += LOOP ? gridDim.x : ntiles) {
         const int base = t * blockDim.x, i = base + threadIdx.x;
-        int4 tp;  // requested with the lookups, not after them
+        int4 tp;  // requested with the lookup, not after it
         if (sizeof(T) == 4) tp = m.topo[i];
-        const int tc = b.chunk_case[base / kChunk];  // the tile's case
-        if (b.ctl[tc].halt) continue;                // uniform over the block
+        const int tc = b.live[base / kChunk];  // the tile's case
+        if (tc < 0) continue;                  // uniform over the block
         const Flow<T> &f = b.flows[tc];
         double v = __longlong_as_double((long long)kDtNone);
         const int frozen = OPT && phi ? b.ctl[tc].frozen : 0;
@@ -1666,7 +1666,7 @@ __global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : Batc
         if constexpr (sizeof(T) == 8)
             v = faces_tile<OPT, 1>(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, dt, phi,
                                 frozen, first, smem);
-        else if (i < b.case_end[tc])
+        else if (tp.w >= 0)
             v = (double)faces_cell<OPT>(m, f, i, W, FS, dt, phi, frozen, first, tp);
         if (OPT && f.global_dt) block_min_dt(v, &b.ctl[tc].dtmin[st]);  // uniform over the block
     }
@@ -1678,15 +1678,15 @@ __global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlock
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += LOOP ? gridDim.x : ntiles) {
         const int base = t * blockDim.x, i = base + threadIdx.x;
-        int4 tp;  // requested with the lookups, not after them
+        int4 tp;  // requested with the lookup, not after it
         if (!FluxTiled<T>::value) tp = m.topo[i];
-        const int tc = b.chunk_case[base / kChunk];  // every cell of a tile is in one case
-        if (b.ctl[tc].halt) continue;                // uniform over the block
+        const int tc = b.live[base / kChunk];  // every cell of a tile is in one case
+        if (tc < 0) continue;                  // uniform over the block
         const Flow<T> &f = b.flows[tc];
         if constexpr (FluxTiled<T>::value) {
             flux_tile(m, f, base, max(0, min((int)blockDim.x, b.case_end[tc] - base)), W, FS, res);
         } else {
-            if (i < b.case_end[tc]) flux_cell(m, f, i, W, FS, res, tp);
+            if (tp.w >= 0) flux_cell(m, f, i, W, FS, res, tp);
         }
     }
 }
@@ -1698,12 +1698,10 @@ __global__ void __launch_bounds__(256) kb_smooth(MeshDev<T> m, BatchDev<T> b, in
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += LOOP ? gridDim.x : ntiles) {
         const int base = t * blockDim.x, i = base + threadIdx.x;
-        const int4 tp = m.topo[i];  // requested with the lookups, not after them
+        const int4 tp = m.topo[i];  // requested with the lookup, not after it
         const V4<T> r = res[i];
-        const int tc = b.chunk_case[base / kChunk];
-        const int end = b.case_end[tc];
-        if (b.ctl[tc].halt) continue;
-        if (i < end) dst[i] = smooth_value(eps, tp.w, nb_sum(tp, src), r);
+        if (b.live[base / kChunk] < 0) continue;
+        if (tp.w >= 0) dst[i] = smooth_value(eps, tp.w, nb_sum(tp, src), r);
     }
 }
 
@@ -1717,13 +1715,12 @@ __global__ void __launch_bounds__(256) kb_update(MeshDev<T> m, BatchDev<T> b, in
     wait_prior_grid();
     for (int t = blockIdx.x; t < ntiles; t += LOOP ? gridDim.x : ntiles) {
         const int base = t * blockDim.x, i = base + threadIdx.x;
-        const int4 tp = m.topo[i];  // requested with the lookups, not after them
-        const int tc = b.chunk_case[base / kChunk];  // the tile's case
-        const int end = b.case_end[tc];
-        if (b.ctl[tc].halt) continue;  // uniform over the block
+        const int4 tp = m.topo[i];  // requested with the lookup, not after it
+        const int tc = b.live[base / kChunk];  // the tile's case
+        if (tc < 0) continue;                  // uniform over the block
         T drho = T(0.0);
         int bad = 0;
-        if (i < end) {
+        if (tp.w >= 0) {
             V4<T> d = {};
             if (smooth) d = nb_sum(tp, src);
             const T dti = GDT ? stage_dt(b.flows[tc], &b.ctl[tc], st, dt, i) : dt[i];
@@ -1754,7 +1751,7 @@ template <typename T, bool LOOP> void enqueue_batch_passes(const BPlan<T> &p, cu
         launch_chained(p.options ? kb_update<T, true, LOOP> : kb_update<T, false, LOOP>, G, B, s, p.m, p.b, NT,
                        p.rk[st], p.sweeps > 0 ? 1 : 0, src, p.res, p.dt, p.W[0], Wout, last ? p.part : nullptr, st);
     }
-    enqueue_batch_resid(p.part, p.case_tiles, p.ncase, p.b.ctl, p.hist, p.hist_cap, sizeof(T) == 4, s);
+    enqueue_batch_resid(p.part, p.case_tiles, p.ncase, p.b.ctl, p.hist, p.hist_cap, sizeof(T) == 4, p.b.live, B, s);
 }
 
 template <typename T> void enqueue_batch_iteration(const BPlan<T> &p, cudaStream_t s) {

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) k_resid(double *__restrict__ part, int np
 // case gets the bits of its own single-case run.
 template <bool PAIRS>
 __global__ void __launch_bounds__(256) kb_resid(const double *__restrict__ part, const int2 *case_tiles,
-                                                Ctl *ctl, double *hist, int hist_cap) {
+                                                Ctl *ctl, double *hist, int hist_cap, int *live, int block) {
     wait_prior_grid();
     const int c = blockIdx.x;
     if (ctl[c].halt) return;
@@ -83,7 +83,19 @@ __global__ void __launch_bounds__(256) kb_resid(const double *__restrict__ part,
         const double s = block_fold<PAIRS>(p, k0, min(ct.y, k0 + kFoldChunk), sh);
         drou += s;  // every thread keeps the same running sum; thread 0's is used
     }
-    if (threadIdx.x == 0) resid_finish(drou, ctl + c, hist + (size_t)c * hist_cap, hist_cap);
+    __shared__ int halt;
+    if (threadIdx.x == 0) {
+        resid_finish(drou, ctl + c, hist + (size_t)c * hist_cap, hist_cap);
+        halt = ctl[c].halt;
+    }
+    __syncthreads();
+    if (!halt) return;
+    for (int k = threadIdx.x; k < (ct.y * block + kChunk - 1) / kChunk; k += blockDim.x) live[ct.x * block / kChunk + k] = -1;
+}
+
+__global__ void __launch_bounds__(256) kb_live(const int *chunk_case, int *live, int nchunk, const Ctl *ctl) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < nchunk) live[k] = ctl[chunk_case[k]].halt ? -1 : chunk_case[k];
 }
 
 void enqueue_resid(double *part, int nparts, Ctl *ctl, double *hist, int hist_cap, bool pairs, cudaStream_t s) {
@@ -93,9 +105,13 @@ void enqueue_resid(double *part, int nparts, Ctl *ctl, double *hist, int hist_ca
 }
 
 void enqueue_batch_resid(double *part, const int2 *case_tiles, int ncase, Ctl *ctl, double *hist, int hist_cap,
-                         bool pairs, cudaStream_t s) {
-    if (pairs) launch_chained(kb_resid<true>, ncase, 256, s, (const double *)part, case_tiles, ctl, hist, hist_cap);
-    else launch_chained(kb_resid<false>, ncase, 256, s, (const double *)part, case_tiles, ctl, hist, hist_cap);
+                         bool pairs, int *live, int block, cudaStream_t s) {
+    launch_chained(pairs ? kb_resid<true> : kb_resid<false>, ncase, 256, s, (const double *)part, case_tiles, ctl, hist,
+                   hist_cap, live, block);
+}
+
+void enqueue_batch_live(const int *chunk_case, int *live, int nchunk, const Ctl *ctl, cudaStream_t s) {
+    kb_live<<<(nchunk + 255) / 256, 256, 0, s>>>(chunk_case, live, nchunk, ctl);
 }
 
 }  // namespace e2d
