@@ -294,7 +294,7 @@ template <typename T> struct SolverT : SolverBase {
                 CK(cudaMemcpy(at, faces.data(), sizeof(int4) * count, cudaMemcpyHostToDevice));
                 enqueue_face_geometry(plan.m, plan.faces, nullptr);
                 CK(cudaGetLastError());
-                CK(cudaDeviceSynchronize());
+                CK(cudaStreamSynchronize(nullptr));
             }
         }
         Flow<T> &f = plan.f;
