@@ -521,9 +521,9 @@ def mlp_record(layers: int, steps: int, warmup: int) -> dict:
             "config": {"workload": f"MLP 32 -> {L} x 256 GELU -> 4, batch {B}, Adam"},
             "roofline": {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak,
                          "peak_source": f"{kind} bf16_tflops (MEASURED_PEAKS.json)", "traffic": None},
-            # per step: step counter, gather, L forward GEMMs, the output layer,
-            # L weight gradients, L - 1 data gradients, L + 1 Adam launches
-            "gpu_launches": (4 * L + 3) * steps}
+            # per step: step counter, gather, the forward chain, the output layer,
+            # the data-gradient chain, L weight gradients, L + 1 Adam launches
+            "gpu_launches": (2 * L + 6) * steps}
 
 
 def run_mlp(args):

@@ -255,7 +255,8 @@ int e2d_set_precision(e2d_solver *s, int32_t precision);
 /* Device time of the kernels of the last e2d_step/e2d_solve call, ms,
  * measured with CUDA events on the solver's stream. */
 int e2d_last_device_ms(e2d_solver *s, double *ms);
-/* Kernel launches per iteration (all passes of all stages). */
+/* Kernel launches per iteration (all passes of all stages); 1 for a small FP32
+ * mesh, whose iterations run many to a launch. */
 int e2d_launches_per_iteration(e2d_solver *s, int32_t *n);
 /* Runs iters iterations launching the kernels one by one (no graph) with a
  * CUDA event pair around every launch, and returns the summed device time per
