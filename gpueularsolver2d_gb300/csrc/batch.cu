@@ -92,6 +92,19 @@ template <typename T> struct BatchT : BatchBase {
                        Arena::up(sizeof(Flow<T>) * ncase) + 2 * Arena::up(sizeof(int) * (n / kChunk + 1)) +
                        2 * Arena::up(sizeof(int2) * ncase) + Arena::up(sizeof(int) * hw.size()) +
                        Arena::up(sizeof(double) * 4 * wmax);
+        // concatenated topology (padding cells have -1 in the last place)
+        std::vector<int32_t> ht(4 * (size_t)n, 0);
+        for (size_t k = 3; k < ht.size(); k += 4) ht[k] = -1;
+        for (int c = 0; c < ncase; c++) {
+            const HostLayout &l = (*L)[c];
+            const int o = (*off)[c];
+            for (size_t k = 0; k < 4 * (size_t)l.n; k++)
+                ht[4 * (size_t)o + k] = (k & 3) < 3 && l.topo[k] >= 0 ? l.topo[k] + (o << 3) : l.topo[k];
+        }
+        std::vector<int4> faces;
+        if (sizeof(T) == 8 && n > face_list_cells) faces = face_list(ht.data(), n);
+        bytes += Arena::up(sizeof(int4) * faces.size()) + Arena::up(sizeof(double) * 6 * faces.size()) +
+                 Arena::up(faces.empty() ? 0 : sizeof(double) * 3 * n);
         CK(cudaMalloc((void **)&arena.base, bytes));
         arena.cap = bytes;
         int4 *topo = (int4 *)arena.take(sizeof(int4) * n);
@@ -118,9 +131,7 @@ template <typename T> struct BatchT : BatchBase {
         wall_dev = (int *)arena.take(sizeof(int) * hw.size());
         wwall_dev = (double *)arena.take(sizeof(double) * 4 * wmax);
         if (!hw.empty()) CK(cudaMemcpy(wall_dev, hw.data(), sizeof(int) * hw.size(), cudaMemcpyHostToDevice));
-        // concatenated mesh (padding cells stay zero, -1 in topo's last place, and are never touched)
-        std::vector<int32_t> ht(4 * (size_t)n, 0);
-        for (size_t k = 3; k < ht.size(); k += 4) ht[k] = -1;
+        // concatenated mesh (padding cells stay zero and are never touched)
         std::vector<T> hS(6 * (size_t)n, T(0)), hR(6 * (size_t)n, T(0)), ha(n, T(1));
         std::vector<int> hp(n, 0), hcc(n / kChunk + 1, 0), hce(ncase);
         std::vector<Flow<T>> hf(ncase);
@@ -129,14 +140,11 @@ template <typename T> struct BatchT : BatchBase {
             const int o = (*off)[c];
             for (int i = 0; i < l.n; i++) {
                 for (int k = 0; k < 3; k++) {
-                    int code = l.topo[4 * (size_t)i + k];
-                    ht[4 * (size_t)(o + i) + k] = code >= 0 ? code + (o << 3) : code;
                     for (int q = 0; q < 2; q++) {
                         hS[2 * ((size_t)k * n + o + i) + q] = (T)l.S[2 * ((size_t)k * l.n + i) + q];
                         hR[2 * ((size_t)k * n + o + i) + q] = (T)l.R[2 * ((size_t)k * l.n + i) + q];
                     }
                 }
-                ht[4 * (size_t)(o + i) + 3] = l.topo[4 * (size_t)i + 3];
                 ha[o + i] = (T)l.area[i];
                 hp[o + i] = l.perm[i];
             }
@@ -163,6 +171,19 @@ template <typename T> struct BatchT : BatchBase {
         CK(cudaMemset(plan.W[0], 0, sizeof(V4<T>) * n));
         CK(cudaMemset(plan.W[1], 0, sizeof(V4<T>) * n));
         plan.m = MeshDev<T>{n, topo, S, R, area};
+        plan.faces = FaceList{};
+        if constexpr (sizeof(T) == 8) {
+            if (!faces.empty()) {
+                const int count = (int)faces.size();
+                int4 *at = (int4 *)arena.take(sizeof(int4) * count);
+                double *geo = (double *)arena.take(sizeof(double) * 6 * count);
+                plan.faces = FaceList{at, geo, (double *)arena.take(sizeof(double) * 3 * n), count};
+                CK(cudaMemcpy(at, faces.data(), sizeof(int4) * count, cudaMemcpyHostToDevice));
+                enqueue_face_geometry(plan.m, plan.faces, nullptr);
+                CK(cudaGetLastError());
+                CK(cudaStreamSynchronize(nullptr));
+            }
+        }
         plan.f = hf[0];
         plan.b = BatchDev<T>{flows, chunk_case, live, case_end, ctl};
         plan.ncase = ncase;

@@ -132,10 +132,11 @@ template <typename T> struct BPlan {
     int block;               // cells per tile = threads per CTA
     bool options = true;     // some case uses a scheme option (pass-A option variant)
     int grid;                // CTAs per launch (persistent when < tiles)
+    FaceList faces;          // of all cases (FP64)
 };
 
 template <typename T> int launches_per_iteration(const BPlan<T> &p) {
-    return p.stages * (3 + (p.sweeps > 1 ? p.sweeps - 1 : 0)) + 1;
+    return p.stages * (3 + (p.faces.count ? 1 : 0) + (p.sweeps > 1 ? p.sweeps - 1 : 0)) + 1;
 }
 
 template <typename T> void enqueue_batch_iteration(const BPlan<T> &p, cudaStream_t s);

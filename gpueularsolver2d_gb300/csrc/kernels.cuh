@@ -1025,15 +1025,14 @@ __global__ void __launch_bounds__(256, 2) k_faces_tile(MeshDev<double> m, Flow<d
 
 // FP64 with a face list: the face states only, LPC threads per cell without tiles;
 // the radii are taken with the fluxes (k_face_flux) and the steps with their sums.
+// Every thread of the warp calls it (live: it has a cell).
 template <bool OPT, int LPC>
-__global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<double> f,
-                                                        const V4<double> *__restrict__ W, V4<double> *FS,
-                                                        const Ctl *__restrict__ ctl, V4<double> *__restrict__ phi) {
-    wait_prior_grid();
-    if (ctl->halt) return;
-    const int n = m.n, t = blockIdx.x * blockDim.x + threadIdx.x, i = t / LPC, part = t % LPC;
-    const int4 tp = i < n ? m.topo[i] : make_int4(0, 0, 0, 0);
-    if ((tp.x | tp.y | tp.z) < 0 && part == 0) {
+__device__ __forceinline__ void faces_listed(const MeshDev<double> &m, const Flow<double> &f, const int i,
+                                             const int part, const bool live, const int4 tp,
+                                             const V4<double> *__restrict__ W, V4<double> *FS,
+                                             V4<double> *__restrict__ phi, const int frozen, const bool first) {
+    const int n = m.n;
+    if (live && (tp.x | tp.y | tp.z) < 0 && part == 0) {
 #pragma unroll 1
         for (int k = 0; k < 3; k++) {
             const int c = k == 0 ? tp.x : k == 1 ? tp.y : tp.z;
@@ -1042,9 +1041,18 @@ __global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<
         }
     }
     if (LPC > 1) __syncwarp();  // the cell's other threads read the ghosts
-    if (i >= n) return;
-    faces_cell64<OPT, LPC>(m, f, i, part, W, FS, phi, OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order,
-                           W + i, tp, FS + i, n);
+    if (live) faces_cell64<OPT, LPC>(m, f, i, part, W, FS, phi, frozen, first, W + i, tp, FS + i, n);
+}
+template <bool OPT, int LPC>
+__global__ void __launch_bounds__(256, 2) k_faces_cells(MeshDev<double> m, Flow<double> f,
+                                                        const V4<double> *__restrict__ W, V4<double> *FS,
+                                                        const Ctl *__restrict__ ctl, V4<double> *__restrict__ phi) {
+    wait_prior_grid();
+    if (ctl->halt) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / LPC;
+    const bool live = i < m.n;
+    faces_listed<OPT, LPC>(m, f, i, t % LPC, live, live ? m.topo[i] : make_int4(0, 0, 0, 0), W, FS, phi,
+                           OPT && phi ? ctl->frozen : 0, OPT && ctl->step < f.first_order);
 }
 
 // FP32.  OPT: the variant with the scheme options (smooth limiter, limiter
@@ -1355,46 +1363,52 @@ static __device__ __noinline__ V4<double> listed_face_ieee(const FaceList l, con
     l.radius[at.x] = r;
     return F;
 }
+__device__ __forceinline__ void face_listed(const FaceList &l, const Flow<double> &f, const int j, const int4 at,
+                                            const V4<double> *__restrict__ W, V4<double> *FS) {
+    FastOps o;
+    double r;
+    V4<double> F = listed_face<true>(o, l, f, j, at, W, FS, r);
+    l.radius[at.x] = r;
+    if (o.bad) F = listed_face_ieee(l, f, j, W, FS);
+    FS[at.x] = F;
+}
 template <typename T>
 __global__ void __launch_bounds__(256, 2) k_face_flux(FaceList l, Flow<T> f, const V4<T> *__restrict__ W, V4<T> *FS,
                                                       const Ctl *__restrict__ ctl) {
     wait_prior_grid();
     if (ctl->halt) return;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= l.count) return;
-    const int4 at = l.at[j];
-    FastOps o;
-    T r;
-    V4<T> F = listed_face<true>(o, l, f, j, at, W, FS, r);
-    l.radius[at.x] = r;
-    if (o.bad) F = listed_face_ieee(l, f, j, W, FS);
-    FS[at.x] = F;
+    if (j < l.count) face_listed(l, f, j, l.at[j], W, FS);
 }
 
+template <typename T>
+__device__ __forceinline__ T face_sum(const MeshDev<T> &m, const Flow<T> &f, const int i, const int4 tp,
+                                      const V4<T> *__restrict__ F, const T *__restrict__ radius,
+                                      V4<T> *__restrict__ res, T *__restrict__ dt) {
+    const int n = m.n;
+    const int code[3] = {tp.x, tp.y, tp.z};
+    V4<T> v[3], r = {};
+    T q[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int c = code[k], j = c >= 0 && ((c >> 2) & 1) ? (c & 3) * n + (c >> 3) : k * n + i;
+        v[k] = F[j];
+        q[k] = radius[j];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) add_flux(r, v[k], code[k] >= 0 && ((code[k] >> 2) & 1));
+    res[i] = r;
+    return dt[i] = local_dt(m, f, i, q[0] + q[1] + q[2]);
+}
 template <typename T>
 __global__ void __launch_bounds__(256) k_face_sum(MeshDev<T> m, Flow<T> f, const V4<T> *__restrict__ F,
                                                   const T *__restrict__ radius, V4<T> *__restrict__ res,
                                                   T *__restrict__ dt, Ctl *ctl, const int st) {
     wait_prior_grid();
     if (ctl->halt) return;
-    const int n = m.n, i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     T dti = T(INFINITY);
-    if (i < n) {
-        const int4 tp = m.topo[i];
-        const int code[3] = {tp.x, tp.y, tp.z};
-        V4<T> v[3], r = {};
-        T q[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int c = code[k], j = c >= 0 && ((c >> 2) & 1) ? (c & 3) * n + (c >> 3) : k * n + i;
-            v[k] = F[j];
-            q[k] = radius[j];
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) add_flux(r, v[k], code[k] >= 0 && ((code[k] >> 2) & 1));
-        res[i] = r;
-        dt[i] = dti = local_dt(m, f, i, q[0] + q[1] + q[2]);
-    }
+    if (i < m.n) dti = face_sum(m, f, i, m.topo[i], F, radius, res, dt);
     if (f.global_dt) block_min_dt(dti, &ctl->dtmin[st]);
 }
 
@@ -1693,6 +1707,50 @@ __global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlock
     }
 }
 
+// FP64 with a face list of all cases: passes A and B as in a single mesh, a thread
+// per cell or face whatever the launch shape.  A block's cells are in one case.
+template <bool OPT, int LPC>
+__global__ void __launch_bounds__(256, 2) kb_faces_cells(MeshDev<double> m, BatchDev<double> b,
+                                                         const V4<double> *__restrict__ W, V4<double> *FS,
+                                                         V4<double> *__restrict__ phi) {
+    wait_prior_grid();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / LPC;
+    if (i >= m.n) return;  // whole warps: n is a multiple of kChunk
+    const int4 tp = m.topo[i];
+    const int tc = b.live[i / kChunk];
+    if (tc < 0) return;
+    const Flow<double> &f = b.flows[tc];
+    faces_listed<OPT, LPC>(m, f, i, t % LPC, tp.w >= 0, tp, W, FS, phi, OPT && phi ? b.ctl[tc].frozen : 0,
+                           OPT && b.ctl[tc].step < f.first_order);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2) kb_face_flux(FaceList l, BatchDev<T> b, const V4<T> *__restrict__ W,
+                                                       V4<T> *FS) {
+    wait_prior_grid();
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= l.count) return;
+    const int4 at = l.at[j];
+    const int tc = b.live[at.z / kChunk];
+    if (tc >= 0) face_listed(l, b.flows[tc], j, at, W, FS);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) kb_face_sum(MeshDev<T> m, BatchDev<T> b, const V4<T> *__restrict__ F,
+                                                   const T *__restrict__ radius, V4<T> *__restrict__ res,
+                                                   T *__restrict__ dt, const int st) {
+    wait_prior_grid();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.n) return;  // whole blocks
+    const int4 tp = m.topo[i];
+    const int tc = b.live[i / kChunk];
+    if (tc < 0) return;  // uniform over the block
+    const Flow<T> &f = b.flows[tc];
+    T dti = T(INFINITY);
+    if (tp.w >= 0) dti = face_sum(m, f, i, tp, F, radius, res, dt);
+    if (f.global_dt) block_min_dt(dti, &b.ctl[tc].dtmin[st]);
+}
+
 template <typename T, bool LOOP>
 __global__ void __launch_bounds__(256) kb_smooth(MeshDev<T> m, BatchDev<T> b, int ntiles, T eps,
                                                  const V4<T> *__restrict__ src, const V4<T> *__restrict__ res,
@@ -1741,9 +1799,22 @@ template <typename T, bool LOOP> void enqueue_batch_passes(const BPlan<T> &p, cu
         const bool last = st == p.stages - 1;
         V4<T> *Wcur = st == 0 ? p.W[0] : p.W[1];
         V4<T> *Wout = last ? p.W[0] : p.W[1];
-        launch_chained_smem(p.options ? kb_faces<T, true, LOOP> : kb_faces<T, false, LOOP>, G, B,
-                            sizeof(T) == 8 ? B * FacesSmem::per_cell : 0, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi, st);
-        launch_chained(kb_flux<T, LOOP>, G, B, s, p.m, p.b, NT, Wcur, p.FS, p.res);
+        if (sizeof(T) == 8 && p.faces.count) {
+            if constexpr (sizeof(T) == 8) {
+                // positivity: one thread per cell (faces_lanes); a case may ask for it
+                const int lanes = p.options || p.m.n > 100000 ? 1 : 2;
+                launch_chained(p.options ? kb_faces_cells<true, 1>
+                               : lanes == 1 ? kb_faces_cells<false, 1> : kb_faces_cells<false, 2>,
+                               NT * lanes, B, s, p.m, p.b, Wcur, p.FS, p.phi);
+                launch_chained(kb_face_flux<T>, (p.faces.count + B - 1) / B, B, s, p.faces, p.b, Wcur, p.FS);
+                launch_chained(kb_face_sum<T>, NT, B, s, p.m, p.b, p.FS, p.faces.radius, p.res, p.dt, st);
+            }
+        } else {
+            launch_chained_smem(p.options ? kb_faces<T, true, LOOP> : kb_faces<T, false, LOOP>, G, B,
+                                sizeof(T) == 8 ? B * FacesSmem::per_cell : 0, s, p.m, p.b, NT, Wcur, p.FS, p.dt, p.phi,
+                                st);
+            launch_chained(kb_flux<T, LOOP>, G, B, s, p.m, p.b, NT, Wcur, p.FS, p.res);
+        }
         const V4<T> *src = p.res;
         for (int sw = 0; sw + 1 < p.sweeps; sw++) {
             V4<T> *dst = p.sm[sw & 1];

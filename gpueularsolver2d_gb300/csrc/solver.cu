@@ -56,6 +56,20 @@ FreeStream free_stream(const e2d_params &p) {
     return s;
 }
 
+std::vector<int4> face_list(const int32_t *topo, int n) {
+    std::vector<int4> v;
+    v.reserve(3 * (size_t)n / 2 + 1024);
+    for (int i = 0; i < n; i++) {
+        const int32_t *t = topo + 4 * (size_t)i;
+        for (int k = 0; k < 3 && t[3] >= 0; k++) {
+            const int c = t[k];
+            if (c < 0) v.push_back(make_int4(k * n + i, -1, i, i));
+            else if (!((c >> 2) & 1)) v.push_back(make_int4(k * n + i, (c & 3) * n + (c >> 3), i, c >> 3));
+        }
+    }
+    return v;
+}
+
 int build_layout(e2d_mesh *m, const e2d_params &p, HostLayout &L) {
     int rc = build_topology(m, p.wall_box);
     if (rc) return rc;
@@ -249,7 +263,7 @@ template <typename T> struct SolverT : SolverBase {
                        Arena::up(sizeof(double) * G) +
                        Arena::up(sizeof(int) * n) + Arena::up(sizeof(double) * 4 * n);
         std::vector<int4> faces;
-        if (sizeof(T) == 8 && n > face_list_cells) faces = face_list();
+        if (sizeof(T) == 8 && n > face_list_cells) faces = face_list(L->topo.data(), n);
         bytes += Arena::up(sizeof(int4) * faces.size()) + Arena::up(sizeof(double) * 6 * faces.size()) +
                  Arena::up(faces.empty() ? 0 : sizeof(double) * 3 * n);
         CK(cudaMalloc((void **)&arena.base, bytes));
@@ -313,20 +327,6 @@ template <typename T> struct SolverT : SolverBase {
         plan.block = block;
         if constexpr (sizeof(T) == 4) small_ = small_iterations(plan, 0, nullptr, true);
         return E2D_OK;
-    }
-
-    // Every face once, at its left cell (see FaceList).
-    std::vector<int4> face_list() const {
-        const int n = L->n;
-        std::vector<int4> v;
-        v.reserve(3 * (size_t)n / 2 + 1024);
-        for (int i = 0; i < n; i++)
-            for (int k = 0; k < 3; k++) {
-                const int c = L->topo[4 * (size_t)i + k];
-                if (c < 0) v.push_back(make_int4(k * n + i, -1, i, i));
-                else if (!((c >> 2) & 1)) v.push_back(make_int4(k * n + i, (c & 3) * n + (c >> 3), i, c >> 3));
-            }
-        return v;
     }
 
     // Caller's FP64 file-order buffer -> device (one copy; from pinned memory

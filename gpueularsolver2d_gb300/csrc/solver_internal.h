@@ -53,6 +53,10 @@ const char *param_error(const e2d_params *p);
 void keep_in_l2(cudaGraph_t g, const void *base, size_t bytes, bool *held);
 void release_l2(bool *held);
 
+// Every face once, at its left cell (FaceList::at), from the topology [4n] of n
+// cells; cells with a negative last entry (padding) have none.
+std::vector<int4> face_list(const int32_t *topo, int n);
+
 // Device arena: one cudaMalloc carved into 256-byte aligned pieces.
 struct Arena {
     char *base = nullptr;
