@@ -67,7 +67,7 @@ struct FaceList {
     int count;  // 0: passes A and B work in tiles of cells
 };
 
-// Cells above which a single FP64 mesh takes a face list.  Below, a launch is as
+// Cells above which an FP64 mesh, or batch in all, takes a face list.  Below, a launch is as
 // long as one thread's chain, and the list's extra launch costs more than it saves.
 // us per iteration in tiles and with the list: 8k cells 141 and 152, 12.8k 158 and
 // 152, 20k 186 and 185, 34k 220 and 207, 80k 436 and 353, 252k 1059 and 907.

@@ -1709,6 +1709,8 @@ __global__ void __launch_bounds__(256, LOOP ? BatchMinBlocks<T>::flux : MinBlock
 
 // FP64 with a face list of all cases: passes A and B as in a single mesh, a thread
 // per cell or face whatever the launch shape.  A block's cells are in one case.
+// An iteration of 60 cases, 1.85M cells, in tiles and so: 7243 and 5763 us; 24 cases of
+// 33k cells with the smooth limiter 3764 and 3164.
 template <bool OPT, int LPC>
 __global__ void __launch_bounds__(256, 2) kb_faces_cells(MeshDev<double> m, BatchDev<double> b,
                                                          const V4<double> *__restrict__ W, V4<double> *FS,
