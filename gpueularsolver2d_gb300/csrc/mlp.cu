@@ -370,10 +370,13 @@ struct e2d_mlp {
         if (X) cudaFree(X);
         if (T) cudaFree(T);
     }
+    // A buffer of zeros, cleared on the training stream: that stream does not wait
+    // for the default one, where a clear behind a caller's own work would come
+    // after what the stream writes into the buffer.
     template <typename P> int alloc(P **p, size_t bytes) {
         CK(cudaMalloc((void **)p, bytes));
-        CK(cudaMemset(*p, 0, bytes));
         allocs.push_back(*p);
+        CK(cudaMemsetAsync(*p, 0, bytes, stream));
         return E2D_OK;
     }
 };
@@ -530,9 +533,9 @@ int ensure_batch(e2d_mlp *m, int B) {
 // (A prediction of 33.6k rows takes 0.17 ms, 1.12 ms when the host converted and
 // padded to the full batch of 65536.)
 int stage_rows(e2d_mlp *m, const float *x, int cnt, int rows, bf16 *dst, int ld) {
-    if (!m->xf) {
-        int rc = m->alloc(&m->xf, sizeof(float) * (size_t)m->cfg.batch * NIN);
-        if (rc) return rc;
+    if (!m->xf) {  // (not cleared: k_pack reads the rows that were copied)
+        CK(cudaMalloc((void **)&m->xf, sizeof(float) * (size_t)m->cfg.batch * NIN));
+        m->allocs.push_back(m->xf);
     }
     CK(cudaMemcpyAsync(m->xf, x, sizeof(float) * (size_t)cnt * NIN, cudaMemcpyHostToDevice, m->stream));
     k_pack<<<(int)(((size_t)rows * (NIN / 8) + 255) / 256), 256, 0, m->stream>>>(cnt, rows, m->xf, dst, ld);
@@ -848,12 +851,14 @@ int e2d_mlp_create(const e2d_mlp_config *cfg, e2d_mlp **out) {
         double u1 = rnd() + 1e-300, u2 = rnd();
         return std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2);
     };
+    std::vector<std::vector<float>> init;  // each layer's weights, until the copies are done
     for (int l = 0; l <= m->nhidden; l++) {
         const bool last = l == m->nhidden;
         const int rows = last ? NOUT : H, cols = l == 0 ? NIN : H;
         const int fan_in = l == 0 ? E2D_MLP_FEATURES : H;
         Tensor W{rows, cols}, b{rows, 1};
-        std::vector<float> hw((size_t)rows * cols, 0.f), hb(rows, 0.f);
+        init.emplace_back((size_t)rows * cols, 0.f);
+        std::vector<float> &hw = init.back();
         const double sd = std::sqrt((last ? 1.0 : 2.0) / fan_in);
         for (int r = 0; r < rows; r++)
             for (int c = 0; c < cols; c++)
@@ -866,8 +871,7 @@ int e2d_mlp_create(const e2d_mlp_config *cfg, e2d_mlp **out) {
             if ((rc = m->alloc(&t->v, sizeof(float) * n))) return rc;
             if (!last && t == &W && (rc = m->alloc(&t->wbf, sizeof(bf16) * (size_t)t->rows * t->wld()))) return rc;
         }
-        CK(cudaMemcpy(W.w32, hw.data(), sizeof(float) * hw.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(b.w32, hb.data(), sizeof(float) * hb.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(W.w32, hw.data(), sizeof(float) * hw.size(), cudaMemcpyHostToDevice, m->stream));
         if (W.wbf)
             k_to_bf16<<<(W.count() + 255) / 256, 256, 0, m->stream>>>(W.count(), W.w32, W.wbf, W.cols, W.wld());
         m->W.push_back(W);
@@ -885,7 +889,7 @@ int e2d_mlp_create(const e2d_mlp_config *cfg, e2d_mlp **out) {
     if ((rc = m->alloc(&m->bc_dev, 2 * sizeof(float)))) return rc;
     if ((rc = m->alloc(&m->lr_dev, sizeof(float)))) return rc;
     const float lr0 = (float)cfg->lr;
-    CK(cudaMemcpy(m->lr_dev, &lr0, sizeof(float), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(m->lr_dev, &lr0, sizeof(float), cudaMemcpyHostToDevice, m->stream));
     if ((rc = m->alloc(&m->grad, sizeof(float) * param_count(m.get())))) return rc;
     CK(cudaStreamSynchronize(m->stream));
     *out = m.release();
@@ -916,7 +920,7 @@ int e2d_mlp_set_params(e2d_mlp *m, const float *in) {
     size_t off = 0;
     for (size_t l = 0; l < m->W.size(); l++)
         for (Tensor *t : {&m->W[l], &m->b[l]}) {
-            CK(cudaMemcpy(t->w32, in + off, sizeof(float) * t->count(), cudaMemcpyHostToDevice));
+            CK(cudaMemcpyAsync(t->w32, in + off, sizeof(float) * t->count(), cudaMemcpyHostToDevice, m->stream));
             if (t->wbf)
                 k_to_bf16<<<(t->count() + 255) / 256, 256, 0, m->stream>>>(t->count(), t->w32, t->wbf, t->cols, t->wld());
             off += t->count();

@@ -1,0 +1,56 @@
+"""A network's first calls while the legacy default stream has work of the
+caller pending: its buffers are cleared, filled and read on its own streams,
+which do not wait for the default one.  Results against the same calls with
+the default stream idle, bit for bit."""
+import numpy as np
+import pytest
+
+import gpueularsolver2d_gb300 as e2d
+
+pytestmark = pytest.mark.gpu
+
+
+def pending():
+    """Queues some tens of milliseconds of work on the default stream."""
+    import torch
+    a = torch.ones(4096, 4096, device="cuda")
+    b = torch.empty_like(a)
+    torch.cuda.synchronize()
+    for _ in range(40):
+        torch.mm(a, a, out=b)
+    return b
+
+
+def rows(n):
+    rng = np.random.default_rng(6)
+    x = np.zeros((n, 32), np.float32)
+    x[:, :22] = rng.normal(size=(n, 22))
+    return x, rng.normal(size=(n, 4)).astype(np.float32)
+
+
+def first_gradient(net):
+    loss, g = net.gradient(*rows(4096))
+    return np.append(g, np.float32(loss))
+
+
+def first_training(net):
+    net.set_data(*rows(20000))
+    net.train(3)
+    return net.params()
+
+
+def copied_params(net):
+    net.set_params(net.params()[::-1].copy())
+    return net.forward(rows(300)[0])
+
+
+@pytest.mark.parametrize("call", [first_gradient, first_training, copied_params, lambda net: net.forward(rows(5000)[0])])
+@pytest.mark.parametrize("made_before", [True, False])
+def test_first_calls_of_a_network(lib, call, made_before):
+    ref = call(e2d.MLP(nhidden=3, batch=4096, seed=4))
+    assert np.all(np.isfinite(ref)) and np.any(ref != 0)
+    net = e2d.MLP(nhidden=3, batch=4096, seed=4) if made_before else None
+    work = pending()
+    got = call(net or e2d.MLP(nhidden=3, batch=4096, seed=4))
+    assert np.array_equal(got, ref)
+    del work
