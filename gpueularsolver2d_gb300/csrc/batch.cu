@@ -181,7 +181,6 @@ template <typename T> struct BatchT : BatchBase {
                 CK(cudaMemcpy(at, faces.data(), sizeof(int4) * count, cudaMemcpyHostToDevice));
                 enqueue_face_geometry(plan.m, plan.faces, nullptr);
                 CK(cudaGetLastError());
-                CK(cudaStreamSynchronize(nullptr));
             }
         }
         plan.f = hf[0];
@@ -193,6 +192,9 @@ template <typename T> struct BatchT : BatchBase {
         plan.stages = P[0].rk_stages;
         for (int k = 0; k < 8; k++) plan.rk[k] = (T)P[0].rk_coef[k];
         plan.sweeps = P[0].irs_sweeps;
+        // the batch's stream does not wait for the default one, which the copies
+        // and clears above were made on
+        CK(cudaStreamSynchronize(nullptr));
         return E2D_OK;
     }
 
@@ -202,6 +204,7 @@ template <typename T> struct BatchT : BatchBase {
         for (int c = 0; c < ncase; c++)
             ct_host[c] = make_int2((*off)[c] / block, ((*L)[c].n + block - 1) / block);
         CK(cudaMemcpy(case_tiles, ct_host.data(), sizeof(int2) * ncase, cudaMemcpyHostToDevice));
+        CK(cudaStreamSynchronize(nullptr));  // as in init
         plan.block = block;
         plan.grid = grid;
         return E2D_OK;

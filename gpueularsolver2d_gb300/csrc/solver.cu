@@ -308,9 +308,11 @@ template <typename T> struct SolverT : SolverBase {
                 CK(cudaMemcpy(at, faces.data(), sizeof(int4) * count, cudaMemcpyHostToDevice));
                 enqueue_face_geometry(plan.m, plan.faces, nullptr);
                 CK(cudaGetLastError());
-                CK(cudaStreamSynchronize(nullptr));
             }
         }
+        // the solver's stream does not wait for the default one, which the copies
+        // and clears above were made on
+        CK(cudaStreamSynchronize(nullptr));
         Flow<T> &f = plan.f;
         f.gamma = (T)p.gamma; f.ui = (T)fs.ui; f.vi = (T)fs.vi; f.ain = (T)fs.ain_test; f.tin = (T)p.tin;
         f.vin = (T)fs.vin; f.R = (T)kR; f.pis = (T)fs.pis; f.cfl = (T)p.cfl; f.dt_cap = (T)p.dt_cap;

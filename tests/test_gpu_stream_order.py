@@ -1,7 +1,7 @@
-"""A network's first calls while the legacy default stream has work of the
-caller pending: its buffers are cleared, filled and read on its own streams,
-which do not wait for the default one.  Results against the same calls with
-the default stream idle, bit for bit."""
+"""A network's, a solver's and a batch's first calls while the legacy default
+stream has work of the caller pending: they read buffers on streams of their
+own, which do not wait for the default one.  Results against the same calls
+with the default stream idle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -53,4 +53,31 @@ def test_first_calls_of_a_network(lib, call, made_before):
     work = pending()
     got = call(net or e2d.MLP(nhidden=3, batch=4096, seed=4))
     assert np.array_equal(got, ref)
+    del work
+
+
+def solver_state(precision):
+    s = e2d.Solver(e2d.Mesh.ogrid(70, 40, seed=2), e2d.default_params(ma=0.6, cfl=1.2, precision=precision, block_size=64))
+    s.step(2)
+    if precision == e2d.E2D_FP32:
+        s.set_precision(e2d.E2D_FP64)
+        s.step(2)
+    return s.state()
+
+
+def batch_state(precision):
+    b = e2d.Batch([e2d.Mesh.ogrid(40, 9, seed=2), e2d.Mesh.ogrid(33, 20, seed=1)],
+                  [e2d.default_params(ma=m, cfl=1.2, precision=precision) for m in (0.5, 0.6)])
+    b.step(2)
+    b.set_launch(64, 8)
+    b.step(2)
+    return np.concatenate([b.state(0), b.state(1)])
+
+
+@pytest.mark.parametrize("call", [solver_state, batch_state])
+@pytest.mark.parametrize("precision", [e2d.E2D_FP32, e2d.E2D_FP64])
+def test_first_steps(lib, call, precision):
+    ref = call(precision)
+    work = pending()
+    assert np.array_equal(call(precision), ref)
     del work
