@@ -776,10 +776,9 @@ struct CellsAndWalls {
         py = (double *)(base + cells);
         CK(cudaMemcpyAsync(px, t.cx.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
         CK(cudaMemcpyAsync(py, t.cy.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-        if (nseg) {
-            CK(cudaMemcpyAsync(base + 2 * cells, seg.data(), sizeof(double4) * nseg, cudaMemcpyHostToDevice));
-            CK(cudaMemcpyAsync(base + 2 * cells + segs, box.data(), sizeof(float4) * box.size(),
-                               cudaMemcpyHostToDevice));
+        if (nseg) {  // (not asynchronous: seg and box end with this function)
+            CK(cudaMemcpy(base + 2 * cells, seg.data(), sizeof(double4) * nseg, cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(base + 2 * cells + segs, box.data(), sizeof(float4) * box.size(), cudaMemcpyHostToDevice));
         }
         out = base + 2 * cells + segs + boxes;
         walls = Walls{nseg, (const double4 *)(base + 2 * cells), (const float4 *)(base + 2 * cells + segs),

@@ -81,3 +81,25 @@ def test_first_steps(lib, call, precision):
     work = pending()
     assert np.array_equal(call(precision), ref)
     del work
+
+
+def test_features_of_many_wall_faces(lib):
+    """4096 wall faces: the copies of their segments and boxes are over the
+    64 KB that a copy from pageable memory takes at once."""
+    mesh = e2d.Mesh.ogrid(4096, 2, seed=3)
+    x, y, tri = mesh.nodes()
+    ei, _, _, _ = mesh.topology()
+    w = ei[ei[:, 0] == 2][:, 5:7] - 1
+    a = np.stack([x[w[:, 0]], y[w[:, 0]]], 1)
+    e = np.stack([x[w[:, 1]], y[w[:, 1]]], 1) - a
+    c = np.stack([x[tri - 1].mean(1), y[tri - 1].mean(1)], 1)
+    assert len(w) == 4096
+    work = pending()
+    f = e2d.MLP.features(mesh, 0.6, 1.5).astype(np.float64)
+    for k in range(0, len(c), 1000):
+        p = c[k:k + 1000, None] - a
+        t = np.clip((p * e).sum(-1) / (e * e).sum(-1), 0.0, 1.0)
+        ref = np.log(np.sqrt(((p - t[..., None] * e) ** 2).sum(-1).min(1)) + 1e-3)
+        # FP32 values: half a unit in the last place is 6e-8 of the value
+        assert np.all(np.abs(f[k:k + 1000, 2] - ref) <= 1e-7 * np.abs(ref) + 1e-12)
+    del work
