@@ -238,10 +238,12 @@ struct Walls {
 // rounding of the coordinates (slack); every other segment is evaluated in
 // FP64, its division on the integer units: 14 FP64 operations each, which is
 // what the kernel is bound by (33.6k cells and 251 segments: 0.3 ms before the
-// boxes).
+// boxes).  No box is passed over where FP32 squares could overflow (sizes from
+// 1e15) or lose more below the normal range (roots under 1e-19) than the slack.
 __device__ __forceinline__ double wall_distance(const Walls &w, const double x, const double y) {
     const float fx = (float)x, fy = (float)y;
-    const float slack = 2e-6f * (fabsf(fx) + fabsf(fy) + w.scale);
+    const float size = fabsf(fx) + fabsf(fy) + w.scale;
+    const float slack = size > 1e-12f && size < 1e15f ? 2e-6f * size : INFINITY;
     const int nbox = (w.nseg + kBox - 1) / kBox;
     float near = INFINITY;  // an upper bound of the distance
     for (int k = 0; k < nbox; k++) {
