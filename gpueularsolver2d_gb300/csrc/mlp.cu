@@ -30,6 +30,7 @@ using namespace e2d::mlp;
     do {                                                                               \
         cudaError_t err_ = (call);                                                     \
         if (err_ != cudaSuccess) {                                                     \
+            cudaGetLastError(); /* reported here, not by a later call's check */       \
             set_error(std::string("CUDA: ") + #call + ": " + cudaGetErrorString(err_)); \
             return E2D_ERR_CUDA;                                                       \
         }                                                                              \
@@ -327,7 +328,7 @@ struct e2d_mlp {
     // batch buffers
     int B = 0;
     bf16 *xb = nullptr;  // [B][KX], the inputs in the first NIN columns
-    float *xf = nullptr;  // [cfg.batch][NIN], the caller's FP32 rows on their way into xb or X
+    float *xf = nullptr;  // the caller's FP32 rows on their way into xb or X (stage_rows)
     float *tb = nullptr, *y = nullptr, *dy = nullptr;
     std::vector<bf16 *> Gd, Hh;  // [nhidden] of [B][H]: gelu'(z) and gelu(z) of each hidden layer
     std::vector<bf16 *> dz;  // [nhidden] of [B][H]: gradient at each hidden layer's pre-activation
@@ -530,18 +531,25 @@ int ensure_batch(e2d_mlp *m, int B) {
     return build_ws_maps(m);
 }
 
-// cnt rows of the caller's inputs (at most cfg.batch) to the device and as bf16
-// to dst (row pitch ld), rows cnt .. rows - 1 zero, on the training stream.
+// cnt rows of the caller's inputs to the device and as bf16 to dst (row pitch
+// ld), rows cnt .. rows - 1 zero, on the training stream, in pieces of a batch, but
+// of 2048 to 65536 rows whatever the batch (8 MB of room at most).
 // (A prediction of 33.6k rows takes 0.17 ms, 1.12 ms when the host converted and
 // padded to the full batch of 65536.)
-int stage_rows(e2d_mlp *m, const float *x, int cnt, int rows, bf16 *dst, int ld) {
+int stage_rows(e2d_mlp *m, const float *x, int64_t cnt, int64_t rows, bf16 *dst, int ld) {
+    const int64_t piece = std::min(std::max(m->cfg.batch, 2048), 65536);
     if (!m->xf) {  // (not cleared: k_pack reads the rows that were copied)
-        CK(cudaMalloc((void **)&m->xf, sizeof(float) * (size_t)m->cfg.batch * NIN));
+        CK(cudaMalloc((void **)&m->xf, sizeof(float) * (size_t)piece * NIN));
         m->allocs.push_back(m->xf);
     }
-    CK(cudaMemcpyAsync(m->xf, x, sizeof(float) * (size_t)cnt * NIN, cudaMemcpyHostToDevice, m->stream));
-    k_pack<<<(int)(((size_t)rows * (NIN / 8) + 255) / 256), 256, 0, m->stream>>>(cnt, rows, m->xf, dst, ld);
-    CK(cudaGetLastError());
+    for (int64_t r0 = 0; r0 < rows; r0 += piece) {
+        const int r = (int)std::min(piece, rows - r0), c = (int)std::max<int64_t>(0, std::min<int64_t>(r, cnt - r0));
+        if (c > 0)
+            CK(cudaMemcpyAsync(m->xf, x + (size_t)r0 * NIN, sizeof(float) * (size_t)c * NIN, cudaMemcpyHostToDevice,
+                               m->stream));
+        k_pack<<<(r * (NIN / 8) + 255) / 256, 256, 0, m->stream>>>(c, r, m->xf, dst + (size_t)r0 * ld, ld);
+        CK(cudaGetLastError());
+    }
     return E2D_OK;
 }
 
@@ -943,24 +951,23 @@ int e2d_mlp_set_lr(e2d_mlp *m, double lr) {
 
 int e2d_mlp_set_data(e2d_mlp *m, int64_t nsamples, const float *x, const float *t) {
     if (!m || !x || !t || nsamples < 1) { set_error("bad argument"); return E2D_ERR_ARG; }
+    // nothing of the previous data stays in use if one of the steps below fails
+    if (m->gexec) { cudaGraphExecDestroy(m->gexec); m->gexec = nullptr; }
+    m->nsamples = 0;
     if (m->X) { cudaFree(m->X); m->X = nullptr; }
     if (m->T) { cudaFree(m->T); m->T = nullptr; }
     CK(cudaMalloc((void **)&m->X, sizeof(bf16) * (size_t)nsamples * NIN));
     CK(cudaMalloc((void **)&m->T, sizeof(float) * (size_t)nsamples * NOUT));
-    for (int64_t r0 = 0; r0 < nsamples; r0 += m->cfg.batch) {
-        const int cnt = (int)std::min<int64_t>(m->cfg.batch, nsamples - r0);
-        int rc = stage_rows(m, x + (size_t)r0 * NIN, cnt, cnt, m->X + (size_t)r0 * NIN, NIN);
-        if (rc) return rc;
-    }
+    int rc = stage_rows(m, x, nsamples, nsamples, m->X, NIN);
+    if (rc) return rc;
     CK(cudaMemcpyAsync(m->T, t, sizeof(float) * (size_t)nsamples * NOUT, cudaMemcpyHostToDevice, m->stream));
     CK(cudaStreamSynchronize(m->stream));
     m->nsamples = nsamples;
-    if (m->gexec) { cudaGraphExecDestroy(m->gexec); m->gexec = nullptr; }
     return E2D_OK;
 }
 
 int e2d_mlp_train(e2d_mlp *m, int32_t steps, double *loss) {
-    if (!m || steps < 1 || !m->X) { set_error("bad argument or no training data"); return E2D_ERR_ARG; }
+    if (!m || steps < 1 || m->nsamples < 1) { set_error("bad argument or no training data"); return E2D_ERR_ARG; }
     int rc = ensure_batch(m, m->cfg.batch);
     if (rc) return rc;
     if ((rc = build_train_graph(m))) return rc;
@@ -991,7 +998,7 @@ int e2d_mlp_forward(e2d_mlp *m, int64_t n, const float *x, float *y) {
     for (int64_t r0 = 0; r0 < n; r0 += m->B) {
         const int64_t cnt = std::min<int64_t>(m->B, n - r0);
         const int rows = (int)((cnt + 255) / 256 * 256);  // whole tiles; B is a multiple of 2048
-        if ((rc = stage_rows(m, x + (size_t)r0 * NIN, (int)cnt, rows, m->xb, KX))) return rc;
+        if ((rc = stage_rows(m, x + (size_t)r0 * NIN, cnt, rows, m->xb, KX))) return rc;
         forward(m, m->stream, false, rows);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(y + (size_t)r0 * NOUT, m->y, sizeof(float) * cnt * NOUT, cudaMemcpyDeviceToHost, m->stream));
