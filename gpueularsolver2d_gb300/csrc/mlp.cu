@@ -430,7 +430,28 @@ bool map_part(CUtensorMap *map, const float *ptr, uint64_t rows, uint64_t cols) 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of the TMA / tcgen05 kernels once the batch buffers exist;
+// Weight- and bias-gradient partials of the hidden layers, nparts of each: kSplits
+// for the per-tile kernel, one per wrows rows of the batch for the TMA one (512
+// rows: 128 CTAs at batch 65536, 20.7 us per layer against 26.9 us for 1024 rows,
+// with Adam summing twice the partials).
+int alloc_partials(e2d_mlp *m, int nparts) {
+    int rc;
+    m->part.assign(m->nhidden, nullptr);
+    m->bpart.assign(m->nhidden, nullptr);
+    for (int l = m->nhidden - 1; l >= 0; l--) {
+        const int share = l + 2;  // the set of the layer two up, unless merged
+        if (!m->merged && share < m->nhidden) {
+            m->part[l] = m->part[share];
+            m->bpart[l] = m->bpart[share];
+            continue;
+        }
+        if ((rc = m->alloc(&m->part[l], sizeof(float) * (size_t)nparts * H * H))) return rc;
+        if ((rc = m->alloc(&m->bpart[l], sizeof(float) * (size_t)nparts * H))) return rc;
+    }
+    return E2D_OK;
+}
+
+// Partials and tensor maps of the TMA / tcgen05 kernels once the batch buffers exist;
 // use_ws stays false (the per-tile kernel runs every layer) when the driver
 // entry point, a map or the shared-memory size is not available, or
 // E2D_MLP_WS=0.  With E2D_MLP_WS=1 that is an error instead.
@@ -447,6 +468,7 @@ int build_ws_maps(e2d_mlp *m) {
         return E2D_OK;
     }
     bool ok = m->wrows >= ws::WCH && m->wrows % ws::WCH == 0 && m->B % m->wrows == 0;
+    if (int rc = alloc_partials(m, m->B / m->wrows)) return rc;
     const int L = m->nhidden;
     const uint64_t B = m->B, prows = (uint64_t)(m->B / m->wrows) * H;
     ok = ok && map_2d(&m->fwd.in, m->xb, B, KX, ws::BM) && map_2d(&m->bwd.in, m->dz[L - 1], B, H, ws::BM);
@@ -508,27 +530,11 @@ int ensure_batch(e2d_mlp *m, int B) {
     m->dz.resize(m->nhidden);
     for (int l = 0; l < m->nhidden; l++)
         if ((rc = m->alloc(&m->dz[l], sizeof(bf16) * (size_t)B * H))) return rc;
-    // weight-gradient partials: kSplits of the per-tile kernel, or one per
-    // wrows rows of the batch for the TMA one (512 rows: 128 CTAs at batch
-    // 65536, 20.7 us per layer against 26.9 us for 1024 rows, with Adam
-    // summing twice the partials)
-    const int nparts = std::max(kSplits, B / m->wrows);
-    m->merged = (size_t)m->nhidden * (B / m->wrows) * H * H * sizeof(float) <= kMergeBytes;
-    m->part.resize(m->nhidden);
-    m->bpart.resize(m->nhidden);
-    for (int l = m->nhidden - 1; l >= 0; l--) {
-        const int share = l + 2;  // the set of the layer two up, unless merged
-        if (!m->merged && share < m->nhidden) {
-            m->part[l] = m->part[share];
-            m->bpart[l] = m->bpart[share];
-            continue;
-        }
-        if ((rc = m->alloc(&m->part[l], sizeof(float) * (size_t)nparts * H * H))) return rc;
-        if ((rc = m->alloc(&m->bpart[l], sizeof(float) * (size_t)nparts * H))) return rc;
-    }
     if ((rc = m->alloc(&m->opart, sizeof(float) * (size_t)(B / 256) * (NOUT * H + NOUT)))) return rc;
     if ((rc = m->alloc(&m->loss_part, sizeof(double) * kLossSlots * (B / 256)))) return rc;
-    return build_ws_maps(m);
+    m->merged = (size_t)m->nhidden * (B / m->wrows) * H * H * sizeof(float) <= kMergeBytes;
+    if ((rc = build_ws_maps(m))) return rc;
+    return m->use_ws ? E2D_OK : alloc_partials(m, kSplits);
 }
 
 // cnt rows of the caller's inputs to the device and as bf16 to dst (row pitch
