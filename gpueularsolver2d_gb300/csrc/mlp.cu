@@ -508,14 +508,9 @@ size_t param_count(const e2d_mlp *m) {
     return c;
 }
 
-int ensure_batch(e2d_mlp *m, int B) {
-    if (m->B == B) return E2D_OK;
-    if (m->B != 0) { set_error("batch size is fixed at the first use"); return E2D_ERR_ARG; }
-    if (B < 2048 || B % 2048 != 0) {  // split-K slices of the batch are multiples of BK
-        set_error("batch must be a positive multiple of 2048");
-        return E2D_ERR_ARG;
-    }
-    m->B = B;
+// The buffers of a batch of m->B rows, and what runs on them.
+int make_batch(e2d_mlp *m) {
+    const int B = m->B;
     int rc;
     if ((rc = m->alloc(&m->xb, sizeof(bf16) * (size_t)B * KX))) return rc;  // columns NIN.. stay zero
     if ((rc = m->alloc(&m->tb, sizeof(float) * (size_t)B * NOUT))) return rc;
@@ -535,6 +530,23 @@ int ensure_batch(e2d_mlp *m, int B) {
     m->merged = (size_t)m->nhidden * (B / m->wrows) * H * H * sizeof(float) <= kMergeBytes;
     if ((rc = build_ws_maps(m))) return rc;
     return m->use_ws ? E2D_OK : alloc_partials(m, kSplits);
+}
+
+int ensure_batch(e2d_mlp *m, int B) {
+    if (m->B == B) return E2D_OK;
+    if (m->B != 0) { set_error("batch size is fixed at the first use"); return E2D_ERR_ARG; }
+    if (B < 2048 || B % 2048 != 0) {  // split-K slices of the batch are multiples of BK
+        set_error("batch must be a positive multiple of 2048");
+        return E2D_ERR_ARG;
+    }
+    const size_t had = m->allocs.size();
+    m->B = B;
+    const int rc = make_batch(m);
+    if (rc) {  // no half-made batch stays behind for the next call
+        m->B = 0;
+        for (; m->allocs.size() > had; m->allocs.pop_back()) cudaFree(m->allocs.back());
+    }
+    return rc;
 }
 
 // cnt rows of the caller's inputs to the device and as bf16 to dst (row pitch

@@ -66,3 +66,14 @@ def test_a_failed_call_leaves_no_data(lib):
         net.train(1)
     net.set_data(x, t)
     assert np.isfinite(net.train(1)[0])
+
+
+def test_a_batch_that_does_not_fit_stays_refused(lib):
+    """The first call's error is every later call's: none runs on a part of the
+    buffers.  (The first hidden layer would take 256 GB.)"""
+    net = e2d.MLP(nhidden=1, batch=2 ** 29)
+    for _ in range(2):
+        with pytest.raises(E2DError, match="out of memory"):
+            net.forward(rows(1)[0])
+    net.close()
+    assert np.all(np.isfinite(e2d.MLP(nhidden=1, batch=2048).forward(rows(1)[0])))
