@@ -485,6 +485,18 @@ def run_batch64(args):
     print(json.dumps(line), flush=True)
 
 
+def mlp_launches(layers: int, batch: int) -> int:
+    """Kernel launches of a training step: step counter, gather, the forward
+    chain, the output layer and, with more than one hidden layer, the
+    data-gradient chain; then the weight gradients and Adam.  While the partials
+    of all layers (one of 256 KB per 512 rows and layer) fit 64 MB, those are one
+    launch for the first layer, one for the others and one Adam; otherwise one
+    each per layer and an Adam of the output layer."""
+    head = 5 if layers > 1 else 4
+    merged = layers * (batch // 512) * 256 * 256 * 4 <= 64 << 20
+    return head + (min(layers, 2) + 1 if merged else 2 * layers + 1)
+
+
 def mlp_record(layers: int, steps: int, warmup: int) -> dict:
     """Training steps of the warm-start MLP (22 features padded to 32 -> L x
     256 GELU -> 4, batch 65536, BF16 tensor-core GEMMs with FP32 accumulate):
@@ -521,9 +533,7 @@ def mlp_record(layers: int, steps: int, warmup: int) -> dict:
             "config": {"workload": f"MLP 32 -> {L} x 256 GELU -> 4, batch {B}, Adam"},
             "roofline": {"bound": "tensor", "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak,
                          "peak_source": f"{kind} bf16_tflops (MEASURED_PEAKS.json)", "traffic": None},
-            # per step: step counter, gather, the forward chain, the output layer,
-            # the data-gradient chain, L weight gradients, L + 1 Adam launches
-            "gpu_launches": (2 * L + 6) * steps}
+            "gpu_launches": mlp_launches(L, B) * steps}
 
 
 def run_mlp(args):
