@@ -652,8 +652,7 @@ void forward(e2d_mlp *m, cudaStream_t s, bool with_loss, int B) {
     // (k_out_train), fused with its gradient
     if (with_loss) return;
     const Tensor &Wo = m->W[m->nhidden], &bo = m->b[m->nhidden];
-    k_out_fwd_loss<H, NOUT><<<(B + 255) / 256, 256, 0, s>>>(B, m->Hh[m->nhidden - 1], Wo.w32, bo.w32, nullptr,
-                                                            m->y, m->dy, nullptr);
+    k_out_fwd<H, NOUT><<<(B + 255) / 256, 256, 0, s>>>(B, m->Hh[m->nhidden - 1], Wo.w32, bo.w32, m->y);
 }
 
 // Backward + Adam with the step size at lr (null: gradient only, written to

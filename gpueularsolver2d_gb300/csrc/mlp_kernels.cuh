@@ -54,11 +54,6 @@ __device__ __forceinline__ void gelu_and_grad2(const float2 x, float2 &h, float2
     g = __ffma2_rn(__fmul2_rn(hx, sech2), du, __ffma2_rn(half, t, half));
 }
 
-__device__ __forceinline__ float gelu(float x) {
-    const float hx = 0.5f * x;
-    return fmaf(hx, tanh_approx(kGeluC0 * x * fmaf(kGeluC1, x * x, 1.0f)), hx);
-}
-
 // Epilogue modes of the GEMM.
 enum Epi : int {
     EPI_BIAS_GELU = 0,  // z = acc + bias[n]; out = gelu(z), zout = gelu'(z) (bf16)
@@ -297,73 +292,32 @@ __global__ void __launch_bounds__(256, GemmOcc<EPI>::value) k_gemm_tc(GemmArgs g
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tmem), "r"(tc::TMEM_COLS));
 }
 
-// Output layer (256 -> NOUT) on the CUDA cores: y[b][o] = h[b] . W[o] + bias[o]
-// (fp32); loss partial per block of MSE against t, and dY = 2 (y - t) / (B NOUT).
+// Output layer (256 -> NOUT) of a prediction on the CUDA cores: y[b][o] = h[b] .
+// W[o] + bias[o] (fp32).
 template <int H, int NOUT>
-__global__ void __launch_bounds__(256) k_out_fwd_loss(int B, const bf16 *__restrict__ h, const float *__restrict__ W,
-                                                      const float *__restrict__ bias, const float *__restrict__ t,
-                                                      float *__restrict__ y, float *__restrict__ dy,
-                                                      double *__restrict__ loss_part) {
+__global__ void __launch_bounds__(256) k_out_fwd(int B, const bf16 *__restrict__ h, const float *__restrict__ W,
+                                                 const float *__restrict__ bias, float *__restrict__ y) {
     __shared__ float Ws[NOUT * H];
     for (int k = threadIdx.x; k < NOUT * H; k += blockDim.x) Ws[k] = W[k];
     __syncthreads();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (b < B) {
-        float acc[NOUT];
+    if (b >= B) return;
+    float acc[NOUT];
 #pragma unroll
-        for (int o = 0; o < NOUT; o++) acc[o] = bias[o];
-        const bf16 *hr = h + (size_t)b * H;
-        for (int k = 0; k < H; k += 8) {
-            const uint4 v = *(const uint4 *)(hr + k);
-            const bf16 *e = (const bf16 *)&v;
+    for (int o = 0; o < NOUT; o++) acc[o] = bias[o];
+    const bf16 *hr = h + (size_t)b * H;
+    for (int k = 0; k < H; k += 8) {
+        const uint4 v = *(const uint4 *)(hr + k);
+        const bf16 *e = (const bf16 *)&v;
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const float x = __bfloat162float(e[q]);
+        for (int q = 0; q < 8; q++) {
+            const float x = __bfloat162float(e[q]);
 #pragma unroll
-                for (int o = 0; o < NOUT; o++) acc[o] += x * Ws[o * H + k + q];
-            }
-        }
-#pragma unroll
-        for (int o = 0; o < NOUT; o++) {
-            y[(size_t)b * NOUT + o] = acc[o];
-            if (t) {
-                const float d = acc[o] - t[(size_t)b * NOUT + o];
-                l += (double)d * d;
-                dy[(size_t)b * NOUT + o] = 2.0f * d / (float)(B * NOUT);
-            }
+            for (int o = 0; o < NOUT; o++) acc[o] += x * Ws[o * H + k + q];
         }
     }
-    if (!loss_part) return;
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    __shared__ double ws[8];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) s += ws[k];
-        loss_part[blockIdx.x] = s;
-    }
-}
-
-// Output layer backward: dz[b][k] = (sum_o dy[b][o] W[o][k]) * gd[b][k] (bf16),
-// gd = gelu'(z) of the last hidden layer as its forward epilogue stored it.
-template <int H, int NOUT>
-__global__ void __launch_bounds__(256) k_out_bwd_data(int B, const float *__restrict__ dy, const float *__restrict__ W,
-                                                      const bf16 *__restrict__ gd, bf16 *__restrict__ dz) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // one (b, pair of k)
-    if (idx >= (size_t)B * (H / 2)) return;
-    const int b = (int)(idx / (H / 2)), k = (int)(idx % (H / 2)) * 2;
-    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-    for (int o = 0; o < NOUT; o++) {
-        const float d = dy[(size_t)b * NOUT + o];
-        s0 += d * W[o * H + k];
-        s1 += d * W[o * H + k + 1];
-    }
-    const __nv_bfloat162 gg = *(const __nv_bfloat162 *)(gd + (size_t)b * H + k);
-    const __nv_bfloat162 d = __floats2bfloat162_rn(s0 * __bfloat162float(gg.x), s1 * __bfloat162float(gg.y));
-    *(__nv_bfloat162 *)(dz + (size_t)b * H + k) = d;
+    for (int o = 0; o < NOUT; o++) y[(size_t)b * NOUT + o] = acc[o];
 }
 
 // Output layer of a training step, forward and backward in one pass over the
@@ -493,51 +447,9 @@ __global__ void __launch_bounds__(256, MINB) k_out_train(int B, const bf16 *__re
     }
 }
 
-// Split partials of the output layer's weight gradient: part[split][o][k] =
-// sum over the split's rows of dy[b][o] h[b][k]; part[split][NOUT*H + o] =
-// sum dy.  Grid (H / 32, splits): lane = column k, the block's 8 warps take
-// every 8th row, then the warps are added in a fixed order (deterministic).
-template <int H, int NOUT>
-__global__ void __launch_bounds__(256) k_out_bwd_weight(int B, int rows_per_split, const float *__restrict__ dy,
-                                                        const bf16 *__restrict__ h, float *__restrict__ part) {
-    __shared__ float red[8][NOUT][32];
-    __shared__ float dred[8][NOUT];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k = blockIdx.x * 32 + lane;
-    const int b0 = blockIdx.y * rows_per_split, b1 = min(B, b0 + rows_per_split);
-    float s[NOUT], ds[NOUT];
-#pragma unroll
-    for (int o = 0; o < NOUT; o++) s[o] = ds[o] = 0.f;
-    for (int b = b0 + warp; b < b1; b += 8) {
-        const float x = __bfloat162float(h[(size_t)b * H + k]);
-#pragma unroll
-        for (int o = 0; o < NOUT; o++) {
-            const float d = dy[(size_t)b * NOUT + o];
-            s[o] += d * x;
-            ds[o] += d;
-        }
-    }
-#pragma unroll
-    for (int o = 0; o < NOUT; o++) red[warp][o][lane] = s[o];
-    if (lane == 0)
-#pragma unroll
-        for (int o = 0; o < NOUT; o++) dred[warp][o] = ds[o];
-    __syncthreads();
-    float *p = part + (size_t)blockIdx.y * (NOUT * H + NOUT);
-    if (warp < NOUT) {
-        float t = 0.f;
-        for (int w = 0; w < 8; w++) t += red[w][warp][lane];
-        p[warp * H + k] = t;
-    }
-    if (blockIdx.x == 0 && threadIdx.x < NOUT) {
-        float t = 0.f;
-        for (int w = 0; w < 8; w++) t += dred[w][threadIdx.x];
-        p[NOUT * H + threadIdx.x] = t;
-    }
-}
-
 // Column sums of a bf16 [B][N] gradient over row splits: part[split][n].
-// Grid (N / 32, splits), same shape as k_out_bwd_weight.
+// Grid (N / 32, splits): block (x, y) takes columns 32 x .. and the rows of split y,
+// a column to a lane, the rows in turn to its eight warps.
 __global__ void __launch_bounds__(256) k_colsum(int B, int N, int rows_per_split, const bf16 *__restrict__ d,
                                                 float *__restrict__ part) {
     __shared__ float red[8][32];
