@@ -462,8 +462,8 @@ __device__ __forceinline__ V4<float> roe<float>(const V4<float> &LW, const V4<fl
 // (the reference's boundary faces are first order: the cell's own side is the
 // cell state, and pass B would evaluate the ghost again from it: on small
 // O-grids most warps hold a boundary cell.  us per iteration without and with
-// this: FP32 4.2M cells 940 and 925, 60 batched cases 508 and 500, 2k cells in one
-// launch 18.4 and 14.7; FP64 33.6k cells 252 and 243).
+// this: FP32 2k cells in one launch 18.4 and 14.7, 131k 54.3 and 52.6, 4.2M 926 and
+// 929 (pass A 76.9 and 78.1, pass B 81.5 and 79.9); FP64 33.6k cells 252 and 243).
 //
 // Limiter freezing (an option with no reference counterpart, off when phi is
 // null): while not frozen the limiter values of every face are recorded in
@@ -667,7 +667,11 @@ __device__ __forceinline__ Limit32 limits32(const Recon32 &c, const Flow<float> 
 // there is the ghost, which the caller leaves in the face's place.)  OPT compiles in
 // the scheme options (smooth limiter, frozen limiter values, first-order faces,
 // positivity fallback); without them the reference configuration runs in fewer
-// registers.  first: this iteration uses first-order faces.
+// registers.  first: this iteration uses first-order faces.  Without the options a
+// boundary face's state is evaluated like the others and only not stored: with a
+// branch around each face the launch spilled 32 bytes per thread instead of 20 (12
+// instead of none in a batch) and took 80.2 instead of 78.1 us at 4.2M cells (an
+// iteration 937 and 929 us, of 60 batched cases 480 and 473).
 template <bool OPT, typename Out>
 __device__ __forceinline__ float faces_cell32(const MeshDev<float> &m, const Flow<float> &f, const int i,
                                               const int *code, const V2<float> *S, const V4<float> &U,
@@ -681,7 +685,7 @@ __device__ __forceinline__ float faces_cell32(const MeshDev<float> &m, const Flo
     const Limit32 lim = limits32<OPT>(c, f, code, S, A, reuse, first);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        if (code[k] < 0) continue;
+        if (OPT && code[k] < 0) continue;
         V4<float> o = U;
         if (!(OPT && first)) {
             V4<float> ph;
@@ -689,7 +693,7 @@ __device__ __forceinline__ float faces_cell32(const MeshDev<float> &m, const Flo
             o = face_state32<OPT>(c, f, lim, offset32(S[(k + 1) % 3], S[(k + 2) % 3]), ph);
             if (OPT && phi && !frozen) phi[k * n + i] = ph;
         }
-        out(k, o);
+        if (code[k] >= 0) out(k, o);
     }
     return tmin(fdiv(A * f.cfl, Tsum), f.dt_cap);
 }
