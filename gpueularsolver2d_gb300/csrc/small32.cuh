@@ -22,6 +22,7 @@ constexpr int kSmallThreads = 512;    // threads with cells at most; one more wa
 constexpr int kSmallPerCta = 1024;    // cells of a CTA at most: two per thread
 constexpr int kSmallCells = kSmallCtas * kSmallPerCta;
 constexpr int kSmallParts = kSmallCells / 128;
+constexpr int kSmallDense = kSmallCtas * 768;  // cells up to which every scheme takes it
 
 struct SmallArgs {
     MeshDev<float> m;
@@ -299,10 +300,18 @@ template <bool OPT, int CPT> bool small_launch(const SmallArgs &a, cudaStream_t 
 // us per iteration of 4 stages, this against one launch per pass: 2k cells 14.7 and
 // 35.6; 8k 21.2 and 36.4, with the cell-wise limiter 27.5 and 38.9; 12k 29.1 and 36.3;
 // 16k 33.6 and 37.8 (two cells to a thread
-// spill with the options: they stop at one).
+// spill with the options: they stop at one).  A pass more costs a launch about 1.5
+// us and this kernel 0.75, a stage's flux and reconstruction of two cells per thread
+// more than the launches: above 768 cells to a CTA the launches win with less than
+// two sweeps and more than three stages.  16k cells (and 12.3k) in file order, without
+// smoothing: 3 stages 20.4 and 20.0 (20.2, 20.5), 4 stages 26.7 and 25.4 (26.5, 25.6),
+// 8 stages 51.8 and 46.5 (51.5, 46.8); one sweep, 4 stages 28.1 and 27.4 (28.4, 27.7);
+// two sweeps, 8 stages 60.5 and 62.5 (61.6, 62.3).  12288 cells, 4 stages, without
+// smoothing: 22.8 and 24.9.
 bool small_iterations(const Plan<float> &p, int iters, cudaStream_t s, bool probe) {
     const bool opt = faces_options(p.f, p.phi);
     if (p.m.n > (opt ? kSmallCtas * kSmallThreads : kSmallCells) || p.block != 128 || p.f.global_dt) return false;
+    if (p.m.n > kSmallDense && p.sweeps < 2 && p.stages > 3) return false;
     SmallArgs a;
     a.m = p.m; a.f = p.f; a.W = p.W[0]; a.phi = p.phi; a.ctl = p.ctl; a.hist = p.hist; a.hist_cap = p.hist_cap;
     a.stages = p.stages; a.sweeps = p.sweeps; a.iters = iters;
