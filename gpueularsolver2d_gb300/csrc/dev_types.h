@@ -157,6 +157,13 @@ template <typename T> void enqueue_iteration(const Plan<T> &p, cudaStream_t s);
 // (probe: asked once, nothing is launched) or the launch failed.
 bool small_iterations(const Plan<float> &p, int iters, cudaStream_t s, bool probe);
 
+// Cells up to which that is the faster way for every scheme and number of
+// iterations (768 to a CTA).  Above, not for schemes that small_iterations leaves
+// out, nor for a call of a single iteration, which has the kernel's loads of the
+// mesh to itself: us per call at 16k cells, in one launch and in passes, 72 and 64
+// for one iteration, 99 and 101 for two, 164 and 174 for four.
+constexpr int small_dense_cells = 12288;
+
 // Same, with an event pair around every launch (per-pass timing).
 template <typename T> int enqueue_iteration_timed(const Plan<T> &p, cudaStream_t s, cudaEvent_t *ev, int *kind);
 

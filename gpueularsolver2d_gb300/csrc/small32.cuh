@@ -22,7 +22,6 @@ constexpr int kSmallThreads = 512;    // threads with cells at most; one more wa
 constexpr int kSmallPerCta = 1024;    // cells of a CTA at most: two per thread
 constexpr int kSmallCells = kSmallCtas * kSmallPerCta;
 constexpr int kSmallParts = kSmallCells / 128;
-constexpr int kSmallDense = kSmallCtas * 768;  // cells up to which every scheme takes it
 
 struct SmallArgs {
     MeshDev<float> m;
@@ -311,7 +310,7 @@ template <bool OPT, int CPT> bool small_launch(const SmallArgs &a, cudaStream_t 
 bool small_iterations(const Plan<float> &p, int iters, cudaStream_t s, bool probe) {
     const bool opt = faces_options(p.f, p.phi);
     if (p.m.n > (opt ? kSmallCtas * kSmallThreads : kSmallCells) || p.block != 128 || p.f.global_dt) return false;
-    if (p.m.n > kSmallDense && p.sweeps < 2 && p.stages > 3) return false;
+    if (p.m.n > small_dense_cells && p.sweeps < 2 && p.stages > 3) return false;
     SmallArgs a;
     a.m = p.m; a.f = p.f; a.W = p.W[0]; a.phi = p.phi; a.ctl = p.ctl; a.hist = p.hist; a.hist_cap = p.hist_cap;
     a.stages = p.stages; a.sweeps = p.sweeps; a.iters = iters;

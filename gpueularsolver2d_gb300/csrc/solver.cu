@@ -536,7 +536,7 @@ int run(e2d_solver *s, int n, bool check, double epsl, int poll_every) {
     if (n <= 0) return E2D_OK;
     int rc = ensure_hist(s, s->ctl_host->step + n);
     if (rc) return rc;
-    const bool small = s->impl->small();
+    const bool small = s->impl->small() && (n > 1 || s->L.n <= small_dense_cells);
     if (small) bind_hist(s);
     else if ((rc = build_graph(s))) return rc;
     Ctl &c = *s->ctl_host;

@@ -26,3 +26,18 @@ def test_line(lib, ni, nj, stages, sweeps, launches):
         s.step(6)
     assert a.launches_per_iteration() == launches
     assert np.array_equal(a.state(), b.state())
+
+
+@pytest.mark.parametrize("ni,nj", [(128, 48), (150, 41), (128, 64)])
+def test_single_iterations(lib, ni, nj):
+    """A call of one iteration takes the passes above 12288 cells; calls of one and
+    of several iterations mix freely, over a growth of the history too."""
+    mesh = e2d.Mesh.ogrid(ni, nj, seed=5)
+    kw = dict(ma=0.5, alpha_deg=1.0, cfl=0.5, precision=e2d.E2D_FP32)
+    a = e2d.Solver(mesh, e2d.default_params(**kw))
+    b = e2d.Solver(mesh, e2d.default_params(**kw, block_size=64))
+    for n in (1, 1, 3, 1, 2, 1, 1100, 1):
+        a.step(n)
+        b.step(n)
+    assert np.array_equal(a.state(), b.state())
+    np.testing.assert_allclose(a.history(), b.history(), rtol=1e-9)  # sums to about 48 bits, grouped otherwise
