@@ -43,8 +43,9 @@ def default_params(**kw) -> Params:
 
 def _result(shape, dtype=np.float64) -> np.ndarray:
     """An array that a download fills whole.  One write a page puts its pages in
-    place first: pages first touched by the GPU took 23 ms for the 59 MB of a
-    60-case sweep, and about as long again to release; so 1.5 ms."""
+    place first: on some hosts pages first touched by the GPU took 23 ms for the
+    59 MB of a 60-case sweep, and about as long again to release, with the pages
+    in place 2.5 ms; on others a new 59 MB array takes 3.0 ms either way."""
     w = np.empty(shape, dtype)
     w.reshape(-1).view(np.uint8)[::4096] = 0
     return w

@@ -227,6 +227,7 @@ E2D_HD double mul_fast(double a, double b, bool &bad) {
     const uint64_t sign = (ua ^ ub) & 0x8000000000000000ULL;
     return double_of(sign | (zero ? 0 : ((uint64_t)(uint32_t)(e - 1 + up) << 52) + m));
 }
+// (A product by itself: the form that the host's test holds against its own.)
 E2D_HD_SLOW double mul_ieee(double a, double b) { return a * b; }
 E2D_HD double imul(double a, double b) {
     bool bad = false;

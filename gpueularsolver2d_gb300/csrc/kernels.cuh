@@ -1666,6 +1666,10 @@ __global__ void __launch_bounds__(256) k_update(MeshDev<T> m, Flow<T> f, T rk, i
 // 24 cases of 33k cells with the smooth limiter 255 -> 241 us.)  With a CTA for every
 // tile (LOOP false, the default launch shape) there is no loop to keep values for
 // and pass B has its single-case registers (540 -> 508 us).
+// In FP64 kb_faces and kb_flux serve batches of at most 12000 cells (above, a face
+// list).  kb_faces with options spills 212 bytes per thread there, at the 128
+// registers of two blocks; 4 cases of 4096 cells in tiles took 196 us an iteration
+// without options, 222 with the smooth limiter.
 
 template <typename T, bool OPT, bool LOOP>
 __global__ void __launch_bounds__(256, OPT && sizeof(T) == 4 ? kOptBlocks : BatchMinBlocks<T>::faces) kb_faces(MeshDev<T> m, BatchDev<T> b, int ntiles, const V4<T> *__restrict__ W,
